@@ -307,8 +307,8 @@ nbody_status fwd_initial(nbody_adjoint* a, cudaStream_t st) {
                                                                nullptr, fp64 ? nullptr : a->jbx);
   AD_TRY(fwd_eval(a, st));
   double* D = a->D;
-  reduce_splits_kernel<<<(a->n + kBlock - 1) / kBlock, kBlock, 0, st>>>(
-      0, a->n, a->ld, a->S, a->P, SoA6{D, D + ld, D + 2 * ld, D + 3 * ld, D + 4 * ld, D + 5 * ld});
+  launch_reduce(st, 0, a->n, a->ld, a->S, a->P,
+                SoA6{D, D + ld, D + 2 * ld, D + 3 * ld, D + 4 * ld, D + 5 * ld});
   AD_CUDA(cudaGetLastError());
   return NBODY_OK;
 }
@@ -322,8 +322,7 @@ nbody_status fwd_step(nbody_adjoint* a, cudaStream_t st, double* xp_out) {
   if (xp_out)
     AD_CUDA(cudaMemcpyAsync(xp_out, a->X, sizeof(double) * 6 * a->ld, cudaMemcpyDeviceToDevice, st));
   AD_TRY(fwd_eval(a, st));
-  correct_kernel<<<(a->n + kBlock - 1) / kBlock, kBlock, 0, st>>>(a->n, a->ld, a->S, a->P, a->X, a->V,
-                                                                 a->D, a->ctl, 1.0);
+  launch_correct(st, a->n, a->ld, a->S, a->P, a->X, a->V, a->D, a->ctl, 1.0);
   AD_CUDA(cudaGetLastError());
   return NBODY_OK;
 }

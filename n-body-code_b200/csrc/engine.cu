@@ -44,6 +44,7 @@
 #include "hermite.cuh"
 #include "pair.cuh"
 #include "reltiles.cuh"
+#include "sympair.cuh"
 #include "trace.h"
 
 using namespace nbody;
@@ -52,6 +53,16 @@ namespace {
 
 constexpr int kPad = 256;        // body padding granularity (multiple of every j-tile)
 constexpr int kMaxSplit = 64;    // split-j upper bound
+// Blocks of the symmetric schedule: nb / 2 partial-sum slots, so at most 64
+// beside the splits.  More blocks would need more slots (48 bytes per row
+// each), fewer would evaluate more of the pairs one-sided (1 / nb of them).
+constexpr int kMaxSymBlocks = 128;
+// Slots of a symmetric pass are further bounded by memory (8 GiB of P, at
+// least 8 slots): larger systems take fewer, larger blocks and fewer splits.
+int max_sym_slots(int n) {
+  const double fit = 8.0 * (1 << 30) / (48.0 * n);
+  return fit > 2 * kMaxSplit ? 2 * kMaxSplit : std::max(8, static_cast<int>(fit));
+}
 // Rate at which the corrector sums split partials (64 splits at N = 65536:
 // 201 MB in 52 us), the autotuner's price for each partial a tiling leaves.
 constexpr double kSplitSumBytesPerMs = 3.9e9;
@@ -102,6 +113,7 @@ struct PairKernel {
   int acc_smem = 0, junroll = 2, minb = 1;
   int near = 0;  // tile-relative: 1 = near tiles in double-single (variant 4), 0 = all far (5)
   int cluster = 1;  // CTAs per thread-block cluster along j (splits summed in the cluster)
+  bool sym = false;  // symmetric kernel (sympair.cuh): full-row passes only
 };
 
 template <int NT, int IPT, int TJ, int JU = 2, int MINB = 1>
@@ -130,6 +142,15 @@ PairKernel make_mixed_nf() {
           MINB, NEAR ? 1 : 0};
 }
 
+template <int IPT, int W, int UNR, int MINB>
+PairKernel make_sym_fp64() {
+  PairKernel k{NBODY_FP64, 32 * W, IPT, kSymTile64, kRecF64,
+               reinterpret_cast<const void*>(&pair_sym_fp64_kernel<IPT, W, UNR, MINB>),
+               sym_fp64_smem<IPT, W, UNR>(), 0, UNR, MINB};
+  k.sym = true;
+  return k;
+}
+
 // Near/far rows on clusters of CL CTAs along j: split count a multiple of CL,
 // S / CL partials (pair_mixed_nf_cluster_kernel).
 template <int NT, int IPT, int TJ, int JU, int MINB, int NEAR, int CL>
@@ -147,6 +168,8 @@ const std::vector<PairKernel>& registry() {
       make_fp64<128, 1, 128, 2>(),  make_fp64<128, 4, 128, 1>(),  make_fp64<256, 1, 128, 4>(),
       make_fp64<256, 2, 128, 1>(),  make_fp64<128, 2, 256, 1>(),  make_fp64<64, 2, 128, 1>(),
       make_fp64<128, 2, 128, 1, 6>(), make_fp64<128, 2, 64, 1, 6>(), make_fp64<128, 1, 128, 4, 8>(),
+      // symmetric (full-row passes; sym_kernel chooses between the two)
+      make_sym_fp64<4, 4, 2, 2>(), make_sym_fp64<2, 4, 4, 4>(),
       // near/far tile-relative packed pairs (bodies in Hilbert order; default
       // mixed: 128 x 4 rows, j-unroll 2, 4 CTAs/SM = 128 registers, no spills)
       make_mixed_nf<128, 4, 128, 1, 2, 4>(), make_mixed_nf<64, 4, 128>(), make_mixed_nf<128, 2, 128>(),
@@ -190,7 +213,7 @@ const PairKernel* find_kernel(int precision, int nt, int ipt, int tj, int varian
                               int cluster = 1) {
   auto match = [&](int fmt, int acc, int near = 1) -> const PairKernel* {
     for (const auto& k : registry())
-      if (k.precision == precision && k.nt == nt && k.ipt == ipt && k.tj == tj &&
+      if (!k.sym && k.precision == precision && k.nt == nt && k.ipt == ipt && k.tj == tj &&
           (fmt < 0 || k.fmt == fmt) && (acc < 0 || k.acc_smem == acc) &&
           (k.fmt != kRecRel || k.near == near) && k.cluster == cluster)
         return &k;
@@ -212,9 +235,30 @@ struct Tiling {
   int source = 0;  // nbody_timers.tiling_source: 1 heuristic/explicit, 2 timed, 3 cached
 };
 
-// Split partials a launch of tiling t leaves in P (cluster kernels sum their
-// CL CTAs' partials into one).
-int partial_count(const Tiling& t) { return t.split / t.k->cluster; }
+// The symmetric schedule of n bodies with kernel k.
+struct SymGrid {
+  int subs, block_rows, nb;
+  SymGrid(const PairKernel& k, int n) {
+    const int rows = k.nt * k.ipt;
+    const long most = static_cast<long>(std::min(kMaxSymBlocks, max_sym_slots(n))) * rows;
+    subs = static_cast<int>((n + most - 1) / most);
+    block_rows = subs * rows;
+    nb = (n + block_rows - 1) / block_rows;
+  }
+};
+
+// Partial-sum slots of each row after a launch of tiling t over n bodies
+// (cluster kernels sum their CL CTAs' partials into one).
+RowSlots row_slots(const Tiling& t, int n) {
+  if (!t.k->sym) return RowSlots(t.split / t.k->cluster);
+  const SymGrid g(*t.k, n);
+  return RowSlots(t.split, g.block_rows, g.nb);
+}
+// Slots of P that such a launch writes.
+int partial_count(const Tiling& t, int n) {
+  const RowSlots r = row_slots(t, n);
+  return r.S + r.nb / 2;
+}
 
 // Autotune results shared by all engines of the process: (device, precision,
 // record format, ld, rows) -> tiling.
@@ -348,6 +392,41 @@ int choose_split(const nbody_engine* e, const PairKernel& k, int rows) {
   return best_s;
 }
 
+// Splits of the symmetric kernel k over n bodies: S CTAs per block share its
+// run of Q tiles, ceil(Q / S) each.  Same wave model, over the tile counts
+// that differ: full waves cost a CTA's tiles, the last one what its fullest
+// SM holds (but at least half: alone on its SM a CTA is latency-bound), and
+// every split another 48 bytes per row to write and sum, at the measured rate
+// of 13 us per (CTA, tile).
+int choose_sym_split(const nbody_engine* e, const PairKernel& k, int n) {
+  prepare_kernel(k);
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, k.nt, k.smem) != cudaSuccess ||
+      occ < 1)
+    occ = 1;
+  const SymGrid g(k, n);
+  const int Q = sym_q_count(g.nb, 0, g.block_rows / k.tj, (n + k.tj - 1) / k.tj);
+  const long slots = static_cast<long>(e->num_sms) * occ;
+  const double tile_ms = 0.013 * (k.nt * k.ipt / 512.0) * (k.tj / 32.0) * (occ / 2.0);
+  const double per_split = 48.0 * n / kSplitSumBytesPerMs / tile_ms;
+  double best = 1e300;
+  int best_s = 1;
+  for (int tps = 1; tps <= Q; ++tps) {
+    const int s = (Q + tps - 1) / tps;
+    if (s > std::min(kMaxSplit, max_sym_slots(n) / 2)) continue;
+    const long ctas = static_cast<long>(g.nb) * s, last = ctas % slots;
+    const double one = tps * g.subs + 0.5;
+    const double share = static_cast<double>((last + e->num_sms - 1) / e->num_sms) / occ;
+    const double cost = (ctas / slots) * one + (last ? one * std::max(0.5, share) : 0.0) + per_split * s;
+    if (cost < best - 1e-9) {
+      best = cost;
+      best_s = s;
+    }
+  }
+  return best_s;
+}
+
+// Grows P to `split` slots.
 nbody_status ensure_partials(nbody_engine* e, int split) {
   if (split <= e->p_splits) return NBODY_OK;
   if (e->P) {
@@ -383,12 +462,34 @@ nbody_status prepare_kernel(const PairKernel& k) {
 
 SoA7 own_inputs(nbody_engine* e);
 
+// A symmetric pass over all rows of n bodies whose records are in place.
+nbody_status launch_sym(nbody_engine* e, const Tiling& t, int n, cudaStream_t st) {
+  const PairKernel& k = *t.k;
+  const SymGrid g(k, n);
+  SymArgs a;
+  a.n = n;
+  a.ld = e->ld;
+  a.nb = g.nb;
+  a.subs = g.subs;
+  a.S = t.split;
+  a.tiles = (n + k.tj - 1) / k.tj;
+  a.eps2 = e->cfg.eps2;
+  a.out = e->P;
+  a.stride = static_cast<size_t>(e->ld);
+  a.status = e->status;
+  const void* jb = e->jb64;
+  void* args[] = {static_cast<void*>(&jb), static_cast<void*>(&a)};
+  NB_CUDA(cudaLaunchKernel(k.fn, dim3(g.nb, t.split), dim3(k.nt), args, k.smem, st));
+  return NBODY_OK;
+}
+
 // src / n_src: the inputs the records were built from (the tile-relative
 // kernel reads its i-rows there); nullptr = the engine's own state.
 nbody_status launch_pair(nbody_engine* e, const Tiling& t, int i_begin, int i_end,
                          cudaStream_t st, const SoA7* src = nullptr, int n_src = 0) {
   const PairKernel& k = *t.k;
   NB_TRY(prepare_kernel(k));
+  if (k.sym) return launch_sym(e, t, i_end, st);  // full rows: [0, i_end)
   PairArgs a;
   a.i_begin = i_begin;
   a.i_end = i_end;
@@ -424,15 +525,28 @@ nbody_status enqueue_reorder_state(nbody_engine* e, cudaStream_t st);
 
 // The tiling the autotuner cached for this engine's (device, precision,
 // record format, ld, rows), if any.
-bool tuned_lookup(const nbody_engine* e, int rows, Tiling* out) {
+bool tuned_lookup(const nbody_engine* e, int rows, Tiling* out, bool full = true) {
   const auto key = std::make_tuple(e->dev, e->cfg.precision, default_format(e), e->ld, rows);
   std::lock_guard<std::mutex> g(g_tune_mu);
   auto it = g_tuned.find(key);
   if (it == g_tuned.end()) return false;
+  if (!full && registry()[it->second.first].sym) return false;  // evaluates all rows only
   out->k = &registry()[it->second.first];
   out->split = it->second.second;
   out->source = 3;
   return true;
+}
+
+// The symmetric kernel an automatic full-row pass over n bodies takes, or null.
+// Four rows per lane from 16384 bodies, two below, where twice the blocks
+// fill the SMs (pair pass: N = 8192 106 us both, 4096 34 vs 36, 2048 19.5 vs
+// 17.5, 1024 13.2 vs 11.3; one-sided 144, 44, 18.2 and 15.0).
+const PairKernel* sym_kernel(const nbody_engine* e, int n) {
+  const int want = n >= 16384 ? 4 : 2;
+  for (const auto& k : registry())
+    if (k.sym && k.precision == e->cfg.precision && k.fmt == default_format(e) && k.ipt == want)
+      return &k;
+  return nullptr;
 }
 
 nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
@@ -444,6 +558,7 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
   float best = 1e30f;
   int best_idx = -1, best_split = 1;
   const auto& reg = registry();
+  const bool use_sym = rows == e->n && sym_kernel(e, rows);
   // the near/far kernel's cost depends on the bodies being in Hilbert order
   if (default_format(e) == kRecRel && e->have_state && !e->sorted)
     NB_TRY(enqueue_reorder_state(e, e->stream));
@@ -454,12 +569,15 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
     // cluster kernels save in the split sums what their pair pass loses
     // (N = 65536: 4.071 vs 4.071 ms with the sums priced in); not timed
     if (k.cluster > 1) continue;
-    const int s0 = choose_split(e, k, rows);
+    // symmetric kernels serve full-row passes (faster than every one-sided
+    // shape there at each size from 1024 to 262144), one-sided ones the rest
+    if (k.sym != use_sym) continue;
+    const int s0 = k.sym ? choose_sym_split(e, k, rows) : choose_split(e, k, rows);
     NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj));
     for (int s : {std::max(1, s0 / 2), s0, std::min(kMaxSplit, s0 * 2)}) {
       s = std::min(kMaxSplit, (s + k.cluster - 1) / k.cluster * k.cluster);
-      NB_TRY(ensure_partials(e, s));
       Tiling t{&k, s};
+      NB_TRY(ensure_partials(e, partial_count(t, rows)));
       NB_TRY(launch_pair(e, t, 0, rows, e->stream));  // warm-up
       NB_CUDA(cudaEventRecord(a, e->stream));
       for (int r = 0; r < 3; ++r) NB_TRY(launch_pair(e, t, 0, rows, e->stream));
@@ -470,7 +588,7 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
       pair_ms /= 3;
       // the split partials are summed after every pass (corrector or
       // reduction): 48 bytes per row and partial at the measured 3.9 TB/s
-      const float ms = pair_ms + static_cast<float>(48.0 * (s / k.cluster) * rows / kSplitSumBytesPerMs);
+      const float ms = pair_ms + static_cast<float>(48.0 * partial_count(t, rows) * rows / kSplitSumBytesPerMs);
       if (getenv("NBODY_TUNE_VERBOSE"))
         fprintf(stderr, "[nbody tune] #%zu prec=%d rows=%d nt=%d ipt=%d tj=%d fmt=%d acc_smem=%d ju=%d minb=%d cluster=%d split=%d  %.4f ms (pair %.4f)\n",
                 idx, k.precision, rows, k.nt, k.ipt, k.tj, k.fmt, k.acc_smem, k.junroll, k.minb,
@@ -495,7 +613,8 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
 }
 
 // Tiling for `rows` i-rows: explicit config, else tuned, else heuristic.
-nbody_status get_tiling(nbody_engine* e, int rows, Tiling* out) {
+// full: the rows are all the bodies of the pass (a symmetric kernel may serve).
+nbody_status get_tiling(nbody_engine* e, int rows, Tiling* out, bool full = true) {
   const nbody_config& c = e->cfg;
   // defaults: the best measured shape of each family (Plummer N = 65536);
   // small systems take half the rows per thread, which doubles their row
@@ -516,8 +635,15 @@ nbody_status get_tiling(nbody_engine* e, int rows, Tiling* out) {
                 ipt, tj, variant);
   const bool automatic = !c.threads && !c.i_per_thread && !c.j_tile && !c.split_j &&
                          !c.pair_variant && !c.j_cluster;
-  if (c.tune && automatic) return autotune(e, rows, out);
-  if (e->tune_lookup && automatic && tuned_lookup(e, rows, out)) return NBODY_OK;
+  if (c.tune && automatic && full) return autotune(e, rows, out);
+  if (e->tune_lookup && automatic && tuned_lookup(e, rows, out, full)) return NBODY_OK;
+  if (full && automatic)
+    if (const PairKernel* ks = sym_kernel(e, rows)) {
+      out->k = ks;
+      out->split = choose_sym_split(e, *ks, rows);
+      out->source = 1;
+      return NBODY_OK;
+    }
   out->k = k;
   out->split = c.split_j ? std::min(c.split_j, kMaxSplit) : choose_split(e, *k, rows);
   out->split = std::min(kMaxSplit, (out->split + cl - 1) / cl * cl);  // whole clusters
@@ -538,7 +664,7 @@ nbody_status hilo_tiling(nbody_engine* e, int rows, Tiling* out) {
 nbody_status ensure_tiling(nbody_engine* e) {
   if (e->tiled) return NBODY_OK;
   NB_TRY(get_tiling(e, e->n, &e->tiling));
-  NB_TRY(ensure_partials(e, e->tiling.split));
+  NB_TRY(ensure_partials(e, partial_count(e->tiling, e->n)));
   e->tiled = true;
   return NBODY_OK;
 }
@@ -648,8 +774,7 @@ nbody_status eval_foreign_rel(nbody_engine* e, const Tiling& t, int n, const SoA
   NB_TRY(build_rel_tiles(e, n, sorted, st, t.k->tj));
   NB_TRY(launch_pair(e, t, 0, n, st, &sorted, n));
   if (!reduce) return NBODY_OK;  // the caller sums the splits (rows in sort_idx + ld order)
-  reduce_splits_kernel<<<(n + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, st>>>(
-      0, n, e->ld, partial_count(t), e->P, out, nullptr, ord);
+  launch_reduce(st, 0, n, e->ld, row_slots(t, n), e->P, out, nullptr, ord);
   NB_CUDA(cudaGetLastError());
   return NBODY_OK;
 }
@@ -691,8 +816,7 @@ nbody_status eval_current(nbody_engine* e) {
   }
   NB_CUDA(cudaEventRecord(e->ev_init[0], e->stream));
   NB_TRY(launch_pair(e, e->tiling, 0, e->n, e->stream));
-  reduce_splits_kernel<<<(e->n + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, e->stream>>>(
-      0, e->n, e->ld, partial_count(e->tiling), e->P, own_derivs(e));
+  launch_reduce(e->stream, 0, e->n, e->ld, row_slots(e->tiling, e->n), e->P, own_derivs(e));
   NB_CUDA(cudaGetLastError());
   NB_CUDA(cudaEventRecord(e->ev_init[1], e->stream));
   if (e->cfg.dt <= 0.0) {
@@ -716,8 +840,8 @@ nbody_status enqueue_predict(nbody_engine* e, cudaStream_t st) {
 }
 
 nbody_status enqueue_correct(nbody_engine* e, cudaStream_t st) {
-  correct_kernel<<<(e->n + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, st>>>(
-      e->n, e->ld, partial_count(e->tiling), e->P, e->X, e->V, e->D, e->ctl, e->cfg.eta);
+  launch_correct(st, e->n, e->ld, row_slots(e->tiling, e->n), e->P, e->X, e->V, e->D, e->ctl,
+                 e->cfg.eta);
   NB_CUDA(cudaGetLastError());
   return NBODY_OK;
 }
@@ -1188,7 +1312,7 @@ nbody_status nbody_acc_jerk_device(nbody_engine* e, int n, const double* x, cons
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : e->stream;
   Tiling t;
   NB_TRY(get_tiling(e, n, &t));
-  NB_TRY(ensure_partials(e, t.split));
+  NB_TRY(ensure_partials(e, partial_count(t, n)));
   const SoA7 in{x, y, z, m, vx, vy, vz};
   const SoA6 out{ax, ay, az, jx, jy, jz};
   if (t.k->fmt == kRecRel) {  // Hilbert order of the caller's bodies, gathered into scratch
@@ -1197,8 +1321,7 @@ nbody_status nbody_acc_jerk_device(nbody_engine* e, int n, const double* x, cons
   }
   NB_TRY(launch_pack(e, n, in, st, t.k->fmt, t.k->tj));
   NB_TRY(launch_pair(e, t, 0, n, st, &in, n));
-  reduce_splits_kernel<<<(n + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, st>>>(
-      0, n, e->ld, partial_count(t), e->P, out);
+  launch_reduce(st, 0, n, e->ld, row_slots(t, n), e->P, out);
   NB_CUDA(cudaGetLastError());
   return NBODY_OK;
 }
@@ -1304,11 +1427,11 @@ extern "C" nbody_status nbody_force_calculation(int n, double eps2, int precisio
   NB_TRY(ensure_tiling(e));
   Tiling t = e->tiling;
   const bool full = i_begin == 0 && i_end == n;
-  if (!full) NB_TRY(get_tiling(e, i_end - i_begin, &t));
+  if (!full) NB_TRY(get_tiling(e, i_end - i_begin, &t, false));
   // a row range: the packed hi/lo kernel, whose rows stay in the caller's
   // order (the near/far kernel evaluates all rows in Hilbert order)
   if (!full && t.k->fmt == kRecRel) NB_TRY(hilo_tiling(e, i_end - i_begin, &t));
-  NB_TRY(ensure_partials(e, t.split));
+  NB_TRY(ensure_partials(e, partial_count(t, n)));
   if (!e->aux) {
     NB_CUDA(cudaStreamCreateWithFlags(&e->aux, cudaStreamNonBlocking));
     for (auto& ev : e->aux_ev) NB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -1345,8 +1468,8 @@ extern "C" nbody_status nbody_force_calculation(int n, double eps2, int precisio
     if (i_begin > 0) memset(out[k], 0, sizeof(double) * i_begin);
     if (i_end < n) memset(out[k] + i_end, 0, sizeof(double) * (n - i_end));
     if (!rows) continue;
-    reduce_split_field_kernel<<<(rows + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, e->stream>>>(
-        i_begin, i_end, e->ld, partial_count(t), e->P + k * ld, e->D + k * ld, index);
+    launch_reduce_field(e->stream, i_begin, i_end, e->ld, row_slots(t, n), e->P + k * ld,
+                        e->D + k * ld, index);
     NB_CUDA(cudaGetLastError());
     NB_CUDA(cudaEventRecord(e->aux_ev[0], e->stream));
     NB_CUDA(cudaStreamWaitEvent(e->aux, e->aux_ev[0], 0));

@@ -81,11 +81,7 @@ __global__ void ens_pack_kernel(int L, const int* __restrict__ cid, const double
   const double x = real ? X[r] : 0, y = real ? X[L + r] : 0, z = real ? X[2 * L + r] : 0;
   const double m = real ? M[r] : 0;
   const double u = real ? V[r] : 0, v = real ? V[L + r] : 0, w = real ? V[2 * L + r] : 0;
-  if (jb64) {
-    JBody64 b;
-    b.x = x; b.y = y; b.z = z; b.m = m; b.vx = u; b.vy = v; b.vz = w; b.pad = 0;
-    jb64[r] = b;
-  }
+  if (jb64) store_jb64(jb64, r, x, y, z, m, u, v, w);
   if (jbx) jbx[r] = make_jbx2(x, y, z, m, u, v, w);
 }
 
@@ -112,11 +108,7 @@ __global__ void ens_predict_kernel(int L, const int* __restrict__ cid,
     V[k * L + r] = u[k];
   }
   const double m = M[r];
-  if (jb64) {
-    JBody64 b;
-    b.x = p[0]; b.y = p[1]; b.z = p[2]; b.m = m; b.vx = u[0]; b.vy = u[1]; b.vz = u[2]; b.pad = 0;
-    jb64[r] = b;
-  }
+  if (jb64) store_jb64(jb64, r, p[0], p[1], p[2], m, u[0], u[1], u[2]);
   if (jbx) jbx[r] = make_jbx2(p[0], p[1], p[2], m, u[0], u[1], u[2]);
 }
 
@@ -219,11 +211,14 @@ __global__ void __launch_bounds__(kBlock) ens_phi_kernel(const int* __restrict__
   __shared__ double4 tile[kBlock];
   const ClusterDev k = cl[blk_cluster[blockIdx.x]];
   const int i = blk_row[blockIdx.x] + threadIdx.x;  // cluster-relative row
-  const JBody64 bi = jb[k.row0 + i];
+  const double2* pi = jb64_at(jb, k.row0 + i);
+  const double2 pi0 = pi[0], pi1 = pi[32];
+  const double4 bi = make_double4(pi0.x, pi0.y, pi1.x, pi1.y);
   double acc = 0.0;
   for (int j0 = 0; j0 < k.ld; j0 += kBlock) {
-    const JBody64 bj = jb[k.row0 + j0 + threadIdx.x];
-    tile[threadIdx.x] = make_double4(bj.x, bj.y, bj.z, bj.m);
+    const double2* pj = jb64_at(jb, k.row0 + j0 + threadIdx.x);
+    const double2 pj0 = pj[0], pj1 = pj[32];
+    tile[threadIdx.x] = make_double4(pj0.x, pj0.y, pj1.x, pj1.y);
     __syncthreads();
 #pragma unroll 4
     for (int t = 0; t < kBlock; ++t) {

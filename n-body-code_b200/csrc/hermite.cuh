@@ -143,12 +143,7 @@ static __global__ void pack_kernel(int n, int ld, SoA7 in, JBody64* __restrict__
     x = in.x[i]; y = in.y[i]; z = in.z[i]; m = in.m[i];
     vx = in.vx[i]; vy = in.vy[i]; vz = in.vz[i];
   }
-  if (jb64) {
-    JBody64 b;
-    b.x = x; b.y = y; b.z = z; b.m = m;
-    b.vx = vx; b.vy = vy; b.vz = vz; b.pad = 0.0;
-    jb64[i] = b;
-  }
+  if (jb64) store_jb64(jb64, i, x, y, z, m, vx, vy, vz);
   if (jb32) jb32[i] = make_jb32(x, y, z, m, vx, vy, vz);
   if (jbx2) jbx2[i] = make_jbx2(x, y, z, m, vx, vy, vz);
 }
@@ -175,57 +170,108 @@ static __global__ void predict_kernel(int n, int ld, const StepCtl* __restrict__
     V[c * ld + i] = u[c];
   }
   const double m = M[i];
-  if (jb64) {
-    JBody64 b;
-    b.x = p[0]; b.y = p[1]; b.z = p[2]; b.m = m;
-    b.vx = u[0]; b.vy = u[1]; b.vz = u[2]; b.pad = 0.0;
-    jb64[i] = b;
-  }
+  if (jb64) store_jb64(jb64, i, p[0], p[1], p[2], m, u[0], u[1], u[2]);
   if (jb32) jb32[i] = make_jb32(p[0], p[1], p[2], m, u[0], u[1], u[2]);
   if (jbx2) jbx2[i] = make_jbx2(p[0], p[1], p[2], m, u[0], u[1], u[2]);
 }
 
-// sum[c] = sum over splits s = 0, 1, ..., S-1 (in that order) of
-// P[s][c][i], for the six fields at once: one pass over the splits with
+// Partial-sum slots of a row: S of every row and, where the symmetric pair
+// kernels (sympair.cuh) wrote them, one per block at distance 1, 2, ... ahead
+// of which the row's block lies.
+struct RowSlots {
+  int S;           // splits
+  int block_rows;  // rows per block of the symmetric schedule
+  int nb;          // its blocks; 0: no such slots
+  __host__ __device__ RowSlots(int splits, int rows = 1, int blocks = 0)
+      : S(splits), block_rows(rows), nb(blocks) {}
+  __device__ __forceinline__ int count(int i) const {
+    if (nb == 0) return S;
+    const int half = nb / 2;  // an even nb's last distance reaches the upper half only
+    return S + ((nb & 1) ? half : half - (i / block_rows < half ? 1 : 0));
+  }
+};
+
+// sum[c] = sum over slots s = 0, 1, ..., S-1 (in that order) of
+// P[s * step][c][i], for the six fields at once: one pass over the splits with
 // several loads in flight, so a small system (few CTAs) is not bound by
 // one load latency per split.
 __device__ __forceinline__ void split_sums(const double* __restrict__ P, int ld, int S, int i,
-                                           double sum[6]) {
+                                           double sum[6], int step = 1) {
 #pragma unroll
   for (int c = 0; c < 6; ++c) sum[c] = 0.0;
 #pragma unroll 4
   for (int s = 0; s < S; ++s) {
-    const double* p = P + static_cast<size_t>(s) * 6 * ld + i;
+    const double* p = P + static_cast<size_t>(s) * step * 6 * ld + i;
 #pragma unroll
     for (int c = 0; c < 6; ++c) sum[c] += p[static_cast<size_t>(c) * ld];
   }
 }
 
+// Threads of the kernels that sum slots: kSumThreads per CTA, as kSumThreads /
+// GR rows times GR groups.  Group g adds the slots g, g + GR, ... of its row,
+// and the groups' sums are added in group order through shared memory, so a
+// result's rounding depends on GR but not on timing.  A small system has few
+// rows and, with the symmetric kernels, dozens of slots: with one thread per
+// row its sums are a chain of loads on a handful of SMs.
+constexpr int kSumThreads = 256;
+template <int GR>
+constexpr int kSumRows = kSumThreads / GR;
+
+// The six sums of row i, valid in the threads of group 0 (threadIdx.x <
+// kSumRows<GR>); sh holds 6 * kSumThreads doubles when GR > 1.
+template <int GR>
+__device__ __forceinline__ void slot_sums(const double* __restrict__ P, int ld, int S, int i,
+                                          double sum[6], double* sh) {
+  constexpr int R = kSumRows<GR>;
+  const int g = threadIdx.x / R, r = threadIdx.x % R;
+  split_sums(P + static_cast<size_t>(g) * 6 * ld, ld, (S - g + GR - 1) / GR, i, sum, GR);
+  if (GR > 1) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) sh[(g * 6 + c) * R + r] = sum[c];
+    __syncthreads();
+    if (g == 0)
+#pragma unroll
+      for (int q = 1; q < GR; ++q)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) sum[c] += sh[(q * 6 + c) * R + r];
+  }
+}
+
 // Corrector fused with the split-j reduction and the Aarseth criterion:
-// a1/j1 = sum over S splits of P; snap/crackle; correct X, V; D <- a1/j1.
-static __global__ void correct_kernel(int n, int ld, int S, const double* __restrict__ P,
-                               double* __restrict__ X, double* __restrict__ V,
-                               double* __restrict__ D, StepCtl* __restrict__ ctl, double eta) {
-  __shared__ double sh[32];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// a1/j1 = sum over the row's slots of P; snap/crackle; correct X, V; D <- a1/j1.
+template <int GR>
+static __global__ void __launch_bounds__(kSumThreads)
+    correct_kernel(int n, int ld, RowSlots slots, const double* __restrict__ P,
+                   double* __restrict__ X, double* __restrict__ V, double* __restrict__ D,
+                   StepCtl* __restrict__ ctl, double eta) {
+  __shared__ double sh[GR > 1 ? 6 * kSumThreads : 32];
+  const int i = blockIdx.x * kSumRows<GR> + threadIdx.x % kSumRows<GR>;
   double crit = __longlong_as_double(static_cast<long long>(kPosInfBits));
-  if (i < n) {
+  const bool mine = i < n && threadIdx.x < kSumRows<GR>;
+  double x[3], v[3], d[6];
+  if (mine)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      x[c] = X[c * ld + i]; v[c] = V[c * ld + i];
+      d[c] = D[c * ld + i]; d[3 + c] = D[(3 + c) * ld + i];
+    }
+  double sum[6];
+  slot_sums<GR>(P, ld, i < n ? slots.count(i) : 0, i, sum, sh);
+  if (mine) {
     const double dt = ctl->dt;
     const double idt2 = 1.0 / (dt * dt);
     const double idt3 = idt2 / dt;
     const double dt3 = dt * dt * dt, dt4 = dt3 * dt, dt5 = dt4 * dt;
     double A2 = 0, J2 = 0, S2 = 0, C2 = 0;
-    double sum[6];
-    split_sums(P, ld, S, i, sum);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const double a1 = sum[c], j1 = sum[3 + c];
-      const double a = D[c * ld + i], j = D[(3 + c) * ld + i];
+      const double a = d[c], j = d[3 + c];
       const double da = a - a1;
       const double a2 = 2.0 * idt2 * (-3.0 * da - (2.0 * j + j1) * dt);
       const double a3 = 6.0 * idt3 * (2.0 * da + (j + j1) * dt);
-      X[c * ld + i] += a2 * dt4 * (1.0 / 24.0) + a3 * dt5 * (1.0 / 120.0);
-      V[c * ld + i] += a2 * dt3 * (1.0 / 6.0) + a3 * dt4 * (1.0 / 24.0);
+      X[c * ld + i] = x[c] + (a2 * dt4 * (1.0 / 24.0) + a3 * dt5 * (1.0 / 120.0));
+      V[c * ld + i] = v[c] + (a2 * dt3 * (1.0 / 6.0) + a3 * dt4 * (1.0 / 24.0));
       D[c * ld + i] = a1;
       D[(3 + c) * ld + i] = j1;
       A2 += a * a; J2 += j * j; S2 += a2 * a2; C2 += a3 * a3;
@@ -234,49 +280,98 @@ static __global__ void correct_kernel(int n, int ld, int S, const double* __rest
     const double den = sqrt(J2) * sqrt(C2) + S2;
     crit = sqrt(eta * num / den);
   }
+  if (GR > 1) __syncthreads();  // sh is reused
   finish_criterion(ctl, crit, true, sh);
 }
 
-// out[c][i] = sum_s P[s][c][i] for rows [i_begin, i_end), splits in order.
+// out[c][i] = sum over the row's slots of P for rows [i_begin, i_end).
 // With a status word (callers that cannot read it back before using the
 // outputs), a non-zero word - a pair kernel gave up a bounded wait - makes
 // every output NaN instead.  With an index map, row i is written to
 // out[c][index[i]] (partials kept in Hilbert order, outputs in the caller's
 // body order).
-static __global__ void reduce_splits_kernel(int i_begin, int i_end, int ld, int S,
-                                     const double* __restrict__ P, SoA6 out,
-                                     const int* __restrict__ status = nullptr,
-                                     const int* __restrict__ index = nullptr) {
-  const int i = i_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= i_end) return;
+template <int GR>
+static __global__ void __launch_bounds__(kSumThreads)
+    reduce_splits_kernel(int i_begin, int i_end, int ld, RowSlots slots,
+                         const double* __restrict__ P, SoA6 out,
+                         const int* __restrict__ status = nullptr,
+                         const int* __restrict__ index = nullptr) {
+  __shared__ double sh[GR > 1 ? 6 * kSumThreads : 1];
+  const int i = i_begin + blockIdx.x * kSumRows<GR> + threadIdx.x % kSumRows<GR>;
+  double sum[6];
+  slot_sums<GR>(P, ld, i < i_end ? slots.count(i) : 0, i, sum, sh);
+  if (i >= i_end || threadIdx.x >= kSumRows<GR>) return;
   double* dst[6] = {out.ax, out.ay, out.az, out.jx, out.jy, out.jz};
   const int o = index ? index[i] : i;
-  if (status && *status != 0) {
+  const bool bad = status && *status != 0;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) dst[c][o] = __longlong_as_double(0x7FF8000000000000ll);
-    return;
-  }
-  double sum[6];
-  split_sums(P, ld, S, i, sum);
-#pragma unroll
-  for (int c = 0; c < 6; ++c) dst[c][o] = sum[c];
+  for (int c = 0; c < 6; ++c)
+    dst[c][o] = bad ? __longlong_as_double(0x7FF8000000000000ll) : sum[c];
 }
 
 // One field of reduce_splits_kernel: out[index ? index[i] : i] = sum over
-// the S splits of P[(s*6 + c)*ld + i], for the field c whose [ld] block of
-// split 0 is Pc.  Same summation order as split_sums, so the same bits.
-// Lets a caller copy each finished field to the host while the next one
-// reduces.
-static __global__ void reduce_split_field_kernel(int i_begin, int i_end, int ld, int S,
-                                                 const double* __restrict__ Pc,
-                                                 double* __restrict__ out,
-                                                 const int* __restrict__ index = nullptr) {
-  const int i = i_begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= i_end) return;
+// the row's slots of P[(s*6 + c)*ld + i], for the field c whose [ld] block of
+// slot 0 is Pc.  Lets a caller copy each finished field to the host while the
+// next one reduces.
+template <int GR>
+static __global__ void __launch_bounds__(kSumThreads)
+    reduce_split_field_kernel(int i_begin, int i_end, int ld, RowSlots slots,
+                              const double* __restrict__ Pc, double* __restrict__ out,
+                              const int* __restrict__ index = nullptr) {
+  constexpr int R = kSumRows<GR>;
+  __shared__ double sh[kSumThreads];
+  const int g = threadIdx.x / R, r = threadIdx.x % R;
+  const int i = i_begin + blockIdx.x * R + r;
+  const int S = i < i_end ? slots.count(i) : 0;
   double sum = 0.0;
 #pragma unroll 8
-  for (int s = 0; s < S; ++s) sum += Pc[static_cast<size_t>(s) * 6 * ld + i];
-  out[index ? index[i] : i] = sum;
+  for (int s = g; s < S; s += GR) sum += Pc[static_cast<size_t>(s) * 6 * ld + i];
+  if (GR > 1) {
+    sh[threadIdx.x] = sum;
+    __syncthreads();
+    if (g == 0)
+#pragma unroll
+      for (int q = 1; q < GR; ++q) sum += sh[q * R + r];
+  }
+  if (g == 0 && i < i_end) out[index ? index[i] : i] = sum;
+}
+
+// Groups per row: eight from kSumGroupSlots slots, one below, where most
+// groups would have nothing to add.  Corrector with eight groups against one:
+// N = 1024 (26 slots) 3.9 against 10 us, N = 5003 (40) 6 against 16; N = 65536
+// (80), which the partials' bandwidth bounds, the same within 0.2 % of a step.
+constexpr int kSumGroupSlots = 8;
+inline bool sum_in_groups(const RowSlots& s) { return s.S + s.nb / 2 >= kSumGroupSlots; }
+
+inline void launch_correct(cudaStream_t st, int n, int ld, RowSlots slots, const double* P,
+                           double* X, double* V, double* D, StepCtl* ctl, double eta) {
+  if (sum_in_groups(slots))
+    correct_kernel<8><<<(n + kSumRows<8> - 1) / kSumRows<8>, kSumThreads, 0, st>>>(
+        n, ld, slots, P, X, V, D, ctl, eta);
+  else
+    correct_kernel<1><<<(n + kSumRows<1> - 1) / kSumRows<1>, kSumThreads, 0, st>>>(
+        n, ld, slots, P, X, V, D, ctl, eta);
+}
+inline void launch_reduce(cudaStream_t st, int i_begin, int i_end, int ld, RowSlots slots,
+                          const double* P, SoA6 out, const int* status = nullptr,
+                          const int* index = nullptr) {
+  const int rows = i_end - i_begin;
+  if (sum_in_groups(slots))
+    reduce_splits_kernel<8><<<(rows + kSumRows<8> - 1) / kSumRows<8>, kSumThreads, 0, st>>>(
+        i_begin, i_end, ld, slots, P, out, status, index);
+  else
+    reduce_splits_kernel<1><<<(rows + kSumRows<1> - 1) / kSumRows<1>, kSumThreads, 0, st>>>(
+        i_begin, i_end, ld, slots, P, out, status, index);
+}
+inline void launch_reduce_field(cudaStream_t st, int i_begin, int i_end, int ld, RowSlots slots,
+                                const double* Pc, double* out, const int* index) {
+  const int rows = i_end - i_begin;
+  if (sum_in_groups(slots))
+    reduce_split_field_kernel<8><<<(rows + kSumRows<8> - 1) / kSumRows<8>, kSumThreads, 0, st>>>(
+        i_begin, i_end, ld, slots, Pc, out, index);
+  else
+    reduce_split_field_kernel<1><<<(rows + kSumRows<1> - 1) / kSumRows<1>, kSumThreads, 0, st>>>(
+        i_begin, i_end, ld, slots, Pc, out, index);
 }
 
 // Initial step criterion min_i eta0 |a| / |j| (published via ctl).
@@ -322,15 +417,18 @@ static __global__ void __launch_bounds__(NT) potential_kernel(int n, int ld, dou
   __shared__ double4 tile[NT];
   __shared__ double sh[32];
   const int i = blockIdx.x * NT + threadIdx.x;
-  const JBody64 bi = jb[min(i, ld - 1)];
+  const double2* pi = jb64_at(jb, min(i, ld - 1));
+  const double2 pi0 = pi[0], pi1 = pi[32];
+  const double4 bi = make_double4(pi0.x, pi0.y, pi1.x, pi1.y);
   const int tiles = ld / NT, tps = (tiles + gridDim.y - 1) / gridDim.y;
   const int jb0 = blockIdx.y * tps * NT, jb1 = min(ld, (blockIdx.y + 1) * tps * NT);
   // four accumulators (partner k adds into acc[k % 4]), combined in a fixed
   // order: four independent add chains instead of one
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int j0 = jb0; j0 < jb1; j0 += NT) {
-    const JBody64 bj = jb[j0 + threadIdx.x];
-    tile[threadIdx.x] = make_double4(bj.x, bj.y, bj.z, bj.m);
+    const double2* pj = jb64_at(jb, j0 + threadIdx.x);
+    const double2 pj0 = pj[0], pj1 = pj[32];
+    tile[threadIdx.x] = make_double4(pj0.x, pj0.y, pj1.x, pj1.y);
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < NT; ++k) {
@@ -345,7 +443,7 @@ static __global__ void __launch_bounds__(NT) potential_kernel(int n, int ld, dou
   }
   const double phi = (acc[0] + acc[1]) + (acc[2] + acc[3]);
   double e = 0.0;
-  if (i < n) e = mode == 0 ? bi.m * phi : bi.m * bi.m * phi;
+  if (i < n) e = mode == 0 ? bi.w * phi : bi.w * bi.w * phi;
   const double b = block_sum(e, sh);
   if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = b;
 }

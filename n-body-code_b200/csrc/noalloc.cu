@@ -227,8 +227,7 @@ extern "C" nbody_status nbody_acc_jerk_noalloc(int n, double eps2, int precision
         reinterpret_cast<const JBodyX2*>(jb), a);
   if ((st = launched("pair kernel launch")) != NBODY_OK) return st;
   // a pair-kernel timeout (status word set) turns every output into NaN
-  reduce_splits_kernel<<<(n + 255) / 256, 256, 0, cs>>>(0, n, ld, split, P,
-                                                        SoA6{ax, ay, az, jx, jy, jz}, status);
+  launch_reduce(cs, 0, n, ld, split, P, SoA6{ax, ay, az, jx, jy, jz}, status);
   if ((st = launched("reduce_splits_kernel launch")) != NBODY_OK) return st;
   return NBODY_OK;
 }

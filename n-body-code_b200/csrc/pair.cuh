@@ -47,10 +47,30 @@ namespace nbody {
 // float (1e36 x m here; 3.4e38 is the float limit), else 0 x inf = NaN.
 constexpr double kMinEps2Mixed = 1e-24;
 
-// j-record, FP64 path: 64 bytes.
+// j-record, FP64 path: 64 bytes per body, in groups of 32 bodies, each group
+// four rows of 32 16-byte chunks (x, y), (z, m), (vx, vy), (vz, -).  A warp
+// writing 32 consecutive bodies, or reading them with one body per lane in
+// any rotation, moves contiguous 512-byte rows (no shared-memory bank
+// conflicts); a broadcast read of one body is four loads at fixed offsets.
+// The struct is only storage for one body's share of its group: records are
+// read and written through jb64_at / store_jb64.
 struct __align__(16) JBody64 {
-  double x, y, z, m, vx, vy, vz, pad;
+  double raw[8];
 };
+static_assert(sizeof(JBody64) == 64, "a group of 32 bodies is 2048 bytes");
+
+// Chunks of body i (a group's base is a multiple of 32): chunk c at [32 * c].
+__device__ __forceinline__ const double2* jb64_at(const JBody64* jb, int i) {
+  return reinterpret_cast<const double2*>(jb + (i & ~31)) + (i & 31);
+}
+__device__ __forceinline__ void store_jb64(JBody64* jb, int i, double x, double y, double z,
+                                           double m, double vx, double vy, double vz) {
+  double2* p = reinterpret_cast<double2*>(jb + (i & ~31)) + (i & 31);
+  p[0] = make_double2(x, y);
+  p[32] = make_double2(z, m);
+  p[64] = make_double2(vx, vy);
+  p[96] = make_double2(vz, 0.0);
+}
 
 // j-record, mixed path: 48 bytes.
 struct __align__(16) JBody32 {
@@ -184,11 +204,17 @@ struct TilePipe {
   }
 
   // Streams tiles src[t*TJ ...] for t < nt through shared memory and calls
-  // consume(tile) with all threads; false if a wait timed out (status
-  // reported, copies in flight drained).
+  // consume(tile) with all threads and, after the CTA barrier that ends the
+  // tile, post(); false if a wait timed out (status reported, copies in
+  // flight drained).
   template <class Consume>
   __device__ __forceinline__ bool run(const JB* __restrict__ src, int nt, int* status,
                                       Consume&& consume) {
+    return run(src, nt, status, consume, [] {});
+  }
+  template <class Consume, class Post>
+  __device__ __forceinline__ bool run(const JB* __restrict__ src, int nt, int* status,
+                                      Consume&& consume, Post&& post) {
     constexpr uint32_t kBytes = TJ * sizeof(JB);
     static_assert(kBytes % 16 == 0, "bulk copies move multiples of 16 bytes");
     const int tid = threadIdx.x;
@@ -215,6 +241,7 @@ struct TilePipe {
         mbar_arrive_expect_tx(&full[b], kBytes);
         bulk_load(buf + b * TJ, src + static_cast<size_t>(t + 2) * TJ, kBytes, &full[b]);
       }
+      post();
     }
     seq += nt;
     return true;
@@ -240,9 +267,8 @@ struct RowsFP64 {
                                         unsigned char*) {
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
-      const int i = min(row + k * NT, row_max);
-      const double2* r = reinterpret_cast<const double2*>(jb + i);
-      const double2 p0 = r[0], p1 = r[1], p2 = r[2], p3 = r[3];
+      const double2* r = jb64_at(jb, min(row + k * NT, row_max));
+      const double2 p0 = r[0], p1 = r[32], p2 = r[64], p3 = r[96];
       xi[k] = p0.x; yi[k] = p0.y; zi[k] = p1.x;
       ui[k] = p2.x; vi[k] = p2.y; wi[k] = p3.x;
       ax[k] = ay[k] = az[k] = 0.0;
@@ -254,8 +280,8 @@ struct RowsFP64 {
   __device__ __forceinline__ void consume(const JB* tile) {
 #pragma unroll JU
     for (int j = 0; j < TJ; ++j) {
-      const double2* r = reinterpret_cast<const double2*>(tile + j);
-      const double2 p0 = r[0], p1 = r[1], p2 = r[2], p3 = r[3];
+      const double2* r = jb64_at(tile, j);
+      const double2 p0 = r[0], p1 = r[32], p2 = r[64], p3 = r[96];
       const double xj = p0.x, yj = p0.y, zj = p1.x, mj = p1.y;
       const double uj = p2.x, vj = p2.y, wj = p3.x;
 #pragma unroll

@@ -1,0 +1,97 @@
+"""The symmetric pair kernels (each unordered pair evaluated once) at the edges
+of their tiles, blocks and schedules, against the oracle's direct sums.
+
+Masses are unequal and some are zero, so a pair that is missed, met twice or
+given the wrong body's mass shows at once.  FP64 bound 1e-12: the parity bound
+of the FP64 engine (sums of n terms of relative error ~2^-52, n <= 2^17)."""
+import numpy as np
+import pytest
+
+import nbody_b200 as nb
+import oracle as O
+from _util import derivs_rel, vec_rel
+
+pytestmark = pytest.mark.gpu
+
+EPS2 = 1e-4
+
+
+def bodies(n, seed=3):
+    s = nb.plummer(max(n, 2), seed=seed)
+    s = {k: v[:n].copy() for k, v in s.items()}
+    s["m"] = s["m"] * np.random.default_rng(seed).uniform(0.0, 2.0, n)
+    s["m"][::7] = 0.0
+    return s
+
+
+def derivs(s, precision, **kw):
+    with nb.Engine(s["x"].size, eps2=EPS2, precision=precision, dt=1.0, **kw) as e:
+        e.set_state(s)
+        e.force_calculation()
+        return e.get_derivs(), e.timers()
+
+
+# one block; tiles of 32; blocks of 256 rows, odd and even counts, short last
+# blocks; the four-row kernel (blocks of 512) from 16384
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 256, 257, 511, 513, 768, 769, 1025, 2047, 4097])
+def test_fp64_small_edges(n):
+    s = bodies(n)
+    d, _ = derivs(s, "fp64")
+    if n == 1:
+        assert np.all(d == 0.0)
+        return
+    ref = O.force(s, EPS2)
+    ok = np.abs(ref[:3]).max(axis=0) > 0  # a body whose partners are all massless feels nothing
+    assert np.all(d[:, ~ok] == 0.0)
+    ea, ej = derivs_rel(d[:, ok], ref[:, ok])
+    assert ea <= 1e-12 and ej <= 1e-12, (n, ea, ej)
+
+
+# the last n of one block size and the first of the next; blocks of two
+# sub-blocks (from 65537), odd and even block counts
+@pytest.mark.parametrize("n", [16383, 16384, 16897, 65536, 65537, 70001])
+def test_fp64_block_edges_sampled_rows(n):
+    s = bodies(n)
+    d, t = derivs(s, "fp64")
+    assert t["i_per_thread"] == (4 if n >= 16384 else 2)
+    rows = np.unique(np.concatenate([np.arange(0, n, n // 60), [n - 1, n - 2, n // 2, n // 2 - 1]]))
+    ref = O.force_rows(s, EPS2, rows)
+    ea, ej = derivs_rel(d[:, rows], ref)
+    assert ea <= 1e-12 and ej <= 1e-12, (n, ea, ej)
+    # the same sums from the one-sided kernel, every row
+    one, _ = derivs(s, "fp64", threads=128, i_per_thread=2, j_tile=128)
+    assert vec_rel(d[:3], one[:3]).max() <= 1e-12 and vec_rel(d[3:], one[3:]).max() <= 1e-11
+
+
+def test_fewer_bodies_than_the_engine_and_row_ranges():
+    """A device-array call on fewer bodies than the engine holds between its
+    own steps, and a drop-in row range after the autotuner cached a symmetric
+    tiling for another size with the same padding and row count."""
+    import torch
+    n, m = 3000, 2500
+    s = bodies(n)
+    sub = {k: v[:m] for k, v in s.items()}
+    t = [torch.tensor(sub[k], dtype=torch.float64, device="cuda") for k in nb.FIELDS]
+    out = torch.empty(6, m, dtype=torch.float64, device="cuda")
+    with nb.Engine(n, eps2=EPS2, dt=1 / 1024) as e, nb.Engine(n, eps2=EPS2, dt=1 / 1024) as f:
+        for g in (e, f):
+            g.set_state(s)
+            g.timestepping(2)
+        e.acc_jerk_device(*t, list(out), stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        for g in (e, f):
+            g.timestepping(2)
+        a, b = e.get_state(), f.get_state()
+    assert all(np.array_equal(a[k], b[k]) for k in a)
+    ea, ej = derivs_rel(out.cpu().numpy(), O.force(sub, EPS2))
+    assert ea <= 1e-12 and ej <= 1e-12, (ea, ej)
+    big = bodies(5100)
+    nb.release_force_cache()
+    try:
+        nb.force_calculation_tune({k: v[:5000] for k, v in big.items()}, eps2=EPS2)
+        part = nb.force_calculation(big, eps2=EPS2, i_begin=0, i_end=5000)
+    finally:
+        nb.release_force_cache()
+    assert np.all(part[:, 5000:] == 0.0)
+    ea, ej = derivs_rel(part[:, :5000], O.force_rows(big, EPS2, np.arange(5000)))
+    assert ea <= 1e-12 and ej <= 1e-12, (ea, ej)
