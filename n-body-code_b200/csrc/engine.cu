@@ -75,6 +75,10 @@ constexpr int kOrderBits = 48;     // Hilbert key width (order_key_kernel)
 // beyond the cell.
 constexpr int kDropInOrderLowBit = 18;
 constexpr int kMaxPotSplit = 32;    // j-splits of the potential diagnostic
+// Calls on caller-owned bodies order them for the near/far kernel from this
+// many bodies: ordering costs about 0.09 ms a call and saves the pair pass
+// 0.02 ms at N = 16384.
+constexpr int kForeignOrderMin = 32768;
 
 thread_local std::string g_last_error;
 
@@ -151,6 +155,16 @@ PairKernel make_sym_fp64() {
   return k;
 }
 
+template <int IPT, int W, int SUB, int UNR, int NUNR, int MINB>
+PairKernel make_sym_nf() {
+  PairKernel k{NBODY_MIXED, 32 * W, IPT, 64 * SUB, kRecSym,
+               reinterpret_cast<const void*>(&pair_sym_nf_kernel<IPT, W, SUB, UNR, NUNR, MINB>),
+               sym_nf_smem<IPT, W, SUB>(), 1, UNR, MINB};
+  k.near = 1;
+  k.sym = true;
+  return k;
+}
+
 // Near/far rows on clusters of CL CTAs along j: split count a multiple of CL,
 // S / CL partials (pair_mixed_nf_cluster_kernel).
 template <int NT, int IPT, int TJ, int JU, int MINB, int NEAR, int CL>
@@ -160,40 +174,34 @@ PairKernel make_mixed_nf_cl() {
           2 * (TJ + 1) * sizeof(JBodyNF) + sizeof(double) * 6 * IPT * NT, 1, JU, MINB, 1, CL};
 }
 
-// The first entry of each shape/variant is the one explicit tilings select
-// (never a cluster kernel); the autotuner times all of them.
+// One-sided kernels: the shapes an explicit tiling may ask for (one entry
+// each) and, for row ranges, the default ones.  Symmetric kernels: full-row
+// passes with an automatic tiling; the autotuner times them.
 const std::vector<PairKernel>& registry() {
   static const std::vector<PairKernel> r = {
-      make_fp64<128, 2, 128, 1>(),  make_fp64<128, 2, 128, 2>(),  make_fp64<128, 1, 128, 4>(),
-      make_fp64<128, 1, 128, 2>(),  make_fp64<128, 4, 128, 1>(),  make_fp64<256, 1, 128, 4>(),
-      make_fp64<256, 2, 128, 1>(),  make_fp64<128, 2, 256, 1>(),  make_fp64<64, 2, 128, 1>(),
-      make_fp64<128, 2, 128, 1, 6>(), make_fp64<128, 2, 64, 1, 6>(), make_fp64<128, 1, 128, 4, 8>(),
-      // symmetric (full-row passes; sym_kernel chooses between the two)
+      // symmetric: sym_kernel chooses by size
       make_sym_fp64<4, 4, 2, 2>(), make_sym_fp64<2, 4, 4, 4>(),
-      // near/far tile-relative packed pairs (bodies in Hilbert order; default
-      // mixed: 128 x 4 rows, j-unroll 2, 4 CTAs/SM = 128 registers, no spills)
+      make_sym_nf<4, 4, 2, 4, 2, 3>(), make_sym_nf<2, 4, 1, 4, 2, 4>(),
+      make_fp64<128, 2, 128, 1>(),  make_fp64<128, 1, 128, 4>(),  make_fp64<128, 4, 128, 1>(),
+      make_fp64<256, 1, 128, 4>(),  make_fp64<256, 2, 128, 1>(),  make_fp64<128, 2, 256, 1>(),
+      make_fp64<64, 2, 128, 1>(),   make_fp64<128, 2, 64, 1, 6>(),
+      // near/far tile-relative packed pairs (bodies in Hilbert order)
       make_mixed_nf<128, 4, 128, 1, 2, 4>(), make_mixed_nf<64, 4, 128>(), make_mixed_nf<128, 2, 128>(),
       make_mixed_nf<256, 2, 128>(), make_mixed_nf<256, 4, 128>(), make_mixed_nf<128, 2, 64>(),
-      make_mixed_nf<128, 4, 64>(),  make_mixed_nf<128, 2, 256>(), make_mixed_nf<128, 4, 128, 0, 2>(),
-      make_mixed_nf<128, 4, 128>(), make_mixed_nf<128, 4, 128, 1, 1, 4>(),
-      make_mixed_nf<64, 4, 128, 1, 1, 8>(),  make_mixed_nf<128, 6, 128, 1, 1>(),
-      make_mixed_nf<64, 6, 128, 1, 1>(),     make_mixed_nf<128, 4, 128, 1, 2>(),
-      make_mixed_nf<128, 4, 64, 1, 2, 4>(),  make_mixed_nf<128, 2, 64, 1, 2, 4>(),
-      make_mixed_nf<128, 4, 128, 1, 2, 4, 2>(), make_mixed_nf<64, 4, 128, 1, 2, 8, 2>(),
+      make_mixed_nf<128, 4, 64>(),  make_mixed_nf<128, 2, 256>(), make_mixed_nf<128, 6, 128>(),
+      make_mixed_nf<64, 6, 128>(),
       // the same kernel with every tile taken as far (plain tile-relative
       // separations; pair_variant 5, a measured comparison)
       make_mixed_nf<128, 4, 128, 1, 2, 4, 0>(), make_mixed_nf<128, 2, 128, 1, 1, 1, 0>(),
       // near/far on thread-block clusters along j (fewer split partials;
-      // selected by nbody_config.j_cluster, not by the autotuner)
+      // selected by nbody_config.j_cluster)
       make_mixed_nf_cl<128, 4, 128, 2, 4, 2, 8>(), make_mixed_nf_cl<128, 4, 128, 2, 4, 2, 4>(),
       make_mixed_nf_cl<128, 4, 128, 2, 4, 2, 2>(),
-      // packed pairs, FP64 accumulators in shared memory (default)
+      // packed hi/lo pairs, FP64 accumulators in shared memory
       make_mixed_x2<128, 4, 128, 1, 1>(), make_mixed_x2<256, 4, 128, 1, 1>(),
-      make_mixed_x2<128, 4, 128, 1, 2>(), make_mixed_x2<64, 4, 128, 1, 1>(),
-      make_mixed_x2<128, 2, 128, 1, 1>(),
-      make_mixed_x2<128, 4, 64, 1, 1, 5>(), make_mixed_x2<128, 4, 64, 1, 1, 6>(),
-      make_mixed_x2<128, 4, 64, 1, 1>(),    make_mixed_x2<64, 4, 64, 1, 1, 10>(),
-      // packed pairs, FP64 accumulators in registers
+      make_mixed_x2<64, 4, 128, 1, 1>(),  make_mixed_x2<128, 2, 128, 1, 1>(),
+      make_mixed_x2<128, 4, 64, 1, 1, 5>(), make_mixed_x2<64, 4, 64, 1, 1, 10>(),
+      // packed hi/lo pairs, FP64 accumulators in registers
       make_mixed_x2<128, 4, 128, 0, 2>(), make_mixed_x2<128, 2, 128, 0, 2>(),
       make_mixed_x2<256, 2, 128, 0, 2>(), make_mixed_x2<64, 4, 128, 0, 2>(),
       make_mixed_x2<128, 4, 64, 0, 2>(),
@@ -308,12 +316,11 @@ struct nbody_engine {
   bool tiled = false;
   cudaGraphExec_t graph = nullptr;
   int graph_kernels = 0;  // kernel nodes of the captured step
-  // automatic mixed kernel (pair_variant 0): near/far from this many bodies,
-  // packed hi/lo below (measured Hermite steps, Plummer spheres: N = 8192
-  // 0.136 vs 0.124 ms, N = 16384 0.352 vs 0.366 ms).  Engines re-order every
-  // sort_every steps; the drop-in re-orders on every call and raises the
-  // threshold.
-  int rel_min_bodies = 16384;
+  // automatic mixed kernel (pair_variant 0): bodies in Hilbert order from this
+  // many, in the caller's below, where too few subtiles would be far to pay
+  // for the ordering.  An engine re-orders every sort_every steps; a drop-in
+  // or device-array call on every call (kForeignOrderMin).
+  int order_min_bodies = 16384;
   // drop-in engines: reuse a tiling the autotuner chose for the same
   // (device, precision, record format, size) in this process; never tune
   bool tune_lookup = false;
@@ -332,18 +339,30 @@ namespace {
 
 int round_up(int a, int b) { return (a + b - 1) / b * b; }
 
-// The mixed kernel family in use: pair_variant, with 0 (automatic)
-// resolved by the system size.
+bool explicit_shape(const nbody_config& c) {
+  return c.threads || c.i_per_thread || c.j_tile || c.split_j || c.j_cluster;
+}
+
+// The mixed kernel family in use: pair_variant, 0 (automatic) being near/far;
+// with an explicit (one-sided) shape, packed hi/lo below order_min_bodies,
+// where the one-sided near/far kernel is the slower of the two.
 int effective_variant(const nbody_engine* e) {
   const nbody_config& c = e->cfg;
   if (c.precision != NBODY_MIXED || c.pair_variant != 0) return c.pair_variant;
-  return e->n >= e->rel_min_bodies ? 4 : 3;
+  return explicit_shape(c) && e->n < e->order_min_bodies ? 3 : 4;
 }
 
 // Record format of the autotuner's family (the automatic choice).
 int default_format(const nbody_engine* e) {
-  if (e->cfg.precision == NBODY_FP64) return kRecF64;
-  return effective_variant(e) >= 4 ? kRecRel : kRecX2;
+  return e->cfg.precision == NBODY_FP64 ? kRecF64 : kRecSym;
+}
+
+bool tile_relative(int fmt) { return fmt == kRecRel || fmt == kRecSym; }
+
+// Whether tile-relative kernels of this engine get their bodies in Hilbert
+// order: the one-sided ones always, the automatic choice from `min` bodies.
+bool wants_order(const nbody_engine* e, int n, int min) {
+  return e->cfg.pair_variant >= 4 || n >= min;
 }
 
 // The engine keeps its bodies in Hilbert order (positions != body indices).
@@ -396,8 +415,7 @@ int choose_split(const nbody_engine* e, const PairKernel& k, int rows) {
 // run of Q tiles, ceil(Q / S) each.  Same wave model, over the tile counts
 // that differ: full waves cost a CTA's tiles, the last one what its fullest
 // SM holds (but at least half: alone on its SM a CTA is latency-bound), and
-// every split another 48 bytes per row to write and sum, at the measured rate
-// of 13 us per (CTA, tile).
+// every split another 48 bytes per row to sum.
 int choose_sym_split(const nbody_engine* e, const PairKernel& k, int n) {
   prepare_kernel(k);
   int occ = 0;
@@ -407,7 +425,8 @@ int choose_sym_split(const nbody_engine* e, const PairKernel& k, int n) {
   const SymGrid g(k, n);
   const int Q = sym_q_count(g.nb, 0, g.block_rows / k.tj, (n + k.tj - 1) / k.tj);
   const long slots = static_cast<long>(e->num_sms) * occ;
-  const double tile_ms = 0.013 * (k.nt * k.ipt / 512.0) * (k.tj / 32.0) * (occ / 2.0);
+  const double per_ms = k.precision == NBODY_FP64 ? 7.6e8 : 1.6e9;  // interactions of a full GPU
+  const double tile_ms = 2.0 * k.nt * k.ipt * k.tj * slots / per_ms;
   const double per_split = 48.0 * n / kSplitSumBytesPerMs / tile_ms;
   double best = 1e300;
   int best_s = 1;
@@ -462,8 +481,9 @@ nbody_status prepare_kernel(const PairKernel& k) {
 
 SoA7 own_inputs(nbody_engine* e);
 
-// A symmetric pass over all rows of n bodies whose records are in place.
-nbody_status launch_sym(nbody_engine* e, const Tiling& t, int n, cudaStream_t st) {
+// A symmetric pass over all rows of n bodies whose records are in place; src:
+// the bodies the records were built from.
+nbody_status launch_sym(nbody_engine* e, const Tiling& t, int n, cudaStream_t st, const SoA7& src) {
   const PairKernel& k = *t.k;
   const SymGrid g(k, n);
   SymArgs a;
@@ -477,7 +497,9 @@ nbody_status launch_sym(nbody_engine* e, const Tiling& t, int n, cudaStream_t st
   a.out = e->P;
   a.stride = static_cast<size_t>(e->ld);
   a.status = e->status;
-  const void* jb = e->jb64;
+  a.rows = src;
+  a.near_count = e->near_count;
+  const void* jb = k.fmt == kRecF64 ? static_cast<const void*>(e->jb64) : e->jb32;
   void* args[] = {static_cast<void*>(&jb), static_cast<void*>(&a)};
   NB_CUDA(cudaLaunchKernel(k.fn, dim3(g.nb, t.split), dim3(k.nt), args, k.smem, st));
   return NBODY_OK;
@@ -489,7 +511,8 @@ nbody_status launch_pair(nbody_engine* e, const Tiling& t, int i_begin, int i_en
                          cudaStream_t st, const SoA7* src = nullptr, int n_src = 0) {
   const PairKernel& k = *t.k;
   NB_TRY(prepare_kernel(k));
-  if (k.sym) return launch_sym(e, t, i_end, st);  // full rows: [0, i_end)
+  if (k.sym)  // full rows: [0, i_end)
+    return launch_sym(e, t, i_end, st, src ? *src : own_inputs(e));
   PairArgs a;
   a.i_begin = i_begin;
   a.i_end = i_end;
@@ -537,15 +560,16 @@ bool tuned_lookup(const nbody_engine* e, int rows, Tiling* out, bool full = true
   return true;
 }
 
-// The symmetric kernel an automatic full-row pass over n bodies takes, or null.
-// Four rows per lane from 16384 bodies, two below, where twice the blocks
-// fill the SMs (pair pass: N = 8192 106 us both, 4096 34 vs 36, 2048 19.5 vs
-// 17.5, 1024 13.2 vs 11.3; one-sided 144, 44, 18.2 and 15.0).
+// The symmetric kernel an automatic full-row pass over n bodies takes.  Four
+// rows per lane from 16384 bodies, two below, where twice the blocks fill the
+// SMs.  Pair pass in us, two / four rows / one-sided: FP64 N = 16384 386 /
+// 380 / 539, 8192 106 / 106 / 144, 4096 36 / 34 / 44, 1024 11.3 / 13.2 / 15;
+// mixed N = 16384 226 / 227 / 300, 8192 73 / 81 / 88, 4096 26 / 34 / 33, 1024
+// 13.5 / 21.5 / 18.
 const PairKernel* sym_kernel(const nbody_engine* e, int n) {
   const int want = n >= 16384 ? 4 : 2;
   for (const auto& k : registry())
-    if (k.sym && k.precision == e->cfg.precision && k.fmt == default_format(e) && k.ipt == want)
-      return &k;
+    if (k.sym && k.precision == e->cfg.precision && k.ipt == want) return &k;
   return nullptr;
 }
 
@@ -558,24 +582,18 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
   float best = 1e30f;
   int best_idx = -1, best_split = 1;
   const auto& reg = registry();
-  const bool use_sym = rows == e->n && sym_kernel(e, rows);
-  // the near/far kernel's cost depends on the bodies being in Hilbert order
-  if (default_format(e) == kRecRel && e->have_state && !e->sorted)
+  // the near/far kernel's cost depends on the order of the bodies
+  if (default_format(e) == kRecSym && e->have_state && !e->sorted &&
+      wants_order(e, e->n, e->order_min_bodies))
     NB_TRY(enqueue_reorder_state(e, e->stream));
   for (size_t idx = 0; idx < reg.size(); ++idx) {
     const PairKernel& k = reg[idx];
-    if (k.precision != e->cfg.precision || k.fmt != default_format(e)) continue;
-    if (k.fmt == kRecRel && !k.near) continue;  // the automatic choice keeps near tiles exact
-    // cluster kernels save in the split sums what their pair pass loses
-    // (N = 65536: 4.071 vs 4.071 ms with the sums priced in); not timed
-    if (k.cluster > 1) continue;
-    // symmetric kernels serve full-row passes (faster than every one-sided
-    // shape there at each size from 1024 to 262144), one-sided ones the rest
-    if (k.sym != use_sym) continue;
-    const int s0 = k.sym ? choose_sym_split(e, k, rows) : choose_split(e, k, rows);
+    // the symmetric kernels: faster than every one-sided shape in full-row
+    // passes at each size from 1024 to 262144
+    if (!k.sym || k.precision != e->cfg.precision) continue;
+    const int s0 = choose_sym_split(e, k, rows);
     NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj));
     for (int s : {std::max(1, s0 / 2), s0, std::min(kMaxSplit, s0 * 2)}) {
-      s = std::min(kMaxSplit, (s + k.cluster - 1) / k.cluster * k.cluster);
       Tiling t{&k, s};
       NB_TRY(ensure_partials(e, partial_count(t, rows)));
       NB_TRY(launch_pair(e, t, 0, rows, e->stream));  // warm-up
@@ -633,17 +651,16 @@ nbody_status get_tiling(nbody_engine* e, int rows, Tiling* out, bool full = true
     return fail(NBODY_ERR_INVALID_ARG,
                 "no compiled pair kernel for threads=%d i_per_thread=%d j_tile=%d variant=%d", nt,
                 ipt, tj, variant);
-  const bool automatic = !c.threads && !c.i_per_thread && !c.j_tile && !c.split_j &&
-                         !c.pair_variant && !c.j_cluster;
+  const bool automatic = !explicit_shape(c) && !c.pair_variant;
   if (c.tune && automatic && full) return autotune(e, rows, out);
   if (e->tune_lookup && automatic && tuned_lookup(e, rows, out, full)) return NBODY_OK;
-  if (full && automatic)
-    if (const PairKernel* ks = sym_kernel(e, rows)) {
-      out->k = ks;
-      out->split = choose_sym_split(e, *ks, rows);
-      out->source = 1;
-      return NBODY_OK;
-    }
+  const bool near_far = c.precision == NBODY_MIXED && c.pair_variant == 4;
+  if (full && (automatic || (near_far && !explicit_shape(c)))) {
+    out->k = sym_kernel(e, rows);
+    out->split = choose_sym_split(e, *out->k, rows);
+    out->source = 1;
+    return NBODY_OK;
+  }
   out->k = k;
   out->split = c.split_j ? std::min(c.split_j, kMaxSplit) : choose_split(e, *k, rows);
   out->split = std::min(kMaxSplit, (out->split + cl - 1) / cl * cl);  // whole clusters
@@ -745,7 +762,11 @@ nbody_status build_rel_tiles(nbody_engine* e, int n, const SoA7& in, cudaStream_
 // then be in Hilbert order.  (The energy diagnostic packs its own records.)
 nbody_status launch_pack(nbody_engine* e, int n, const SoA7& in, cudaStream_t st, int fmt,
                          int tj) {
-  if (fmt != kRecRel) {
+  if (fmt == kRecSym) {
+    sym_tile_kernel<false><<<e->ld / 64, 64, 0, st>>>(n, in, static_cast<SymSub*>(e->jb32), 0, nullptr,
+                                                      nullptr, nullptr, nullptr, e->near_count);
+    NB_CUDA(cudaGetLastError());
+  } else if (fmt != kRecRel) {
     pack_kernel<<<(e->ld + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, st>>>(
         n, e->ld, in, e->jb64, fmt == kRecF32 ? static_cast<JBody32*>(e->jb32) : nullptr,
         fmt == kRecX2 ? static_cast<JBodyX2*>(e->jb32) : nullptr);
@@ -771,7 +792,7 @@ nbody_status eval_foreign_rel(nbody_engine* e, const Tiling& t, int n, const SoA
   gather_rows_kernel<<<(n + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, st>>>(n, ord, g, nullptr, nullptr);
   NB_CUDA(cudaGetLastError());
   const SoA7 sorted{g.dst[0], g.dst[1], g.dst[2], g.dst[3], g.dst[4], g.dst[5], g.dst[6]};
-  NB_TRY(build_rel_tiles(e, n, sorted, st, t.k->tj));
+  NB_TRY(launch_pack(e, n, sorted, st, t.k->fmt, t.k->tj));
   NB_TRY(launch_pair(e, t, 0, n, st, &sorted, n));
   if (!reduce) return NBODY_OK;  // the caller sums the splits (rows in sort_idx + ld order)
   launch_reduce(st, 0, n, e->ld, row_slots(t, n), e->P, out, nullptr, ord);
@@ -783,7 +804,9 @@ int tiling_fmt(const nbody_engine* e) { return e->tiled ? e->tiling.k->fmt : kRe
 int tiling_tj(const nbody_engine* e) { return e->tiled ? e->tiling.k->tj : 0; }
 int sort_period(const nbody_engine* e) { return e->cfg.sort_every > 0 ? e->cfg.sort_every : 16; }
 
-bool curve_resident(const nbody_engine* e) { return tiling_fmt(e) == kRecRel; }
+bool curve_resident(const nbody_engine* e) {
+  return tile_relative(tiling_fmt(e)) && wants_order(e, e->n, e->order_min_bodies);
+}
 
 // Before a step of the engine's own state: re-order when the order is stale
 // (never made since set_state, or sort_every steps old).
@@ -830,6 +853,12 @@ nbody_status eval_current(nbody_engine* e) {
 
 nbody_status enqueue_predict(nbody_engine* e, cudaStream_t st) {
   const int fmt = tiling_fmt(e);
+  if (fmt == kRecSym) {
+    sym_tile_kernel<true><<<e->ld / 64, 64, 0, st>>>(e->n, own_inputs(e), static_cast<SymSub*>(e->jb32),
+                                                     e->ld, e->X, e->V, e->D, e->ctl, e->near_count);
+    NB_CUDA(cudaGetLastError());
+    return NBODY_OK;
+  }
   predict_kernel<<<(e->n + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, st>>>(
       e->n, e->ld, e->ctl, e->X, e->V, e->M, e->D, fmt == kRecF64 ? e->jb64 : nullptr,
       fmt == kRecF32 ? static_cast<JBody32*>(e->jb32) : nullptr,
@@ -895,7 +924,7 @@ nbody_status build_step_graph(nbody_engine* e) {
     e->graph = nullptr;
     return fail(NBODY_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ce));
   }
-  if (tiling_fmt(e) == kRecRel && !e->order_graph) {
+  if (curve_resident(e) && !e->order_graph) {
     // the Hilbert re-ordering of the engine's own state, replayed every
     // sort_every steps ahead of the step graph
     const bool sorted = e->sorted, permuted = e->permuted;
@@ -1254,15 +1283,25 @@ nbody_status nbody_get_timers(nbody_engine* e, nbody_timers* out) {
     out->j_tile = e->tiling.k->tj;
     out->split_j = e->tiling.split;
     out->j_cluster = e->tiling.k->cluster;
-    out->record_format = e->tiling.k->fmt;
+    out->record_format = e->tiling.k->fmt == kRecSym ? kRecRel : e->tiling.k->fmt;
     out->tiling_source = e->tiling.source;
     const PairKernel& k = *e->tiling.k;
-    if (k.fmt == kRecRel && k.near) {
+    if (tile_relative(k.fmt) && k.near) {
       unsigned long long near = 0;
       NB_CUDA(cudaMemcpy(&near, e->near_count, sizeof near, cudaMemcpyDeviceToHost));
-      // classified per (warp, tile): warps = row blocks x NT / 32
-      const double pairs = static_cast<double>((e->n + k.nt * k.ipt - 1) / (k.nt * k.ipt)) *
-                           (k.nt / 32) * static_cast<double>(e->ld / k.tj);
+      // classified per (warp, tile): warps = row blocks x NT / 32; the
+      // symmetric kernel's 64-body subtiles, over the runs of its blocks
+      double pairs = static_cast<double>((e->n + k.nt * k.ipt - 1) / (k.nt * k.ipt)) *
+                     (k.nt / 32) * static_cast<double>(e->ld / k.tj);
+      if (k.sym) {
+        const SymGrid g(k, e->n);
+        pairs = 0.0;
+        for (int I = 0; I < g.nb; ++I) {
+          const int rows = std::min(g.block_rows, e->n - I * g.block_rows);
+          pairs += static_cast<double>((rows + 32 * k.ipt - 1) / (32 * k.ipt)) * (k.tj / 64) *
+                   sym_q_count(g.nb, I, g.block_rows / k.tj, (e->n + k.tj - 1) / k.tj);
+        }
+      }
       out->near_tile_fraction = static_cast<double>(near) / pairs;
     }
   }
@@ -1315,7 +1354,8 @@ nbody_status nbody_acc_jerk_device(nbody_engine* e, int n, const double* x, cons
   NB_TRY(ensure_partials(e, partial_count(t, n)));
   const SoA7 in{x, y, z, m, vx, vy, vz};
   const SoA6 out{ax, ay, az, jx, jy, jz};
-  if (t.k->fmt == kRecRel) {  // Hilbert order of the caller's bodies, gathered into scratch
+  if (tile_relative(t.k->fmt) && wants_order(e, n, kForeignOrderMin)) {
+    // Hilbert order of the caller's bodies, gathered into scratch
     NB_TRY(enqueue_curve_order(e, n, in, st, kDropInOrderLowBit));
     return eval_foreign_rel(e, t, n, in, out, st);
   }
@@ -1368,9 +1408,7 @@ nbody_status dropin_engine(int n, double eps2, int precision, nbody_engine** out
     c.device = dev;
     c.dt = 1.0;  // fixed: no initial-dt pass on the drop-in path
     NB_TRY(nbody_create(&d.e, &c));
-    // every call re-orders: tile-relative pays off only above ~24k bodies
-    // (measured per call: N = 16384 428 vs 357 us hi/lo; N = 65536 it wins)
-    d.e->rel_min_bodies = 32768;
+    d.e->order_min_bodies = kForeignOrderMin;  // every call re-orders
     d.e->tune_lookup = true;
     d.n = n;
     d.eps2 = eps2;
@@ -1430,14 +1468,14 @@ extern "C" nbody_status nbody_force_calculation(int n, double eps2, int precisio
   if (!full) NB_TRY(get_tiling(e, i_end - i_begin, &t, false));
   // a row range: the packed hi/lo kernel, whose rows stay in the caller's
   // order (the near/far kernel evaluates all rows in Hilbert order)
-  if (!full && t.k->fmt == kRecRel) NB_TRY(hilo_tiling(e, i_end - i_begin, &t));
+  if (!full && tile_relative(t.k->fmt)) NB_TRY(hilo_tiling(e, i_end - i_begin, &t));
   NB_TRY(ensure_partials(e, partial_count(t, n)));
   if (!e->aux) {
     NB_CUDA(cudaStreamCreateWithFlags(&e->aux, cudaStreamNonBlocking));
     for (auto& ev : e->aux_ev) NB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
   const int* index = nullptr;  // row -> output position (the near/far rows are in Hilbert order)
-  if (t.k->fmt == kRecRel) {
+  if (tile_relative(t.k->fmt) && wants_order(e, n, kForeignOrderMin)) {
     // positions first: their Hilbert ordering runs while the masses and
     // velocities upload on a second stream
     NB_CUDA(cudaEventRecord(e->aux_ev[0], e->stream));

@@ -121,7 +121,7 @@ __device__ __forceinline__ JBodyX2 make_jbx2(double x, double y, double z, doubl
 }
 
 // j-record formats of the pair kernels.
-enum RecordFormat { kRecF64 = 0, kRecF32 = 1, kRecX2 = 2, kRecRel = 3 };
+enum RecordFormat { kRecF64 = 0, kRecF32 = 1, kRecX2 = 2, kRecRel = 3, kRecSym = 4 };
 
 // Seven SoA input arrays (caller's or the engine's own).
 struct SoA7 {
@@ -148,18 +148,12 @@ static __global__ void pack_kernel(int n, int ld, SoA7 in, JBody64* __restrict__
   if (jbx2) jbx2[i] = make_jbx2(x, y, z, m, vx, vy, vz);
 }
 
-// Predictor: in place on X, V (rows < n) and writes the j-records of the
-// predicted state (jb64 or jb32, whichever is non-null).
-static __global__ void predict_kernel(int n, int ld, const StepCtl* __restrict__ ctl, double* __restrict__ X,
-                               double* __restrict__ V, const double* __restrict__ M,
-                               const double* __restrict__ D, JBody64* __restrict__ jb64,
-                               JBody32* __restrict__ jb32, JBodyX2* __restrict__ jbx2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double dt = ctl->dt;
+// Predicted position p and velocity u of row i, written back to X, V.
+__device__ __forceinline__ void predict_body(double dt, int ld, int i, double* __restrict__ X,
+                                             double* __restrict__ V, const double* __restrict__ D,
+                                             double p[3], double u[3]) {
   const double h2 = 0.5 * dt * dt;
   const double h3 = dt * dt * dt * (1.0 / 6.0);
-  double p[3], u[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const double x = X[c * ld + i], v = V[c * ld + i];
@@ -169,6 +163,18 @@ static __global__ void predict_kernel(int n, int ld, const StepCtl* __restrict__
     X[c * ld + i] = p[c];
     V[c * ld + i] = u[c];
   }
+}
+
+// Predictor: in place on X, V (rows < n) and writes the j-records of the
+// predicted state (jb64 or jb32, whichever is non-null).
+static __global__ void predict_kernel(int n, int ld, const StepCtl* __restrict__ ctl, double* __restrict__ X,
+                               double* __restrict__ V, const double* __restrict__ M,
+                               const double* __restrict__ D, JBody64* __restrict__ jb64,
+                               JBody32* __restrict__ jb32, JBodyX2* __restrict__ jbx2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double p[3], u[3];
+  predict_body(ctl->dt, ld, i, X, V, D, p, u);
   const double m = M[i];
   if (jb64) store_jb64(jb64, i, p[0], p[1], p[2], m, u[0], u[1], u[2]);
   if (jb32) jb32[i] = make_jb32(p[0], p[1], p[2], m, u[0], u[1], u[2]);

@@ -3,8 +3,9 @@
 // The one-sided kernels (pair.cuh) evaluate each pair twice, once for either
 // body.  Here the pair's separation, 1/sqrt, and tidal vector are formed once
 // and added to both bodies (Newton's third law): 38 FP64 operations per pair
-// instead of 2 x 31.  The pair kernels are bound by their arithmetic pipe, so
-// the fewer operations are the gain.
+// instead of 2 x 31, 32 FP32 lane operations (38 near) instead of 2 x 25 (31).
+// The pair kernels are bound by their arithmetic pipe, so the fewer operations
+// are the gain.
 //
 // Schedule.  Rows are cut into nb blocks of `block_rows` rows.  Block I meets
 // the D(I) blocks that follow it cyclically (all blocks at distance 1 ..
@@ -32,9 +33,11 @@
 // it wrote itself; this bounds the slots (nb / 2 + S) whatever N is.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "hermite.cuh"
 #include "pair.cuh"
+#include "reltiles.cuh"
 
 namespace nbody {
 
@@ -47,6 +50,8 @@ struct SymArgs {
   double* out;     // P
   size_t stride;
   int* status;
+  SoA7 rows;       // near/far kernel: the bodies its tiles were built from
+  unsigned long long* near_count;  // near/far kernel: += near (warp, subtile) pairs (nullable)
 };
 
 __host__ __device__ __forceinline__ int sym_distances(int nb, int I) {
@@ -137,12 +142,14 @@ constexpr size_t sym_fp64_smem() {
   return 2 * kSymTile64 * sizeof(JBody64) + 2 * 6 * W * 32 * sizeof(double);
 }
 
+// UNR: unrolled steps; MINB: CTAs per SM asked of the register allocator.
 template <int IPT, int W, int UNR, int MINB>
 __global__ void __launch_bounds__(32 * W, MINB)
     pair_sym_fp64_kernel(const JBody64* __restrict__ jb, SymArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint64_t full[2];
   constexpr int kRows = 32 * IPT * W;
+  static_assert(kRows % kSymTile64 == 0, "blocks are whole tiles");
   TilePipe<JBody64, kSymTile64> pipe;
   pipe.init(reinterpret_cast<JBody64*>(smem_raw), full);
   double* red = reinterpret_cast<double*>(smem_raw + 2 * kSymTile64 * sizeof(JBody64));  // [2][6][W][32]
@@ -167,9 +174,15 @@ __global__ void __launch_bounds__(32 * W, MINB)
 #pragma unroll
       for (int c = 0; c < 6; ++c) acc[k][c] = 0.0;
     }
+    const bool idle = row0 >= a.n;  // a warp of padding rows adds nothing
     int t = 0;
     auto consume = [&](const JBody64* tile) {
       const double2* p = reinterpret_cast<const double2*>(tile);
+      if (idle) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) red[((half * 6 + c) * W + warp) * 32 + lane] = 0.0;
+        return;
+      }
       if (run.distance(run.tile(t)) == 0) {
 #pragma unroll 1
         for (int k = 0; k < 32; ++k) {
@@ -227,6 +240,377 @@ __global__ void __launch_bounds__(32 * W, MINB)
         for (int c = 0; c < 6; ++c) out[static_cast<size_t>(c) * a.stride + r] = acc[k][c];
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// Mixed precision, near/far tile-relative
+// ---------------------------------------------------------------------------
+// Subtile of 64 bodies.  Header: centre c, radius R >= max |x_j - c|, bounding
+// box rounded outward (as JBodyNF's header).  Bodies: lane l holds bodies l and
+// l + 32 as packed pairs, so each 64-bit word is an f32x2 operand: chunks
+// 0 (-Dx, -Dy), 1 (-Dz, m), 2 (vx, vy), 3 (vz, -), 4 (-Dx_lo, -Dy_lo),
+// 5 (-Dz_lo, -), with (D, D_lo) = ds_offset(c, x_hi, x_lo).  50 bytes per body.
+struct __align__(128) SymSub {
+  float c[3], R, lo[3], hi[3], pad[22];
+  ulonglong2 v[6][32];
+};
+static_assert(sizeof(SymSub) == 3200, "subtiles start 128-byte aligned");
+
+// Subtile blockIdx.x of the bodies of `in` (64 threads, one per body; bodies
+// >= n are zero-mass padding at the centre).  PREDICT: `in` is the state X, V
+// (written), with its derivatives D and step ctl, and the subtile is that of
+// the predicted state (predict_kernel's arithmetic): one pass instead of two.
+// Bound by its launch below some 10^5 bodies (104 B read, 48 + 50 written per
+// body): N = 5003 5 us instead of 5 + 5.  Zeroes near_count for the pair pass
+// that follows.
+template <bool PREDICT>
+__global__ void __launch_bounds__(64)
+    sym_tile_kernel(int n, SoA7 in, SymSub* __restrict__ out, int ld = 0, double* X = nullptr,
+                    double* V = nullptr, const double* __restrict__ D = nullptr,
+                    const StepCtl* __restrict__ ctl = nullptr,
+                    unsigned long long* near_count = nullptr) {
+  __shared__ double box[6][2];
+  __shared__ float rmax[2];
+  __shared__ SymSub stage;  // written out in one bulk copy
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slot = blockIdx.x * 64 + tid;
+  const bool valid = slot < n;
+  if (near_count && slot == 0) *near_count = 0;
+  double p[3] = {0.0, 0.0, 0.0}, u[3] = {0.0, 0.0, 0.0}, m = 0.0;
+  if (valid) {
+    m = in.m[slot];
+    if (PREDICT) {
+      predict_body(ctl->dt, ld, slot, X, V, D, p, u);
+    } else {
+      p[0] = in.x[slot]; p[1] = in.y[slot]; p[2] = in.z[slot];
+      u[0] = in.vx[slot]; u[1] = in.vy[slot]; u[2] = in.vz[slot];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {  // bounding box in double (empty subtile: +inf/-inf)
+    double w = k < 3 ? (valid ? p[k] : INFINITY) : (valid ? p[k - 3] : -INFINITY);
+    w = k < 3 ? warp_min(w) : warp_max(w);
+    if (lane == 0) box[k][warp] = w;
+  }
+  __syncthreads();
+  double lo[3], hi[3];
+  float c[3];
+  double r2 = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = fmin(box[k][0], box[k][1]);
+    hi[k] = fmax(box[3 + k][0], box[3 + k][1]);
+    const double mid = 0.5 * lo[k] + 0.5 * hi[k];
+    c[k] = isfinite(mid) ? static_cast<float>(mid) : 0.0f;
+    const double d = p[k] - static_cast<double>(c[k]);
+    r2 += valid ? d * d : 0.0;
+  }
+  float R = __double2float_ru(sqrt(r2));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
+  if (lane == 0) rmax[warp] = R;
+  __syncthreads();
+  if (tid == 0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      stage.c[k] = c[k];
+      stage.lo[k] = __double2float_rd(lo[k]);
+      stage.hi[k] = __double2float_ru(hi[k]);
+    }
+    stage.R = fmaxf(rmax[0], rmax[1]);
+  }
+  float oh[3], ol[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    float h, l, dh = 0.f, dl = 0.f;
+    split_hilo(p[k], h, l);
+    if (valid) ds_offset(c[k], h, l, dh, dl);
+    oh[k] = -dh;
+    ol[k] = -dl;
+  }
+  // body tid = half `warp` of lane `lane`'s pairs; word w of chunk q at [128 q + 2 w]
+  float* f = reinterpret_cast<float*>(&stage.v[0][lane]) + warp;
+  f[0] = oh[0];
+  f[2] = oh[1];
+  f[128] = oh[2];
+  f[130] = __double2float_rn(m);
+  f[256] = __double2float_rn(u[0]);
+  f[258] = __double2float_rn(u[1]);
+  f[384] = __double2float_rn(u[2]);
+  f[386] = 0.f;
+  f[512] = ol[0];
+  f[514] = ol[1];
+  f[640] = ol[2];
+  f[642] = 0.f;
+  if (tid < 22) stage.pad[tid] = 0.f;
+  bulk_store_fence();
+  __syncthreads();
+  if (tid == 0) bulk_store(out + blockIdx.x, &stage, static_cast<uint32_t>(sizeof stage));
+}
+
+__device__ __forceinline__ uint64_t f2_dup(float v) { return f2_pack(v, v); }
+
+// One i-row (its values in both halves) against two j-bodies, separations
+// (dx, dy, dz) given.  MUFU rsqrt and rcp (1/s) as in the one-sided kernels.
+template <bool SYM>
+__device__ __forceinline__ void sym_pair_x2(uint64_t dx, uint64_t dy, uint64_t dz, uint64_t mj,
+                                            uint64_t vxj, uint64_t vyj, uint64_t vzj, uint64_t ui,
+                                            uint64_t vi, uint64_t wi, uint64_t mi, uint64_t eps2,
+                                            uint64_t m3, uint64_t* ai, uint64_t* bj) {
+  const uint64_t du = f2_sub(vxj, ui), dv = f2_sub(vyj, vi), dw = f2_sub(vzj, wi);
+  const uint64_t s = f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, eps2)));
+  const uint64_t rv = f2_fma(dx, du, f2_fma(dy, dv, f2_mul(dz, dw)));
+  float s0, s1;
+  f2_unpack(s, s0, s1);
+  const uint64_t y = f2_pack(rsqrt_mufu(s0), rsqrt_mufu(s1));
+  const uint64_t y2 = f2_pack(rcp_mufu(s0), rcp_mufu(s1));
+  const uint64_t y3 = f2_mul(y, y2);
+  const uint64_t q = f2_mul(mj, y3);
+  const uint64_t c = f2_mul(rv, f2_mul(y2, m3));
+  const uint64_t ex = f2_fma(c, dx, du), ey = f2_fma(c, dy, dv), ez = f2_fma(c, dz, dw);
+  ai[0] = f2_fma(q, dx, ai[0]); ai[1] = f2_fma(q, dy, ai[1]); ai[2] = f2_fma(q, dz, ai[2]);
+  ai[3] = f2_fma(q, ex, ai[3]); ai[4] = f2_fma(q, ey, ai[4]); ai[5] = f2_fma(q, ez, ai[5]);
+  if (SYM) {
+    const uint64_t h = f2_mul(mi, y3);
+    bj[0] = f2_fma(h, dx, bj[0]); bj[1] = f2_fma(h, dy, bj[1]); bj[2] = f2_fma(h, dz, bj[2]);
+    bj[3] = f2_fma(h, ex, bj[3]); bj[4] = f2_fma(h, ey, bj[4]); bj[5] = f2_fma(h, ez, bj[5]);
+  }
+}
+
+// Sums of a lane's j-bodies, handed to the next lane's.
+__device__ __forceinline__ void sym_rotate(uint64_t* b, int next) {
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    float l, h;
+    f2_unpack(b[c], l, h);
+    b[c] = f2_pack(__shfl_sync(0xffffffffu, l, next), __shfl_sync(0xffffffffu, h, next));
+  }
+}
+
+// Near/far form of a pair (pair.cuh, RowsMixedNF): far subtiles form the
+// separation with one add per component, near ones in double-single; a
+// (warp, subtile) pair is far when their boxes are apart by at least R / 2.
+// Float sums (a row's over one tile of 64 SUB bodies in two halves, a
+// j-body's over the warp's 32 IPT rows) are flushed into double: fewer terms
+// per float sum than the one-sided kernel's 128, and smaller errors (N =
+// 65536 median / p99 / rms acc error 2.3e-8 / 1.2e-7 / 3.8e-8, one-sided
+// 3.0e-8 / 1.6e-7 / 5.0e-8).  Jerk likewise.
+//
+// Two j-bodies per lane are packed, the i-rows are held in both halves of
+// their registers: the packed j-operands and their sums come from shared
+// memory and shuffles as they are, and 12 shuffles serve 2 IPT pairs.  At four
+// rows per lane a step is 64 cycles of the FP32 pipe against 28 of the shared
+// pipe; 168 registers leave three CTAs of four warps per SM (two with more
+// registers per thread: 3.0 ms; two rows per lane and four CTAs: 2.9 ms at N
+// = 65536).  FP32 pipe 68-72 % active, stalls on the pipe and on fixed
+// latencies.  Measured against the one-sided kernel at its tuned tiling: N =
+// 65536 2.70 vs 4.00 ms, 262144 41.1 vs 60.8, 16384 0.226 vs 0.300.
+// xhl: the rows' (x_hi, x_lo), in shared memory, read once per subtile.
+template <int IPT, int W, int SUB>
+constexpr size_t sym_nf_smem() {
+  return 2 * SUB * sizeof(SymSub) + 6 * IPT * 32 * W * (sizeof(double) + sizeof(float)) +
+         2 * SUB * 6 * W * 32 * sizeof(uint64_t);
+}
+
+// SUB subtiles per tile (one barrier each); UNR / NUNR: unrolled steps of the
+// far / near loop (two bodies per lane and step).
+template <int IPT, int W, int SUB, int UNR, int NUNR, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB)
+    pair_sym_nf_kernel(const SymSub* __restrict__ jt, SymArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ uint64_t full[2];
+  constexpr int NT = 32 * W, kRows = 32 * IPT * W, TJ = 64 * SUB;
+  static_assert(kRows % TJ == 0, "blocks are whole tiles");
+  TilePipe<SymSub, SUB> pipe;
+  pipe.init(reinterpret_cast<SymSub*>(smem_raw), full);
+  double* acc = reinterpret_cast<double*>(smem_raw + 2 * SUB * sizeof(SymSub));  // [6 IPT][NT]
+  float* xhl = reinterpret_cast<float*>(acc + 6 * IPT * NT);                     // [6 IPT][NT]
+  uint64_t* red = reinterpret_cast<uint64_t*>(xhl + 6 * IPT * NT);  // [2][SUB][6][W][32]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, next = (lane + 1) & 31;
+  const SymRun run(a, a.subs * (kRows / TJ));
+  const float e2 = static_cast<float>(a.eps2);
+  const uint64_t eps2 = f2_dup(e2), m3 = f2_dup(-3.0f);
+  int half = 0;  // half of `red` of the current tile, alternating over the CTA's life
+  int near_subs = 0;
+  for (int g = 0; g < a.subs; ++g) {
+    const int row0 = (run.I * a.subs + g) * kRows + warp * 32 * IPT;
+    if ((run.I * a.subs + g) * kRows >= a.n) break;  // a short last block
+    uint64_t ui[IPT], vi[IPT], wi[IPT], mi[IPT], fa[IPT][6];
+    float blo[3], bhi[3];
+    {
+      double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int k = 0; k < IPT; ++k) {
+        const int r = row0 + 32 * k + lane;
+        const bool ok = r < a.n;  // rows >= n: massless copies of the last body, not stored
+        const int i = min(r, a.n - 1);
+        const double x[3] = {a.rows.x[i], a.rows.y[i], a.rows.z[i]};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (ok) { lo[c] = fmin(lo[c], x[c]); hi[c] = fmax(hi[c], x[c]); }
+          float h, l;
+          split_hilo(x[c], h, l);
+          xhl[(k * 6 + c) * NT + tid] = h;
+          xhl[(k * 6 + 3 + c) * NT + tid] = l;
+        }
+        ui[k] = f2_dup(static_cast<float>(a.rows.vx[i]));
+        vi[k] = f2_dup(static_cast<float>(a.rows.vy[i]));
+        wi[k] = f2_dup(static_cast<float>(a.rows.vz[i]));
+        mi[k] = f2_dup(ok ? static_cast<float>(a.rows.m[i]) : 0.f);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          fa[k][c] = 0ull;
+          acc[(c * IPT + k) * NT + tid] = 0.0;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {  // the warp's box, rounded outward
+        float l = __double2float_rd(lo[c]), h = __double2float_ru(hi[c]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          l = fminf(l, __shfl_xor_sync(0xffffffffu, l, o));
+          h = fmaxf(h, __shfl_xor_sync(0xffffffffu, h, o));
+        }
+        blo[c] = l;
+        bhi[c] = h;
+      }
+    }
+    // (D, D_lo)(x_i) relative to the subtile's centre, bit-identical to the records'
+    auto offsets = [&](const SymSub* t, int k, uint64_t oh[3], uint64_t ol[3]) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        float h, l;
+        ds_offset(t->c[c], xhl[(k * 6 + c) * NT + tid], xhl[(k * 6 + 3 + c) * NT + tid], h, l);
+        oh[c] = f2_dup(h);
+        ol[c] = f2_dup(l);
+      }
+    };
+    auto near_sub = [&](const SymSub* t, auto sym, uint64_t* b) {
+      constexpr bool SYM = decltype(sym)::value;
+      uint64_t oh[IPT][3], ol[IPT][3];
+#pragma unroll
+      for (int k = 0; k < IPT; ++k) offsets(t, k, oh[k], ol[k]);
+#pragma unroll NUNR
+      for (int k = 0; k < 32; ++k) {
+        const int j = (lane + k) & 31;
+        const ulonglong2 r0 = t->v[0][j], r1 = t->v[1][j], r2 = t->v[2][j], r3 = t->v[3][j];
+        const ulonglong2 r4 = t->v[4][j], r5 = t->v[5][j];
+#pragma unroll
+        for (int r = 0; r < IPT; ++r)
+          sym_pair_x2<SYM>(f2_add(f2_add(r0.x, oh[r][0]), f2_add(r4.x, ol[r][0])),
+                           f2_add(f2_add(r0.y, oh[r][1]), f2_add(r4.y, ol[r][1])),
+                           f2_add(f2_add(r1.x, oh[r][2]), f2_add(r5.x, ol[r][2])), r1.y, r2.x,
+                           r2.y, r3.x, ui[r], vi[r], wi[r], mi[r], eps2, m3, fa[r], b);
+        if (SYM) sym_rotate(b, next);
+      }
+    };
+    auto far_sub = [&](const SymSub* t, uint64_t* b) {
+      uint64_t o[IPT][3];  // D(x_i) to float accuracy: fl(fl(c - x_hi) - x_lo)
+#pragma unroll
+      for (int k = 0; k < IPT; ++k)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          o[k][c] = f2_dup(__fsub_rn(__fsub_rn(t->c[c], xhl[(k * 6 + c) * NT + tid]),
+                                     xhl[(k * 6 + 3 + c) * NT + tid]));
+#pragma unroll UNR
+      for (int k = 0; k < 32; ++k) {
+        const int j = (lane + k) & 31;
+        const ulonglong2 r0 = t->v[0][j], r1 = t->v[1][j], r2 = t->v[2][j], r3 = t->v[3][j];
+#pragma unroll
+        for (int r = 0; r < IPT; ++r)
+          sym_pair_x2<true>(f2_add(r0.x, o[r][0]), f2_add(r0.y, o[r][1]), f2_add(r1.x, o[r][2]),
+                            r1.y, r2.x, r2.y, r3.x, ui[r], vi[r], wi[r], mi[r], eps2, m3, fa[r], b);
+        sym_rotate(b, next);
+      }
+    };
+    const bool idle = row0 >= a.n;  // a warp of padding rows adds nothing
+    int t = 0;
+    auto consume = [&](const SymSub* tile) {
+      const bool own = run.distance(run.tile(t)) == 0;
+      if (idle) {
+#pragma unroll
+        for (int s = 0; s < SUB; ++s)
+#pragma unroll
+          for (int c = 0; c < 6; ++c)
+            red[(((half * SUB + s) * 6 + c) * W + warp) * 32 + lane] = 0ull;
+        return;
+      }
+#pragma unroll 1
+      for (int s = 0; s < SUB; ++s) {
+        const SymSub* sub = tile + s;
+        // far: boxes apart by d > 0 with d^2 >= R^2 / 4 (gaps rounded down, R up)
+        float d2 = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float gap = fmaxf(0.f, fmaxf(__fsub_rd(blo[c], sub->hi[c]), __fsub_rd(sub->lo[c], bhi[c])));
+          d2 = __fmaf_rd(gap, gap, d2);
+        }
+        const bool far = d2 > 0.f && d2 >= __fmul_ru(0.25f, __fmul_ru(sub->R, sub->R));
+        uint64_t b[6] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
+        if (own) {
+          ++near_subs;
+          near_sub(sub, std::false_type{}, b);
+          continue;
+        }
+        if (far) {
+          far_sub(sub, b);
+        } else {
+          ++near_subs;
+          near_sub(sub, std::true_type{}, b);
+        }
+        uint64_t* o = red + ((half * SUB + s) * 6 * W + warp) * 32 + lane;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) o[c * W * 32] = b[c];
+      }
+#pragma unroll
+      for (int k = 0; k < IPT; ++k)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          float l, h;
+          f2_unpack(fa[k][c], l, h);
+          acc[(c * IPT + k) * NT + tid] += static_cast<double>(l + h);
+          fa[k][c] = 0ull;
+        }
+    };
+    // after the tile's barrier: the W warps' sums of the tile's bodies, in warp
+    // order, into their slot (double from here on)
+    auto post = [&]() {
+      const int tt = run.tile(t), d = run.distance(tt);
+      if (d != 0) {
+        double* out = a.out + static_cast<size_t>(a.S + d - 1) * 6 * a.stride +
+                      static_cast<size_t>(tt) * TJ;
+        for (int e = tid; e < SUB * 6 * 32; e += NT) {
+          const int l = e & 31, c = (e >> 5) % 6, s = e / (6 * 32);
+          const uint64_t* o = red + ((half * SUB + s) * 6 + c) * W * 32 + l;
+          double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            float x, y;
+            f2_unpack(o[w * 32], x, y);
+            v0 -= static_cast<double>(x);
+            v1 -= static_cast<double>(y);
+          }
+          double* dst = out + static_cast<size_t>(c) * a.stride + s * 64 + l;
+          dst[0] = g ? dst[0] + v0 : v0;  // a later sub-block adds to this thread's own store
+          dst[32] = g ? dst[32] + v1 : v1;
+        }
+      }
+      ++t;
+      half ^= 1;
+    };
+    if (!run.stream(pipe, jt, a.status, consume, post)) return;
+    double* out = a.out + static_cast<size_t>(blockIdx.y) * 6 * a.stride;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+      const int r = row0 + 32 * k + lane;
+      if (r < a.n)
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+          out[static_cast<size_t>(c) * a.stride + r] = acc[(c * IPT + k) * NT + tid];
+    }
+  }
+  if (a.near_count && lane == 0 && near_subs)
+    atomicAdd(a.near_count, static_cast<unsigned long long>(near_subs));
 }
 
 }  // namespace nbody

@@ -95,3 +95,68 @@ def test_fewer_bodies_than_the_engine_and_row_ranges():
     assert np.all(part[:, 5000:] == 0.0)
     ea, ej = derivs_rel(part[:, :5000], O.force_rows(big, EPS2, np.arange(5000)))
     assert ea <= 1e-12 and ej <= 1e-12, (ea, ej)
+
+
+# subtiles of 64, tiles of 64 (two rows per lane) and 128 bodies (four rows),
+# a last tile whose second subtile is empty, odd and even block counts; bodies
+# in the caller's order (automatic, below 16384) and in Hilbert order
+# (pair_variant 4, or from 16384).  Bounds: those of the mixed kernels against
+# FP64 (median 2e-6, worst 2e-4 acc; median 1e-5 jerk).
+@pytest.mark.parametrize("variant", [0, 4])
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 255, 257, 513, 1025, 4097, 5003])
+def test_mixed_small_edges(n, variant):
+    s = bodies(n)
+    d, _ = derivs(s, "mixed", pair_variant=variant)
+    if n == 1:
+        assert np.all(d == 0.0)
+        return
+    ref = O.force(s, EPS2)
+    ok = np.abs(ref[:3]).max(axis=0) > 0
+    assert np.all(d[:, ~ok] == 0.0)
+    ea, ej = vec_rel(d[:3, ok], ref[:3, ok]), vec_rel(d[3:, ok], ref[3:, ok])
+    assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4, (n, np.median(ea), ea.max())
+    assert np.median(ej) <= 1e-5, (n, np.median(ej))
+
+
+@pytest.mark.parametrize("n", [16384, 20000, 65537, 70017])
+def test_mixed_block_edges_against_the_one_sided_kernel(n):
+    """Every row against the packed hi/lo kernel of the same float arithmetic
+    class: a pair missed or met twice would be off by its whole term.  Bounds:
+    the mixed kernels' against FP64, twice."""
+    s = bodies(n)
+    d, t = derivs(s, "mixed")
+    assert t["record_format"] == 3
+    one, _ = derivs(s, "mixed", pair_variant=3)
+    ea, ej = vec_rel(d[:3], one[:3]), vec_rel(d[3:], one[3:])
+    assert np.median(ea) <= 4e-6 and ea.max() <= 4e-4, (n, np.median(ea), ea.max())
+    assert np.median(ej) <= 2e-5, (n, np.median(ej))
+    again, _ = derivs(s, "mixed")
+    assert np.array_equal(d, again)
+
+
+@pytest.mark.parametrize("n", [3001, 33000])
+def test_mixed_calls_on_the_callers_arrays(n):
+    """Host and device calls in the caller's order (below 32768 bodies) and
+    through the Hilbert order (from there) give the engine's accuracy, and
+    leave a stepping engine's own bodies alone."""
+    import torch
+    s = bodies(n)
+    rows = np.arange(0, n, max(1, n // 200))
+    ref = O.force_rows(s, EPS2, rows)
+    ok = np.abs(ref[:3]).max(axis=0) > 0
+    t = [torch.tensor(s[k], dtype=torch.float64, device="cuda") for k in nb.FIELDS]
+    out = torch.empty(6, n, dtype=torch.float64, device="cuda")
+    with nb.Engine(n, eps2=EPS2, dt=1 / 1024, precision="mixed") as e, \
+            nb.Engine(n, eps2=EPS2, dt=1 / 1024, precision="mixed") as f:
+        for g in (e, f):
+            g.set_state(s)
+            g.timestepping(2)
+        e.acc_jerk_device(*t, list(out), stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        for g in (e, f):
+            g.timestepping(2)
+        a, b = e.get_state(), f.get_state()
+    assert all(np.array_equal(a[k], b[k]) for k in a)
+    for d in (out.cpu().numpy(), nb.force_calculation(s, eps2=EPS2, precision="mixed")):
+        ea = vec_rel(d[:3, rows][:, ok], ref[:3, ok])
+        assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4, (n, np.median(ea), ea.max())
