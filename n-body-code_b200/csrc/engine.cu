@@ -412,10 +412,15 @@ int choose_split(const nbody_engine* e, const PairKernel& k, int rows) {
 }
 
 // Splits of the symmetric kernel k over n bodies: S CTAs per block share its
-// run of Q tiles, ceil(Q / S) each.  Same wave model, over the tile counts
-// that differ: full waves cost a CTA's tiles, the last one what its fullest
-// SM holds (but at least half: alone on its SM a CTA is latency-bound), and
-// every split another 48 bytes per row to sum.
+// run of Q tiles, ceil(Q / S) each.  Cost in units of one (CTA, tile).  FP64
+// CTAs take the same time each and run in waves, the last of which takes what
+// its fullest SM holds (three quarters of a tile's time are throughput).  The
+// near/far kernel's differ with their near subtiles: the work of more CTAs
+// than are resident spreads over the slots, and the last ones leave SMs idle
+// for about a third of a CTA's time.  Every split is another 48 bytes per row
+// to sum.  Pair pass in ms by splits: FP64 N = 16384 0.464 (8) 0.39 (23) 0.405
+// (31), 65536 5.79 (8) 5.69 (31); mixed 16384 0.265 (9) 0.223 (31), 65536 2.91
+// (9) 2.77 (31).
 int choose_sym_split(const nbody_engine* e, const PairKernel& k, int n) {
   prepare_kernel(k);
   int occ = 0;
@@ -433,10 +438,14 @@ int choose_sym_split(const nbody_engine* e, const PairKernel& k, int n) {
   for (int tps = 1; tps <= Q; ++tps) {
     const int s = (Q + tps - 1) / tps;
     if (s > std::min(kMaxSplit, max_sym_slots(n) / 2)) continue;
-    const long ctas = static_cast<long>(g.nb) * s, last = ctas % slots;
+    const long ctas = static_cast<long>(g.nb) * s;
     const double one = tps * g.subs + 0.5;
-    const double share = static_cast<double>((last + e->num_sms - 1) / e->num_sms) / occ;
-    const double cost = (ctas / slots) * one + (last ? one * std::max(0.5, share) : 0.0) + per_split * s;
+    const bool waves = k.precision == NBODY_FP64 || ctas <= slots;
+    const long last = waves ? ctas % slots : 0;
+    const double per_sm = static_cast<double>((last + e->num_sms - 1) / e->num_sms) / occ;
+    double work = waves ? one * (ctas / slots) : one * ctas / slots;
+    if (last) work += one * (0.25 + 0.75 * per_sm);
+    const double cost = work + (k.precision == NBODY_FP64 ? 0.1 : 0.35) * one + per_split * s;
     if (cost < best - 1e-9) {
       best = cost;
       best_s = s;

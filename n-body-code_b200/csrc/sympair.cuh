@@ -116,13 +116,12 @@ __device__ __forceinline__ void sym_pair_fp64(const double2& p0, const double2& 
   const double y = rsqrt_f64(s);
   const double y2 = y * y;
   const double y3 = y * y2;
-  const double q = p1.y * y3;
+  const double q = p1.y * y3, h = SYM ? mi * y3 : 0.0;
   const double c = rv * (-3.0 * y2);
   const double ex = fma(c, dx, du), ey = fma(c, dy, dv), ez = fma(c, dz, dw);
   ai[0] = fma(q, dx, ai[0]); ai[1] = fma(q, dy, ai[1]); ai[2] = fma(q, dz, ai[2]);
   ai[3] = fma(q, ex, ai[3]); ai[4] = fma(q, ey, ai[4]); ai[5] = fma(q, ez, ai[5]);
   if (SYM) {
-    const double h = mi * y3;
     bj[0] = fma(h, dx, bj[0]); bj[1] = fma(h, dy, bj[1]); bj[2] = fma(h, dz, bj[2]);
     bj[3] = fma(h, ex, bj[3]); bj[4] = fma(h, ey, bj[4]); bj[5] = fma(h, ez, bj[5]);
   }
@@ -174,15 +173,9 @@ __global__ void __launch_bounds__(32 * W, MINB)
 #pragma unroll
       for (int c = 0; c < 6; ++c) acc[k][c] = 0.0;
     }
-    const bool idle = row0 >= a.n;  // a warp of padding rows adds nothing
     int t = 0;
     auto consume = [&](const JBody64* tile) {
       const double2* p = reinterpret_cast<const double2*>(tile);
-      if (idle) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c) red[((half * 6 + c) * W + warp) * 32 + lane] = 0.0;
-        return;
-      }
       if (run.distance(run.tile(t)) == 0) {
 #pragma unroll 1
         for (int k = 0; k < 32; ++k) {
@@ -365,13 +358,12 @@ __device__ __forceinline__ void sym_pair_x2(uint64_t dx, uint64_t dy, uint64_t d
   const uint64_t y = f2_pack(rsqrt_mufu(s0), rsqrt_mufu(s1));
   const uint64_t y2 = f2_pack(rcp_mufu(s0), rcp_mufu(s1));
   const uint64_t y3 = f2_mul(y, y2);
-  const uint64_t q = f2_mul(mj, y3);
+  const uint64_t q = f2_mul(mj, y3), h = SYM ? f2_mul(mi, y3) : 0ull;
   const uint64_t c = f2_mul(rv, f2_mul(y2, m3));
   const uint64_t ex = f2_fma(c, dx, du), ey = f2_fma(c, dy, dv), ez = f2_fma(c, dz, dw);
   ai[0] = f2_fma(q, dx, ai[0]); ai[1] = f2_fma(q, dy, ai[1]); ai[2] = f2_fma(q, dz, ai[2]);
   ai[3] = f2_fma(q, ex, ai[3]); ai[4] = f2_fma(q, ey, ai[4]); ai[5] = f2_fma(q, ez, ai[5]);
   if (SYM) {
-    const uint64_t h = f2_mul(mi, y3);
     bj[0] = f2_fma(h, dx, bj[0]); bj[1] = f2_fma(h, dy, bj[1]); bj[2] = f2_fma(h, dz, bj[2]);
     bj[3] = f2_fma(h, ex, bj[3]); bj[4] = f2_fma(h, ey, bj[4]); bj[5] = f2_fma(h, ez, bj[5]);
   }
