@@ -22,14 +22,16 @@
 // both precisions (for a mixed-precision forward it is the FP64 adjoint of
 // the same trajectory).
 //
-// Pair VJP (gather form, no atomics).  For rows k, partners p, with
-// r = x_p - x_k, u = v_p - v_k, s = r^2 + eps2, y2 = 1/s, q = s^(-3/2),
-// w = r.u, c = -3 w y2, and the term T = m q (a.r + b.u + c b.r) that row k's
-// acc/jerk adjoint (a, b) = (ab_k, jb_k) sees from partner p:
-//   dT/dr = m q [a + c b - 3 y2 B u + (6 w y2^2 B - 3 y2 G) r],  dT/du = m q (b - 3 y2 B r),
-//   dT/dm = q G,  with B = b.r, G = a.r + b.u + c B.
-// Row k collects -dT_kp/dr (its own term, m = m_p) and +dT_pk/dr' (the
-// partner's term, r' = -r, m = m_k), and dT_pk/dm_k for its mass.
+// Pair VJP (no atomics).  For an unordered pair (k, p) with r = x_p - x_k,
+// u = v_p - v_k, s = r^2 + eps2, y2 = 1/s, q = s^(-3/2), w = r.u, c = -3 w y2
+// and the adjoints (a, b) = (ab, jb) of acc and jerk, both bodies' terms are
+//   T = q (m_p G_k - m_k G_p),  G_i = a_i.r + b_i.u + c B_i,  B_i = b_i.r
+// (body p sees -r and -u).  With A = m_p a_k - m_k a_p, J = m_p b_k - m_k b_p,
+// B = m_p B_k - m_k B_p and G = m_p G_k - m_k G_p:
+//   dT/dr = q [A + c J - 3 y2 B u - 3 y2 (G + 2/3 c B) r],  dT/du = q (J - 3 y2 B r),
+//   dT/dm_p = q G_k,  dT/dm_k = -q G_p.
+// x_p collects +dT/dr and x_k -dT/dr, likewise v.  The symmetric schedule
+// (sympair.cuh) meets every pair once: 87 FP64 operations for both bodies.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,6 +42,7 @@
 #include "errors.h"
 #include "hermite.cuh"
 #include "pair.cuh"
+#include "sympair.cuh"
 #include "trace.h"
 
 using namespace nbody;
@@ -48,172 +51,245 @@ namespace {
 
 constexpr int kPad = 256;
 constexpr int kBlock = 256;
-constexpr int kTile = 128;
+constexpr int kPredictBlock = 64;  // a few thousand rows reach more SMs
 
-// j-record of the pair VJP: position, mass, velocity and the acc/jerk adjoints.
+// j-record of the pair VJP, in groups of 32 bodies, each seven rows of 32
+// 16-byte chunks: (x, y) (z, m) (vx, vy) (vz, ax) (ay, az) (bx, by) (bz, -)
+// with (a, b) the acc/jerk adjoints.  JAdj is one body's share of a group.
+constexpr int kAdjChunks = 7;
 struct __align__(16) JAdj {
-  double x, y, z, m, vx, vy, vz, ax, ay, az, bx, by, bz, pad0, pad1, pad2;
+  double raw[2 * kAdjChunks];
 };
+constexpr int kVjpTile = 32;
 
-constexpr int kVjpNT = 128, kVjpTile = 64;
+__device__ __forceinline__ double2* jadj_at(JAdj* jb, int i) {
+  return reinterpret_cast<double2*>(jb + (i & ~31)) + (i & 31);
+}
 
-// Row block of the pair VJP: one row per thread.
-struct RowsVJP {
-  static constexpr int TJ = kVjpTile;
-  using JB = JAdj;
+// One body's values.
+struct VjpBody {
   double x, y, z, m, u, v, w, ax, ay, az, bx, by, bz;
-  double rpk[3], upk[3], rkp[3], ukp[3], mb;
-  double eps2;
-  int row;
-
-  __device__ __forceinline__ void begin(const JB* __restrict__ jb, int r, int row_max, double e2,
-                                        unsigned char*) {
-    row = r;
-    const JAdj o = jb[min(r, row_max)];
-    x = o.x; y = o.y; z = o.z; m = o.m; u = o.vx; v = o.vy; w = o.vz;
-    ax = o.ax; ay = o.ay; az = o.az; bx = o.bx; by = o.by; bz = o.bz;
-    for (int c = 0; c < 3; ++c) rpk[c] = upk[c] = rkp[c] = ukp[c] = 0.0;
-    mb = 0.0;
-    eps2 = e2;
-  }
-
-  __device__ __forceinline__ void consume(const JB* tile, int tile_row0) {
-    // Two partners per iteration.  The self pair (r = u = 0, s = eps2) has
-    // finite terms; q = 0 removes them without a branch, which lets the
-    // compiler interleave the two pairs (measured 6 % faster backward).
-#pragma unroll 2
-    for (int t = 0; t < TJ; ++t) {
-      const JAdj p = tile[t];
-      const bool self = tile_row0 + t == row;
-      const double r0 = p.x - x, r1 = p.y - y, r2 = p.z - z;
-      const double u0 = p.vx - u, u1 = p.vy - v, u2 = p.vz - w;
-      const double s = fma(r0, r0, fma(r1, r1, fma(r2, r2, eps2)));
-      const double yy = rsqrt_f64(s);
-      const double y2 = yy * yy;
-      const double q = self ? 0.0 : yy * y2;
-      const double wr = fma(r0, u0, fma(r1, u1, r2 * u2));
-      const double c = -3.0 * wr * y2;
-      // own term (adjoints of row k, partner mass m_p)
-      {
-        const double B = bx * r0 + by * r1 + bz * r2;
-        const double G = (ax * r0 + ay * r1 + az * r2) + (bx * u0 + by * u1 + bz * u2) + c * B;
-        const double kr = 6.0 * wr * y2 * y2 * B - 3.0 * y2 * G;
-        const double mq = p.m * q;
-        rkp[0] += mq * (ax + c * bx - 3.0 * y2 * B * u0 + kr * r0);
-        rkp[1] += mq * (ay + c * by - 3.0 * y2 * B * u1 + kr * r1);
-        rkp[2] += mq * (az + c * bz - 3.0 * y2 * B * u2 + kr * r2);
-        ukp[0] += mq * (bx - 3.0 * y2 * B * r0);
-        ukp[1] += mq * (by - 3.0 * y2 * B * r1);
-        ukp[2] += mq * (bz - 3.0 * y2 * B * r2);
-      }
-      // partner's term (adjoints of p, mass m_k applied at the end)
-      {
-        const double B = p.bx * r0 + p.by * r1 + p.bz * r2;
-        const double G = -((p.ax * r0 + p.ay * r1 + p.az * r2) + (p.bx * u0 + p.by * u1 + p.bz * u2) + c * B);
-        const double kr = 6.0 * wr * y2 * y2 * B + 3.0 * y2 * G;
-        rpk[0] += q * (p.ax + c * p.bx - 3.0 * y2 * B * u0 + kr * r0);
-        rpk[1] += q * (p.ay + c * p.by - 3.0 * y2 * B * u1 + kr * r1);
-        rpk[2] += q * (p.az + c * p.bz - 3.0 * y2 * B * u2 + kr * r2);
-        upk[0] += q * (p.bx - 3.0 * y2 * B * r0);
-        upk[1] += q * (p.by - 3.0 * y2 * B * r1);
-        upk[2] += q * (p.bz - 3.0 * y2 * B * r2);
-        mb += q * G;
-      }
-    }
-  }
-
-  // out: [7][stride] = d(xbar) (3), d(vbar) (3), d(mbar)
-  __device__ __forceinline__ void store(double* out, size_t stride, int row_end) const {
-    if (row >= row_end) return;
-    for (int c = 0; c < 3; ++c) {
-      out[c * stride + row] = m * rpk[c] - rkp[c];
-      out[(3 + c) * stride + row] = m * upk[c] - ukp[c];
-    }
-    out[6 * stride + row] = mb;
+  __device__ __forceinline__ void load(const double2* p) {
+    const double2 p0 = p[0], p1 = p[32], p2 = p[64], p3 = p[96], p4 = p[128], p5 = p[160], p6 = p[192];
+    x = p0.x; y = p0.y; z = p1.x; m = p1.y; u = p2.x; v = p2.y; w = p3.x;
+    ax = p3.y; ay = p4.x; az = p4.y; bx = p5.x; by = p5.y; bz = p6.x;
   }
 };
 
-__global__ void __launch_bounds__(kVjpNT) vjp_pair_kernel(const JAdj* __restrict__ jb, int n, int ld,
-                                                          int tiles_per_split, double eps2,
-                                                          double* __restrict__ P, int* status) {
+// The pair (k, p): ai and (SYM) bj collect q dT/dr, q dT/du and the masses'
+// terms; the row's sums change sign when they are stored.  skip: the self
+// pair, whose terms are finite and taken out by q = 0.
+template <bool SYM>
+__device__ __forceinline__ void vjp_pair(const VjpBody& k, const VjpBody& p, double eps2, bool skip,
+                                         double* ai, double* bj) {
+  const double r0 = p.x - k.x, r1 = p.y - k.y, r2 = p.z - k.z;
+  const double u0 = p.u - k.u, u1 = p.v - k.v, u2 = p.w - k.w;
+  const double s = fma(r0, r0, fma(r1, r1, fma(r2, r2, eps2)));
+  const double wr = fma(r0, u0, fma(r1, u1, r2 * u2));
+  const double y = rsqrt_f64(s);
+  const double y2 = y * y;
+  const double q = !SYM && skip ? 0.0 : y * y2;
+  const double t = -3.0 * y2, c = wr * t;
+  const double Bk = fma(k.bx, r0, fma(k.by, r1, k.bz * r2));
+  const double Bp = fma(p.bx, r0, fma(p.by, r1, p.bz * r2));
+  const double Gk = fma(c, Bk, fma(k.ax, r0, fma(k.ay, r1, fma(k.az, r2, fma(k.bx, u0, fma(k.by, u1, k.bz * u2))))));
+  const double Gp = fma(c, Bp, fma(p.ax, r0, fma(p.ay, r1, fma(p.az, r2, fma(p.bx, u0, fma(p.by, u1, p.bz * u2))))));
+  const double B = fma(p.m, Bk, -(k.m * Bp)), G = fma(p.m, Gk, -(k.m * Gp));
+  const double J0 = fma(p.m, k.bx, -(k.m * p.bx)), J1 = fma(p.m, k.by, -(k.m * p.by)),
+               J2 = fma(p.m, k.bz, -(k.m * p.bz));
+  const double A0 = fma(c, J0, fma(p.m, k.ax, -(k.m * p.ax))), A1 = fma(c, J1, fma(p.m, k.ay, -(k.m * p.ay))),
+               A2 = fma(c, J2, fma(p.m, k.az, -(k.m * p.az)));
+  const double e = t * B, kr = t * fma(c * (2.0 / 3.0), B, G);
+  const double d0 = fma(kr, r0, fma(e, u0, A0)), d1 = fma(kr, r1, fma(e, u1, A1)), d2 = fma(kr, r2, fma(e, u2, A2));
+  const double g0 = fma(e, r0, J0), g1 = fma(e, r1, J1), g2 = fma(e, r2, J2);
+  ai[0] = fma(q, d0, ai[0]); ai[1] = fma(q, d1, ai[1]); ai[2] = fma(q, d2, ai[2]);
+  ai[3] = fma(q, g0, ai[3]); ai[4] = fma(q, g1, ai[4]); ai[5] = fma(q, g2, ai[5]);
+  ai[6] = fma(q, Gp, ai[6]);
+  if (SYM) {
+    bj[0] = fma(q, d0, bj[0]); bj[1] = fma(q, d1, bj[1]); bj[2] = fma(q, d2, bj[2]);
+    bj[3] = fma(q, g0, bj[3]); bj[4] = fma(q, g1, bj[4]); bj[5] = fma(q, g2, bj[5]);
+    bj[6] = fma(q, Gk, bj[6]);
+  }
+}
+
+// Slots [slot][7][ld]: d(xbar) (3), d(vbar) (3), d(mbar).  Bound by the FP64
+// pipe; two rows per lane put the 14 shuffles and seven 16-byte shared loads
+// of a step (42 cycles of the shared pipe) under 2 x 87 FP64 instructions (87
+// cycles).  One row or three CTAs per SM time the same within 3 %.  Whole call
+// against the one-sided gather form: N = 4096 224 vs 297 us, 8192 399 vs 639,
+// 20000 1543 vs 3121.
+template <int IPT, int W>
+constexpr size_t vjp_smem() {
+  return 2 * kVjpTile * sizeof(JAdj) + 2 * 7 * W * 32 * sizeof(double);
+}
+template <int IPT, int W, int UNR, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB) vjp_sym_kernel(JAdj* __restrict__ jb, SymArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint64_t full[2];
+  constexpr int kRows = 32 * IPT * W;
+  static_assert(kRows % kVjpTile == 0, "blocks are whole tiles");
   TilePipe<JAdj, kVjpTile> pipe;
   pipe.init(reinterpret_cast<JAdj*>(smem_raw), full);
-  const int n_tiles = ld / kVjpTile;
-  const int split = blockIdx.y;
-  const int t_begin = split * tiles_per_split;
-  const int nt = max(0, min(tiles_per_split, n_tiles - t_begin));
-  RowsVJP r;
-  r.begin(jb, blockIdx.x * kVjpNT + threadIdx.x, ld - 1, eps2, nullptr);
-  int tile_row0 = t_begin * kVjpTile;
-  if (!pipe.run(jb + static_cast<size_t>(t_begin) * kVjpTile, nt, status, [&](const JAdj* tile) {
-        r.consume(tile, tile_row0);
-        tile_row0 += kVjpTile;
-      }))
-    return;
-  r.store(P + static_cast<size_t>(split) * 7 * ld, ld, n);
+  double* red = reinterpret_cast<double*>(smem_raw + 2 * kVjpTile * sizeof(JAdj));  // [2][7][W][32]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, next = (lane + 1) & 31;
+  const SymRun run(a, a.subs * (kRows / kVjpTile));
+  const double eps2 = a.eps2;
+  int half = 0;
+  grid_wait();
+  for (int g = 0; g < a.subs; ++g) {
+    const int row0 = (run.I * a.subs + g) * kRows + warp * 32 * IPT;
+    if ((run.I * a.subs + g) * kRows >= a.n) break;  // a short last block
+    VjpBody me[IPT];
+    double acc[IPT][7];
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+      const int r = row0 + 32 * k + lane;
+      // rows in [n, ld) are zero records; rows past ld have none (zero mass and
+      // adjoints add nothing, and they are not stored)
+      me[k] = VjpBody{};
+      if (r < a.ld) me[k].load(jadj_at(jb, r));
+#pragma unroll
+      for (int c = 0; c < 7; ++c) acc[k][c] = 0.0;
+    }
+    int t = 0;
+    auto consume = [&](const JAdj* tile) {
+      const double2* p = reinterpret_cast<const double2*>(tile);
+      const int tt = run.tile(t);
+      VjpBody o;
+      if (run.distance(tt) == 0) {
+#pragma unroll 1
+        for (int k = 0; k < 32; ++k) {
+          o.load(p + k);
+          const int j = tt * kVjpTile + k;
+#pragma unroll
+          for (int r = 0; r < IPT; ++r)
+            vjp_pair<false>(me[r], o, eps2, j == row0 + 32 * r + lane, acc[r], nullptr);
+        }
+      } else {
+        double b[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll UNR
+        for (int k = 0; k < 32; ++k) {
+          o.load(p + ((lane + k) & 31));
+#pragma unroll
+          for (int r = 0; r < IPT; ++r) vjp_pair<true>(me[r], o, eps2, false, acc[r], b);
+#pragma unroll
+          for (int c = 0; c < 7; ++c) b[c] = __shfl_sync(0xffffffffu, b[c], next);
+        }
+        double* w = red + half * 7 * W * 32 + warp * 32 + lane;
+#pragma unroll
+        for (int c = 0; c < 7; ++c) w[c * W * 32] = b[c];
+      }
+    };
+    auto post = [&]() {  // the tile's sums over the W warps, into their slot
+      const int tt = run.tile(t), d = run.distance(tt);
+      if (d != 0) {
+        const double* o = red + half * 7 * W * 32;
+        double* out = a.out + static_cast<size_t>(a.S + d - 1) * 7 * a.stride +
+                      static_cast<size_t>(tt) * kVjpTile;
+        for (int e = threadIdx.x; e < 7 * 32; e += 32 * W) {
+          const int l = e & 31, c = e >> 5;
+          double v = 0.0;
+#pragma unroll
+          for (int w = 0; w < W; ++w) v += o[(c * W + w) * 32 + l];
+          double* dst = out + static_cast<size_t>(c) * a.stride + l;
+          *dst = g ? *dst + v : v;  // a later sub-block adds to this thread's own store
+        }
+      }
+      ++t;
+      half ^= 1;
+    };
+    if (!run.stream(pipe, jb, a.status, consume, post)) return;
+    if (g + 1 == a.subs) grid_release();
+    double* out = a.out + static_cast<size_t>(blockIdx.y) * 7 * a.stride;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+      const int r = row0 + 32 * k + lane;
+      if (r < a.n)
+#pragma unroll
+        for (int c = 0; c < 7; ++c) out[static_cast<size_t>(c) * a.stride + r] = -acc[k][c];
+    }
+  }
 }
 
-// Packs the VJP records from a predicted state and the acc/jerk adjoints;
-// rows >= n are zero (zero mass and zero adjoints contribute nothing).
-__global__ void vjp_pack_kernel(int n, int ld, const double* __restrict__ XV, const double* __restrict__ M,
-                                const double* __restrict__ AB, JAdj* __restrict__ jb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ld) return;
-  JAdj o;
+// Everything between two pair VJPs, per row, in one pass (it was five: slot
+// sums, reverse predictor, reverse corrector, adjoint and record packing, each
+// a launch on a handful of SMs for systems of a few thousand bodies).  ADJ =
+// [xb(3) vb(3) ab(3) jb(3)][ld], MB the mass adjoint.
+//   sum   adds the finished VJP's slots to xb, vb and MB
+//   post  reverse predictor: (xbp, vbp) -> (xb0, vb0), ab0/jb0 completed
+//   pack  the next VJP's records at state XV ([6][ld]), with the acc/jerk adjoints
+//         kPackStep  of the reverse corrector of the step whose outputs ADJ now
+//                    holds (its own part of ab0/jb0 goes to ADJ's ab/jb slots)
+//         kPackFrom  AB ([6][ld])
+// Rows >= n pack as zero records.
+enum AdjPack { kPackNone, kPackStep, kPackFrom };
+__global__ void __launch_bounds__(kSumThreads)
+    adj_link_kernel(int n, int ld, double h, RowSlots slots, bool sum, const double* __restrict__ P,
+                    bool post, double* ADJ, double* __restrict__ MB, int pack,
+                    const double* __restrict__ XV, const double* __restrict__ M, const double* AB,
+                    JAdj* __restrict__ jb) {
+  constexpr int GR = 8;
+  __shared__ double sh[7 * kSumThreads];
+  grid_wait();
+  grid_release();
+  const int i = blockIdx.x * kSumRows<GR> + threadIdx.x % kSumRows<GR>;
+  double d[7];
+  if (sum) slot_sums<GR, 7>(P, ld, i < n ? slots.count(i) : 0, i, d, sh);
+  if (threadIdx.x >= kSumRows<GR> || i >= ld) return;
   const bool real = i < n;
-  o.x = real ? XV[i] : 0; o.y = real ? XV[ld + i] : 0; o.z = real ? XV[2 * ld + i] : 0;
-  o.vx = real ? XV[3 * ld + i] : 0; o.vy = real ? XV[4 * ld + i] : 0; o.vz = real ? XV[5 * ld + i] : 0;
-  o.m = real ? M[i] : 0;
-  o.ax = real ? AB[i] : 0; o.ay = real ? AB[ld + i] : 0; o.az = real ? AB[2 * ld + i] : 0;
-  o.bx = real ? AB[3 * ld + i] : 0; o.by = real ? AB[4 * ld + i] : 0; o.bz = real ? AB[5 * ld + i] : 0;
-  o.pad0 = o.pad1 = o.pad2 = 0;
-  jb[i] = o;
-}
-
-// Adds the VJP split partials into xb/vb ([6][ld]) and mb.
-__global__ void vjp_reduce_kernel(int n, int ld, int S, const double* __restrict__ P,
-                                  double* __restrict__ XVB, double* __restrict__ MB) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  for (int c = 0; c < 7; ++c) {
-    double v = 0.0;
-    for (int s = 0; s < S; ++s) v += P[(static_cast<size_t>(s) * 7 + c) * ld + i];
-    if (c < 6) XVB[c * ld + i] += v;
-    else MB[i] += v;
-  }
-}
-
-// Reverse corrector: ADJ = [xb(3) vb(3) ab(3) jb(3)] holds the adjoint of the
-// step's outputs; writes ab1/jb1 into AB1 and the corrector part of ab0/jb0
-// into ADJ's ab/jb slots (xb, vb stay as xbp, vbp).
-__global__ void adj_pre_kernel(int n, int ld, double h, double* __restrict__ ADJ,
-                               double* __restrict__ AB1) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
   const double h2 = h * h, h3 = h2 * h;
-  for (int c = 0; c < 3; ++c) {
-    const double xb = ADJ[c * ld + i], vb = ADJ[(3 + c) * ld + i];
-    const double ab_out = ADJ[(6 + c) * ld + i], jb_out = ADJ[(9 + c) * ld + i];
-    AB1[c * ld + i] = 0.15 * h2 * xb + 0.5 * h * vb + ab_out;
-    AB1[(3 + c) * ld + i] = -(h3 / 30.0) * xb - (h2 / 12.0) * vb + jb_out;
-    ADJ[(6 + c) * ld + i] = -0.15 * h2 * xb - 0.5 * h * vb;
-    ADJ[(9 + c) * ld + i] = -(7.0 * h3 / 60.0) * xb - (5.0 * h2 / 12.0) * vb;
+  double a[3] = {0.0, 0.0, 0.0}, b[3] = {0.0, 0.0, 0.0};
+  if (real) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      double xb = ADJ[c * ld + i], vb = ADJ[(3 + c) * ld + i];
+      double ab = ADJ[(6 + c) * ld + i], jb_ = ADJ[(9 + c) * ld + i];
+      if (sum) {
+        xb += d[c];
+        vb += d[3 + c];
+      }
+      if (post) {
+        ab += 0.5 * h2 * xb + h * vb;
+        jb_ += (h3 / 6.0) * xb + 0.5 * h2 * vb;
+        vb = h * xb + vb;
+      }
+      if (pack == kPackStep) {
+        a[c] = 0.15 * h2 * xb + 0.5 * h * vb + ab;
+        b[c] = -(h3 / 30.0) * xb - (h2 / 12.0) * vb + jb_;
+        ab = -0.15 * h2 * xb - 0.5 * h * vb;
+        jb_ = -(7.0 * h3 / 60.0) * xb - (5.0 * h2 / 12.0) * vb;
+      } else if (pack == kPackFrom) {
+        a[c] = AB[c * ld + i];
+        b[c] = AB[(3 + c) * ld + i];
+      }
+      ADJ[c * ld + i] = xb;
+      ADJ[(3 + c) * ld + i] = vb;
+      ADJ[(6 + c) * ld + i] = ab;
+      ADJ[(9 + c) * ld + i] = jb_;
+    }
+    if (sum) MB[i] += d[6];
+  }
+  if (pack != kPackNone) {
+    double2* o = jadj_at(jb, i);
+    const double z = 0.0;
+    o[0] = make_double2(real ? XV[i] : z, real ? XV[ld + i] : z);
+    o[32] = make_double2(real ? XV[2 * ld + i] : z, real ? M[i] : z);
+    o[64] = make_double2(real ? XV[3 * ld + i] : z, real ? XV[4 * ld + i] : z);
+    o[96] = make_double2(real ? XV[5 * ld + i] : z, a[0]);
+    o[128] = make_double2(a[1], a[2]);
+    o[160] = make_double2(b[0], b[1]);
+    o[192] = make_double2(b[2], z);
   }
 }
 
-// Reverse predictor: (xbp, vbp) -> (xb0, vb0), ab0/jb0 completed.
-__global__ void adj_post_kernel(int n, int ld, double h, double* __restrict__ ADJ) {
+// dst[a][i] = src[a][i] for rows i < n of g.arrays arrays (one launch instead
+// of a copy per array); rows [n, ld) of `dst` become zero when pad is set.
+__global__ void copy_rows_kernel(int n, int ld, GatherArgs g, bool pad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double h2 = h * h, h3 = h2 * h;
-  for (int c = 0; c < 3; ++c) {
-    const double xbp = ADJ[c * ld + i], vbp = ADJ[(3 + c) * ld + i];
-    ADJ[(3 + c) * ld + i] = h * xbp + vbp;
-    ADJ[(6 + c) * ld + i] += 0.5 * h2 * xbp + h * vbp;
-    ADJ[(9 + c) * ld + i] += (h3 / 6.0) * xbp + 0.5 * h2 * vbp;
-  }
+  if (i >= (pad ? ld : n)) return;
+#pragma unroll
+  for (int a = 0; a < kMaxGather; ++a)
+    if (a < g.arrays) g.dst[a][i] = i < n && g.src[a] ? g.src[a][i] : 0.0;
 }
 
 #define AD_CUDA(call)                                                                      \
@@ -229,22 +305,56 @@ __global__ void adj_post_kernel(int n, int ld, double h, double* __restrict__ AD
     if (s_ != NBODY_OK) return s_; \
   } while (0)
 
-using FwdFP64 = RowsFP64<128, 2, kTile, 1>;
-using FwdFP64Small = RowsFP64<128, 1, kTile, 2>;  // n < kSmallN: twice the row blocks
-constexpr int kSmallN = 32768;
-using FwdMixed = RowsMixedX2<128, 4, kTile, 1, 1>;
-
-template <class R>
-__global__ void __launch_bounds__(R::NT) adj_pair_kernel(const typename R::JB* __restrict__ jb, PairArgs a) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ uint64_t full[2];
-  pair_system<R>(jb, a, smem_raw, full);
+// Symmetric kernels of the forward (four rows per lane from kWideN bodies, two
+// below, as the engine) and of the VJP.
+constexpr int kWideN = 16384;
+constexpr int kW = 4;  // warps per CTA
+const void* fwd_fp64(bool wide) {
+  return wide ? reinterpret_cast<const void*>(&pair_sym_fp64_kernel<4, kW, 2, 2>)
+              : reinterpret_cast<const void*>(&pair_sym_fp64_kernel<2, kW, 4, 4>);
 }
-
-int splits_for(int sms, int row_blocks, int n_tiles, int ctas_per_sm) {
-  const int target = sms * ctas_per_sm;
-  return std::max(1, std::min(n_tiles, (target + row_blocks - 1) / row_blocks));
+const void* fwd_mixed(bool wide) {
+  return wide ? reinterpret_cast<const void*>(&pair_sym_nf_kernel<4, kW, 2, 4, 2, 3>)
+              : reinterpret_cast<const void*>(&pair_sym_nf_kernel<2, kW, 1, 4, 2, 4>);
 }
+const void* vjp_fn() { return reinterpret_cast<const void*>(&vjp_sym_kernel<2, kW, 2, 2>); }
+
+// A symmetric kernel with its grid for one system size.
+struct SymLaunch {
+  const void* fn = nullptr;
+  size_t smem = 0;
+  int rows = 0, tj = 0, S = 1, subs = 1, nb = 1, block_rows = 1;
+  cudaError_t plan(const void* f, size_t sm, int rows_, int tj_, int n, int sms, double per_ms, bool waves) {
+    fn = f; smem = sm; rows = rows_; tj = tj_;
+    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+    if (e != cudaSuccess) return e;
+    int occ = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, 32 * kW, sm);
+    if (e != cudaSuccess) return e;
+    S = sym_splits(sms, std::max(occ, 1), rows, tj, n, per_ms, waves);
+    const SymGrid g(rows, n);
+    subs = g.subs; nb = g.nb; block_rows = g.block_rows;
+    return cudaSuccess;
+  }
+  RowSlots slots() const { return RowSlots(S, block_rows, nb); }
+  size_t count() const { return S + nb / 2; }
+  cudaError_t launch(const void* records, SymArgs a, cudaStream_t st) const {
+    a.nb = nb; a.subs = subs; a.S = S;
+    a.tiles = (a.n + tj - 1) / tj;
+    void* args[] = {static_cast<void*>(&records), static_cast<void*>(&a)};
+    cudaLaunchAttribute at{};  // as launch_chained
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(nb, S);
+    c.blockDim = dim3(32 * kW);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelExC(&c, fn, args);
+  }
+};
 
 }  // namespace
 
@@ -255,88 +365,112 @@ struct nbody_adjoint {
   double *X = nullptr, *V = nullptr, *M = nullptr, *D = nullptr;
   double* ckpt = nullptr;   // [nseg][13][ld]
   double* segxv = nullptr;  // [checkpoint_every][6][ld] predicted states of a segment
-  double* adj = nullptr;    // [12][ld] xb vb ab jb
-  double* ab1 = nullptr;    // [6][ld]
-  double* mb = nullptr;     // [ld]
-  double* P = nullptr;      // forward partials [S][6][ld]
-  double* Pv = nullptr;     // VJP partials [Sv][7][ld]
+  double* adj = nullptr;    // [13][ld] xb vb ab jb, mb
+  double* ab1 = nullptr;    // [6][ld] caller's acc/jerk adjoints (vjp_acc_jerk)
+  double* mb = nullptr;     // adj's last array
+  double* P = nullptr;      // forward slots [..][6][ld]
+  double* Pv = nullptr;     // VJP slots [..][7][ld]
   JBody64* jb64 = nullptr;
-  JBodyX2* jbx = nullptr;
+  SymSub* jsub = nullptr;
   JAdj* jadj = nullptr;
   StepCtl* ctl = nullptr;
   int* status = nullptr;
-  int S = 1, Sv = 1;
+  SymLaunch fwd, rev;
   bool have_forward = false;
 };
 
 namespace {
 
-nbody_status fwd_eval(nbody_adjoint* a, cudaStream_t st) {
-  const bool fp64 = a->cfg.precision == NBODY_FP64;
+SymArgs sym_args(const nbody_adjoint* a, double* out) {
+  SymArgs s{};
+  s.n = a->n;
+  s.ld = a->ld;
+  s.eps2 = a->cfg.eps2;
+  s.out = out;
+  s.stride = static_cast<size_t>(a->ld);
+  s.status = a->status;
+  return s;
+}
+
+SoA7 own_state(const nbody_adjoint* a) {
   const size_t ld = a->ld;
-  PairArgs pa;
-  pa.i_begin = 0;
-  pa.i_end = a->n;
-  pa.n_rows_pad = a->ld;
-  pa.n_tiles = a->ld / kTile;
-  pa.tiles_per_split = (pa.n_tiles + a->S - 1) / a->S;
-  pa.eps2 = a->cfg.eps2;
-  pa.out = a->P;
-  pa.stride = ld;
-  pa.status = a->status;
-  if (fp64 && a->n < kSmallN) {
-    const dim3 grid((a->n + FwdFP64Small::ROWS - 1) / FwdFP64Small::ROWS, a->S);
-    adj_pair_kernel<FwdFP64Small><<<grid, FwdFP64Small::NT, pair_smem_bytes<FwdFP64Small>(), st>>>(
-        a->jb64, pa);
-  } else if (fp64) {
-    const dim3 grid((a->n + FwdFP64::ROWS - 1) / FwdFP64::ROWS, a->S);
-    adj_pair_kernel<FwdFP64><<<grid, FwdFP64::NT, pair_smem_bytes<FwdFP64>(), st>>>(a->jb64, pa);
-  } else {
-    const dim3 grid((a->n + FwdMixed::ROWS - 1) / FwdMixed::ROWS, a->S);
-    adj_pair_kernel<FwdMixed><<<grid, FwdMixed::NT, pair_smem_bytes<FwdMixed>(), st>>>(a->jbx, pa);
-  }
-  AD_CUDA(cudaGetLastError());
+  return SoA7{a->X, a->X + ld, a->X + 2 * ld, a->M, a->V, a->V + ld, a->V + 2 * ld};
+}
+
+nbody_status fwd_eval(nbody_adjoint* a, cudaStream_t st) {
+  SymArgs s = sym_args(a, a->P);
+  s.rows = own_state(a);
+  AD_CUDA(a->fwd.launch(a->cfg.precision == NBODY_FP64 ? static_cast<const void*>(a->jb64) : a->jsub, s, st));
   return NBODY_OK;
 }
 
 nbody_status fwd_initial(nbody_adjoint* a, cudaStream_t st) {
-  const bool fp64 = a->cfg.precision == NBODY_FP64;
   const size_t ld = a->ld;
-  SoA7 in{a->X, a->X + ld, a->X + 2 * ld, a->M, a->V, a->V + ld, a->V + 2 * ld};
-  pack_kernel<<<(a->ld + kBlock - 1) / kBlock, kBlock, 0, st>>>(a->n, a->ld, in, fp64 ? a->jb64 : nullptr,
-                                                               nullptr, fp64 ? nullptr : a->jbx);
+  if (a->cfg.precision == NBODY_FP64)
+    pack_kernel<<<(a->ld + kBlock - 1) / kBlock, kBlock, 0, st>>>(a->n, a->ld, own_state(a), a->jb64, nullptr);
+  else
+    sym_tile_kernel<false><<<a->ld / 64, 64, 0, st>>>(a->n, own_state(a), a->jsub);
+  AD_CUDA(cudaGetLastError());
   AD_TRY(fwd_eval(a, st));
   double* D = a->D;
-  launch_reduce(st, 0, a->n, a->ld, a->S, a->P,
+  launch_reduce(st, 0, a->n, a->ld, a->fwd.slots(), a->P,
                 SoA6{D, D + ld, D + 2 * ld, D + 3 * ld, D + 4 * ld, D + 5 * ld});
   AD_CUDA(cudaGetLastError());
   return NBODY_OK;
 }
 
-// One Hermite step; if xp_out, the predicted X/V ([6][ld]) are copied there.
+// One Hermite step; if xp_out, the predicted X/V ([6][ld]) go there too.
 nbody_status fwd_step(nbody_adjoint* a, cudaStream_t st, double* xp_out) {
-  const bool fp64 = a->cfg.precision == NBODY_FP64;
-  predict_kernel<<<(a->n + kBlock - 1) / kBlock, kBlock, 0, st>>>(
-      a->n, a->ld, a->ctl, a->X, a->V, a->M, a->D, fp64 ? a->jb64 : nullptr, nullptr,
-      fp64 ? nullptr : a->jbx);
-  if (xp_out)
-    AD_CUDA(cudaMemcpyAsync(xp_out, a->X, sizeof(double) * 6 * a->ld, cudaMemcpyDeviceToDevice, st));
+  if (a->cfg.precision == NBODY_FP64)
+    AD_CUDA(launch_chained(predict_kernel, (a->n + kPredictBlock - 1) / kPredictBlock, kPredictBlock, 0, st,
+                           a->n, a->ld, a->ctl, a->X, a->V, a->M, a->D, a->jb64, nullptr, nullptr, xp_out));
+  else
+    AD_CUDA(launch_chained(sym_tile_kernel<true>, a->ld / 64, 64, 0, st, a->n, own_state(a), a->jsub, a->ld,
+                           a->X, a->V, a->D, a->ctl, nullptr, xp_out));
   AD_TRY(fwd_eval(a, st));
-  launch_correct(st, a->n, a->ld, a->S, a->P, a->X, a->V, a->D, a->ctl, 1.0);
+  launch_correct(st, a->n, a->ld, a->fwd.slots(), a->P, a->X, a->V, a->D, a->ctl, 1.0, true);
   AD_CUDA(cudaGetLastError());
   return NBODY_OK;
 }
 
-// (xb, vb, mb) += VJP of the pair acc/jerk at state XV ([6][ld]) with
-// acc/jerk adjoints AB ([6][ld]).
-nbody_status vjp(nbody_adjoint* a, cudaStream_t st, const double* XV, const double* AB) {
-  vjp_pack_kernel<<<(a->ld + kBlock - 1) / kBlock, kBlock, 0, st>>>(a->n, a->ld, XV, a->M, AB, a->jadj);
-  const int n_tiles = a->ld / kVjpTile;
-  const int tps = (n_tiles + a->Sv - 1) / a->Sv;
-  const dim3 grid((a->n + kVjpNT - 1) / kVjpNT, a->Sv);
-  vjp_pair_kernel<<<grid, kVjpNT, 2 * kVjpTile * sizeof(JAdj), st>>>(a->jadj, a->n, a->ld, tps,
-                                                                    a->cfg.eps2, a->Pv, a->status);
-  vjp_reduce_kernel<<<(a->n + kBlock - 1) / kBlock, kBlock, 0, st>>>(a->n, a->ld, a->Sv, a->Pv, a->adj, a->mb);
+// The pass between two VJPs (adj_link_kernel).
+nbody_status link(nbody_adjoint* a, cudaStream_t st, bool sum, bool post, AdjPack pack,
+                  const double* XV = nullptr, const double* AB = nullptr) {
+  constexpr int rows = kSumRows<8>;
+  AD_CUDA(launch_chained(adj_link_kernel, (a->ld + rows - 1) / rows, kSumThreads, 0, st, a->n, a->ld,
+                         a->cfg.dt, a->rev.slots(), sum, a->Pv, post, a->adj, a->mb,
+                         static_cast<int>(pack), XV, a->M, AB, a->jadj));
+  return NBODY_OK;
+}
+
+// Slots of the pair VJP at the packed records.
+nbody_status vjp(nbody_adjoint* a, cudaStream_t st) {
+  AD_CUDA(a->rev.launch(a->jadj, sym_args(a, a->Pv), st));
+  return NBODY_OK;
+}
+
+// The caller's `count` arrays (n each; null: zeros) into consecutive [ld]
+// arrays, padding rows zero.
+nbody_status copy_rows(nbody_adjoint* a, cudaStream_t st, const double* const* src, double* dst, int count) {
+  GatherArgs g{};
+  g.arrays = count;
+  for (int k = 0; k < count; ++k) {
+    g.src[k] = src[k];
+    g.dst[k] = dst + static_cast<size_t>(k) * a->ld;
+  }
+  copy_rows_kernel<<<(a->ld + kBlock - 1) / kBlock, kBlock, 0, st>>>(a->n, a->ld, g, true);
+  AD_CUDA(cudaGetLastError());
+  return NBODY_OK;
+}
+// And back: consecutive [ld] arrays to the caller's.
+nbody_status copy_out(nbody_adjoint* a, cudaStream_t st, const double* src, double* const* dst, int count) {
+  GatherArgs g{};
+  g.arrays = count;
+  for (int k = 0; k < count; ++k) {
+    g.src[k] = src + static_cast<size_t>(k) * a->ld;
+    g.dst[k] = dst[k];
+  }
+  copy_rows_kernel<<<(a->ld + kBlock - 1) / kBlock, kBlock, 0, st>>>(a->n, a->ld, g, false);
   AD_CUDA(cudaGetLastError());
   return NBODY_OK;
 }
@@ -369,8 +503,8 @@ nbody_status nbody_adjoint_destroy(nbody_adjoint* a) {
   if (!a) return NBODY_OK;
   cudaSetDevice(a->cfg.device);
   cudaDeviceSynchronize();
-  void* bufs[] = {a->state, a->ckpt, a->segxv, a->adj, a->ab1, a->mb, a->P, a->Pv,
-                  a->jb64, a->jbx, a->jadj, a->ctl, a->status};
+  void* bufs[] = {a->state, a->ckpt, a->segxv, a->adj, a->ab1, a->P, a->Pv,
+                  a->jb64, a->jsub, a->jadj, a->ctl, a->status};
   for (void* p : bufs) cudaFree(p);
   delete a;
   return NBODY_OK;
@@ -402,16 +536,16 @@ nbody_status nbody_adjoint_create(nbody_adjoint** out, const nbody_adjoint_confi
   a->ld = (cfg->n + kPad - 1) / kPad * kPad;
   a->nseg = std::max(1, (cfg->nsteps + cfg->checkpoint_every - 1) / cfg->checkpoint_every);
   cudaDeviceGetAttribute(&a->sms, cudaDevAttrMultiProcessorCount, cfg->device);
-  const int rows_fwd = cfg->precision == NBODY_FP64
-                           ? (cfg->n < kSmallN ? FwdFP64Small::ROWS : FwdFP64::ROWS)
-                           : FwdMixed::ROWS;
-  // forward: small systems take as many j-splits as the wave allows (the
-  // pair pass is latency-bound there); VJP: about 4 CTAs per SM
-  a->S = splits_for(a->sms, (a->n + rows_fwd - 1) / rows_fwd, a->ld / kTile, 8);
-  a->Sv = splits_for(a->sms, (a->n + kVjpNT - 1) / kVjpNT, a->ld / kVjpTile, 4);
   nbody_adjoint* r = a.get();
   auto body = [&]() -> nbody_status {
     const size_t ld = r->ld;
+    const bool fp64 = cfg->precision == NBODY_FP64, wide = r->n >= kWideN;
+    const int ipt = wide ? 4 : 2;
+    const size_t fwd_smem = fp64 ? (wide ? sym_fp64_smem<4, kW, 2>() : sym_fp64_smem<2, kW, 4>())
+                                 : (wide ? sym_nf_smem<4, kW, 2>() : sym_nf_smem<2, kW, 1>());
+    AD_CUDA(r->fwd.plan(fp64 ? fwd_fp64(wide) : fwd_mixed(wide), fwd_smem, 32 * kW * ipt,
+                        fp64 ? kSymTile64 : wide ? 128 : 64, r->n, r->sms, fp64 ? 7.6e8 : 1.6e9, fp64));
+    AD_CUDA(r->rev.plan(vjp_fn(), vjp_smem<2, kW>(), 32 * kW * 2, kVjpTile, r->n, r->sms, 3.3e8, true));
     AD_CUDA(cudaMalloc(&r->state, sizeof(double) * 13 * ld));
     AD_CUDA(cudaMemset(r->state, 0, sizeof(double) * 13 * ld));
     r->X = r->state;
@@ -420,29 +554,17 @@ nbody_status nbody_adjoint_create(nbody_adjoint** out, const nbody_adjoint_confi
     r->D = r->state + 7 * ld;
     AD_CUDA(cudaMalloc(&r->ckpt, sizeof(double) * 13 * ld * r->nseg));
     AD_CUDA(cudaMalloc(&r->segxv, sizeof(double) * 6 * ld * cfg->checkpoint_every));
-    AD_CUDA(cudaMalloc(&r->adj, sizeof(double) * 12 * ld));
+    AD_CUDA(cudaMalloc(&r->adj, sizeof(double) * 13 * ld));
+    r->mb = r->adj + 12 * ld;
     AD_CUDA(cudaMalloc(&r->ab1, sizeof(double) * 6 * ld));
-    AD_CUDA(cudaMalloc(&r->mb, sizeof(double) * ld));
-    AD_CUDA(cudaMalloc(&r->P, sizeof(double) * 6 * ld * r->S));
-    AD_CUDA(cudaMalloc(&r->Pv, sizeof(double) * 7 * ld * r->Sv));
-    AD_CUDA(cudaMalloc(&r->jb64, sizeof(JBody64) * ld));
-    AD_CUDA(cudaMalloc(&r->jbx, sizeof(JBodyX2) * ld));
+    AD_CUDA(cudaMalloc(&r->P, sizeof(double) * 6 * ld * r->fwd.count()));
+    AD_CUDA(cudaMalloc(&r->Pv, sizeof(double) * 7 * ld * r->rev.count()));
+    if (fp64) AD_CUDA(cudaMalloc(&r->jb64, sizeof(JBody64) * ld));
+    else AD_CUDA(cudaMalloc(&r->jsub, sizeof(SymSub) * (ld / 64)));
     AD_CUDA(cudaMalloc(&r->jadj, sizeof(JAdj) * ld));
     AD_CUDA(cudaMalloc(&r->ctl, sizeof(StepCtl)));
     AD_CUDA(cudaMalloc(&r->status, sizeof(int)));
     AD_CUDA(cudaMemset(r->status, 0, sizeof(int)));
-    AD_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(&adj_pair_kernel<FwdMixed>),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(pair_smem_bytes<FwdMixed>())));
-    AD_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(&adj_pair_kernel<FwdFP64>),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(pair_smem_bytes<FwdFP64>())));
-    AD_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(&adj_pair_kernel<FwdFP64Small>),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(pair_smem_bytes<FwdFP64Small>())));
-    AD_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(&vjp_pair_kernel),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(2 * kVjpTile * sizeof(JAdj))));
     return NBODY_OK;
   };
   nbody_status s = body();
@@ -465,11 +587,9 @@ nbody_status nbody_adjoint_forward(nbody_adjoint* a, const double* x, const doub
     if (!p) return nbody_set_error(NBODY_ERR_INVALID_ARG, "null device array");
   AD_CUDA(cudaSetDevice(a->cfg.device));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t ld = a->ld, b = sizeof(double) * a->n;
-  AD_CUDA(cudaMemsetAsync(a->state, 0, sizeof(double) * 13 * ld, st));
-  const double* src[7] = {x, y, z, vx, vy, vz, m};
-  double* dst[7] = {a->X, a->X + ld, a->X + 2 * ld, a->V, a->V + ld, a->V + 2 * ld, a->M};
-  for (int k = 0; k < 7; ++k) AD_CUDA(cudaMemcpyAsync(dst[k], src[k], b, cudaMemcpyDeviceToDevice, st));
+  const size_t ld = a->ld;
+  const double* src[13] = {x, y, z, vx, vy, vz, m};  // the derivatives start at zero
+  AD_TRY(copy_rows(a, st, src, a->state, 13));
   AD_TRY(set_ctl(a, st));
   AD_TRY(fwd_initial(a, st));
   const int K = a->cfg.checkpoint_every;
@@ -482,8 +602,7 @@ nbody_status nbody_adjoint_forward(nbody_adjoint* a, const double* x, const doub
   if (a->cfg.nsteps == 0)
     AD_CUDA(cudaMemcpyAsync(a->ckpt, a->state, sizeof(double) * 13 * ld, cudaMemcpyDeviceToDevice, st));
   double* outs[6] = {x1, y1, z1, vx1, vy1, vz1};
-  const double* res[6] = {a->X, a->X + ld, a->X + 2 * ld, a->V, a->V + ld, a->V + 2 * ld};
-  for (int k = 0; k < 6; ++k) AD_CUDA(cudaMemcpyAsync(outs[k], res[k], b, cudaMemcpyDeviceToDevice, st));
+  AD_TRY(copy_out(a, st, a->X, outs, 6));
   a->have_forward = true;
   return check_status(a, st);
 }
@@ -501,15 +620,11 @@ nbody_status nbody_adjoint_backward(nbody_adjoint* a, const double* gx, const do
     if (!p) return nbody_set_error(NBODY_ERR_INVALID_ARG, "null device array");
   AD_CUDA(cudaSetDevice(a->cfg.device));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t ld = a->ld, b = sizeof(double) * a->n;
-  const double h = a->cfg.dt;
+  const size_t ld = a->ld;
   const int K = a->cfg.checkpoint_every, NS = a->cfg.nsteps;
-  AD_CUDA(cudaMemsetAsync(a->adj, 0, sizeof(double) * 12 * ld, st));
-  AD_CUDA(cudaMemsetAsync(a->mb, 0, sizeof(double) * ld, st));
-  const double* g[6] = {gx, gy, gz, gvx, gvy, gvz};
-  for (int k = 0; k < 6; ++k) AD_CUDA(cudaMemcpyAsync(a->adj + k * ld, g[k], b, cudaMemcpyDeviceToDevice, st));
+  const double* g[13] = {gx, gy, gz, gvx, gvy, gvz};  // the rest of adj and mb start at zero
+  AD_TRY(copy_rows(a, st, g, a->adj, 13));
   AD_TRY(set_ctl(a, st));
-  const int nb = (a->n + kBlock - 1) / kBlock;
   for (int seg = a->nseg - 1; seg >= 0; --seg) {
     const int s0 = seg * K, s1 = std::min(NS, s0 + K);
     if (s1 <= s0) continue;
@@ -517,17 +632,19 @@ nbody_status nbody_adjoint_backward(nbody_adjoint* a, const double* gx, const do
                             sizeof(double) * 13 * ld, cudaMemcpyDeviceToDevice, st));
     for (int s = s0; s < s1; ++s) AD_TRY(fwd_step(a, st, a->segxv + static_cast<size_t>(s - s0) * 6 * ld));
     for (int s = s1 - 1; s >= s0; --s) {
-      adj_pre_kernel<<<nb, kBlock, 0, st>>>(a->n, a->ld, h, a->adj, a->ab1);
-      AD_TRY(vjp(a, st, a->segxv + static_cast<size_t>(s - s0) * 6 * ld, a->ab1));
-      adj_post_kernel<<<nb, kBlock, 0, st>>>(a->n, a->ld, h, a->adj);
-      AD_CUDA(cudaGetLastError());
+      const bool inside = s < s1 - 1;  // a VJP of this segment's next step to finish first
+      AD_TRY(link(a, st, inside, inside, kPackStep, a->segxv + static_cast<size_t>(s - s0) * 6 * ld));
+      AD_TRY(vjp(a, st));
     }
+    AD_TRY(link(a, st, true, true, kPackNone));
   }
   // the initial acc/jerk: (a0, j0) = F(x_init, v_init, m), x_init in checkpoint 0
-  AD_TRY(vjp(a, st, a->ckpt, a->adj + 6 * ld));
-  double* outs[7] = {gx0, gy0, gz0, gvx0, gvy0, gvz0, gm};
-  for (int k = 0; k < 6; ++k) AD_CUDA(cudaMemcpyAsync(outs[k], a->adj + k * ld, b, cudaMemcpyDeviceToDevice, st));
-  AD_CUDA(cudaMemcpyAsync(gm, a->mb, b, cudaMemcpyDeviceToDevice, st));
+  AD_TRY(link(a, st, false, false, kPackFrom, a->ckpt, a->adj + 6 * ld));
+  AD_TRY(vjp(a, st));
+  AD_TRY(link(a, st, true, false, kPackNone));
+  double* outs[6] = {gx0, gy0, gz0, gvx0, gvy0, gvz0};
+  AD_TRY(copy_out(a, st, a->adj, outs, 6));
+  AD_TRY(copy_out(a, st, a->mb, &gm, 1));
   return check_status(a, st);
 }
 
@@ -544,24 +661,20 @@ nbody_status nbody_adjoint_vjp_acc_jerk(nbody_adjoint* a, const double* x, const
     if (!p) return nbody_set_error(NBODY_ERR_INVALID_ARG, "null device array");
   AD_CUDA(cudaSetDevice(a->cfg.device));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t ld = a->ld, b = sizeof(double) * a->n;
   // inputs go to the segment buffer (state) and ab1 (adjoints); outputs via adj/mb
-  AD_CUDA(cudaMemsetAsync(a->segxv, 0, sizeof(double) * 6 * ld, st));
-  AD_CUDA(cudaMemsetAsync(a->ab1, 0, sizeof(double) * 6 * ld, st));
-  AD_CUDA(cudaMemsetAsync(a->adj, 0, sizeof(double) * 6 * ld, st));
-  AD_CUDA(cudaMemsetAsync(a->mb, 0, sizeof(double) * ld, st));
-  AD_CUDA(cudaMemsetAsync(a->M, 0, sizeof(double) * ld, st));
   const double* xv[6] = {x, y, z, vx, vy, vz};
   const double* ab[6] = {abx, aby, abz, jbx, jby, jbz};
-  for (int k = 0; k < 6; ++k) {
-    AD_CUDA(cudaMemcpyAsync(a->segxv + k * ld, xv[k], b, cudaMemcpyDeviceToDevice, st));
-    AD_CUDA(cudaMemcpyAsync(a->ab1 + k * ld, ab[k], b, cudaMemcpyDeviceToDevice, st));
-  }
-  AD_CUDA(cudaMemcpyAsync(a->M, m, b, cudaMemcpyDeviceToDevice, st));
-  AD_TRY(vjp(a, st, a->segxv, a->ab1));
+  const double* zero[13] = {};
+  AD_TRY(copy_rows(a, st, xv, a->segxv, 6));
+  AD_TRY(copy_rows(a, st, ab, a->ab1, 6));
+  AD_TRY(copy_rows(a, st, zero, a->adj, 13));
+  AD_TRY(copy_rows(a, st, &m, a->M, 1));
+  AD_TRY(link(a, st, false, false, kPackFrom, a->segxv, a->ab1));
+  AD_TRY(vjp(a, st));
+  AD_TRY(link(a, st, true, false, kPackNone));
   double* outs[6] = {gx, gy, gz, gvx, gvy, gvz};
-  for (int k = 0; k < 6; ++k) AD_CUDA(cudaMemcpyAsync(outs[k], a->adj + k * ld, b, cudaMemcpyDeviceToDevice, st));
-  AD_CUDA(cudaMemcpyAsync(gm, a->mb, b, cudaMemcpyDeviceToDevice, st));
+  AD_TRY(copy_out(a, st, a->adj, outs, 6));
+  AD_TRY(copy_out(a, st, a->mb, &gm, 1));
   a->have_forward = false;  // the state buffers now hold this call's inputs
   return check_status(a, st);
 }

@@ -53,19 +53,6 @@ namespace {
 
 constexpr int kPad = 256;        // body padding granularity (multiple of every j-tile)
 constexpr int kMaxSplit = 64;    // split-j upper bound
-// Blocks of the symmetric schedule: nb / 2 partial-sum slots, so at most 64
-// beside the splits.  More blocks would need more slots (48 bytes per row
-// each), fewer would evaluate more of the pairs one-sided (1 / nb of them).
-constexpr int kMaxSymBlocks = 128;
-// Slots of a symmetric pass are further bounded by memory (8 GiB of P, at
-// least 8 slots): larger systems take fewer, larger blocks and fewer splits.
-int max_sym_slots(int n) {
-  const double fit = 8.0 * (1 << 30) / (48.0 * n);
-  return fit > 2 * kMaxSplit ? 2 * kMaxSplit : std::max(8, static_cast<int>(fit));
-}
-// Rate at which the corrector sums split partials (64 splits at N = 65536:
-// 201 MB in 52 us), the autotuner's price for each partial a tiling leaves.
-constexpr double kSplitSumBytesPerMs = 3.9e9;
 constexpr int kBlockO1 = 256;    // threads per CTA of the O(N) kernels
 constexpr int kMaxBBoxParts = 512;  // CTAs of the bounding-box pass
 constexpr int kOrderBits = 48;     // Hilbert key width (order_key_kernel)
@@ -243,23 +230,11 @@ struct Tiling {
   int source = 0;  // nbody_timers.tiling_source: 1 heuristic/explicit, 2 timed, 3 cached
 };
 
-// The symmetric schedule of n bodies with kernel k.
-struct SymGrid {
-  int subs, block_rows, nb;
-  SymGrid(const PairKernel& k, int n) {
-    const int rows = k.nt * k.ipt;
-    const long most = static_cast<long>(std::min(kMaxSymBlocks, max_sym_slots(n))) * rows;
-    subs = static_cast<int>((n + most - 1) / most);
-    block_rows = subs * rows;
-    nb = (n + block_rows - 1) / block_rows;
-  }
-};
-
 // Partial-sum slots of each row after a launch of tiling t over n bodies
 // (cluster kernels sum their CL CTAs' partials into one).
 RowSlots row_slots(const Tiling& t, int n) {
   if (!t.k->sym) return RowSlots(t.split / t.k->cluster);
-  const SymGrid g(*t.k, n);
+  const SymGrid g(t.k->nt * t.k->ipt, n);
   return RowSlots(t.split, g.block_rows, g.nb);
 }
 // Slots of P that such a launch writes.
@@ -411,47 +386,15 @@ int choose_split(const nbody_engine* e, const PairKernel& k, int rows) {
   return best_s;
 }
 
-// Splits of the symmetric kernel k over n bodies: S CTAs per block share its
-// run of Q tiles, ceil(Q / S) each.  Cost in units of one (CTA, tile).  FP64
-// CTAs take the same time each and run in waves, the last of which takes what
-// its fullest SM holds (three quarters of a tile's time are throughput).  The
-// near/far kernel's differ with their near subtiles: the work of more CTAs
-// than are resident spreads over the slots, and the last ones leave SMs idle
-// for about a third of a CTA's time.  Every split is another 48 bytes per row
-// to sum.  Pair pass in ms by splits: FP64 N = 16384 0.464 (8) 0.39 (23) 0.405
-// (31), 65536 5.79 (8) 5.69 (31); mixed 16384 0.265 (9) 0.223 (31), 65536 2.91
-// (9) 2.77 (31).
+// Splits of the symmetric kernel k over n bodies.
 int choose_sym_split(const nbody_engine* e, const PairKernel& k, int n) {
   prepare_kernel(k);
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, k.nt, k.smem) != cudaSuccess ||
       occ < 1)
     occ = 1;
-  const SymGrid g(k, n);
-  const int Q = sym_q_count(g.nb, 0, g.block_rows / k.tj, (n + k.tj - 1) / k.tj);
-  const long slots = static_cast<long>(e->num_sms) * occ;
-  const double per_ms = k.precision == NBODY_FP64 ? 7.6e8 : 1.6e9;  // interactions of a full GPU
-  const double tile_ms = 2.0 * k.nt * k.ipt * k.tj * slots / per_ms;
-  const double per_split = 48.0 * n / kSplitSumBytesPerMs / tile_ms;
-  double best = 1e300;
-  int best_s = 1;
-  for (int tps = 1; tps <= Q; ++tps) {
-    const int s = (Q + tps - 1) / tps;
-    if (s > std::min(kMaxSplit, max_sym_slots(n) / 2)) continue;
-    const long ctas = static_cast<long>(g.nb) * s;
-    const double one = tps * g.subs + 0.5;
-    const bool waves = k.precision == NBODY_FP64 || ctas <= slots;
-    const long last = waves ? ctas % slots : 0;
-    const double per_sm = static_cast<double>((last + e->num_sms - 1) / e->num_sms) / occ;
-    double work = waves ? one * (ctas / slots) : one * ctas / slots;
-    if (last) work += one * (0.25 + 0.75 * per_sm);
-    const double cost = work + (k.precision == NBODY_FP64 ? 0.1 : 0.35) * one + per_split * s;
-    if (cost < best - 1e-9) {
-      best = cost;
-      best_s = s;
-    }
-  }
-  return best_s;
+  const bool fp64 = k.precision == NBODY_FP64;
+  return sym_splits(e->num_sms, occ, k.nt * k.ipt, k.tj, n, fp64 ? 7.6e8 : 1.6e9, fp64);
 }
 
 // Grows P to `split` slots.
@@ -494,7 +437,7 @@ SoA7 own_inputs(nbody_engine* e);
 // the bodies the records were built from.
 nbody_status launch_sym(nbody_engine* e, const Tiling& t, int n, cudaStream_t st, const SoA7& src) {
   const PairKernel& k = *t.k;
-  const SymGrid g(k, n);
+  const SymGrid g(k.nt * k.ipt, n);
   SymArgs a;
   a.n = n;
   a.ld = e->ld;
@@ -1303,7 +1246,7 @@ nbody_status nbody_get_timers(nbody_engine* e, nbody_timers* out) {
       double pairs = static_cast<double>((e->n + k.nt * k.ipt - 1) / (k.nt * k.ipt)) *
                      (k.nt / 32) * static_cast<double>(e->ld / k.tj);
       if (k.sym) {
-        const SymGrid g(k, e->n);
+        const SymGrid g(k.nt * k.ipt, e->n);
         pairs = 0.0;
         for (int I = 0; I < g.nb; ++I) {
           const int rows = std::min(g.block_rows, e->n - I * g.block_rows);

@@ -14,7 +14,10 @@
 //                            with the pre-step a, j
 //   initialdt       131-150  min_i eta0 |a| / |j|
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cstdint>
+#include <utility>
 
 #include "pair.cuh"
 
@@ -31,6 +34,25 @@ struct StepCtl {
   int adaptive;                    // 1: adopt dt_crit as the next dt
   long long steps;                 // completed steps
 };
+
+// Launches a kernel that begins with grid_wait right behind the kernel before
+// it on the stream: its launch overlaps that kernel's tail (three small
+// kernels 7.4 us instead of 12.5).
+template <class... P, class... A>
+cudaError_t launch_chained(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                           A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, std::forward<A>(args)...);
+}
 
 constexpr unsigned long long kPosInfBits = 0x7FF0000000000000ull;
 
@@ -148,10 +170,12 @@ static __global__ void pack_kernel(int n, int ld, SoA7 in, JBody64* __restrict__
   if (jbx2) jbx2[i] = make_jbx2(x, y, z, m, vx, vy, vz);
 }
 
-// Predicted position p and velocity u of row i, written back to X, V.
+// Predicted position p and velocity u of row i, written back to X, V and, if
+// not null, to XP ([6][ld]).
 __device__ __forceinline__ void predict_body(double dt, int ld, int i, double* __restrict__ X,
                                              double* __restrict__ V, const double* __restrict__ D,
-                                             double p[3], double u[3]) {
+                                             double p[3], double u[3],
+                                             double* __restrict__ XP = nullptr) {
   const double h2 = 0.5 * dt * dt;
   const double h3 = dt * dt * dt * (1.0 / 6.0);
 #pragma unroll
@@ -162,6 +186,10 @@ __device__ __forceinline__ void predict_body(double dt, int ld, int i, double* _
     u[c] = v + (a * dt + j * h2);
     X[c * ld + i] = p[c];
     V[c * ld + i] = u[c];
+    if (XP) {
+      XP[c * ld + i] = p[c];
+      XP[(3 + c) * ld + i] = u[c];
+    }
   }
 }
 
@@ -170,11 +198,14 @@ __device__ __forceinline__ void predict_body(double dt, int ld, int i, double* _
 static __global__ void predict_kernel(int n, int ld, const StepCtl* __restrict__ ctl, double* __restrict__ X,
                                double* __restrict__ V, const double* __restrict__ M,
                                const double* __restrict__ D, JBody64* __restrict__ jb64,
-                               JBody32* __restrict__ jb32, JBodyX2* __restrict__ jbx2) {
+                               JBody32* __restrict__ jb32, JBodyX2* __restrict__ jbx2,
+                               double* __restrict__ XP = nullptr) {
+  grid_wait();
+  grid_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double p[3], u[3];
-  predict_body(ctl->dt, ld, i, X, V, D, p, u);
+  predict_body(ctl->dt, ld, i, X, V, D, p, u, XP);
   const double m = M[i];
   if (jb64) store_jb64(jb64, i, p[0], p[1], p[2], m, u[0], u[1], u[2]);
   if (jb32) jb32[i] = make_jb32(p[0], p[1], p[2], m, u[0], u[1], u[2]);
@@ -198,18 +229,19 @@ struct RowSlots {
 };
 
 // sum[c] = sum over slots s = 0, 1, ..., S-1 (in that order) of
-// P[s * step][c][i], for the six fields at once: one pass over the splits with
+// P[s * step][c][i], for the F fields at once: one pass over the splits with
 // several loads in flight, so a small system (few CTAs) is not bound by
 // one load latency per split.
+template <int F = 6>
 __device__ __forceinline__ void split_sums(const double* __restrict__ P, int ld, int S, int i,
-                                           double sum[6], int step = 1) {
+                                           double sum[F], int step = 1) {
 #pragma unroll
-  for (int c = 0; c < 6; ++c) sum[c] = 0.0;
+  for (int c = 0; c < F; ++c) sum[c] = 0.0;
 #pragma unroll 4
   for (int s = 0; s < S; ++s) {
-    const double* p = P + static_cast<size_t>(s) * step * 6 * ld + i;
+    const double* p = P + static_cast<size_t>(s) * step * F * ld + i;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) sum[c] += p[static_cast<size_t>(c) * ld];
+    for (int c = 0; c < F; ++c) sum[c] += p[static_cast<size_t>(c) * ld];
   }
 }
 
@@ -223,23 +255,23 @@ constexpr int kSumThreads = 256;
 template <int GR>
 constexpr int kSumRows = kSumThreads / GR;
 
-// The six sums of row i, valid in the threads of group 0 (threadIdx.x <
-// kSumRows<GR>); sh holds 6 * kSumThreads doubles when GR > 1.
-template <int GR>
+// The F sums of row i, valid in the threads of group 0 (threadIdx.x <
+// kSumRows<GR>); sh holds F * kSumThreads doubles when GR > 1.
+template <int GR, int F = 6>
 __device__ __forceinline__ void slot_sums(const double* __restrict__ P, int ld, int S, int i,
-                                          double sum[6], double* sh) {
+                                          double sum[F], double* sh) {
   constexpr int R = kSumRows<GR>;
   const int g = threadIdx.x / R, r = threadIdx.x % R;
-  split_sums(P + static_cast<size_t>(g) * 6 * ld, ld, (S - g + GR - 1) / GR, i, sum, GR);
+  split_sums<F>(P + static_cast<size_t>(g) * F * ld, ld, (S - g + GR - 1) / GR, i, sum, GR);
   if (GR > 1) {
 #pragma unroll
-    for (int c = 0; c < 6; ++c) sh[(g * 6 + c) * R + r] = sum[c];
+    for (int c = 0; c < F; ++c) sh[(g * F + c) * R + r] = sum[c];
     __syncthreads();
     if (g == 0)
 #pragma unroll
       for (int q = 1; q < GR; ++q)
 #pragma unroll
-        for (int c = 0; c < 6; ++c) sum[c] += sh[(q * 6 + c) * R + r];
+        for (int c = 0; c < F; ++c) sum[c] += sh[(q * F + c) * R + r];
   }
 }
 
@@ -251,6 +283,8 @@ static __global__ void __launch_bounds__(kSumThreads)
                    double* __restrict__ X, double* __restrict__ V, double* __restrict__ D,
                    StepCtl* __restrict__ ctl, double eta) {
   __shared__ double sh[GR > 1 ? 6 * kSumThreads : 32];
+  grid_wait();
+  grid_release();
   const int i = blockIdx.x * kSumRows<GR> + threadIdx.x % kSumRows<GR>;
   double crit = __longlong_as_double(static_cast<long long>(kPosInfBits));
   const bool mine = i < n && threadIdx.x < kSumRows<GR>;
@@ -350,8 +384,12 @@ constexpr int kSumGroupSlots = 8;
 inline bool sum_in_groups(const RowSlots& s) { return s.S + s.nb / 2 >= kSumGroupSlots; }
 
 inline void launch_correct(cudaStream_t st, int n, int ld, RowSlots slots, const double* P,
-                           double* X, double* V, double* D, StepCtl* ctl, double eta) {
-  if (sum_in_groups(slots))
+                           double* X, double* V, double* D, StepCtl* ctl, double eta,
+                           bool chained = false) {
+  if (sum_in_groups(slots) && chained)
+    launch_chained(correct_kernel<8>, (n + kSumRows<8> - 1) / kSumRows<8>, kSumThreads, 0, st, n, ld,
+                   slots, P, X, V, D, ctl, eta);
+  else if (sum_in_groups(slots))
     correct_kernel<8><<<(n + kSumRows<8> - 1) / kSumRows<8>, kSumThreads, 0, st>>>(
         n, ld, slots, P, X, V, D, ctl, eta);
   else

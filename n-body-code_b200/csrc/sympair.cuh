@@ -32,6 +32,7 @@
 // CTA works through one after another over the same tiles, adding to the slots
 // it wrote itself; this bounds the slots (nb / 2 + S) whatever N is.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -98,6 +99,75 @@ struct SymRun {
   }
 };
 
+// ---- host side of the schedule --------------------------------------------
+
+// Blocks of a schedule: nb / 2 partial-sum slots, so at most 64 beside the
+// splits.  More blocks would need more slots (48 bytes per row each), fewer
+// would evaluate more of the pairs one-sided (1 / nb of them).
+constexpr int kMaxSymBlocks = 128;
+constexpr int kMaxSymSplits = 64;
+// Slots are further bounded by memory (8 GiB of P, at least 8 slots): larger
+// systems take fewer, larger blocks and fewer splits.
+inline int max_sym_slots(int n) {
+  const double fit = 8.0 * (1 << 30) / (48.0 * n);
+  return fit > 2 * kMaxSymSplits ? 2 * kMaxSymSplits : std::max(8, static_cast<int>(fit));
+}
+
+// The blocks of n bodies for a kernel whose CTAs hold `rows` rows.
+struct SymGrid {
+  int subs, block_rows, nb;
+  SymGrid(int rows, int n) {
+    const long most = static_cast<long>(std::min(kMaxSymBlocks, max_sym_slots(n))) * rows;
+    subs = static_cast<int>((n + most - 1) / most);
+    block_rows = subs * rows;
+    nb = (n + block_rows - 1) / block_rows;
+  }
+  RowSlots slots(int S) const { return RowSlots(S, block_rows, nb); }
+  int count(int S) const { return S + nb / 2; }
+};
+
+// Rate at which the corrector sums slots (104 slots at N = 65536: 327 MB in 84
+// us): the price of each partial a tiling leaves.
+constexpr double kSplitSumBytesPerMs = 3.9e9;
+
+// Splits of a symmetric kernel over n bodies: S CTAs per block share its run
+// of Q tiles, ceil(Q / S) each.  Cost in units of one (CTA, tile); per_ms:
+// interactions a full GPU evaluates per ms.  FP64 CTAs (waves) take the same
+// time each and run in waves, the last of which takes what its fullest SM
+// holds (three quarters of a tile's time are throughput).  The near/far
+// kernel's differ with their near subtiles: the work of more CTAs than are
+// resident spreads over the slots, and the last ones leave SMs idle for about
+// a third of a CTA's time.  Every split is another 48 bytes per row to sum.
+// Pair pass in ms by splits: FP64 N = 16384 0.464 (8) 0.39 (23) 0.405 (31),
+// 65536 5.79 (8) 5.69 (31); mixed 16384 0.265 (9) 0.223 (31), 65536 2.91 (9)
+// 2.77 (31).
+inline int sym_splits(int sms, int occ, int rows, int tj, int n, double per_ms, bool waves) {
+  const SymGrid g(rows, n);
+  const int Q = sym_q_count(g.nb, 0, g.block_rows / tj, (n + tj - 1) / tj);
+  const long slots = static_cast<long>(sms) * occ;
+  const double tile_ms = 2.0 * rows * tj * slots / per_ms;
+  const double per_split = 48.0 * n / kSplitSumBytesPerMs / tile_ms;
+  double best = 1e300;
+  int best_s = 1;
+  for (int tps = 1; tps <= Q; ++tps) {
+    const int s = (Q + tps - 1) / tps;
+    if (s > std::min(kMaxSymSplits, max_sym_slots(n) / 2)) continue;
+    const long ctas = static_cast<long>(g.nb) * s;
+    const double one = tps * g.subs + 0.5;
+    const bool in_waves = waves || ctas <= slots;
+    const long last = in_waves ? ctas % slots : 0;
+    const double per_sm = static_cast<double>((last + sms - 1) / sms) / occ;
+    double work = in_waves ? one * (ctas / slots) : one * ctas / slots;
+    if (last) work += one * (0.25 + 0.75 * per_sm);
+    const double cost = work + (waves ? 0.1 : 0.35) * one + per_split * s;
+    if (cost < best - 1e-9) {
+      best = cost;
+      best_s = s;
+    }
+  }
+  return best_s;
+}
+
 // ---------------------------------------------------------------------------
 // FP64
 // ---------------------------------------------------------------------------
@@ -156,6 +226,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
   const SymRun run(a, a.subs * (kRows / kSymTile64));
   const double eps2 = a.eps2;
   int half = 0;  // half of `red` of the current tile, alternating over the CTA's life
+  grid_wait();
   for (int g = 0; g < a.subs; ++g) {
     const int row0 = (run.I * a.subs + g) * kRows + warp * 32 * IPT;
     if ((run.I * a.subs + g) * kRows >= a.n) break;  // a short last block
@@ -224,6 +295,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
       half ^= 1;
     };
     if (!run.stream(pipe, jb, a.status, consume, post)) return;
+    if (g + 1 == a.subs) grid_release();
     double* out = a.out + static_cast<size_t>(blockIdx.y) * 6 * a.stride;
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
@@ -261,10 +333,12 @@ __global__ void __launch_bounds__(64)
     sym_tile_kernel(int n, SoA7 in, SymSub* __restrict__ out, int ld = 0, double* X = nullptr,
                     double* V = nullptr, const double* __restrict__ D = nullptr,
                     const StepCtl* __restrict__ ctl = nullptr,
-                    unsigned long long* near_count = nullptr) {
+                    unsigned long long* near_count = nullptr, double* __restrict__ XP = nullptr) {
   __shared__ double box[6][2];
   __shared__ float rmax[2];
   __shared__ SymSub stage;  // written out in one bulk copy
+  grid_wait();
+  grid_release();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int slot = blockIdx.x * 64 + tid;
   const bool valid = slot < n;
@@ -273,7 +347,7 @@ __global__ void __launch_bounds__(64)
   if (valid) {
     m = in.m[slot];
     if (PREDICT) {
-      predict_body(ctl->dt, ld, slot, X, V, D, p, u);
+      predict_body(ctl->dt, ld, slot, X, V, D, p, u, XP);
     } else {
       p[0] = in.x[slot]; p[1] = in.y[slot]; p[2] = in.z[slot];
       u[0] = in.vx[slot]; u[1] = in.vy[slot]; u[2] = in.vz[slot];
@@ -424,6 +498,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
   const uint64_t eps2 = f2_dup(e2), m3 = f2_dup(-3.0f);
   int half = 0;  // half of `red` of the current tile, alternating over the CTA's life
   int near_subs = 0;
+  grid_wait();
   for (int g = 0; g < a.subs; ++g) {
     const int row0 = (run.I * a.subs + g) * kRows + warp * 32 * IPT;
     if ((run.I * a.subs + g) * kRows >= a.n) break;  // a short last block
@@ -591,6 +666,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
       half ^= 1;
     };
     if (!run.stream(pipe, jt, a.status, consume, post)) return;
+    if (g + 1 == a.subs) grid_release();
     double* out = a.out + static_cast<size_t>(blockIdx.y) * 6 * a.stride;
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {

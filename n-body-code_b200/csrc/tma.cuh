@@ -99,6 +99,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return mbar_wait_for(bar, parity, kWaitLimitNs);
 }
 
+// Programmatic dependent launch.  A kernel launched with launch_chained
+// (hermite.cuh) may start before its predecessor on the stream has finished:
+// grid_wait returns once that has, its writes visible, and comes before the
+// kernel touches any memory others write; grid_release lets the successor be
+// scheduled.  Without such a launch both do nothing.  A kernel whose
+// predecessor waited so itself runs after everything earlier on the stream.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ void report_status(int* status, int code) {
   if (status) atomicCAS(status, kKernelOk, code);
 }

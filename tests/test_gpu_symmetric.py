@@ -160,3 +160,51 @@ def test_mixed_calls_on_the_callers_arrays(n):
     for d in (out.cpu().numpy(), nb.force_calculation(s, eps2=EPS2, precision="mixed")):
         ea = vec_rel(d[:3, rows][:, ok], ref[:3, ok])
         assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4, (n, np.median(ea), ea.max())
+
+
+def _vjp_rows(s, ab, jb, rows):
+    """d/d(x_k, v_k, m_k) of sum_i ab_i . acc_i + jb_i . jerk_i for the given
+    rows k, by autograd of the terms that contain body k (plain torch, FP64)."""
+    import torch
+    dev = "cuda"
+    X = torch.tensor(np.stack([s["x"], s["y"], s["z"]]), device=dev)
+    V = torch.tensor(np.stack([s["vx"], s["vy"], s["vz"]]), device=dev)
+    M = torch.tensor(s["m"], device=dev)
+    A, J = torch.tensor(ab, device=dev), torch.tensor(jb, device=dev)
+    k = torch.tensor(rows, device=dev)
+    x, v, m = (t[..., k].clone().requires_grad_() for t in (X, V, M))
+    d = X[:, None, :] - x[:, :, None]
+    u = V[:, None, :] - v[:, :, None]
+    s2 = (d * d).sum(0) + EPS2
+    q = s2 ** -1.5
+    q = torch.where(torch.arange(M.numel(), device=dev)[None, :] == k[:, None], torch.zeros_like(q), q)
+    c = -3.0 * (d * u).sum(0) / s2
+    own = ((A[:, k, None] * d).sum(0) + (J[:, k, None] * (u + c * d)).sum(0)) * q * M[None, :]
+    partner = -((A[:, None, :] * d).sum(0) + (J[:, None, :] * (u + c * d)).sum(0)) * q * m[:, None]
+    gx, gv, gm = torch.autograd.grad((own + partner).sum(), (x, v, m))
+    return gx.cpu().numpy(), gv.cpu().numpy(), gm.cpu().numpy()
+
+
+# blocks of 256 rows, odd and even counts, tiles of 32; blocks of two
+# sub-blocks from 32769.  Sums of n terms of relative error a few 2^-52: 1e-11
+# of each kind's largest value.
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 257, 513, 1000, 4097, 33001])
+def test_pair_vjp_edges(n):
+    import torch
+    s = bodies(n)
+    rng = np.random.default_rng(n)
+    ab, jb = rng.normal(size=(3, n)), rng.normal(size=(3, n))
+    t = {k: torch.tensor(v, device="cuda") for k, v in
+         dict(x=np.stack([s["x"], s["y"], s["z"]]), v=np.stack([s["vx"], s["vy"], s["vz"]]),
+              m=s["m"], a=ab, j=jb).items()}
+    gx, gv = torch.empty(3, n, dtype=torch.float64, device="cuda"), torch.empty(3, n, dtype=torch.float64, device="cuda")
+    gm = torch.empty(n, dtype=torch.float64, device="cuda")
+    adj = nb.Adjoint(n, EPS2, 1 / 256, 1, 1)
+    adj.vjp_acc_jerk(t["x"], t["v"], t["m"], t["a"], t["j"], gx, gv, gm,
+                     torch.cuda.current_stream().cuda_stream)
+    rows = np.arange(n) if n <= 1000 else np.unique(np.concatenate([np.arange(0, n, n // 100), [n - 2, n - 1]]))
+    for got, want in zip((gx, gv, gm), _vjp_rows(s, ab, jb, rows)):
+        got = got.cpu().numpy()
+        err = np.abs(got[..., rows] - want).max()
+        assert err <= 1e-11 * max(np.abs(want).max(), np.abs(got).max()) + (0.0 if n > 1 else 1e-300), (n, err)
+    adj.close()
