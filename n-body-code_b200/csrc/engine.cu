@@ -62,6 +62,9 @@ constexpr int kOrderBits = 48;     // Hilbert key width (order_key_kernel)
 // beyond the cell.
 constexpr int kDropInOrderLowBit = 18;
 constexpr int kMaxPotSplit = 32;    // j-splits of the potential diagnostic
+// Steps captured together: launching a graph costs the GPU about 2.5 us, which
+// a small system's step (three kernels, 20 us at N = 1024) notices.
+constexpr int kStepsPerGraph = 8;
 // Calls on caller-owned bodies order them for the near/far kernel from this
 // many bodies: ordering costs about 0.09 ms a call and saves the pair pass
 // 0.02 ms at N = 16384.
@@ -289,7 +292,11 @@ struct nbody_engine {
   int* status = nullptr;
   Tiling tiling;
   bool tiled = false;
-  cudaGraphExec_t graph = nullptr;
+  // The captured step.  Event-record nodes take about 3.6 us each, so only the
+  // last step of a call, whose phases nbody_get_timers reports, has them.
+  cudaGraphExec_t graph = nullptr;      // one step with its event records
+  cudaGraphExec_t plain = nullptr;      // one step
+  cudaGraphExec_t many = nullptr;       // kStepsPerGraph steps
   int graph_kernels = 0;  // kernel nodes of the captured step
   // automatic mixed kernel (pair_variant 0): bodies in Hilbert order from this
   // many, in the caller's below, where too few subtiles would be far to pay
@@ -397,6 +404,13 @@ int choose_sym_split(const nbody_engine* e, const PairKernel& k, int n) {
   return sym_splits(e->num_sms, occ, k.nt * k.ipt, k.tj, n, fp64 ? 7.6e8 : 1.6e9, fp64);
 }
 
+void drop_step_graphs(nbody_engine* e) {
+  for (cudaGraphExec_t* g : {&e->graph, &e->plain, &e->many}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
+}
+
 // Grows P to `split` slots.
 nbody_status ensure_partials(nbody_engine* e, int split) {
   if (split <= e->p_splits) return NBODY_OK;
@@ -404,10 +418,7 @@ nbody_status ensure_partials(nbody_engine* e, int split) {
     NB_CUDA(cudaStreamSynchronize(e->stream));
     cudaFree(e->P);
   }
-  if (e->graph) {  // the captured step refers to the old buffer
-    cudaGraphExecDestroy(e->graph);
-    e->graph = nullptr;
-  }
+  drop_step_graphs(e);  // the captured steps refer to the old buffer
   e->P = nullptr;
   e->p_splits = 0;
   NB_CUDA(cudaMalloc(&e->P, sizeof(double) * 6 * static_cast<size_t>(e->ld) * split));
@@ -842,10 +853,12 @@ int count_kernel_nodes(cudaGraph_t g) {
   return kernels;
 }
 
-nbody_status build_step_graph(nbody_engine* e) {
-  if (e->graph) return NBODY_OK;
+// Captures `steps` steps (timed: one, with its event records) into *out.
+nbody_status capture_steps(nbody_engine* e, int steps, bool timed, cudaGraphExec_t* out) {
+  if (*out) return NBODY_OK;
   NB_TRY(ensure_tiling(e));
-  if (!e->step_events) {
+  NB_TRY(prepare_kernel(*e->tiling.k));
+  if (timed && !e->step_events) {
     for (auto& ev : e->ev) NB_CUDA(cudaEventCreate(&ev));
     e->step_events = true;
   }
@@ -853,29 +866,41 @@ nbody_status build_step_graph(nbody_engine* e) {
   NB_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
   nbody_status s = NBODY_OK;
   auto rec = [&](cudaEvent_t ev) {
-    if (s == NBODY_OK && cudaEventRecordWithFlags(ev, e->stream, cudaEventRecordExternal) != cudaSuccess)
+    if (timed && s == NBODY_OK &&
+        cudaEventRecordWithFlags(ev, e->stream, cudaEventRecordExternal) != cudaSuccess)
       s = fail(NBODY_ERR_CUDA, "event record during capture failed");
   };
-  rec(e->ev[0]);
-  if (s == NBODY_OK) s = enqueue_predict(e, e->stream);
-  rec(e->ev[1]);
-  if (s == NBODY_OK) s = launch_pair(e, e->tiling, 0, e->n, e->stream);
-  rec(e->ev[2]);
-  if (s == NBODY_OK) s = enqueue_correct(e, e->stream);
-  rec(e->ev[3]);
+  for (int k = 0; k < steps && s == NBODY_OK; ++k) {
+    rec(e->ev[0]);
+    if (s == NBODY_OK) s = enqueue_predict(e, e->stream);
+    rec(e->ev[1]);
+    if (s == NBODY_OK) s = launch_pair(e, e->tiling, 0, e->n, e->stream);
+    rec(e->ev[2]);
+    if (s == NBODY_OK) s = enqueue_correct(e, e->stream);
+    rec(e->ev[3]);
+  }
   cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
   if (s != NBODY_OK) {
     if (g) cudaGraphDestroy(g);
     return s;
   }
   if (ce != cudaSuccess) return fail(NBODY_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
-  e->graph_kernels = count_kernel_nodes(g);
-  ce = cudaGraphInstantiate(&e->graph, g, 0);
+  if (timed) e->graph_kernels = count_kernel_nodes(g);
+  ce = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   if (ce != cudaSuccess) {
-    e->graph = nullptr;
+    *out = nullptr;
     return fail(NBODY_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ce));
   }
+  return NBODY_OK;
+}
+
+nbody_status build_step_graph(nbody_engine* e) {
+  if (e->graph) return NBODY_OK;
+  NB_TRY(capture_steps(e, 1, true, &e->graph));
+  cudaGraph_t g = nullptr;
+  nbody_status s = NBODY_OK;
+  cudaError_t ce = cudaSuccess;
   if (curve_resident(e) && !e->order_graph) {
     // the Hilbert re-ordering of the engine's own state, replayed every
     // sort_every steps ahead of the step graph
@@ -883,7 +908,6 @@ nbody_status build_step_graph(nbody_engine* e) {
     const int since = e->since_sort;
     NB_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     s = enqueue_reorder_state(e, e->stream);
-    g = nullptr;
     ce = cudaStreamEndCapture(e->stream, &g);
     e->sorted = sorted;  // capturing ran nothing
     e->permuted = permuted;
@@ -1029,6 +1053,11 @@ nbody_status nbody_create(nbody_engine** out, const nbody_config* cfg) {
     NB_CUDA(cudaMalloc(&e->partial, sizeof(double) * (ld / kBlockO1 * kMaxPotSplit + 8)));
     NB_CUDA(cudaMalloc(&e->status, sizeof(int)));
     NB_CUDA(cudaMemsetAsync(e->status, 0, sizeof(int), e->stream));
+    if (!explicit_shape(e->cfg) && e->cfg.tune == 0) {  // the slots of its own passes
+      Tiling t;
+      NB_TRY(get_tiling(e.get(), e->n, &t));
+      NB_TRY(ensure_partials(e.get(), partial_count(t, e->n)));
+    }
     NB_CUDA(cudaStreamSynchronize(e->stream));
     return NBODY_OK;
   }();
@@ -1041,7 +1070,7 @@ nbody_status nbody_destroy(nbody_engine* e) {
   if (!e) return NBODY_OK;
   cudaSetDevice(e->dev);
   if (e->stream) cudaStreamSynchronize(e->stream);
-  if (e->graph) cudaGraphExecDestroy(e->graph);
+  drop_step_graphs(e);
   if (e->order_graph) cudaGraphExecDestroy(e->order_graph);
   for (auto ev : e->aux_ev)
     if (ev) cudaEventDestroy(ev);
@@ -1174,9 +1203,24 @@ nbody_status nbody_step(nbody_engine* e, int nsteps) {
   if (nsteps < 0) return fail(NBODY_ERR_INVALID_ARG, "nsteps < 0");
   if (!e->have_derivs) NB_TRY(eval_current(e));
   NB_TRY(build_step_graph(e));
-  for (int k = 0; k < nsteps; ++k) {
-    NB_TRY(maybe_reorder(e, e->stream));
-    NB_CUDA(cudaGraphLaunch(e->graph, e->stream));
+  for (int k = 0; k < nsteps;) {
+    NB_TRY(maybe_reorder(e, e->stream));  // counts this step
+    // steps from here that need neither event records nor a re-ordering
+    int run = nsteps - 1 - k;
+    if (curve_resident(e)) run = std::min(run, 1 + sort_period(e) - e->since_sort);
+    if (run <= 0) {
+      NB_CUDA(cudaGraphLaunch(e->graph, e->stream));
+      ++k;
+    } else if (run >= kStepsPerGraph) {
+      NB_TRY(capture_steps(e, kStepsPerGraph, false, &e->many));
+      NB_CUDA(cudaGraphLaunch(e->many, e->stream));
+      if (curve_resident(e)) e->since_sort += kStepsPerGraph - 1;
+      k += kStepsPerGraph;
+    } else {
+      NB_TRY(capture_steps(e, 1, false, &e->plain));
+      NB_CUDA(cudaGraphLaunch(e->plain, e->stream));
+      ++k;
+    }
   }
   return NBODY_OK;
 }

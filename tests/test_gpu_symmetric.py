@@ -208,3 +208,25 @@ def test_pair_vjp_edges(n):
         err = np.abs(got[..., rows] - want).max()
         assert err <= 1e-11 * max(np.abs(want).max(), np.abs(got).max()) + (0.0 if n > 1 else 1e-300), (n, err)
     adj.close()
+
+
+@pytest.mark.parametrize("precision,kw", [("fp64", {}), ("mixed", {}), ("mixed", dict(pair_variant=4, sort_every=3)),
+                                          ("mixed", dict(pair_variant=4, sort_every=10))])
+def test_steps_of_one_call_equal_single_steps(precision, kw):
+    """A call's steps run from graphs of one and of eight steps, re-ordered
+    when due; the result, the step count and the number of re-orderings are
+    those of one call per step."""
+    s = bodies(1300)
+    args = dict(eps2=EPS2, dt=1 / 1024, precision=precision, **kw)
+    with nb.Engine(1300, **args) as a, nb.Engine(1300, **args) as b:
+        for e in (a, b):
+            e.set_state(s)
+            e.force_calculation()
+        for k in (1, 2, 9, 10, 25):
+            a.timestepping(k)
+            for _ in range(k):
+                b.timestepping(1)
+        sa, sb, ta, tb = a.get_state(), b.get_state(), a.timers(), b.timers()
+    assert all(np.array_equal(sa[k], sb[k]) for k in sa)
+    assert ta["steps"] == tb["steps"] == 47 and ta["t"] == tb["t"] and ta["reorders"] == tb["reorders"]
+    assert ta["pred_ms"] > 0 and ta["eval_ms"] > 0 and ta["corr_ms"] > 0
