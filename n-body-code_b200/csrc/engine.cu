@@ -42,6 +42,7 @@
 #include "../../include/nbody_cuda.h"
 #include "errors.h"
 #include "hermite.cuh"
+#include "hoststage.h"
 #include "pair.cuh"
 #include "reltiles.cuh"
 #include "sympair.cuh"
@@ -65,6 +66,16 @@ constexpr int kMaxPotSplit = 32;    // j-splits of the potential diagnostic
 // Steps captured together: launching a graph costs the GPU about 2.5 us, which
 // a small system's step (three kernels, 20 us at N = 1024) notices.
 constexpr int kStepsPerGraph = 8;
+// Up to these many bodies host arrays go through the engine's pinned staging
+// buffer, one copy each way.  A copy from or to pageable memory costs several
+// us whatever its size; above the limits the extra pass over the bytes costs
+// more (set_state at 16384 bodies 99 us staged, 92 direct, at 1024 33 and 70;
+// get_state at 65536 265 and 314, at 1024 26 and 92).  The drop-in downloads
+// field by field beside its sums from kDropInStageBodies on (30011: 1.55 ms
+// staged, 1.63 not; 65536: equal).
+constexpr int kStageInBodies = 16384;
+constexpr int kStageOutBodies = 65536;
+constexpr int kDropInStageBodies = 32768;
 // Calls on caller-owned bodies order them for the near/far kernel from this
 // many bodies: ordering costs about 0.09 ms a call and saves the pair pass
 // 0.02 ms at N = 16384.
@@ -290,6 +301,7 @@ struct nbody_engine {
   StepCtl* ctl = nullptr;
   double* partial = nullptr;  // reduction scratch: ld / 256 + 1 doubles + 4 scalars
   int* status = nullptr;
+  HostStage stage;  // host side of small transfers, idle between calls
   Tiling tiling;
   bool tiled = false;
   // The captured step.  Event-record nodes take about 3.6 us each, so only the
@@ -350,15 +362,54 @@ bool wants_order(const nbody_engine* e, int n, int min) {
 // The engine keeps its bodies in Hilbert order (positions != body indices).
 bool curve_resident(const nbody_engine* e);
 
-nbody_status check_status_word(nbody_engine* e) {
-  int h = 0;
-  NB_CUDA(cudaMemcpyAsync(&h, e->status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-  NB_CUDA(cudaStreamSynchronize(e->stream));
+nbody_status status_result(nbody_engine* e, int h) {
   if (h == kKernelTimeout) {
     cudaMemsetAsync(e->status, 0, sizeof(int), e->stream);
     return fail(NBODY_ERR_TIMEOUT, "a pair-kernel shared-memory wait exceeded its limit");
   }
   return NBODY_OK;
+}
+
+nbody_status check_status_word(nbody_engine* e) {
+  int h = 0;
+  NB_CUDA(cudaMemcpyAsync(&h, e->status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+  NB_CUDA(cudaStreamSynchronize(e->stream));
+  return status_result(e, h);
+}
+
+// The caller's seven arrays (state order: x, y, z, vx, vy, vz, m) into the
+// engine's state arrays; staged: one copy, padding rows zero.
+nbody_status upload_state(nbody_engine* e, const double* const src[7]) {
+  const size_t ld = e->ld, n = e->n;
+  if (e->n > kStageInBodies) {
+    for (int k = 0; k < 7; ++k)
+      NB_CUDA(cudaMemcpyAsync(e->state + k * ld, src[k], sizeof(double) * n, cudaMemcpyHostToDevice,
+                              e->stream));
+    return NBODY_OK;
+  }
+  NB_CUDA(e->stage.need(sizeof(double) * (7 * ld + 1)));
+  double* h = e->stage.doubles();
+  for (int k = 0; k < 7; ++k) {
+    memcpy(h + k * ld, src[k], sizeof(double) * n);
+    memset(h + k * ld + n, 0, sizeof(double) * (ld - n));
+  }
+  NB_CUDA(cudaMemcpyAsync(e->state, h, sizeof(double) * 7 * ld, cudaMemcpyHostToDevice, e->stream));
+  return NBODY_OK;
+}
+
+// `count` consecutive [ld] device arrays, rows [lo, hi), to dst (entries may be
+// null), with the status word: one wait.
+nbody_status stage_out(nbody_engine* e, const double* src, double* const* dst, int count, int lo, int hi) {
+  const size_t ld = e->ld;
+  NB_CUDA(e->stage.need(sizeof(double) * (count * ld + 1)));
+  double* h = e->stage.doubles();
+  int* status = reinterpret_cast<int*>(h + count * ld);
+  NB_CUDA(cudaMemcpyAsync(h, src, sizeof(double) * count * ld, cudaMemcpyDeviceToHost, e->stream));
+  NB_CUDA(cudaMemcpyAsync(status, e->status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+  NB_CUDA(cudaStreamSynchronize(e->stream));
+  for (int k = 0; k < count; ++k)
+    if (dst[k]) memcpy(dst[k] + lo, h + k * ld + lo, sizeof(double) * (hi - lo));
+  return status_result(e, *status);
 }
 
 // Split count from a wave model: CTAs = i_blocks * S run in waves of
@@ -1002,11 +1053,14 @@ nbody_status nbody_create(nbody_engine** out, const nbody_config* cfg) {
     return fail(NBODY_ERR_NO_DEVICE, "no CUDA device visible");
   if (cfg->device < 0 || cfg->device >= ndev)
     return fail(NBODY_ERR_INVALID_ARG, "device %d of %d", cfg->device, ndev);
-  cudaDeviceProp prop;
-  NB_CUDA(cudaGetDeviceProperties(&prop, cfg->device));
-  if (prop.major != 10)
+  // single attributes: cudaGetDeviceProperties takes 2.5 ms
+  int major = 0, minor = 0, sms = 0;
+  NB_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, cfg->device));
+  NB_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, cfg->device));
+  NB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device));
+  if (major != 10)
     return fail(NBODY_ERR_NO_DEVICE, "device %d is sm_%d%d; this library is built for sm_100a",
-                cfg->device, prop.major, prop.minor);
+                cfg->device, major, minor);
   NB_CUDA(cudaSetDevice(cfg->device));
 
   std::unique_ptr<nbody_engine> e(new nbody_engine);
@@ -1014,7 +1068,7 @@ nbody_status nbody_create(nbody_engine** out, const nbody_config* cfg) {
   e->n = cfg->n;
   e->ld = round_up(cfg->n, kPad);
   e->dev = cfg->device;
-  e->num_sms = prop.multiProcessorCount;
+  e->num_sms = sms;
   const size_t ld = e->ld;
   auto cleanup_on_fail = [&](nbody_status s) {
     nbody_destroy(e.release());
@@ -1107,10 +1161,8 @@ nbody_status nbody_set_state(nbody_engine* e, const double* x, const double* y, 
   const double* src[7] = {x, y, z, vx, vy, vz, m};
   for (auto p : src)
     if (!p) return fail(NBODY_ERR_INVALID_ARG, "null state array");
-  const size_t ld = e->ld, b = sizeof(double) * e->n;
-  double* dst[7] = {e->X, e->X + ld, e->X + 2 * ld, e->V, e->V + ld, e->V + 2 * ld, e->M};
-  for (int k = 0; k < 7; ++k)
-    NB_CUDA(cudaMemcpyAsync(dst[k], src[k], b, cudaMemcpyHostToDevice, e->stream));
+  const size_t ld = e->ld;
+  NB_TRY(upload_state(e, src));
   StepCtl c{};
   c.dt = e->cfg.dt > 0 ? e->cfg.dt : 0.0;
   c.t = 0.0;
@@ -1136,7 +1188,8 @@ nbody_status nbody_set_state(nbody_engine* e, const double* x, const double* y, 
 
 namespace {
 // Downloads `count` [ld] arrays starting at `src` (engine positions) to the
-// caller's arrays in body order: through scratch when the state is permuted.
+// caller's arrays in body order, through scratch when the state is permuted,
+// and checks the status word.
 nbody_status download_rows(nbody_engine* e, const double* src, double* const* dst, int count) {
   const size_t ld = e->ld, b = sizeof(double) * e->n;
   const double* from = src;
@@ -1146,10 +1199,11 @@ nbody_status download_rows(nbody_engine* e, const double* src, double* const* ds
     NB_CUDA(cudaGetLastError());
     from = e->scratch;
   }
+  if (e->n <= kStageOutBodies) return stage_out(e, from, dst, count, 0, e->n);
   for (int k = 0; k < count; ++k)
     if (dst[k]) NB_CUDA(cudaMemcpyAsync(dst[k], from + k * ld, b, cudaMemcpyDeviceToHost, e->stream));
   NB_CUDA(cudaStreamSynchronize(e->stream));
-  return NBODY_OK;
+  return check_status_word(e);
 }
 }  // namespace
 
@@ -1158,8 +1212,7 @@ nbody_status nbody_get_state(nbody_engine* e, double* x, double* y, double* z, d
   TraceRange trace_("nbody_get_state");
   NB_TRY(need_state(e));
   double* dst[6] = {x, y, z, vx, vy, vz};
-  NB_TRY(download_rows(e, e->X, dst, 6));  // X(3) and V(3) are consecutive state arrays
-  return check_status_word(e);
+  return download_rows(e, e->X, dst, 6);  // X(3) and V(3) are consecutive state arrays
 }
 
 nbody_status nbody_get_derivs(nbody_engine* e, double* ax, double* ay, double* az, double* jx,
@@ -1167,8 +1220,7 @@ nbody_status nbody_get_derivs(nbody_engine* e, double* ax, double* ay, double* a
   NB_TRY(need_state(e));
   if (!e->have_derivs) return fail(NBODY_ERR_STATE, "no derivatives yet (call nbody_acc_jerk)");
   double* dst[6] = {ax, ay, az, jx, jy, jz};
-  NB_TRY(download_rows(e, e->D, dst, 6));
-  return check_status_word(e);
+  return download_rows(e, e->D, dst, 6);
 }
 
 nbody_status nbody_acc_jerk(nbody_engine* e) {
@@ -1466,12 +1518,28 @@ extern "C" nbody_status nbody_force_calculation(int n, double eps2, int precisio
   // order (the near/far kernel evaluates all rows in Hilbert order)
   if (!full && tile_relative(t.k->fmt)) NB_TRY(hilo_tiling(e, i_end - i_begin, &t));
   NB_TRY(ensure_partials(e, partial_count(t, n)));
+  const bool order = tile_relative(t.k->fmt) && wants_order(e, n, kForeignOrderMin);
+  if (n <= kDropInStageBodies && !order) {
+    double* out[6] = {ax, ay, az, jx, jy, jz};
+    NB_TRY(upload_state(e, src));
+    NB_TRY(launch_pack(e, n, own_inputs(e), e->stream, t.k->fmt, t.k->tj));
+    NB_TRY(launch_pair(e, t, i_begin, i_end, e->stream));
+    if (i_end > i_begin) {
+      launch_reduce(e->stream, i_begin, i_end, e->ld, row_slots(t, n), e->P, own_derivs(e));
+      NB_CUDA(cudaGetLastError());
+    }
+    for (double* o : out) {  // while the GPU works
+      memset(o, 0, sizeof(double) * i_begin);
+      memset(o + i_end, 0, sizeof(double) * (n - i_end));
+    }
+    return stage_out(e, e->D, out, 6, i_begin, i_end);
+  }
   if (!e->aux) {
     NB_CUDA(cudaStreamCreateWithFlags(&e->aux, cudaStreamNonBlocking));
     for (auto& ev : e->aux_ev) NB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
   const int* index = nullptr;  // row -> output position (the near/far rows are in Hilbert order)
-  if (tile_relative(t.k->fmt) && wants_order(e, n, kForeignOrderMin)) {
+  if (order) {
     // positions first: their Hilbert ordering runs while the masses and
     // velocities upload on a second stream
     NB_CUDA(cudaEventRecord(e->aux_ev[0], e->stream));

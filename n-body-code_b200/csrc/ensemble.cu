@@ -112,6 +112,29 @@ __global__ void ens_predict_kernel(int L, const int* __restrict__ cid,
   if (jbx) jbx[r] = make_jbx2(p[0], p[1], p[2], m, u[0], u[1], u[2]);
 }
 
+// Between the caller's concatenated arrays ([count][total]) and the padded
+// ones ([count][L]): idx[row] is a padded row's index in the caller's order, -1
+// on padding.  One launch instead of a copy per cluster and array.
+__global__ void ens_expand_kernel(int L, int total, int count, const int* __restrict__ idx,
+                                  const double* __restrict__ src, double* __restrict__ dst) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= L) return;
+  const int o = idx[r];
+  for (int k = 0; k < count; ++k)
+    dst[static_cast<size_t>(k) * L + r] = o >= 0 ? src[static_cast<size_t>(k) * total + o] : 0.0;
+}
+// perm (nullable): row r holds the body of padded row perm[r].
+__global__ void ens_compact_kernel(int L, int total, int count, const int* __restrict__ idx,
+                                   const int* __restrict__ perm, const double* __restrict__ src,
+                                   double* __restrict__ dst) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= L) return;
+  const int o = idx[perm ? perm[r] : r];
+  if (o < 0) return;
+  for (int k = 0; k < count; ++k)
+    dst[static_cast<size_t>(k) * total + o] = src[static_cast<size_t>(k) * L + r];
+}
+
 // bbox[c*6 + k]: min (k < 3) / max of cluster c's positions (one CTA each).
 __global__ void __launch_bounds__(kBlock) ens_bbox_kernel(const ClusterDev* __restrict__ cl,
                                                          const double* __restrict__ X, int L,
@@ -328,6 +351,9 @@ struct nbody_ensemble {
   JBody64* jb64 = nullptr;
   JBodyX2* jbx = nullptr;
   int* cid = nullptr;
+  int* idx = nullptr;    // [L] padded row -> index in the caller's arrays, -1 on padding
+  double* io = nullptr;  // [7][total] the caller's arrays on their way in or out
+  int total = 0;         // bodies
   ClusterDev* cl = nullptr;
   EnsItem* items = nullptr;
   int n_items = 0;
@@ -486,29 +512,15 @@ nbody_status ens_tiles(nbody_ensemble* e, cudaStream_t st) {
 }
 
 // Copies `count` [L] arrays starting at src to the caller's concatenated
-// arrays (cluster c's n_c bodies in turn), through scratch when permuted.
+// arrays (cluster c's n_c bodies in turn).
 nbody_status ens_download(nbody_ensemble* e, const double* src, double* const* dst, int count) {
-  const size_t L = e->L;
-  const double* from = src;
-  if (e->permuted) {
-    GatherArgs g;
-    g.arrays = count;
-    for (int a = 0; a < count; ++a) {
-      g.src[a] = src + a * L;
-      g.dst[a] = e->scratch + a * L;
-    }
-    scatter_rows_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(e->L, e->perm, g);
-    EN_CUDA(cudaGetLastError());
-    from = e->scratch;
-  }
-  long long off = 0;
-  for (int c = 0; c < e->C; ++c) {
-    for (int k = 0; k < count; ++k)
-      if (dst[k])
-        EN_CUDA(cudaMemcpyAsync(dst[k] + off, from + k * L + e->row0[c], sizeof(double) * e->n[c],
-                                cudaMemcpyDeviceToHost, e->stream));
-    off += e->n[c];
-  }
+  ens_compact_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(
+      e->L, e->total, count, e->idx, e->permuted ? e->perm : nullptr, src, e->io);
+  EN_CUDA(cudaGetLastError());
+  const size_t n = e->total;
+  for (int k = 0; k < count; ++k)
+    if (dst[k])
+      EN_CUDA(cudaMemcpyAsync(dst[k], e->io + k * n, sizeof(double) * n, cudaMemcpyDeviceToHost, e->stream));
   EN_CUDA(cudaStreamSynchronize(e->stream));
   return NBODY_OK;
 }
@@ -678,7 +690,7 @@ nbody_status nbody_ensemble_destroy(nbody_ensemble* e) {
     if (ev) cudaEventDestroy(ev);
   void* bufs[] = {e->state, e->P, e->jb64, e->jbx, e->cid, e->cl, e->items, e->counter,
                   e->status, e->blk_cluster, e->blk_row, e->phi, e->Tc, e->Uc,
-                  e->seg, e->bbox, e->sort_keys, e->sort_idx, e->sort_tmp, e->perm, e->scratch};
+                  e->idx, e->io, e->seg, e->bbox, e->sort_keys, e->sort_idx, e->sort_tmp, e->perm, e->scratch};
   for (void* p : bufs) cudaFree(p);
   if (e->stream) cudaStreamDestroy(e->stream);
   delete e;
@@ -745,13 +757,16 @@ nbody_status nbody_ensemble_create(nbody_ensemble** out, const nbody_ensemble_co
   e->n.assign(cfg->n, cfg->n + C);
   e->eps2.assign(cfg->eps2, cfg->eps2 + C);
   e->dt.assign(cfg->dt, cfg->dt + C);
-  std::vector<int> cid(e->L, -1), seg(e->L, 0), blk_cluster, blk_row;
+  std::vector<int> cid(e->L, -1), idx(e->L, -1), seg(e->L, 0), blk_cluster, blk_row;
   int r0 = 0;
   for (int c = 0; c < C; ++c) {
     const int ld = (e->n[c] + kPadRows - 1) / kPadRows * kPadRows;
     e->row0.push_back(r0);
     e->ld.push_back(ld);
-    for (int i = 0; i < e->n[c]; ++i) cid[r0 + i] = c;
+    for (int i = 0; i < e->n[c]; ++i) {
+      cid[r0 + i] = c;
+      idx[r0 + i] = e->total++;
+    }
     for (int i = 0; i < ld; ++i) seg[r0 + i] = c;
     for (int b = 0; b < ld; b += kPadRows) {
       blk_cluster.push_back(c);
@@ -776,6 +791,9 @@ nbody_status nbody_ensemble_create(nbody_ensemble** out, const nbody_ensemble_co
     if (raw->precision == NBODY_MIXED) EN_CUDA(cudaMalloc(&raw->jbx, sizeof(JBodyNF) * (Ls / 64) * 65));
     EN_CUDA(cudaMalloc(&raw->cid, sizeof(int) * Ls));
     EN_CUDA(cudaMemcpy(raw->cid, cid.data(), sizeof(int) * Ls, cudaMemcpyHostToDevice));
+    EN_CUDA(cudaMalloc(&raw->idx, sizeof(int) * Ls));
+    EN_CUDA(cudaMemcpy(raw->idx, idx.data(), sizeof(int) * Ls, cudaMemcpyHostToDevice));
+    EN_CUDA(cudaMalloc(&raw->io, sizeof(double) * 7 * raw->total));
     EN_CUDA(cudaMalloc(&raw->cl, sizeof(ClusterDev) * raw->C));
     EN_CUDA(cudaMalloc(&raw->counter, sizeof(unsigned int)));
     EN_CUDA(cudaMalloc(&raw->status, sizeof(int)));
@@ -829,14 +847,12 @@ nbody_status nbody_ensemble_set_state(nbody_ensemble* e, const double* x, const 
   for (auto p : src)
     if (!p) return nbody_set_error(NBODY_ERR_INVALID_ARG, "null state array");
   const size_t L = e->L;
-  double* dst[7] = {e->X, e->X + L, e->X + 2 * L, e->V, e->V + L, e->V + 2 * L, e->M};
-  long long off = 0;
-  for (int c = 0; c < e->C; ++c) {
-    for (int k = 0; k < 7; ++k)
-      EN_CUDA(cudaMemcpyAsync(dst[k] + e->row0[c], src[k] + off, sizeof(double) * e->n[c],
-                              cudaMemcpyHostToDevice, e->stream));
-    off += e->n[c];
-  }
+  const size_t n = e->total;
+  for (int k = 0; k < 7; ++k)  // state order: x, y, z, vx, vy, vz, m
+    EN_CUDA(cudaMemcpyAsync(e->io + k * n, src[k], sizeof(double) * n, cudaMemcpyHostToDevice, e->stream));
+  ens_expand_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(e->L, e->total, 7, e->idx,
+                                                                          e->io, e->state);
+  EN_CUDA(cudaGetLastError());
   EN_CUDA(cudaMemsetAsync(e->D, 0, sizeof(double) * 6 * L, e->stream));
   if (e->perm) {  // the caller's order again; re-ordered before the next evaluation
     iota_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(e->L, e->perm);
