@@ -62,7 +62,6 @@ constexpr int kOrderBits = 48;     // Hilbert key width (order_key_kernel)
 // that share a cell keep their input order, which moves no tile boundary
 // beyond the cell.
 constexpr int kDropInOrderLowBit = 18;
-constexpr int kMaxPotSplit = 32;    // j-splits of the potential diagnostic
 // Steps captured together: launching a graph costs the GPU about 2.5 us, which
 // a small system's step (three kernels, 20 us at N = 1024) notices.
 constexpr int kStepsPerGraph = 8;
@@ -299,7 +298,7 @@ struct nbody_engine {
   bool permuted = false;          // perm is not the identity
   int since_sort = 0;             // steps since the last re-ordering
   StepCtl* ctl = nullptr;
-  double* partial = nullptr;  // reduction scratch: ld / 256 + 1 doubles + 4 scalars
+  double* partial = nullptr;  // energy: kinetic and potential partials, two sums
   int* status = nullptr;
   HostStage stage;  // host side of small transfers, idle between calls
   Tiling tiling;
@@ -979,6 +978,25 @@ nbody_status build_step_graph(nbody_engine* e) {
   return NBODY_OK;
 }
 
+// The potential kernels: four rows per thread and tiles of 128 from 16384
+// bodies, two rows and tiles of 64 below.
+constexpr int kPotWarps = 4;
+struct PotKernel {
+  const void* fn;
+  int rows, tj;
+  size_t smem;
+};
+template <int COMPAT, int IPT, int TJ>
+PotKernel make_pot() {
+  return {reinterpret_cast<const void*>(&potential_sym_kernel<COMPAT, IPT, kPotWarps, TJ>),
+          32 * IPT * kPotWarps, TJ, 2 * TJ * sizeof(JBody64)};
+}
+const PotKernel& pot_kernel(bool compat, bool wide) {
+  static const PotKernel k[2][2] = {{make_pot<0, 2, 64>(), make_pot<0, 4, 128>()},
+                                    {make_pot<1, 2, 64>(), make_pot<1, 4, 128>()}};
+  return k[compat][wide];
+}
+
 nbody_status check_engine(nbody_engine* e) {
   if (!e) return fail(NBODY_ERR_INVALID_ARG, "null engine");
   if (cudaSetDevice(e->dev) != cudaSuccess) return fail(NBODY_ERR_CUDA, "cudaSetDevice(%d) failed", e->dev);
@@ -1104,7 +1122,7 @@ nbody_status nbody_create(nbody_engine** out, const nbody_config* cfg) {
       NB_CUDA(cudaMalloc(&e->sort_tmp, std::max<size_t>(e->sort_tmp_bytes, 16)));
     }
     NB_CUDA(cudaMalloc(&e->ctl, sizeof(StepCtl)));
-    NB_CUDA(cudaMalloc(&e->partial, sizeof(double) * (ld / kBlockO1 * kMaxPotSplit + 8)));
+    NB_CUDA(cudaMalloc(&e->partial, sizeof(double) * (ld / kBlockO1 + kMaxSymBlocks * kMaxSymSplits + 2)));
     NB_CUDA(cudaMalloc(&e->status, sizeof(int)));
     NB_CUDA(cudaMemsetAsync(e->status, 0, sizeof(int), e->stream));
     if (!explicit_shape(e->cfg) && e->cfg.tune == 0) {  // the slots of its own passes
@@ -1287,21 +1305,35 @@ nbody_status nbody_energy(nbody_engine* e, int ref_compat, double* T, double* U)
   TraceRange trace_("nbody_energy");
   NB_TRY(need_state(e));
   const int nb = e->ld / kBlockO1;
-  // j-splits of the potential: about 8 CTAs per SM in all
-  const int ps = std::max(1, std::min({kMaxPotSplit, nb, (8 * e->num_sms + nb - 1) / nb}));
-  double* scal = e->partial + nb * kMaxPotSplit;  // two result slots after the partials
-  kinetic_kernel<<<nb, kBlockO1, 0, e->stream>>>(e->n, e->ld, e->V, e->M, e->partial);
-  sum_partials_kernel<<<1, 256, 0, e->stream>>>(nb, e->partial, scal);
-  pack_kernel<<<nb, kBlockO1, 0, e->stream>>>(e->n, e->ld, own_inputs(e), e->jbe, nullptr, nullptr);
-  potential_kernel<kBlockO1><<<dim3(nb, ps), kBlockO1, 0, e->stream>>>(
-      e->n, e->ld, e->cfg.eps2, ref_compat ? 1 : 0, e->jbe, e->partial);
-  sum_partials_kernel<<<1, 256, 0, e->stream>>>(nb * ps, e->partial, scal + 1);
+  double* pot = e->partial + nb;  // after the kinetic partials
+  double* scal = pot + kMaxSymBlocks * kMaxSymSplits;
+  energy_pack_kernel<<<nb, kBlockO1, 0, e->stream>>>(e->n, e->ld, own_inputs(e), e->jbe, e->partial);
+  const PotKernel& k = pot_kernel(ref_compat != 0, e->n >= 16384);
+  SymArgs a{};
+  const SymGrid g(k.rows, e->n);
+  a.n = e->n;
+  a.ld = e->ld;
+  a.nb = g.nb;
+  a.subs = g.subs;
+  a.tiles = (e->n + k.tj - 1) / k.tj;
+  int occ = 0;
+  NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, 32 * kPotWarps, k.smem));
+  a.S = sym_splits(e->num_sms, std::max(1, occ), k.rows, k.tj, e->n, 2.4e9, true);
+  a.eps2 = e->cfg.eps2;
+  a.status = e->status;
+  const void* jb = e->jbe;
+  void* args[] = {static_cast<void*>(&jb), static_cast<void*>(&a), static_cast<void*>(&pot)};
+  NB_CUDA(cudaLaunchKernel(k.fn, dim3(g.nb, a.S), dim3(32 * kPotWarps), args, k.smem, e->stream));
+  sum_partials_kernel<<<2, 256, 0, e->stream>>>(nb, e->partial, g.nb * a.S, pot, scal);
   NB_CUDA(cudaGetLastError());
   double h[2];
+  int status = 0;
   NB_CUDA(cudaMemcpyAsync(h, scal, sizeof h, cudaMemcpyDeviceToHost, e->stream));
+  NB_CUDA(cudaMemcpyAsync(&status, e->status, sizeof status, cudaMemcpyDeviceToHost, e->stream));
   NB_CUDA(cudaStreamSynchronize(e->stream));
+  NB_TRY(status_result(e, status));
   const double t = h[0];
-  const double u = ref_compat ? -h[1] : -0.5 * h[1];
+  const double u = -h[1];
   if (T) *T = t;
   if (U) *U = u;
   if (!std::isfinite(t) || !std::isfinite(u))

@@ -432,74 +432,35 @@ static __global__ void initialdt_kernel(int n, int ld, const double* __restrict_
   finish_criterion(ctl, crit, false, sh);
 }
 
-// Per-CTA partial of 0.5 m v^2.
-static __global__ void kinetic_kernel(int n, int ld, const double* __restrict__ V,
-                               const double* __restrict__ M, double* __restrict__ partial) {
+// FP64 records of the energy diagnostic (rows [0, ld), padding zero) and per-CTA
+// partials of 0.5 m v^2.
+static __global__ void energy_pack_kernel(int n, int ld, SoA7 in, JBody64* __restrict__ jb,
+                                          double* __restrict__ partial) {
   __shared__ double sh[32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double e = 0.0;
   if (i < n) {
-    const double u = V[i], v = V[ld + i], w = V[2 * ld + i];
-    e = 0.5 * M[i] * (u * u + v * v + w * w);
+    const double m = in.m[i], u = in.vx[i], v = in.vy[i], w = in.vz[i];
+    e = 0.5 * m * (u * u + v * v + w * w);
+    store_jb64(jb, i, in.x[i], in.y[i], in.z[i], m, u, v, w);
+  } else if (i < ld) {
+    store_jb64(jb, i, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
   }
   const double b = block_sum(e, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = b;
 }
 
-// Potential: per row i, phi_i = sum_{j != i} m_j / sqrt(r^2 + eps2)
-// (mode 0; CTA partial of m_i phi_i) or psi_i = sum_{j < i} 1/sqrt(.)
-// (mode 1, the reference's printed potential sum_i sum_{j>i} m_j^2/r_ij
-// regrouped by j; CTA partial of m_i^2 psi_i).  FP64, j-tiles staged
-// through shared memory by the CTA's threads.  The j-range is split over
-// gridDim.y (CTA (x, y) takes tiles [y*tps, (y+1)*tps)), so a system of few
-// row blocks still fills the GPU; partial[y*gridDim.x + x] holds each CTA's
-// sum and sum_partials_kernel adds them in that fixed order.
-template <int NT>
-static __global__ void __launch_bounds__(NT) potential_kernel(int n, int ld, double eps2, int mode,
-                                                       const JBody64* __restrict__ jb,
-                                                       double* __restrict__ partial) {
-  __shared__ double4 tile[NT];
+// out[b] = the sum of count[b] partials, in a fixed order (CTA b of two).
+static __global__ void sum_partials_kernel(int count0, const double* __restrict__ partial0, int count1,
+                                           const double* __restrict__ partial1,
+                                           double* __restrict__ out) {
   __shared__ double sh[32];
-  const int i = blockIdx.x * NT + threadIdx.x;
-  const double2* pi = jb64_at(jb, min(i, ld - 1));
-  const double2 pi0 = pi[0], pi1 = pi[32];
-  const double4 bi = make_double4(pi0.x, pi0.y, pi1.x, pi1.y);
-  const int tiles = ld / NT, tps = (tiles + gridDim.y - 1) / gridDim.y;
-  const int jb0 = blockIdx.y * tps * NT, jb1 = min(ld, (blockIdx.y + 1) * tps * NT);
-  // four accumulators (partner k adds into acc[k % 4]), combined in a fixed
-  // order: four independent add chains instead of one
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int j0 = jb0; j0 < jb1; j0 += NT) {
-    const double2* pj = jb64_at(jb, j0 + threadIdx.x);
-    const double2 pj0 = pj[0], pj1 = pj[32];
-    tile[threadIdx.x] = make_double4(pj0.x, pj0.y, pj1.x, pj1.y);
-    __syncthreads();
-#pragma unroll 4
-    for (int k = 0; k < NT; ++k) {
-      const double4 p = tile[k];
-      const int j = j0 + k;
-      const double dx = p.x - bi.x, dy = p.y - bi.y, dz = p.z - bi.z;
-      const double y = rsqrt_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
-      const bool take = mode == 0 ? (j != i) : (j < i);
-      acc[k & 3] += take ? (mode == 0 ? p.w * y : y) : 0.0;
-    }
-    __syncthreads();
-  }
-  const double phi = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-  double e = 0.0;
-  if (i < n) e = mode == 0 ? bi.w * phi : bi.w * bi.w * phi;
-  const double b = block_sum(e, sh);
-  if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = b;
-}
-
-// Sums `count` partials in a fixed order (one CTA).
-static __global__ void sum_partials_kernel(int count, const double* __restrict__ partial,
-                                    double* __restrict__ out) {
-  __shared__ double sh[32];
+  const int count = blockIdx.x ? count1 : count0;
+  const double* p = blockIdx.x ? partial1 : partial0;
   double v = 0.0;
-  for (int k = threadIdx.x; k < count; k += blockDim.x) v += partial[k];
+  for (int k = threadIdx.x; k < count; k += blockDim.x) v += p[k];
   const double b = block_sum(v, sh);
-  if (threadIdx.x == 0) *out = b;
+  if (threadIdx.x == 0) out[blockIdx.x] = b;
 }
 
 }  // namespace nbody

@@ -308,6 +308,89 @@ __global__ void __launch_bounds__(32 * W, MINB)
 }
 
 // ---------------------------------------------------------------------------
+// Potential energy (FP64)
+// ---------------------------------------------------------------------------
+// partial[y * gridDim.x + x]: the CTA's sum over its unordered pairs (i, j) of
+// m_i m_j / sqrt(r^2 + eps2) (COMPAT = 0) or, the reference's printed potential,
+// m_k^2 / sqrt(.) with k the later of the two (COMPAT = 1).  Only the total is
+// wanted, so the pair goes to the row's sum alone and nothing rotates: rows in
+// registers, bodies of TJ-body tiles broadcast from shared memory, 12 FP64
+// operations per pair (the one-sided form spent them on each ordered pair: N =
+// 32768 1.23 ms).  Off its own block a tile lies wholly after or before the
+// rows, so COMPAT's later body is the same side for a whole tile.
+template <int COMPAT, int IPT, int W, int TJ>
+__global__ void __launch_bounds__(32 * W)
+    potential_sym_kernel(const JBody64* __restrict__ jb, SymArgs a, double* __restrict__ partial) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ uint64_t full[2];
+  __shared__ double sh[32];
+  constexpr int kRows = 32 * IPT * W;
+  static_assert(kRows % TJ == 0 && TJ % 32 == 0, "blocks are whole tiles of whole groups");
+  TilePipe<JBody64, TJ> pipe;
+  pipe.init(reinterpret_cast<JBody64*>(smem_raw), full);
+  const SymRun run(a, a.subs * (kRows / TJ));
+  const double eps2 = a.eps2;
+  double total = 0.0;
+  for (int g = 0; g < a.subs; ++g) {
+    const int row0 = (run.I * a.subs + g) * kRows + threadIdx.x;  // rows row0 + k * 32 W
+    if (row0 - static_cast<int>(threadIdx.x) >= a.n) break;
+    double xi[IPT], yi[IPT], zi[IPT], mi[IPT], after[IPT], before[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+      const int r = row0 + 32 * W * k;
+      double2 p0{0, 0}, p1{0, 0};
+      if (r < a.ld) {
+        const double2* p = jb64_at(jb, r);
+        p0 = p[0];
+        p1 = p[32];
+      }
+      xi[k] = p0.x; yi[k] = p0.y; zi[k] = p1.x; mi[k] = p1.y;
+      after[k] = before[k] = 0.0;
+    }
+    int t = 0;
+    auto consume = [&](const JBody64* tile) {
+      const int tt = run.tile(t);
+      const bool own = run.distance(tt) == 0;
+      const int j0 = tt * TJ;
+      auto pair = [&](int j, auto&& add) {
+        const double2* p = jb64_at(tile, j);
+        const double2 p0 = p[0], p1 = p[32];
+#pragma unroll
+        for (int k = 0; k < IPT; ++k) {
+          const double dx = p0.x - xi[k], dy = p0.y - yi[k], dz = p1.x - zi[k];
+          add(k, p1.y, rsqrt_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)))));
+        }
+      };
+      if (own) {  // each pair from its later row; padding bodies have no mass
+#pragma unroll 2
+        for (int j = 0; j < TJ; ++j)
+          pair(j, [&](int k, double m, double y) {
+            const bool take = j0 + j < row0 + 32 * W * k;
+            if (COMPAT) before[k] += take ? y : 0.0;
+            else after[k] = fma(take ? m : 0.0, y, after[k]);
+          });
+      } else if (COMPAT && j0 < run.I * a.subs * kRows) {  // the row is the later body
+#pragma unroll 2
+        for (int j = 0; j < TJ; ++j)
+          pair(j, [&](int k, double, double y) { before[k] += y; });
+      } else {
+#pragma unroll 2
+        for (int j = 0; j < TJ; ++j)
+          pair(j, [&](int k, double m, double y) {
+            after[k] = fma(COMPAT ? m * m : m, y, after[k]);
+          });
+      }
+    };
+    if (!run.stream(pipe, jb, a.status, consume, [&] { ++t; })) return;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k)
+      total += COMPAT ? fma(mi[k] * mi[k], before[k], after[k]) : mi[k] * after[k];
+  }
+  const double b = block_sum(total, sh);
+  if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = b;
+}
+
+// ---------------------------------------------------------------------------
 // Mixed precision, near/far tile-relative
 // ---------------------------------------------------------------------------
 // Subtile of 64 bodies.  Header: centre c, radius R >= max |x_j - c|, bounding

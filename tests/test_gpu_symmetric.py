@@ -230,3 +230,20 @@ def test_steps_of_one_call_equal_single_steps(precision, kw):
     assert all(np.array_equal(sa[k], sb[k]) for k in sa)
     assert ta["steps"] == tb["steps"] == 47 and ta["t"] == tb["t"] and ta["reorders"] == tb["reorders"]
     assert ta["pred_ms"] > 0 and ta["eval_ms"] > 0 and ta["corr_ms"] > 0
+
+
+# blocks of 256 rows with tiles of 64, of 512 rows with tiles of 128 (from
+# 16384), odd and even counts.  A sum of positive terms of relative error a few
+# 2^-52: 1e-12.
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 255, 257, 513, 1024, 4097, 16383, 16384, 20001])
+def test_energy_edges(n):
+    s = bodies(n)
+    with nb.Engine(n, eps2=EPS2, dt=1.0) as e:
+        e.set_state(s)
+        T, U = e.energy()
+        _, Uc = e.energy(ref_compat=True)
+    kin = 0.5 * (s["m"] * (s["vx"] ** 2 + s["vy"] ** 2 + s["vz"] ** 2)).sum()
+    assert abs(T - kin) <= 1e-12 * kin
+    for got, compat in ((U, False), (Uc, True)):
+        want = O.potential(s, EPS2, compat=compat) if n > 1 else 0.0
+        assert abs(got - want) <= 1e-12 * abs(want), (n, compat, got, want)
