@@ -6,21 +6,24 @@
 // clusters and padding rows are zero-mass bodies that add nothing.  A row's
 // cluster comes from cid[row] (-1 on padding rows).
 //
-// Work list: item = (cluster, 256-row block, j-tile range of at most
-// `tiles_per_item` tiles).  Items are sorted by cost (longest first) and a
-// fixed grid of SMs x resident CTAs takes them from an atomic counter, so a
-// 256-body cluster and an 8192-body cluster share one launch without the
-// small one idling the GPU.  Split partial sums of cluster c live at
-// P + p_off_c ([S_c][6][ld_c]) and are added in a fixed order by the
-// corrector, so results are bitwise reproducible.
+// Work list: item = (cluster, 256-row block, range of at most `tiles_per_item`
+// j-tiles; in the symmetric schedule, sympair.cuh, of the block's run).  Items are sorted by cost (longest first) and a fixed grid of
+// SMs x resident CTAs takes them from an atomic counter, so a 256-body cluster
+// and an 8192-body cluster share one launch without the small one idling the
+// GPU.  The partial-sum slots of cluster c live at P + p_off_c ([slot][6][ld_c])
+// and are added in a fixed order by the corrector, so results are bitwise
+// reproducible.
 //
-// A step is memset(counter) -> predict -> persistent pair -> correct,
-// captured once into a CUDA graph.  Mixed ensembles use the near/far
-// tile-relative kernel (pair.cuh RowsMixedNF): each cluster keeps its bodies
-// in Hilbert order within its own padded segment (every sort_every steps a
-// second captured graph sorts (cluster, Hilbert code) keys over all rows and
-// gathers the state into that order; perm maps positions back to the
-// caller's rows), and the j-tile records are rebuilt right after predict.
+// A step is memset(counter) -> predict -> persistent pair -> correct, captured
+// into a CUDA graph; only the last step of a call carries the event records of
+// last_step_ms (about 3.6 us each).  FP64 ensembles and pair_variant 4 run the
+// symmetric kernels, mixed ones by default (and pair_variant 3) the one-sided
+// packed hi/lo kernel, pair_variant 5 the one-sided near/far kernel with every
+// tile taken as far.  pair_variant 4 and 5 use tile-relative records: each
+// cluster then keeps its bodies in Hilbert order within its own padded segment (every
+// sort_every steps a second captured graph sorts (cluster, Hilbert code) keys
+// over all rows and gathers the state into that order; perm maps positions
+// back to the caller's rows).
 // Each cluster has its own softening and fixed shared step (the adaptive
 // criterion is per system in the reference, src/nbody.cpp:198-222; ensembles
 // here run fixed steps).
@@ -42,17 +45,27 @@
 #include "hermite.cuh"
 #include "pair.cuh"
 #include "reltiles.cuh"
+#include "sympair.cuh"
 #include "trace.h"
 
 using namespace nbody;
 
 namespace {
 
-constexpr int kPadRows = 256;  // cluster padding = rows per work item
+constexpr int kPadRows = kEnsRows;  // cluster padding = rows per work item
 constexpr int kBlock = 256;
+// Bodies of an item's tile range by default: the most of these that leaves
+// several items per resident CTA, so that the last ones are short.  Steps by
+// bodies per item, packed hi/lo: 256 clusters of 256-8192 bodies 2.87 ms (1024),
+// 2.89 (512); 256 of 256-1024 302 us (1024), 193 (512); 16 of 256-2048 284 us
+// (1024), 152 (512), 56 (128).
+constexpr int kItemBodies[] = {1024, 512, 256, 128, 64};
+constexpr double kItemsPerCta = 2.5;
+constexpr int kWideCtasPerSm = 6;  // resident CTAs of the four-row near/far shape
 
 struct ClusterDev {
-  int row0, n, ld, S;
+  int row0, n, ld;
+  int S, block_rows, nb;  // slots of a row: RowSlots(S, block_rows, nb)
   long long p_off;
   double eps2, dt;
 };
@@ -74,7 +87,7 @@ struct ClusterDev {
 
 __global__ void ens_pack_kernel(int L, const int* __restrict__ cid, const double* __restrict__ X,
                                 const double* __restrict__ V, const double* __restrict__ M,
-                                JBody64* __restrict__ jb64, JBodyX2* __restrict__ jbx) {
+                                JBody64* __restrict__ jb64, JBodyX2* __restrict__ jbx = nullptr) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= L) return;
   const bool real = cid[r] >= 0;
@@ -85,6 +98,33 @@ __global__ void ens_pack_kernel(int L, const int* __restrict__ cid, const double
   if (jbx) jbx[r] = make_jbx2(x, y, z, m, u, v, w);
 }
 
+// Near/far subtile blockIdx.x of the state; PREDICT: of the predicted state,
+// which is written back to X, V.
+template <bool PREDICT>
+__global__ void __launch_bounds__(64)
+    ens_tile_kernel(int L, const int* __restrict__ cid, const ClusterDev* __restrict__ cl,
+                    double* __restrict__ X, double* __restrict__ V, const double* __restrict__ M,
+                    const double* __restrict__ D, SymSub* __restrict__ out) {
+  const int r = blockIdx.x * 64 + threadIdx.x;
+  const int c = cid[r];  // L is a multiple of 256
+  double p[3] = {0.0, 0.0, 0.0}, u[3] = {0.0, 0.0, 0.0}, m = 0.0;
+  if (c >= 0) {
+    m = M[r];
+    if (PREDICT) {
+      predict_body(cl[c].dt, L, r, X, V, D, p, u);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        p[k] = X[k * L + r];
+        u[k] = V[k * L + r];
+      }
+    }
+  }
+  write_subtile(out + blockIdx.x, c >= 0, p, u, m);
+}
+
+// Predictor of the FP64 ensemble and of the one-sided kernels, with the records
+// that are not null.
 __global__ void ens_predict_kernel(int L, const int* __restrict__ cid,
                                    const ClusterDev* __restrict__ cl, double* __restrict__ X,
                                    double* __restrict__ V, const double* __restrict__ M,
@@ -94,22 +134,10 @@ __global__ void ens_predict_kernel(int L, const int* __restrict__ cid,
   if (r >= L) return;
   const int c = cid[r];
   if (c < 0) return;
-  const double dt = cl[c].dt;
-  const double h2 = 0.5 * dt * dt;
-  const double h3 = dt * dt * dt * (1.0 / 6.0);
   double p[3], u[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double x = X[k * L + r], v = V[k * L + r];
-    const double a = D[k * L + r], j = D[(3 + k) * L + r];
-    p[k] = x + (v * dt + (a * h2 + j * h3));
-    u[k] = v + (a * dt + j * h2);
-    X[k * L + r] = p[k];
-    V[k * L + r] = u[k];
-  }
-  const double m = M[r];
-  if (jb64) store_jb64(jb64, r, p[0], p[1], p[2], m, u[0], u[1], u[2]);
-  if (jbx) jbx[r] = make_jbx2(p[0], p[1], p[2], m, u[0], u[1], u[2]);
+  predict_body(cl[c].dt, L, r, X, V, D, p, u);
+  if (jb64) store_jb64(jb64, r, p[0], p[1], p[2], M[r], u[0], u[1], u[2]);
+  if (jbx) jbx[r] = make_jbx2(p[0], p[1], p[2], M[r], u[0], u[1], u[2]);
 }
 
 // Between the caller's concatenated arrays ([count][total]) and the padded
@@ -182,21 +210,30 @@ __global__ void ens_key_kernel(int L, const int* __restrict__ cid, const int* __
   vals[r] = r;
 }
 
-__global__ void ens_correct_kernel(int L, const int* __restrict__ cid,
-                                   const ClusterDev* __restrict__ cl, const double* __restrict__ P,
-                                   double* __restrict__ X, double* __restrict__ V,
-                                   double* __restrict__ D) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= L) return;
+// The slot sums of row r (CTAs of kSumThreads: kSumRows<8> rows of one cluster,
+// eight groups), valid in group 0 of real rows; returns the row's cluster or -1.
+__device__ __forceinline__ int ens_slot_sums(int r, const int* __restrict__ cid,
+                                             const ClusterDev* __restrict__ cl,
+                                             const double* __restrict__ P, double sum[6], double* sh) {
   const int c = cid[r];
+  const ClusterDev k = cl[max(c, 0)];
+  const int i = c >= 0 ? r - k.row0 : 0;
+  slot_sums<8>(P + k.p_off, k.ld, c >= 0 ? RowSlots(k.S, k.block_rows, k.nb).count(i) : 0, i, sum, sh);
+  return threadIdx.x < kSumRows<8> ? c : -1;
+}
+
+__global__ void __launch_bounds__(kSumThreads)
+    ens_correct_kernel(int L, const int* __restrict__ cid, const ClusterDev* __restrict__ cl,
+                       const double* __restrict__ P, double* __restrict__ X, double* __restrict__ V,
+                       double* __restrict__ D) {
+  __shared__ double sh[6 * kSumThreads];
+  const int r = blockIdx.x * kSumRows<8> + threadIdx.x % kSumRows<8>;
+  double sum[6];
+  const int c = ens_slot_sums(r, cid, cl, P, sum, sh);
   if (c < 0) return;
-  const ClusterDev k = cl[c];
-  const int i = r - k.row0;
-  const double dt = k.dt;
+  const double dt = cl[c].dt;
   const double idt2 = 1.0 / (dt * dt), idt3 = idt2 / dt;
   const double dt3 = dt * dt * dt, dt4 = dt3 * dt, dt5 = dt4 * dt;
-  double sum[6];
-  split_sums(P + k.p_off, k.ld, k.S, i, sum);  // cluster partials: [S_c][6][ld_c]
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
     const double a1 = sum[q], j1 = sum[3 + q];
@@ -211,16 +248,14 @@ __global__ void ens_correct_kernel(int L, const int* __restrict__ cid,
   }
 }
 
-__global__ void ens_reduce_kernel(int L, const int* __restrict__ cid,
-                                  const ClusterDev* __restrict__ cl, const double* __restrict__ P,
-                                  double* __restrict__ D) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= L) return;
-  const int c = cid[r];
-  if (c < 0) return;
-  const ClusterDev k = cl[c];
+__global__ void __launch_bounds__(kSumThreads)
+    ens_reduce_kernel(int L, const int* __restrict__ cid, const ClusterDev* __restrict__ cl,
+                      const double* __restrict__ P, double* __restrict__ D) {
+  __shared__ double sh[6 * kSumThreads];
+  const int r = blockIdx.x * kSumRows<8> + threadIdx.x % kSumRows<8>;
   double sum[6];
-  split_sums(P + k.p_off, k.ld, k.S, r - k.row0, sum);
+  if (ens_slot_sums(r, cid, cl, P, sum, sh) < 0) return;
+#pragma unroll
   for (int f = 0; f < 6; ++f) D[f * L + r] = sum[f];
 }
 
@@ -277,57 +312,57 @@ __global__ void ens_energy_sum_kernel(const ClusterDev* __restrict__ cl, const d
 }
 
 // Persistent-kernel shapes (all with 256-row items = one padding unit); the
-// first of each precision is the default, the autotuner times all of them.
+// default is the first of a (precision, record format) or, for large near/far
+// ensembles, the second; the autotuner times all of them.  The packed hi/lo
+// default stays one-sided with tiles of 128: its float sums are those of the
+// single-system hi/lo kernel bit for bit, and in clusters with close pairs
+// (softening 4/N) any other order of them moves a body's result by more than
+// its own error against FP64.  Two rows per thread, j-loop unrolled four
+// times: pair launch of 256 clusters of 256-8192 bodies 2.64 ms, four rows
+// 2.74; the symmetric near/far kernel (pair_variant 4) takes 1.92.
 struct EnsKernel {
   int precision, nt, tile;
   int fmt;  // RecordFormat of its j-records
   const void* fn;
   size_t smem;
-  int near = 0;  // tile-relative: 1 = near tiles in double-single, 0 = every tile far
+  bool sym = true;
 };
 
+template <int IPT, int W, int UNR, int MINB>
+EnsKernel ens_sym_fp64() {
+  return {NBODY_FP64, 32 * W, kSymTile64, kRecF64,
+          reinterpret_cast<const void*>(&ensemble_sym_fp64_kernel<IPT, W, UNR, MINB>),
+          sym_fp64_smem<IPT, W, UNR>()};
+}
+template <int IPT, int W, int SUB, int UNR, int NUNR, int MINB>
+EnsKernel ens_sym_nf() {
+  return {NBODY_MIXED, 32 * W, 64 * SUB, kRecSym,
+          reinterpret_cast<const void*>(&ensemble_sym_nf_kernel<IPT, W, SUB, UNR, NUNR, MINB>),
+          sym_nf_smem<IPT, W, SUB>()};
+}
 template <class R>
-EnsKernel ens_kernel(int precision) {
+EnsKernel ens_hilo() {
   static_assert(R::ROWS == kPadRows, "an item's row block is one padding unit");
-  return {precision, R::NT, R::TJ, precision == NBODY_FP64 ? kRecF64 : kRecX2,
-          reinterpret_cast<const void*>(&ensemble_pair_kernel<R>), pair_smem_bytes<R>()};
+  return {NBODY_MIXED, R::NT, R::TJ, kRecX2, reinterpret_cast<const void*>(&ensemble_pair_kernel<R>),
+          pair_smem_bytes<R>(), false};
+}
+template <class R>
+EnsKernel ens_all_far() {
+  static_assert(R::ROWS == kPadRows, "an item's row block is one padding unit");
+  return {NBODY_MIXED, R::NT, R::TJ, kRecRel, reinterpret_cast<const void*>(&ensemble_pair_nf_kernel<R, 1>),
+          2 * (R::TJ + 1) * sizeof(JBodyNF) + R::kExtraSmem, false};
 }
 
-template <class R, int MINB = 1>
-EnsKernel ens_kernel_nf() {
-  static_assert(R::ROWS == kPadRows, "an item's row block is one padding unit");
-  return {NBODY_MIXED, R::NT, R::TJ, kRecRel,
-          reinterpret_cast<const void*>(&ensemble_pair_nf_kernel<R, MINB>),
-          2 * (R::TJ + 1) * sizeof(JBodyNF) + R::kExtraSmem, R::kNear ? 1 : 0};
-}
-
-// The first entry of each (precision, record format, near) is its default.
 const std::vector<EnsKernel>& ens_registry() {
   static const std::vector<EnsKernel> r = {
-      ens_kernel<RowsFP64<128, 2, 128, 1>>(NBODY_FP64),
-      ens_kernel<RowsFP64<256, 1, 128, 4>>(NBODY_FP64),
-      ens_kernel_nf<RowsMixedNF<64, 4, 64, 1, 1, 1>>(),
-      ens_kernel_nf<RowsMixedNF<64, 4, 128, 1, 1, 1>>(),
-      ens_kernel_nf<RowsMixedNF<128, 2, 128, 1, 1, 1>>(),
-      ens_kernel_nf<RowsMixedNF<128, 2, 64, 1, 1, 1>>(),
-      ens_kernel_nf<RowsMixedNF<64, 4, 64, 1, 2, 1>>(),
-      ens_kernel_nf<RowsMixedNF<128, 2, 128, 1, 2, 1>>(),
-      ens_kernel_nf<RowsMixedNF<64, 4, 128, 1, 2, 1>>(),
-      ens_kernel_nf<RowsMixedNF<64, 4, 64, 1, 1, 2>>(),
-      // 64 threads capped at 128 registers: 8 CTAs (16 warps) per SM
-      ens_kernel_nf<RowsMixedNF<64, 4, 64, 1, 1, 1>, 8>(),
-      ens_kernel_nf<RowsMixedNF<64, 4, 64, 1, 2, 1>, 8>(),
-      ens_kernel_nf<RowsMixedNF<64, 4, 64, 1, 1, 2>, 8>(),
-      ens_kernel_nf<RowsMixedNF<64, 4, 128, 1, 1, 1>, 8>(),
-      ens_kernel_nf<RowsMixedNF<64, 4, 64, 1, 1, 0>>(),
-      ens_kernel_nf<RowsMixedNF<128, 2, 128, 1, 1, 0>>(),
-      ens_kernel<RowsMixedX2<64, 4, 128, 1, 1>>(NBODY_MIXED),
-      ens_kernel<RowsMixedX2<128, 2, 128, 1, 1>>(NBODY_MIXED),
-      ens_kernel<RowsMixedX2<64, 4, 64, 1, 1>>(NBODY_MIXED),
-      ens_kernel<RowsMixedX2<64, 4, 64, 1, 2>>(NBODY_MIXED),
-      ens_kernel<RowsMixedX2<128, 2, 64, 1, 1>>(NBODY_MIXED),
-      ens_kernel<RowsMixedX2<128, 2, 64, 1, 2>>(NBODY_MIXED),
-      ens_kernel<RowsMixedX2<64, 4, 64, 0, 2>>(NBODY_MIXED),
+      ens_sym_fp64<2, 4, 4, 4>(),
+      ens_sym_nf<2, 4, 1, 4, 8, 4>(),
+      ens_sym_nf<4, 2, 1, 4, 2, 6>(),
+      ens_hilo<RowsMixedX2<128, 2, 128, 1, 4>>(),
+      ens_hilo<RowsMixedX2<64, 4, 128, 1, 1>>(),
+      ens_hilo<RowsMixedX2<128, 2, 64, 1, 2>>(),
+      ens_all_far<RowsMixedNF<64, 4, 64, 1, 1, 0>>(),
+      ens_all_far<RowsMixedNF<128, 2, 128, 1, 1, 0>>(),
   };
   return r;
 }
@@ -336,7 +371,8 @@ const std::vector<EnsKernel>& ens_registry() {
 
 struct nbody_ensemble {
   int C = 0, L = 0, dev = 0, sms = 0, precision = 0;
-  int fmt = kRecF64;  // record format of the pair kernels in use
+  int fmt = kRecF64;      // record format of the pair kernels in use
+  bool ordered = false;   // clusters kept in Hilbert order (pair_variant 4, 5)
   int tiles_per_item = 8;
   const EnsKernel* kern = nullptr;  // persistent pair kernel in use
   int grid = 0;
@@ -349,7 +385,7 @@ struct nbody_ensemble {
   double* P = nullptr;
   size_t p_doubles = 0;
   JBody64* jb64 = nullptr;
-  JBodyX2* jbx = nullptr;
+  void* jmix = nullptr;  // mixed records: SymSub, JBodyX2 or tiles of JBodyNF
   int* cid = nullptr;
   int* idx = nullptr;    // [L] padded row -> index in the caller's arrays, -1 on padding
   double* io = nullptr;  // [7][total] the caller's arrays on their way in or out
@@ -362,7 +398,8 @@ struct nbody_ensemble {
   int *blk_cluster = nullptr, *blk_row = nullptr;
   int n_blk = 0;
   double *phi = nullptr, *Tc = nullptr, *Uc = nullptr;
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph = nullptr;  // one step with the event records of last_step_ms
+  cudaGraphExec_t plain = nullptr;  // one step
   int step_kernels = 0;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   bool have_derivs = false;
@@ -370,7 +407,6 @@ struct nbody_ensemble {
   // Hilbert ordering (mixed, tile-relative variants): each cluster keeps its
   // bodies in Hilbert order within its segment; position r holds the body of
   // padded row perm[r] (the caller's order).
-  int near = 1;                   // near/far kernel (variant 4) or every tile far (5)
   int* perm = nullptr;            // [2][L]
   double* scratch = nullptr;      // [13][L]
   bool sorted = false, permuted = false;
@@ -399,39 +435,82 @@ nbody_status ens_status(nbody_ensemble* e) {
   return NBODY_OK;
 }
 
+void drop_graphs(nbody_ensemble* e) {
+  for (cudaGraphExec_t* g : {&e->graph, &e->plain}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
+}
+
+// How cluster c is cut for kernel k: tiles that hold bodies (the padding rows of
+// a segment come last, in the tile-relative order too, so whole padding tiles
+// are skipped), blocks of 256 rows or, in clusters of more than kMaxSymBlocks
+// of those, of several times that, and the splits of a block's run.
+struct ClusterCut {
+  int tiles, subs, block, nb, S;
+  ClusterCut(const EnsKernel& k, int n, int tpi) {
+    tiles = (n + k.tile - 1) / k.tile;
+    subs = k.sym ? (n + kMaxSymBlocks * kPadRows - 1) / (kMaxSymBlocks * kPadRows) : 1;
+    block = kPadRows * subs;
+    nb = (n + block - 1) / block;
+    S = (run(k, 0) + tpi - 1) / tpi;
+  }
+  int run(const EnsKernel& k, int I) const {  // tiles of block I's run
+    return k.sym ? sym_q_count(nb, I, block / k.tile, tiles) : tiles;
+  }
+};
+
+long count_items(const nbody_ensemble* e, int tpi) {
+  long items = 0;
+  for (int c = 0; c < e->C; ++c) {
+    const ClusterCut k(*e->kern, e->n[c], tpi);
+    items += static_cast<long>(k.nb) * k.S;
+  }
+  return items;
+}
+
+int default_tiles_per_item(const nbody_ensemble* e) {
+  int tpi = 1;
+  for (int bodies : kItemBodies) {
+    tpi = std::max(1, bodies / e->kern->tile);
+    if (count_items(e, tpi) >= kItemsPerCta * e->grid) break;
+  }
+  return tpi;
+}
+
 // (Re)builds the work list and partial-sum layout for `tpi` tiles per item.
 nbody_status build_items(nbody_ensemble* e, int tpi) {
   std::vector<ClusterDev> cl(e->C);
   std::vector<EnsItem> items;
   long long p_off = 0;
   for (int c = 0; c < e->C; ++c) {
-    // j-tiles that hold bodies: the padding rows of a segment come last (in
-    // the tile-relative order too), so whole padding tiles are skipped
-    const int tiles = (e->n[c] + e->kern->tile - 1) / e->kern->tile;
-    const int S = (tiles + tpi - 1) / tpi;
-    cl[c] = ClusterDev{e->row0[c], e->n[c], e->ld[c], S, p_off, e->eps2[c], e->dt[c]};
-    for (int rb = 0; rb < e->ld[c] / kPadRows; ++rb)
-      for (int s = 0; s < S; ++s) {
+    const EnsKernel& kern = *e->kern;
+    const ClusterCut k(kern, e->n[c], tpi);
+    cl[c] = ClusterDev{e->row0[c], e->n[c], e->ld[c], k.S, k.block, kern.sym ? k.nb : 0, p_off, e->eps2[c], e->dt[c]};
+    for (int rb = 0; rb < k.nb; ++rb)
+      for (int s = 0; s < k.S; ++s) {
         EnsItem it;
         it.jrow0 = e->row0[c];
-        it.row0 = rb * kPadRows;
+        it.row0 = rb * k.block;
         it.rows_end = e->n[c];
         it.ld = e->ld[c];
-        it.t_begin = s * tpi;
-        it.nt = std::min(tpi, tiles - it.t_begin);
-        it.out_off = p_off + static_cast<long long>(s) * 6 * e->ld[c];
+        it.S = k.S;
+        it.nb = k.nb;
+        it.subs = k.subs;
+        it.split = s;
+        it.p_off = p_off;
         it.eps2 = e->eps2[c];
+        const int q0 = s * tpi;
+        it.t_begin = kern.sym ? rb * (k.block / kern.tile) + q0 : q0;
+        it.nt = std::max(0, std::min(tpi, k.run(kern, rb) - q0));  // 0: the item writes zeros to its slot
         items.push_back(it);
       }
-    p_off += static_cast<long long>(S) * 6 * e->ld[c];
+    p_off += static_cast<long long>(k.S + (kern.sym ? k.nb / 2 : 0)) * 6 * e->ld[c];
   }
   // longest items first, then by cluster so neighbours share L2 lines
   std::stable_sort(items.begin(), items.end(),
-                   [](const EnsItem& a, const EnsItem& b) { return a.nt > b.nt; });
-  if (e->graph) {
-    cudaGraphExecDestroy(e->graph);
-    e->graph = nullptr;
-  }
+                   [](const EnsItem& a, const EnsItem& b) { return a.nt * a.subs > b.nt * b.subs; });
+  drop_graphs(e);
   EN_CUDA(cudaStreamSynchronize(e->stream));
   cudaFree(e->P);
   cudaFree(e->items);
@@ -447,14 +526,19 @@ nbody_status build_items(nbody_ensemble* e, int tpi) {
   return NBODY_OK;
 }
 
+SoA7 ens_state(nbody_ensemble* e) {
+  const size_t L = e->L;
+  return SoA7{e->X, e->X + L, e->X + 2 * L, e->M, e->V, e->V + L, e->V + 2 * L};
+}
+
 nbody_status launch_ens_pair(nbody_ensemble* e) {
   EN_CUDA(cudaMemsetAsync(e->counter, 0, sizeof(unsigned int), e->stream));
-  const bool fp64 = e->precision == NBODY_FP64;
-  const void* jb = fp64 ? static_cast<const void*>(e->jb64) : static_cast<const void*>(e->jbx);
-  const size_t L = e->L;
-  RowSrc rows{e->X, e->X + L, e->X + 2 * L, e->V, e->V + L, e->V + 2 * L};
+  const void* jb = e->fmt == kRecF64 ? static_cast<const void*>(e->jb64) : e->jmix;
+  SoA7 rows = ens_state(e);
+  RowSrc src{rows.x, rows.y, rows.z, rows.vx, rows.vy, rows.vz};
   void* args[] = {const_cast<void*>(static_cast<const void*>(&jb)), &e->items, &e->n_items,
-                  &e->counter, &e->P, &e->status, &rows};
+                  &e->counter, &e->P, &e->status,
+                  e->kern->sym ? static_cast<void*>(&rows) : static_cast<void*>(&src)};
   EN_CUDA(cudaLaunchKernel(e->kern->fn, dim3(e->grid), dim3(e->kern->nt), args, e->kern->smem,
                            e->stream));
   return NBODY_OK;
@@ -495,19 +579,37 @@ nbody_status ens_reorder_state(nbody_ensemble* e, cudaStream_t st) {
   return NBODY_OK;
 }
 
-// Near/far tile records (tiles of the kernel's TJ) of the state, which is in
-// Hilbert order within each cluster segment.
-nbody_status ens_tiles(nbody_ensemble* e, cudaStream_t st) {
-  const size_t L = e->L;
-  const SoA7 in{e->X, e->X + L, e->X + 2 * L, e->M, e->V, e->V + L, e->V + 2 * L};
-  JBodyNF* out = reinterpret_cast<JBodyNF*>(e->jbx);
-  const int tiles = e->L / e->kern->tile;
-  switch (e->kern->tile) {
-    case 64: rel_tile_nf_kernel<64><<<tiles, 64, 0, st>>>(e->L, in, out, e->cid); break;
-    case 128: rel_tile_nf_kernel<128><<<tiles, 128, 0, st>>>(e->L, in, out, e->cid); break;
-    default: return nbody_set_error(NBODY_ERR_INVALID_ARG, "no record builder for tile %d", e->kern->tile);
+// Records of the pair kernel in use from the state (tile-relative ones: in
+// Hilbert order within each cluster segment); predict: of the predicted state.
+nbody_status ens_records(nbody_ensemble* e, cudaStream_t st, bool predict) {
+  const int blocks = (e->L + kBlock - 1) / kBlock;
+  JBodyX2* jbx = e->fmt == kRecX2 ? static_cast<JBodyX2*>(e->jmix) : nullptr;
+  if (e->fmt == kRecSym) {
+    SymSub* out = static_cast<SymSub*>(e->jmix);
+    if (predict)
+      ens_tile_kernel<true><<<e->L / 64, 64, 0, st>>>(e->L, e->cid, e->cl, e->X, e->V, e->M, e->D, out);
+    else
+      ens_tile_kernel<false><<<e->L / 64, 64, 0, st>>>(e->L, e->cid, e->cl, e->X, e->V, e->M, e->D, out);
+    EN_CUDA(cudaGetLastError());
+    return NBODY_OK;
   }
+  if (predict)
+    ens_predict_kernel<<<blocks, kBlock, 0, st>>>(e->L, e->cid, e->cl, e->X, e->V, e->M, e->D,
+                                                  e->fmt == kRecF64 ? e->jb64 : nullptr, jbx);
+  else if (e->fmt != kRecRel)
+    ens_pack_kernel<<<blocks, kBlock, 0, st>>>(e->L, e->cid, e->X, e->V, e->M,
+                                               e->fmt == kRecF64 ? e->jb64 : nullptr, jbx);
   EN_CUDA(cudaGetLastError());
+  if (e->fmt == kRecRel) {
+    JBodyNF* out = static_cast<JBodyNF*>(e->jmix);
+    const int tiles = e->L / e->kern->tile;
+    switch (e->kern->tile) {
+      case 64: rel_tile_nf_kernel<64><<<tiles, 64, 0, st>>>(e->L, ens_state(e), out, e->cid); break;
+      case 128: rel_tile_nf_kernel<128><<<tiles, 128, 0, st>>>(e->L, ens_state(e), out, e->cid); break;
+      default: return nbody_set_error(NBODY_ERR_INVALID_ARG, "no record builder for tile %d", e->kern->tile);
+    }
+    EN_CUDA(cudaGetLastError());
+  }
   return NBODY_OK;
 }
 
@@ -538,14 +640,12 @@ nbody_status use_kernel(nbody_ensemble* e, const EnsKernel* k) {
 }
 
 nbody_status launch_ens_pack(nbody_ensemble* e) {
-  if (e->fmt == kRecRel && !e->sorted)  // tile-relative: bodies into Hilbert order first
+  if (e->ordered && !e->sorted)  // tile-relative: bodies into Hilbert order first
     EN_TRY(ens_reorder_state(e, e->stream));
-  ens_pack_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(
-      e->L, e->cid, e->X, e->V, e->M, e->jb64, e->fmt == kRecX2 ? e->jbx : nullptr);
-  EN_CUDA(cudaGetLastError());
-  if (e->fmt == kRecRel) EN_TRY(ens_tiles(e, e->stream));
-  return NBODY_OK;
+  return ens_records(e, e->stream, false);
 }
+
+int sum_blocks(const nbody_ensemble* e) { return e->L / kSumRows<8>; }  // L is a multiple of 256
 
 int count_graph_kernels(cudaGraph_t g) {
   size_t nodes = 0;
@@ -565,29 +665,25 @@ int count_graph_kernels(cudaGraph_t g) {
 nbody_status ens_eval_current(nbody_ensemble* e) {
   EN_TRY(launch_ens_pack(e));
   EN_TRY(launch_ens_pair(e));
-  ens_reduce_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(e->L, e->cid, e->cl,
-                                                                          e->P, e->D);
+  ens_reduce_kernel<<<sum_blocks(e), kSumThreads, 0, e->stream>>>(e->L, e->cid, e->cl, e->P, e->D);
   EN_CUDA(cudaGetLastError());
   e->have_derivs = true;
   return NBODY_OK;
 }
 
-nbody_status ens_build_graph(nbody_ensemble* e) {
-  if (e->graph) return NBODY_OK;
-  const bool fp64 = e->precision == NBODY_FP64;
+// Captures one step (timed: with its event records) into *out.
+nbody_status ens_capture(nbody_ensemble* e, bool timed, cudaGraphExec_t* out) {
+  if (*out) return NBODY_OK;
   cudaGraph_t g = nullptr;
   EN_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
   nbody_status s = NBODY_OK;
-  if (cudaEventRecordWithFlags(e->ev[0], e->stream, cudaEventRecordExternal) != cudaSuccess)
+  if (timed && cudaEventRecordWithFlags(e->ev[0], e->stream, cudaEventRecordExternal) != cudaSuccess)
     s = nbody_set_error(NBODY_ERR_CUDA, "event record during capture failed");
-  ens_predict_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(
-      e->L, e->cid, e->cl, e->X, e->V, e->M, e->D, fp64 ? e->jb64 : nullptr,
-      e->fmt == kRecX2 ? e->jbx : nullptr);
-  if (s == NBODY_OK && e->fmt == kRecRel) s = ens_tiles(e, e->stream);
+  if (s == NBODY_OK) s = ens_records(e, e->stream, true);
   if (s == NBODY_OK) s = launch_ens_pair(e);
-  ens_correct_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(e->L, e->cid, e->cl,
-                                                                           e->P, e->X, e->V, e->D);
-  if (s == NBODY_OK && cudaEventRecordWithFlags(e->ev[1], e->stream, cudaEventRecordExternal) != cudaSuccess)
+  ens_correct_kernel<<<sum_blocks(e), kSumThreads, 0, e->stream>>>(e->L, e->cid, e->cl, e->P, e->X, e->V, e->D);
+  if (timed && s == NBODY_OK &&
+      cudaEventRecordWithFlags(e->ev[1], e->stream, cudaEventRecordExternal) != cudaSuccess)
     s = nbody_set_error(NBODY_ERR_CUDA, "event record during capture failed");
   cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
   if (s != NBODY_OK) {
@@ -595,19 +691,27 @@ nbody_status ens_build_graph(nbody_ensemble* e) {
     return s;
   }
   if (ce != cudaSuccess) return nbody_set_error(NBODY_ERR_CUDA, "capture: %s", cudaGetErrorString(ce));
-  e->step_kernels = count_graph_kernels(g);
-  ce = cudaGraphInstantiate(&e->graph, g, 0);
+  if (timed) e->step_kernels = count_graph_kernels(g);
+  ce = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   if (ce != cudaSuccess) {
-    e->graph = nullptr;
+    *out = nullptr;
     return nbody_set_error(NBODY_ERR_CUDA, "instantiate: %s", cudaGetErrorString(ce));
   }
-  if (e->fmt == kRecRel && !e->order_graph) {
+  return NBODY_OK;
+}
+
+nbody_status ens_build_graph(nbody_ensemble* e) {
+  if (e->graph) return NBODY_OK;
+  EN_TRY(ens_capture(e, true, &e->graph));
+  cudaGraph_t g = nullptr;
+  nbody_status s = NBODY_OK;
+  cudaError_t ce = cudaSuccess;
+  if (e->ordered && !e->order_graph) {
     const bool sorted = e->sorted, permuted = e->permuted;
     const int since = e->since_sort;
     EN_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     s = ens_reorder_state(e, e->stream);
-    g = nullptr;
     ce = cudaStreamEndCapture(e->stream, &g);
     e->sorted = sorted;  // capturing ran nothing
     e->permuted = permuted;
@@ -639,9 +743,9 @@ nbody_status ens_autotune(nbody_ensemble* e) {
   const EnsKernel* best_k = e->kern;
   int best_tpi = 8;
   for (const EnsKernel& k : ens_registry()) {
-    if (k.precision != e->precision || k.fmt != e->fmt || (k.fmt == kRecRel && k.near != e->near)) continue;
+    if (k.precision != e->precision || k.fmt != e->fmt) continue;
     EN_TRY(use_kernel(e, &k));
-    if (e->fmt == kRecRel) EN_TRY(ens_tiles(e, e->stream));  // this kernel's tile size
+    if (e->fmt == kRecRel) EN_TRY(ens_records(e, e->stream, false));  // this kernel's tile size
     for (int j_per_item : {256, 512, 1024, 2048, 4096, 8192}) {
       const int tpi = std::max(1, j_per_item / k.tile);
       EN_TRY(build_items(e, tpi));
@@ -666,7 +770,7 @@ nbody_status ens_autotune(nbody_ensemble* e) {
   cudaEventDestroy(b);
   EN_TRY(ens_status(e));
   EN_TRY(use_kernel(e, best_k));
-  if (e->fmt == kRecRel) EN_TRY(ens_tiles(e, e->stream));
+  if (e->fmt == kRecRel) EN_TRY(ens_records(e, e->stream, false));
   return build_items(e, best_tpi);
 }
 
@@ -684,11 +788,11 @@ nbody_status nbody_ensemble_destroy(nbody_ensemble* e) {
   if (!e) return NBODY_OK;
   cudaSetDevice(e->dev);
   if (e->stream) cudaStreamSynchronize(e->stream);
-  if (e->graph) cudaGraphExecDestroy(e->graph);
+  drop_graphs(e);
   if (e->order_graph) cudaGraphExecDestroy(e->order_graph);
   for (auto ev : e->ev)
     if (ev) cudaEventDestroy(ev);
-  void* bufs[] = {e->state, e->P, e->jb64, e->jbx, e->cid, e->cl, e->items, e->counter,
+  void* bufs[] = {e->state, e->P, e->jb64, e->jmix, e->cid, e->cl, e->items, e->counter,
                   e->status, e->blk_cluster, e->blk_row, e->phi, e->Tc, e->Uc,
                   e->idx, e->io, e->seg, e->bbox, e->sort_keys, e->sort_idx, e->sort_tmp, e->perm, e->scratch};
   for (void* p : bufs) cudaFree(p);
@@ -712,12 +816,6 @@ nbody_status nbody_ensemble_create(nbody_ensemble** out, const nbody_ensemble_co
                            "ensemble pair_variant = %d (0 automatic = packed hi/lo, 3 packed hi/lo, "
                            "4 near/far tile-relative, 5 plain tile-relative)", cfg->pair_variant);
   if (cfg->sort_every < 0) return nbody_set_error(NBODY_ERR_INVALID_ARG, "sort_every < 0");
-  // Mixed default: packed hi/lo.  In clusters of 256-8192 bodies a 64-body
-  // tile is rarely far from a warp's 128 rows (near share of a Plummer
-  // sphere: 0.48 at 8192 bodies, 0.73 at 4096, 0.93 at 2048), so the
-  // near/far kernel saves less than its tile building and re-ordering cost
-  // (measured 855 vs 878 G interactions/s on 512 Plummer clusters of
-  // 256-8192 bodies).
   const bool rel = cfg->precision == NBODY_MIXED && (cfg->pair_variant == 4 || cfg->pair_variant == 5);
   if (rel && C > 65536)
     return nbody_set_error(NBODY_ERR_INVALID_ARG,
@@ -749,8 +847,11 @@ nbody_status nbody_ensemble_create(nbody_ensemble** out, const nbody_ensemble_co
   e->L = static_cast<int>(L);
   e->dev = cfg->device;
   e->precision = cfg->precision;
-  e->fmt = cfg->precision == NBODY_FP64 ? kRecF64 : (rel ? kRecRel : kRecX2);
-  e->near = cfg->pair_variant == 4 ? 1 : 0;
+  e->fmt = cfg->precision == NBODY_FP64 ? kRecF64
+           : cfg->pair_variant == 4     ? kRecSym
+           : cfg->pair_variant == 5     ? kRecRel
+                                        : kRecX2;
+  e->ordered = rel;
   e->sort_every = cfg->sort_every > 0 ? cfg->sort_every : 16;
   while ((1LL << (e->sort_bits - 48)) < C) ++e->sort_bits;  // cluster id above the 48-bit code
   cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, e->dev);
@@ -787,8 +888,10 @@ nbody_status nbody_ensemble_create(nbody_ensemble** out, const nbody_ensemble_co
     raw->M = raw->state + 6 * Ls;
     raw->D = raw->state + 7 * Ls;
     EN_CUDA(cudaMalloc(&raw->jb64, sizeof(JBody64) * Ls));
-    // JBodyX2 records, or tiles of TJ + 1 JBodyNF records (TJ >= 64)
-    if (raw->precision == NBODY_MIXED) EN_CUDA(cudaMalloc(&raw->jbx, sizeof(JBodyNF) * (Ls / 64) * 65));
+    // subtiles of 64 bodies, packed hi/lo records, or tiles of TJ + 1 JBodyNF (TJ >= 64)
+    static_assert(sizeof(JBodyNF) >= sizeof(JBodyX2), "jmix sized by the larger record");
+    if (raw->precision == NBODY_MIXED)
+      EN_CUDA(cudaMalloc(&raw->jmix, (Ls / 64) * (raw->fmt == kRecSym ? sizeof(SymSub) : 65 * sizeof(JBodyNF))));
     EN_CUDA(cudaMalloc(&raw->cid, sizeof(int) * Ls));
     EN_CUDA(cudaMemcpy(raw->cid, cid.data(), sizeof(int) * Ls, cudaMemcpyHostToDevice));
     EN_CUDA(cudaMalloc(&raw->idx, sizeof(int) * Ls));
@@ -805,7 +908,7 @@ nbody_status nbody_ensemble_create(nbody_ensemble** out, const nbody_ensemble_co
     EN_CUDA(cudaMalloc(&raw->phi, sizeof(double) * Ls));
     EN_CUDA(cudaMalloc(&raw->Tc, sizeof(double) * raw->C));
     EN_CUDA(cudaMalloc(&raw->Uc, sizeof(double) * raw->C));
-    if (raw->fmt == kRecRel) {
+    if (raw->ordered) {
       EN_CUDA(cudaMalloc(&raw->seg, sizeof(int) * Ls));
       EN_CUDA(cudaMemcpy(raw->seg, seg.data(), sizeof(int) * Ls, cudaMemcpyHostToDevice));
       EN_CUDA(cudaMalloc(&raw->bbox, sizeof(double) * 6 * raw->C));
@@ -822,12 +925,18 @@ nbody_status nbody_ensemble_create(nbody_ensemble** out, const nbody_ensemble_co
       EN_CUDA(cudaMalloc(&raw->sort_tmp, std::max<size_t>(raw->sort_tmp_bytes, 16)));
     }
     for (auto& ev : raw->ev) EN_CUDA(cudaEventCreate(&ev));
-    for (const EnsKernel& k : ens_registry())
-      if (k.precision == raw->precision && k.fmt == raw->fmt && (k.fmt != kRecRel || k.near == raw->near)) {
-        EN_TRY(use_kernel(raw, &k));
-        break;
-      }
-    return build_items(raw, cfg->tiles_per_item > 0 ? cfg->tiles_per_item : 8);
+    // the first shape, or the second where there are several long items for
+    // each of its CTAs (pair launch of 256 clusters of 256-8192 bodies 2.04 vs
+    // 1.96 ms, of 64 0.543 vs 0.539, of 256 of 256-2048 0.27 vs 0.28)
+    const EnsKernel* first = nullptr;
+    for (const EnsKernel& k : ens_registry()) {
+      if (k.precision != raw->precision || k.fmt != raw->fmt) continue;
+      if (first && (!k.sym || count_items(raw, kItemBodies[0] / k.tile) < 4L * raw->sms * kWideCtasPerSm)) break;
+      EN_TRY(use_kernel(raw, &k));
+      if (first) break;
+      first = &k;
+    }
+    return build_items(raw, cfg->tiles_per_item > 0 ? cfg->tiles_per_item : default_tiles_per_item(raw));
   };
   nbody_status s = body();
   if (s != NBODY_OK) {
@@ -896,12 +1005,13 @@ nbody_status nbody_ensemble_step(nbody_ensemble* e, int nsteps) {
   if (!e->have_derivs) EN_TRY(ens_eval_current(e));
   EN_TRY(ens_build_graph(e));
   for (int k = 0; k < nsteps; ++k) {
-    if (e->fmt == kRecRel && e->since_sort >= e->sort_every) {
+    if (e->ordered && e->since_sort >= e->sort_every) {
       EN_CUDA(cudaGraphLaunch(e->order_graph, e->stream));
       e->since_sort = 0;
       ++e->reorders;
     }
-    EN_CUDA(cudaGraphLaunch(e->graph, e->stream));
+    if (k + 1 < nsteps) EN_TRY(ens_capture(e, false, &e->plain));
+    EN_CUDA(cudaGraphLaunch(k + 1 < nsteps ? e->plain : e->graph, e->stream));
     ++e->since_sort;
   }
   e->steps += nsteps;
@@ -918,7 +1028,7 @@ nbody_status nbody_ensemble_energy(nbody_ensemble* e, double* T, double* U) {
   EN_TRY(ens_check(e));
   if (!T || !U) return nbody_set_error(NBODY_ERR_INVALID_ARG, "null energy arrays");
   ens_pack_kernel<<<(e->L + kBlock - 1) / kBlock, kBlock, 0, e->stream>>>(e->L, e->cid, e->X, e->V,
-                                                                        e->M, e->jb64, nullptr);
+                                                                        e->M, e->jb64);
   ens_phi_kernel<<<e->n_blk, kBlock, 0, e->stream>>>(e->blk_cluster, e->blk_row, e->cl, e->jb64, e->phi);
   ens_energy_sum_kernel<<<e->C, kBlock, 0, e->stream>>>(e->cl, e->V, e->M, e->phi, e->L, e->Tc, e->Uc);
   EN_CUDA(cudaGetLastError());
@@ -945,7 +1055,7 @@ nbody_status nbody_ensemble_info(nbody_ensemble* e, nbody_ensemble_info_t* out) 
   float ms = 0;
   if (e->graph && cudaEventElapsedTime(&ms, e->ev[0], e->ev[1]) == cudaSuccess) out->last_step_ms = ms;
   cudaGetLastError();
-  out->record_format = e->fmt;
+  out->record_format = e->fmt == kRecSym ? kRecRel : e->fmt;
   out->step_kernels = e->step_kernels;
   out->reorders = e->reorders;
   out->order_kernels = e->order_kernels;

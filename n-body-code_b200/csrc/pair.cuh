@@ -897,47 +897,55 @@ __global__ void __cluster_dims__(1, CL, 1) __launch_bounds__(NT, MINB)
 }
 
 // ---------------------------------------------------------------------------
-// Ensemble: one persistent launch over a work list of (cluster, row block,
-// j-tile range) items; CTAs take items from an atomic counter (zeroed before
-// each launch) until the list is exhausted.
+// Ensemble: work items of the persistent launches (cluster, 256-row block,
+// j-tile range); CTAs take items from an atomic counter (zeroed before each
+// launch) until the list is exhausted.
 // ---------------------------------------------------------------------------
+constexpr int kEnsRows = 256;  // rows of an item = padding unit of a cluster's segment
 struct EnsItem {
   int jrow0;          // first padded row of the cluster (its j-records and rows)
   int row0;           // first i-row of the item, cluster-relative
   int rows_end;       // the cluster's bodies: rows >= rows_end are not stored
   int ld;             // padded rows of the cluster = stride of its partials
-  int t_begin, nt;    // j-tile range, cluster-relative
-  long long out_off;  // doubles from the partial-sum base to this split's [6][ld] block
+  int t_begin, nt;    // first j-tile (cluster-relative; symmetric kernels: cyclic) and count
+  int S, nb, subs;    // the cluster's splits, (symmetric) blocks and 256-row sub-blocks per block
+  int split;          // the item's split
+  long long p_off;    // doubles from the partial-sum base to the cluster's slots
   double eps2;
 };
 
+// One-sided packed hi/lo ensemble kernel (R: a RowsMixedX2).
 template <class R>
-__device__ __forceinline__ void pair_ensemble(const typename R::JB* __restrict__ jb,
-                                              const EnsItem* __restrict__ items, int n_items,
-                                              unsigned int* counter, double* P, int* status,
-                                              unsigned char* smem, uint64_t* full, int* s_item) {
+__global__ void __launch_bounds__(R::NT) ensemble_pair_kernel(const typename R::JB* __restrict__ jb,
+                                                              const EnsItem* __restrict__ items,
+                                                              int n_items, unsigned int* counter,
+                                                              double* P, int* status, RowSrc) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ uint64_t full[2];
+  __shared__ int s_item;
   using JB = typename R::JB;
   TilePipe<JB, R::TJ> pipe;
-  pipe.init(reinterpret_cast<JB*>(smem), full);
+  pipe.init(reinterpret_cast<JB*>(smem_raw), full);
   for (;;) {
-    if (threadIdx.x == 0) *s_item = static_cast<int>(atomicAdd(counter, 1u));
+    if (threadIdx.x == 0) s_item = static_cast<int>(atomicAdd(counter, 1u));
     __syncthreads();
-    const int k = *s_item;
+    const int k = s_item;
     __syncthreads();
     if (k >= n_items) return;
     const EnsItem it = items[k];
     const JB* cj = jb + it.jrow0;
     const int row = it.row0 + threadIdx.x;
     R r;
-    r.begin(cj, row, it.ld - 1, it.eps2, smem + 2 * R::TJ * sizeof(JB));
+    r.begin(cj, row, it.ld - 1, it.eps2, smem_raw + 2 * R::TJ * sizeof(JB));
     if (!pipe.run(cj + static_cast<size_t>(it.t_begin) * R::TJ, it.nt, status,
                   [&](const JB* tile) { r.consume(tile); }))
       return;
-    r.store(P + it.out_off, static_cast<size_t>(it.ld), row, it.rows_end);
+    r.store(P + it.p_off + static_cast<long long>(it.split) * 6 * it.ld, static_cast<size_t>(it.ld), row,
+            it.rows_end);
   }
 }
 
-// Near/far tile-relative ensemble: tiles of TJ + 1 records over the whole
+// Plain tile-relative ensemble kernel: tiles of TJ + 1 records over the whole
 // padded array (cluster segments are multiples of 256 rows, so a tile never
 // spans two clusters); i-rows from the FP64 state `rows`, whose bodies each
 // cluster keeps in Hilbert order within its segment.  R is a RowsMixedNF.
@@ -965,19 +973,9 @@ __global__ void __launch_bounds__(R::NT, MINB) ensemble_pair_nf_kernel(
                  smem_raw + 2 * kRecs * sizeof(JBodyNF));
     const JBodyNF* ct = jt + static_cast<size_t>(it.jrow0 / R::TJ + it.t_begin) * kRecs;
     if (!pipe.run(ct, it.nt, status, [&](const JBodyNF* tile) { r.consume(tile); })) return;
-    r.store(P + it.out_off, static_cast<size_t>(it.ld), it.rows_end);
+    r.store(P + it.p_off + static_cast<long long>(it.split) * 6 * it.ld, static_cast<size_t>(it.ld),
+            it.rows_end);
   }
-}
-
-template <class R>
-__global__ void __launch_bounds__(R::NT) ensemble_pair_kernel(const typename R::JB* __restrict__ jb,
-                                                              const EnsItem* __restrict__ items,
-                                                              int n_items, unsigned int* counter,
-                                                              double* P, int* status) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ uint64_t full[2];
-  __shared__ int s_item;
-  pair_ensemble<R>(jb, items, n_items, counter, P, status, smem_raw, full, &s_item);
 }
 
 }  // namespace nbody

@@ -67,10 +67,15 @@ __host__ __device__ __forceinline__ int sym_q_count(int nb, int I, int tb, int t
   return E < nb ? (whole < tiles ? whole : tiles) - I * tb : tiles - I * tb + (E - nb + 1) * tb;
 }
 
-// The tile run of one CTA: tiles (first + t) mod tiles, t < nq.
+// The tile run of one CTA: tiles (first + t) mod tiles, t < nq, for the rows of
+// block I; its own sums go to slot `split`.
 struct SymRun {
-  int I, nb, tb, tiles, first, nq;
-  __device__ __forceinline__ SymRun(const SymArgs& a, int tb_) : I(blockIdx.x), nb(a.nb), tb(tb_), tiles(a.tiles) {
+  int I, nb, tb, tiles, first, nq, split;
+  __device__ __forceinline__ SymRun(int I_, int nb_, int tb_, int tiles_, int first_, int nq_, int split_)
+      : I(I_), nb(nb_), tb(tb_), tiles(tiles_), first(first_), nq(nq_), split(split_) {}
+  // CTA (blockIdx.x, blockIdx.y) = (block, split) of a grid
+  __device__ __forceinline__ SymRun(const SymArgs& a, int tb_)
+      : I(blockIdx.x), nb(a.nb), tb(tb_), tiles(a.tiles), split(blockIdx.y) {
     const int Q = sym_q_count(nb, I, tb, tiles);
     const int tps = (Q + a.S - 1) / a.S;
     const int q0 = blockIdx.y * tps;
@@ -211,22 +216,16 @@ constexpr size_t sym_fp64_smem() {
   return 2 * kSymTile64 * sizeof(JBody64) + 2 * 6 * W * 32 * sizeof(double);
 }
 
-// UNR: unrolled steps; MINB: CTAs per SM asked of the register allocator.
-template <int IPT, int W, int UNR, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB)
-    pair_sym_fp64_kernel(const JBody64* __restrict__ jb, SymArgs a) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ uint64_t full[2];
+// One run of a CTA of W warps: `half` is the half of `red` ([2][6][W][32]) of
+// the current tile, alternating over the CTA's life.  False if a wait timed out.
+template <int IPT, int W, int UNR>
+__device__ __forceinline__ bool sym_fp64_rows(TilePipe<JBody64, kSymTile64>& pipe, double* red, int& half,
+                                              const JBody64* __restrict__ jb, const SymRun& run,
+                                              const SymArgs& a) {
   constexpr int kRows = 32 * IPT * W;
   static_assert(kRows % kSymTile64 == 0, "blocks are whole tiles");
-  TilePipe<JBody64, kSymTile64> pipe;
-  pipe.init(reinterpret_cast<JBody64*>(smem_raw), full);
-  double* red = reinterpret_cast<double*>(smem_raw + 2 * kSymTile64 * sizeof(JBody64));  // [2][6][W][32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, next = (lane + 1) & 31;
-  const SymRun run(a, a.subs * (kRows / kSymTile64));
   const double eps2 = a.eps2;
-  int half = 0;  // half of `red` of the current tile, alternating over the CTA's life
-  grid_wait();
   for (int g = 0; g < a.subs; ++g) {
     const int row0 = (run.I * a.subs + g) * kRows + warp * 32 * IPT;
     if ((run.I * a.subs + g) * kRows >= a.n) break;  // a short last block
@@ -294,9 +293,8 @@ __global__ void __launch_bounds__(32 * W, MINB)
       ++t;
       half ^= 1;
     };
-    if (!run.stream(pipe, jb, a.status, consume, post)) return;
-    if (g + 1 == a.subs) grid_release();
-    double* out = a.out + static_cast<size_t>(blockIdx.y) * 6 * a.stride;
+    if (!run.stream(pipe, jb, a.status, consume, post)) return false;
+    double* out = a.out + static_cast<size_t>(run.split) * 6 * a.stride;
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
       const int r = row0 + 32 * k + lane;
@@ -305,6 +303,23 @@ __global__ void __launch_bounds__(32 * W, MINB)
         for (int c = 0; c < 6; ++c) out[static_cast<size_t>(c) * a.stride + r] = acc[k][c];
     }
   }
+  return true;
+}
+
+// UNR: unrolled steps; MINB: CTAs per SM asked of the register allocator.
+template <int IPT, int W, int UNR, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB)
+    pair_sym_fp64_kernel(const JBody64* __restrict__ jb, SymArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ uint64_t full[2];
+  TilePipe<JBody64, kSymTile64> pipe;
+  pipe.init(reinterpret_cast<JBody64*>(smem_raw), full);
+  const SymRun run(a, a.subs * (32 * IPT * W / kSymTile64));
+  int half = 0;
+  grid_wait();
+  if (sym_fp64_rows<IPT, W, UNR>(pipe, reinterpret_cast<double*>(smem_raw + 2 * kSymTile64 * sizeof(JBody64)),
+                                 half, jb, run, a))
+    grid_release();
 }
 
 // ---------------------------------------------------------------------------
@@ -404,38 +419,14 @@ struct __align__(128) SymSub {
 };
 static_assert(sizeof(SymSub) == 3200, "subtiles start 128-byte aligned");
 
-// Subtile blockIdx.x of the bodies of `in` (64 threads, one per body; bodies
-// >= n are zero-mass padding at the centre).  PREDICT: `in` is the state X, V
-// (written), with its derivatives D and step ctl, and the subtile is that of
-// the predicted state (predict_kernel's arithmetic): one pass instead of two.
-// Bound by its launch below some 10^5 bodies (104 B read, 48 + 50 written per
-// body): N = 5003 5 us instead of 5 + 5.  Zeroes near_count for the pair pass
-// that follows.
-template <bool PREDICT>
-__global__ void __launch_bounds__(64)
-    sym_tile_kernel(int n, SoA7 in, SymSub* __restrict__ out, int ld = 0, double* X = nullptr,
-                    double* V = nullptr, const double* __restrict__ D = nullptr,
-                    const StepCtl* __restrict__ ctl = nullptr,
-                    unsigned long long* near_count = nullptr, double* __restrict__ XP = nullptr) {
+// Writes one subtile from the values of the calling CTA's 64 bodies (one per
+// thread; invalid ones are zero-mass padding at the centre).
+__device__ __forceinline__ void write_subtile(SymSub* __restrict__ out, bool valid, const double p[3],
+                                              const double u[3], double m) {
   __shared__ double box[6][2];
   __shared__ float rmax[2];
   __shared__ SymSub stage;  // written out in one bulk copy
-  grid_wait();
-  grid_release();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int slot = blockIdx.x * 64 + tid;
-  const bool valid = slot < n;
-  if (near_count && slot == 0) *near_count = 0;
-  double p[3] = {0.0, 0.0, 0.0}, u[3] = {0.0, 0.0, 0.0}, m = 0.0;
-  if (valid) {
-    m = in.m[slot];
-    if (PREDICT) {
-      predict_body(ctl->dt, ld, slot, X, V, D, p, u, XP);
-    } else {
-      p[0] = in.x[slot]; p[1] = in.y[slot]; p[2] = in.z[slot];
-      u[0] = in.vx[slot]; u[1] = in.vy[slot]; u[2] = in.vz[slot];
-    }
-  }
 #pragma unroll
   for (int k = 0; k < 6; ++k) {  // bounding box in double (empty subtile: +inf/-inf)
     double w = k < 3 ? (valid ? p[k] : INFINITY) : (valid ? p[k - 3] : -INFINITY);
@@ -495,7 +486,37 @@ __global__ void __launch_bounds__(64)
   if (tid < 22) stage.pad[tid] = 0.f;
   bulk_store_fence();
   __syncthreads();
-  if (tid == 0) bulk_store(out + blockIdx.x, &stage, static_cast<uint32_t>(sizeof stage));
+  if (tid == 0) bulk_store(out, &stage, static_cast<uint32_t>(sizeof stage));
+}
+
+// Subtile blockIdx.x of the bodies of `in` (64 threads, one per body).
+// PREDICT: `in` is the state X, V (written), with its derivatives D and step
+// ctl, and the subtile is that of the predicted state (predict_kernel's
+// arithmetic): one pass instead of two.  Bound by its launch below some 10^5
+// bodies (104 B read, 48 + 50 written per body): N = 5003 5 us instead of 5 +
+// 5.  Zeroes near_count for the pair pass that follows.
+template <bool PREDICT>
+__global__ void __launch_bounds__(64)
+    sym_tile_kernel(int n, SoA7 in, SymSub* __restrict__ out, int ld = 0, double* X = nullptr,
+                    double* V = nullptr, const double* __restrict__ D = nullptr,
+                    const StepCtl* __restrict__ ctl = nullptr,
+                    unsigned long long* near_count = nullptr, double* __restrict__ XP = nullptr) {
+  grid_wait();
+  grid_release();
+  const int slot = blockIdx.x * 64 + threadIdx.x;
+  const bool valid = slot < n;
+  if (near_count && slot == 0) *near_count = 0;
+  double p[3] = {0.0, 0.0, 0.0}, u[3] = {0.0, 0.0, 0.0}, m = 0.0;
+  if (valid) {
+    m = in.m[slot];
+    if (PREDICT) {
+      predict_body(ctl->dt, ld, slot, X, V, D, p, u, XP);
+    } else {
+      p[0] = in.x[slot]; p[1] = in.y[slot]; p[2] = in.z[slot];
+      u[0] = in.vx[slot]; u[1] = in.vy[slot]; u[2] = in.vz[slot];
+    }
+  }
+  write_subtile(out + blockIdx.x, valid, p, u, m);
 }
 
 __device__ __forceinline__ uint64_t f2_dup(float v) { return f2_pack(v, v); }
@@ -561,27 +582,36 @@ constexpr size_t sym_nf_smem() {
          2 * SUB * 6 * W * 32 * sizeof(uint64_t);
 }
 
-// SUB subtiles per tile (one barrier each); UNR / NUNR: unrolled steps of the
-// far / near loop (two bodies per lane and step).
-template <int IPT, int W, int SUB, int UNR, int NUNR, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB)
-    pair_sym_nf_kernel(const SymSub* __restrict__ jt, SymArgs a) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ uint64_t full[2];
+// A CTA's shared memory.
+template <int IPT, int W, int SUB>
+struct SymNfSmem {
+  SymSub* tiles;   // [2][SUB]
+  double* acc;     // [6 IPT][NT]
+  float* xhl;      // [6 IPT][NT]
+  uint64_t* red;   // [2][SUB][6][W][32]
+  __device__ __forceinline__ explicit SymNfSmem(unsigned char* raw)
+      : tiles(reinterpret_cast<SymSub*>(raw)),
+        acc(reinterpret_cast<double*>(raw + 2 * SUB * sizeof(SymSub))),
+        xhl(reinterpret_cast<float*>(acc + 6 * IPT * 32 * W)),
+        red(reinterpret_cast<uint64_t*>(xhl + 6 * IPT * 32 * W)) {}
+};
+
+// One run of a CTA of W warps: SUB subtiles per tile (one barrier each); UNR /
+// NUNR: unrolled steps of the far / near loop (two bodies per lane and step).
+// `half` is the half of `red` of the current tile, alternating over the CTA's
+// life; near_subs counts this warp's near subtiles.  False if a wait timed out.
+template <int IPT, int W, int SUB, int UNR, int NUNR>
+__device__ __forceinline__ bool sym_nf_rows(TilePipe<SymSub, SUB>& pipe, const SymNfSmem<IPT, W, SUB>& sm,
+                                            int& half, int& near_subs, const SymSub* __restrict__ jt,
+                                            const SymRun& run, const SymArgs& a) {
   constexpr int NT = 32 * W, kRows = 32 * IPT * W, TJ = 64 * SUB;
   static_assert(kRows % TJ == 0, "blocks are whole tiles");
-  TilePipe<SymSub, SUB> pipe;
-  pipe.init(reinterpret_cast<SymSub*>(smem_raw), full);
-  double* acc = reinterpret_cast<double*>(smem_raw + 2 * SUB * sizeof(SymSub));  // [6 IPT][NT]
-  float* xhl = reinterpret_cast<float*>(acc + 6 * IPT * NT);                     // [6 IPT][NT]
-  uint64_t* red = reinterpret_cast<uint64_t*>(xhl + 6 * IPT * NT);  // [2][SUB][6][W][32]
+  double* const acc = sm.acc;
+  float* const xhl = sm.xhl;
+  uint64_t* const red = sm.red;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, next = (lane + 1) & 31;
-  const SymRun run(a, a.subs * (kRows / TJ));
   const float e2 = static_cast<float>(a.eps2);
   const uint64_t eps2 = f2_dup(e2), m3 = f2_dup(-3.0f);
-  int half = 0;  // half of `red` of the current tile, alternating over the CTA's life
-  int near_subs = 0;
-  grid_wait();
   for (int g = 0; g < a.subs; ++g) {
     const int row0 = (run.I * a.subs + g) * kRows + warp * 32 * IPT;
     if ((run.I * a.subs + g) * kRows >= a.n) break;  // a short last block
@@ -748,9 +778,8 @@ __global__ void __launch_bounds__(32 * W, MINB)
       ++t;
       half ^= 1;
     };
-    if (!run.stream(pipe, jt, a.status, consume, post)) return;
-    if (g + 1 == a.subs) grid_release();
-    double* out = a.out + static_cast<size_t>(blockIdx.y) * 6 * a.stride;
+    if (!run.stream(pipe, jt, a.status, consume, post)) return false;
+    double* out = a.out + static_cast<size_t>(run.split) * 6 * a.stride;
 #pragma unroll
     for (int k = 0; k < IPT; ++k) {
       const int r = row0 + 32 * k + lane;
@@ -760,8 +789,102 @@ __global__ void __launch_bounds__(32 * W, MINB)
           out[static_cast<size_t>(c) * a.stride + r] = acc[(c * IPT + k) * NT + tid];
     }
   }
-  if (a.near_count && lane == 0 && near_subs)
+  return true;
+}
+
+template <int IPT, int W, int SUB, int UNR, int NUNR, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB)
+    pair_sym_nf_kernel(const SymSub* __restrict__ jt, SymArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ uint64_t full[2];
+  const SymNfSmem<IPT, W, SUB> sm(smem_raw);
+  TilePipe<SymSub, SUB> pipe;
+  pipe.init(sm.tiles, full);
+  const SymRun run(a, a.subs * (32 * IPT * W / (64 * SUB)));
+  int half = 0, near_subs = 0;
+  grid_wait();
+  if (!sym_nf_rows<IPT, W, SUB, UNR, NUNR>(pipe, sm, half, near_subs, jt, run, a)) return;
+  grid_release();
+  if (a.near_count && (threadIdx.x & 31) == 0 && near_subs)
     atomicAdd(a.near_count, static_cast<unsigned long long>(near_subs));
+}
+
+// ---------------------------------------------------------------------------
+// Ensembles: one persistent launch over a work list of (cluster, block of 256
+// rows, part of its tile run) items; CTAs take items from an atomic counter
+// (zeroed before each launch) until the list is exhausted.  Cluster segments
+// are padded to whole blocks, so a cluster's records are its own tiles.
+// ---------------------------------------------------------------------------
+// The item's run; TJ: bodies per tile.
+__device__ __forceinline__ SymRun item_run(const EnsItem& it, int TJ) {
+  const int block = kEnsRows * it.subs;
+  return SymRun(it.row0 / block, it.nb, block / TJ, (it.rows_end + TJ - 1) / TJ, it.t_begin, it.nt, it.split);
+}
+__device__ __forceinline__ SymArgs item_args(const EnsItem& it, double* P, int* status) {
+  SymArgs a{};
+  a.n = it.rows_end;
+  a.ld = it.ld;
+  a.nb = it.nb;
+  a.subs = it.subs;
+  a.S = it.S;
+  a.eps2 = it.eps2;
+  a.out = P + it.p_off;
+  a.stride = static_cast<size_t>(it.ld);
+  a.status = status;
+  return a;
+}
+
+template <int IPT, int W, int UNR, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB) ensemble_sym_fp64_kernel(
+    const JBody64* __restrict__ jb, const EnsItem* __restrict__ items, int n_items, unsigned int* counter,
+    double* P, int* status, SoA7) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ uint64_t full[2];
+  __shared__ int s_item;
+  static_assert(32 * IPT * W == kEnsRows, "an item's rows are one padding unit");
+  TilePipe<JBody64, kSymTile64> pipe;
+  pipe.init(reinterpret_cast<JBody64*>(smem_raw), full);
+  int half = 0;
+  for (;;) {
+    if (threadIdx.x == 0) s_item = static_cast<int>(atomicAdd(counter, 1u));
+    __syncthreads();
+    const int k = s_item;
+    __syncthreads();
+    if (k >= n_items) return;
+    const EnsItem it = items[k];
+    if (!sym_fp64_rows<IPT, W, UNR>(
+            pipe, reinterpret_cast<double*>(smem_raw + 2 * kSymTile64 * sizeof(JBody64)), half,
+            jb + it.jrow0, item_run(it, kSymTile64), item_args(it, P, status)))
+      return;
+  }
+}
+
+template <int IPT, int W, int SUB, int UNR, int NUNR, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB) ensemble_sym_nf_kernel(
+    const SymSub* __restrict__ jt, const EnsItem* __restrict__ items, int n_items, unsigned int* counter,
+    double* P, int* status, SoA7 rows) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ uint64_t full[2];
+  __shared__ int s_item;
+  static_assert(32 * IPT * W == kEnsRows, "an item's rows are one padding unit");
+  const SymNfSmem<IPT, W, SUB> sm(smem_raw);
+  TilePipe<SymSub, SUB> pipe;
+  pipe.init(sm.tiles, full);
+  int half = 0, near_subs = 0;
+  for (;;) {
+    if (threadIdx.x == 0) s_item = static_cast<int>(atomicAdd(counter, 1u));
+    __syncthreads();
+    const int k = s_item;
+    __syncthreads();
+    if (k >= n_items) return;
+    const EnsItem it = items[k];
+    SymArgs a = item_args(it, P, status);
+    a.rows = SoA7{rows.x + it.jrow0, rows.y + it.jrow0, rows.z + it.jrow0, rows.m + it.jrow0,
+                  rows.vx + it.jrow0, rows.vy + it.jrow0, rows.vz + it.jrow0};
+    if (!sym_nf_rows<IPT, W, SUB, UNR, NUNR>(pipe, sm, half, near_subs, jt + it.jrow0 / 64,
+                                             item_run(it, 64 * SUB), a))
+      return;
+  }
 }
 
 }  // namespace nbody

@@ -247,3 +247,36 @@ def test_energy_edges(n):
     for got, compat in ((U, False), (Uc, True)):
         want = O.potential(s, EPS2, compat=compat) if n > 1 else 0.0
         assert abs(got - want) <= 1e-12 * abs(want), (n, compat, got, want)
+
+
+# clusters around the edges of tiles (32, 64) and blocks (256), odd and even
+# block counts, one of more than 128 blocks (two 256-row sub-blocks per block);
+# items of one tile and of more than a run.  Bounds of the FP64 and mixed
+# kernels against the oracle.
+@pytest.mark.parametrize("precision,variant", [("fp64", 0), ("mixed", 0), ("mixed", 4)])
+@pytest.mark.parametrize("tpi", [0, 1, 1000])
+def test_ensemble_edges(precision, variant, tpi):
+    sizes = [1, 31, 33, 64, 255, 256, 257, 513, 1000, 1281, 2] + ([33000] if tpi != 1 else [])
+    parts = [bodies(n, seed=5 + c) for c, n in enumerate(sizes)]
+    cat = {k: np.concatenate([p[k] for p in parts]) for k in nb.FIELDS}
+    with nb.Ensemble(sizes, EPS2, 1 / 512, precision=precision, pair_variant=variant, tiles_per_item=tpi) as e:
+        e.set_state(cat)
+        e.force_calculation()
+        d, off = e.get_derivs(), e.offsets
+        st = e.get_state()
+    for k in st:
+        assert np.array_equal(st[k], cat[k]), k
+    for c, n in enumerate(sizes):
+        if n == 1:
+            assert np.all(d[:, off[c]] == 0.0)
+            continue
+        rows = np.arange(n) if n <= 2000 else np.arange(0, n, 331)
+        ref = O.force_rows(parts[c], EPS2, rows)
+        ok = np.abs(ref[:3]).max(axis=0) > 0
+        got = d[:, off[c]:off[c + 1]][:, rows]
+        assert np.all(got[:, ~ok] == 0.0)
+        ea, ej = vec_rel(got[:3, ok], ref[:3, ok]), vec_rel(got[3:, ok], ref[3:, ok])
+        if precision == "fp64":
+            assert ea.max() <= 1e-12 and ej.max() <= 1e-12, (c, n, ea.max(), ej.max())
+        else:
+            assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4 and np.median(ej) <= 1e-5, (c, n)
