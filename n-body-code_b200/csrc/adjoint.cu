@@ -315,7 +315,7 @@ const void* fwd_fp64(bool wide) {
 }
 const void* fwd_mixed(bool wide) {
   return wide ? reinterpret_cast<const void*>(&pair_sym_nf_kernel<4, kW, 2, 4, 2, 3>)
-              : reinterpret_cast<const void*>(&pair_sym_nf_kernel<2, kW, 1, 4, 2, 4>);
+              : reinterpret_cast<const void*>(&pair_sym_nf_kernel<2, kW, 1, 4, 8, 4>);
 }
 const void* vjp_fn() { return reinterpret_cast<const void*>(&vjp_sym_kernel<2, kW, 2, 2>); }
 

@@ -181,7 +181,7 @@ const std::vector<PairKernel>& registry() {
   static const std::vector<PairKernel> r = {
       // symmetric: sym_kernel chooses by size
       make_sym_fp64<4, 4, 2, 2>(), make_sym_fp64<2, 4, 4, 4>(),
-      make_sym_nf<4, 4, 2, 4, 2, 3>(), make_sym_nf<2, 4, 1, 4, 2, 4>(),
+      make_sym_nf<4, 4, 2, 4, 2, 3>(), make_sym_nf<2, 4, 1, 4, 8, 4>(),
       make_fp64<128, 2, 128, 1>(),  make_fp64<128, 1, 128, 4>(),  make_fp64<128, 4, 128, 1>(),
       make_fp64<256, 1, 128, 4>(),  make_fp64<256, 2, 128, 1>(),  make_fp64<128, 2, 256, 1>(),
       make_fp64<64, 2, 128, 1>(),   make_fp64<128, 2, 64, 1, 6>(),
@@ -577,8 +577,11 @@ bool tuned_lookup(const nbody_engine* e, int rows, Tiling* out, bool full = true
 // rows per lane from 16384 bodies, two below, where twice the blocks fill the
 // SMs.  Pair pass in us, two / four rows / one-sided: FP64 N = 16384 386 /
 // 380 / 539, 8192 106 / 106 / 144, 4096 36 / 34 / 44, 1024 11.3 / 13.2 / 15;
-// mixed N = 16384 226 / 227 / 300, 8192 73 / 81 / 88, 4096 26 / 34 / 33, 1024
-// 13.5 / 21.5 / 18.
+// mixed N = 16384 218 / 224 / 300, 8192 69 / 71 / 88, 4096 24 / 38 / 33, 1024
+// 11.2 / 28 / 18.  The mixed two-row kernel unrolls its near loop eight times
+// instead of twice: without an order of the bodies every subtile is near, and
+// its chain of 32 rotations is what a small system waits for (N = 5003 36 ->
+// 32 us, 14000 184 -> 168 us).
 const PairKernel* sym_kernel(const nbody_engine* e, int n) {
   const int want = n >= 16384 ? 4 : 2;
   for (const auto& k : registry())
