@@ -305,9 +305,8 @@ __global__ void copy_rows_kernel(int n, int ld, GatherArgs g, bool pad) {
     if (s_ != NBODY_OK) return s_; \
   } while (0)
 
-// Symmetric kernels of the forward (four rows per lane from kWideN bodies, two
-// below, as the engine) and of the VJP.
-constexpr int kWideN = 16384;
+// Symmetric kernels of the forward (two and four rows per lane, as the engine)
+// and of the VJP.
 constexpr int kW = 4;  // warps per CTA
 const void* fwd_fp64(bool wide) {
   return wide ? reinterpret_cast<const void*>(&pair_sym_fp64_kernel<4, kW, 2, 2>)
@@ -324,14 +323,17 @@ struct SymLaunch {
   const void* fn = nullptr;
   size_t smem = 0;
   int rows = 0, tj = 0, S = 1, subs = 1, nb = 1, block_rows = 1;
-  cudaError_t plan(const void* f, size_t sm, int rows_, int tj_, int n, int sms, double per_ms, bool waves) {
+  double ms = 0;  // predicted
+  cudaError_t plan(const void* f, size_t sm, int rows_, int tj_, int n, int sms, double rate, double tail) {
     fn = f; smem = sm; rows = rows_; tj = tj_;
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
     if (e != cudaSuccess) return e;
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, 32 * kW, sm);
     if (e != cudaSuccess) return e;
-    S = sym_splits(sms, std::max(occ, 1), rows, tj, n, per_ms, waves);
+    const SymPlan p = sym_plan(sms, std::max(occ, 1), rows, tj, n, rate, tail);
+    S = p.S;
+    ms = p.ms;
     const SymGrid g(rows, n);
     subs = g.subs; nb = g.nb; block_rows = g.block_rows;
     return cudaSuccess;
@@ -539,13 +541,18 @@ nbody_status nbody_adjoint_create(nbody_adjoint** out, const nbody_adjoint_confi
   nbody_adjoint* r = a.get();
   auto body = [&]() -> nbody_status {
     const size_t ld = r->ld;
-    const bool fp64 = cfg->precision == NBODY_FP64, wide = r->n >= kWideN;
-    const int ipt = wide ? 4 : 2;
-    const size_t fwd_smem = fp64 ? (wide ? sym_fp64_smem<4, kW, 2>() : sym_fp64_smem<2, kW, 4>())
-                                 : (wide ? sym_nf_smem<4, kW, 2>() : sym_nf_smem<2, kW, 1>());
-    AD_CUDA(r->fwd.plan(fp64 ? fwd_fp64(wide) : fwd_mixed(wide), fwd_smem, 32 * kW * ipt,
-                        fp64 ? kSymTile64 : wide ? 128 : 64, r->n, r->sms, fp64 ? 7.6e8 : 1.6e9, fp64));
-    AD_CUDA(r->rev.plan(vjp_fn(), vjp_smem<2, kW>(), 32 * kW * 2, kVjpTile, r->n, r->sms, 3.3e8, true));
+    const bool fp64 = cfg->precision == NBODY_FP64;
+    for (const bool wide : {false, true}) {  // the engine's choice
+      if (r->n < sym_min_bodies(wide)) continue;
+      const size_t smem = fp64 ? (wide ? sym_fp64_smem<4, kW, 2>() : sym_fp64_smem<2, kW, 4>())
+                               : (wide ? sym_nf_smem<4, kW, 2>() : sym_nf_smem<2, kW, 1>());
+      SymLaunch l;
+      AD_CUDA(l.plan(fp64 ? fwd_fp64(wide) : fwd_mixed(wide), smem, 32 * kW * (wide ? 4 : 2),
+                     fp64 ? kSymTile64 : wide ? 128 : 64, r->n, r->sms, sym_rate(fp64, wide),
+                     fp64 ? kSymTail64 : kSymTailNF));
+      if (!wide || l.ms < r->fwd.ms) r->fwd = l;
+    }
+    AD_CUDA(r->rev.plan(vjp_fn(), vjp_smem<2, kW>(), 32 * kW * 2, kVjpTile, r->n, r->sms, 3.3e8, kSymTail64));
     AD_CUDA(cudaMalloc(&r->state, sizeof(double) * 13 * ld));
     AD_CUDA(cudaMemset(r->state, 0, sizeof(double) * 13 * ld));
     r->X = r->state;

@@ -179,7 +179,7 @@ PairKernel make_mixed_nf_cl() {
 // passes with an automatic tiling; the autotuner times them.
 const std::vector<PairKernel>& registry() {
   static const std::vector<PairKernel> r = {
-      // symmetric: sym_kernel chooses by size
+      // symmetric: choose_sym chooses by predicted time
       make_sym_fp64<4, 4, 2, 2>(), make_sym_fp64<2, 4, 4, 4>(),
       make_sym_nf<4, 4, 2, 4, 2, 3>(), make_sym_nf<2, 4, 1, 4, 8, 4>(),
       make_fp64<128, 2, 128, 1>(),  make_fp64<128, 1, 128, 4>(),  make_fp64<128, 4, 128, 1>(),
@@ -443,15 +443,16 @@ int choose_split(const nbody_engine* e, const PairKernel& k, int rows) {
   return best_s;
 }
 
-// Splits of the symmetric kernel k over n bodies.
-int choose_sym_split(const nbody_engine* e, const PairKernel& k, int n) {
+// Splits and predicted time of the symmetric kernel k over n bodies.
+SymPlan plan_sym(const nbody_engine* e, const PairKernel& k, int n) {
   prepare_kernel(k);
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, k.nt, k.smem) != cudaSuccess ||
       occ < 1)
     occ = 1;
   const bool fp64 = k.precision == NBODY_FP64;
-  return sym_splits(e->num_sms, occ, k.nt * k.ipt, k.tj, n, fp64 ? 7.6e8 : 1.6e9, fp64);
+  return sym_plan(e->num_sms, occ, k.nt * k.ipt, k.tj, n, sym_rate(fp64, k.ipt == 4),
+                  fp64 ? kSymTail64 : kSymTailNF);
 }
 
 void drop_step_graphs(nbody_engine* e) {
@@ -573,20 +574,27 @@ bool tuned_lookup(const nbody_engine* e, int rows, Tiling* out, bool full = true
   return true;
 }
 
-// The symmetric kernel an automatic full-row pass over n bodies takes.  Four
-// rows per lane from 16384 bodies, two below, where twice the blocks fill the
-// SMs.  Pair pass in us, two / four rows / one-sided: FP64 N = 16384 386 /
-// 380 / 539, 8192 106 / 106 / 144, 4096 36 / 34 / 44, 1024 11.3 / 13.2 / 15;
-// mixed N = 16384 218 / 224 / 300, 8192 69 / 71 / 88, 4096 24 / 38 / 33, 1024
-// 11.2 / 28 / 18.  The mixed two-row kernel unrolls its near loop eight times
-// instead of twice: without an order of the bodies every subtile is near, and
-// its chain of 32 rotations is what a small system waits for (N = 5003 36 ->
-// 32 us, 14000 184 -> 168 us).
-const PairKernel* sym_kernel(const nbody_engine* e, int n) {
-  const int want = n >= 16384 ? 4 : 2;
-  for (const auto& k : registry())
-    if (k.sym && k.precision == e->cfg.precision && k.ipt == want) return &k;
-  return nullptr;
+// The symmetric kernel and splits of an automatic full-row pass over n bodies:
+// of two and four rows per lane the one whose predicted time is less.  Twice
+// the blocks of two rows fill the SMs where four leave them idle; four rows
+// read each j-body half as often.  Pair pass in us at the best split, two /
+// four rows / one-sided: FP64 N = 16384 397 / 385 / 539, 8192 107 / 104 / 144,
+// 4096 36 / 34 / 44, 1024 8.7 / 12 / 15; mixed N = 65536 3040 / 2770 / 4000,
+// 16384 209 / 219 / 300, 8192 66 / 71 / 88, 4096 24 / 38 / 33, 1024 11 / 28 /
+// 18.  The mixed two-row kernel unrolls its near loop eight times instead of
+// twice: without an order of the bodies every subtile is near, and its chain
+// of 32 rotations is what a small system waits for (N = 5003 36 -> 32 us,
+// 14000 184 -> 168 us).
+void choose_sym(const nbody_engine* e, int n, Tiling* out) {
+  double best = 1e300;
+  for (const auto& k : registry()) {
+    if (!k.sym || k.precision != e->cfg.precision || n < sym_min_bodies(k.ipt == 4)) continue;
+    const SymPlan p = plan_sym(e, k, n);
+    if (p.ms >= best) continue;
+    best = p.ms;
+    out->k = &k;
+    out->split = p.S;
+  }
 }
 
 nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
@@ -607,7 +615,7 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
     // the symmetric kernels: faster than every one-sided shape in full-row
     // passes at each size from 1024 to 262144
     if (!k.sym || k.precision != e->cfg.precision) continue;
-    const int s0 = choose_sym_split(e, k, rows);
+    const int s0 = plan_sym(e, k, rows).S;
     NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj));
     for (int s : {std::max(1, s0 / 2), s0, std::min(kMaxSplit, s0 * 2)}) {
       Tiling t{&k, s};
@@ -672,8 +680,7 @@ nbody_status get_tiling(nbody_engine* e, int rows, Tiling* out, bool full = true
   if (e->tune_lookup && automatic && tuned_lookup(e, rows, out, full)) return NBODY_OK;
   const bool near_far = c.precision == NBODY_MIXED && c.pair_variant == 4;
   if (full && (automatic || (near_far && !explicit_shape(c)))) {
-    out->k = sym_kernel(e, rows);
-    out->split = choose_sym_split(e, *out->k, rows);
+    choose_sym(e, rows, out);
     out->source = 1;
     return NBODY_OK;
   }
@@ -1319,9 +1326,7 @@ nbody_status nbody_energy(nbody_engine* e, int ref_compat, double* T, double* U)
   a.nb = g.nb;
   a.subs = g.subs;
   a.tiles = (e->n + k.tj - 1) / k.tj;
-  int occ = 0;
-  NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, 32 * kPotWarps, k.smem));
-  a.S = sym_splits(e->num_sms, std::max(1, occ), k.rows, k.tj, e->n, 2.4e9, true);
+  a.S = potential_splits(e->num_sms, k.rows, k.tj, e->n);
   a.eps2 = e->cfg.eps2;
   a.status = e->status;
   const void* jb = e->jbe;

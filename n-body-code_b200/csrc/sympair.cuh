@@ -135,41 +135,108 @@ struct SymGrid {
 // us): the price of each partial a tiling leaves.
 constexpr double kSplitSumBytesPerMs = 3.9e9;
 
-// Splits of a symmetric kernel over n bodies: S CTAs per block share its run
-// of Q tiles, ceil(Q / S) each.  Cost in units of one (CTA, tile); per_ms:
-// interactions a full GPU evaluates per ms.  FP64 CTAs (waves) take the same
-// time each and run in waves, the last of which takes what its fullest SM
-// holds (three quarters of a tile's time are throughput).  The near/far
-// kernel's differ with their near subtiles: the work of more CTAs than are
-// resident spreads over the slots, and the last ones leave SMs idle for about
-// a third of a CTA's time.  Every split is another 48 bytes per row to sum.
-// Pair pass in ms by splits: FP64 N = 16384 0.464 (8) 0.39 (23) 0.405 (31),
-// 65536 5.79 (8) 5.69 (31); mixed 16384 0.265 (9) 0.223 (31), 65536 2.91 (9)
-// 2.77 (31).
-inline int sym_splits(int sms, int occ, int rows, int tj, int n, double per_ms, bool waves) {
-  const SymGrid g(rows, n);
-  const int Q = sym_q_count(g.nb, 0, g.block_rows / tj, (n + tj - 1) / tj);
-  const long slots = static_cast<long>(sms) * occ;
-  const double tile_ms = 2.0 * rows * tj * slots / per_ms;
-  const double per_split = 48.0 * n / kSplitSumBytesPerMs / tile_ms;
-  double best = 1e300;
-  int best_s = 1;
-  for (int tps = 1; tps <= Q; ++tps) {
-    const int s = (Q + tps - 1) / tps;
-    if (s > std::min(kMaxSymSplits, max_sym_slots(n) / 2)) continue;
-    const long ctas = static_cast<long>(g.nb) * s;
-    const double one = tps * g.subs + 0.5;
-    const bool in_waves = waves || ctas <= slots;
-    const long last = in_waves ? ctas % slots : 0;
-    const double per_sm = static_cast<double>((last + sms - 1) / sms) / occ;
-    double work = in_waves ? one * (ctas / slots) : one * ctas / slots;
-    if (last) work += one * (0.25 + 0.75 * per_sm);
-    const double cost = work + (waves ? 0.1 : 0.35) * one + per_split * s;
-    if (cost < best - 1e-9) {
-      best = cost;
-      best_s = s;
-    }
+// Interactions per ms of a GPU full of a pass's CTAs (fitted, see sym_plan).
+inline double sym_rate(bool fp64, bool wide) {
+  return fp64 ? (wide ? 7.87e8 : 7.44e8) : (wide ? 1.667e9 : 1.505e9);
+}
+// Smallest system for a kernel.  With one or two tiles a CTA, latency counts,
+// which the prediction leaves out: a four-row CTA's tile takes 11.5 us alone on
+// its SM, a two-row one's 6 (FP64 N = 1831, a step: 31.3 us against 27.9).
+inline int sym_min_bodies(bool wide) { return wide ? 4096 : 0; }
+// Time of the last CTAs that leave SMs idle, in units of one CTA's time: the
+// near/far kernel's CTAs differ with their near subtiles.
+constexpr double kSymTail64 = 0.12, kSymTailNF = 0.2;
+constexpr double kSymCtaTiles = 0.2;  // overhead of a CTA in tiles
+
+// One way of splitting the blocks' runs: S CTAs per block, tps tiles each.
+struct SymSplit {
+  int S, tps;   // tps: of the longest run
+  long ctas;    // with tiles
+  double mean;  // tiles of one
+};
+// Calls f for every split into at most max_s CTAs per block that differs from
+// the ones into fewer.
+template <class F>
+inline void for_sym_splits(const SymGrid& g, int tj, int n, int max_s, F&& f) {
+  const int tb = g.block_rows / tj, tiles = (n + tj - 1) / tj;
+  int Q = 0;
+  long total = 0;
+  for (int I = 0; I < g.nb; ++I) {
+    const int q = sym_q_count(g.nb, I, tb, tiles);
+    Q = std::max(Q, q);
+    total += q;
   }
+  for (int s = 1; s <= max_s; ++s) {
+    const int tps = (Q + s - 1) / s;
+    if ((Q + tps - 1) / tps != s) continue;
+    long ctas = 0;
+    for (int I = 0; I < g.nb; ++I) {  // as SymRun
+      const int q = sym_q_count(g.nb, I, tb, tiles), own = (q + s - 1) / s;
+      ctas += (q + own - 1) / own;
+    }
+    f(SymSplit{s, tps, ctas, static_cast<double>(total) / ctas});
+  }
+}
+
+// Splits of a symmetric kernel over n bodies and the predicted time of the
+// pass and of the sum over its slots.  rate: interactions per ms; tail: below.
+//
+// A CTA's time is its tiles and a small overhead.  C CTAs on `slots` places take
+// whole waves and one more that lasts by what its fullest SM holds, a tile's
+// time being nearly all throughput; CTAs are not equally long, so past the
+// first wave up to a third of the work does not keep to waves.  A wave that
+// would fill the last place spills (N = 2721, four rows, 296 CTAs of one tile on
+// 296 places: 24 us, two waves' time).  Each slot is 48
+// bytes per row to sum.  Fitted to the pass's time over every split of both
+// kernels at 19 (mixed, 1500 to 262144 bodies) and 13 sizes (FP64, 1024 to
+// 100000): 5 % rms; the kernel and split with the least time are on average
+// 0.6 % (4 % at most) slower than the measured best of all, at 12 sizes not
+// fitted (FP64, 1500 to 10000) 3 %, at worst 26 % (N = 4679).  Pass and sums in
+// us against a fixed line between the kernels at 16384 bodies and a model that
+// counted idle CTAs: FP64 N = 3000 25 / 28, 5003 48 / 51, 8192 107 / 122, 12000
+// 219 / 234, 65536 5744 / 5794; mixed 5003 33 / 34, 8192 69 / 73, 18001 267 /
+// 294, 32768 768 / 802, 65536 2855 / 2874.
+struct SymPlan {
+  int S;
+  double ms;
+};
+inline SymPlan sym_plan(int sms, int occ, int rows, int tj, int n, double rate, double tail) {
+  const SymGrid g(rows, n);
+  const long slots = static_cast<long>(sms) * occ;
+  const double tile_ms = 2.0 * rows * tj * slots / rate;
+  SymPlan best{1, 1e300};
+  for_sym_splits(g, tj, n, std::min(kMaxSymSplits, max_sym_slots(n) / 2), [&](const SymSplit& p) {
+    const double one = static_cast<double>(p.tps) * g.subs + kSymCtaTiles;
+    const double mean = p.mean * g.subs + kSymCtaTiles;
+    const long last = (p.ctas + 1) % slots;
+    double work = one * ((p.ctas + 1) / slots);
+    if (last) work += one * (0.08 + 0.92 * ((last + sms - 1) / sms) / occ);
+    if (p.ctas > slots) {
+      const double waves = static_cast<double>(p.ctas) / slots;
+      work += (mean * waves - work) * (1.0 - 1.0 / waves) / 3.0;
+    }
+    const double ms = tile_ms * (work + tail * one) + 48.0 * n * g.count(p.S) / kSplitSumBytesPerMs;
+    if (ms < best.ms) best = {p.S, ms};
+  });
+  return best;
+}
+
+// Splits of the potential kernel, which leaves no slots and keeps 7 to 10 CTAs
+// on an SM: the fewest tiles on the fullest SM and, for the last CTAs, two more
+// CTAs' time.  In us against sym_plan, which prices slots and waves: N = 8192
+// 77 / 88, 16384 169 / 195, 24000 292 / 305; within 4 % of the best split at 12
+// sizes from 4097 to 131072.
+inline int potential_splits(int sms, int rows, int tj, int n) {
+  const SymGrid g(rows, n);
+  long best = -1;
+  int best_s = 1;
+  for_sym_splits(g, tj, n, kMaxSymSplits, [&](const SymSplit& p) {
+    const long cost = p.tps * ((p.ctas + sms - 1) / sms + 2);
+    if (best < 0 || cost < best) {
+      best = cost;
+      best_s = p.S;
+    }
+  });
   return best_s;
 }
 

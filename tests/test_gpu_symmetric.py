@@ -32,7 +32,7 @@ def derivs(s, precision, **kw):
 
 
 # one block; tiles of 32; blocks of 256 rows, odd and even counts, short last
-# blocks; the four-row kernel (blocks of 512) from 16384
+# blocks
 @pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 256, 257, 511, 513, 768, 769, 1025, 2047, 4097])
 def test_fp64_small_edges(n):
     s = bodies(n)
@@ -49,11 +49,15 @@ def test_fp64_small_edges(n):
 
 # the last n of one block size and the first of the next; blocks of two
 # sub-blocks (from 65537), odd and even block counts
-@pytest.mark.parametrize("n", [16383, 16384, 16897, 65536, 65537, 70001])
+# (the four-row kernel serves 8192 and up, smaller ones where it fills the GPU better)
+@pytest.mark.parametrize("n", [3001, 5003, 8192, 8193, 16383, 16384, 16897, 65536, 65537, 70001])
 def test_fp64_block_edges_sampled_rows(n):
     s = bodies(n)
     d, t = derivs(s, "fp64")
-    assert t["i_per_thread"] == (4 if n >= 16384 else 2)
+    if n in (8192, 65536):  # the choice by predicted time reaches both kernels
+        assert t["i_per_thread"] == 4
+    if n == 3001:
+        assert t["i_per_thread"] == 2
     rows = np.unique(np.concatenate([np.arange(0, n, n // 60), [n - 1, n - 2, n // 2, n // 2 - 1]]))
     ref = O.force_rows(s, EPS2, rows)
     ea, ej = derivs_rel(d[:, rows], ref)
