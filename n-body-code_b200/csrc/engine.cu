@@ -898,6 +898,32 @@ nbody_status enqueue_correct(nbody_engine* e, cudaStream_t st) {
   return NBODY_OK;
 }
 
+// Whether a corrector goes straight on to the next step's predictor, one launch
+// and one pass over the state less: with a fixed step (an adaptive one is known
+// when every row is done) and slot sums in groups (correct_kernel<8>,
+// correct_tile_kernel).  A step in us, separate / joined: FP64 N = 1024 14.6 /
+// 12.9, 3000 31.8 / 29.2, 16384 408 / 405; mixed 1024 19.3 / 17.8, 3000 27.8 /
+// 26.4, 5003 42.5 / 42.7.  Larger systems do not notice the launch, and the
+// subtiles' barriers cost the sums bandwidth (mixed 65536 2879 / 2895).
+bool can_chain_steps(const nbody_engine* e) {
+  const int fmt = tiling_fmt(e);
+  const int below = fmt == kRecF64 ? 32768 : fmt == kRecSym ? 4096 : 0;
+  return e->n < below && e->cfg.dt > 0 && sum_in_groups(row_slots(e->tiling, e->n));
+}
+
+nbody_status enqueue_correct_predict(nbody_engine* e, cudaStream_t st) {
+  const RowSlots slots = row_slots(e->tiling, e->n);
+  if (tiling_fmt(e) == kRecSym)
+    correct_tile_kernel<<<e->ld / 64, kCorrectTileThreads, 0, st>>>(
+        e->n, e->ld, slots, e->P, e->X, e->V, e->D, e->ctl, e->cfg.eta, e->M,
+        static_cast<SymSub*>(e->jb32), e->near_count);
+  else
+    correct_kernel<8, true><<<(e->n + kSumRows<8> - 1) / kSumRows<8>, kSumThreads, 0, st>>>(
+        e->n, e->ld, slots, e->P, e->X, e->V, e->D, e->ctl, e->cfg.eta, e->M, e->jb64);
+  NB_CUDA(cudaGetLastError());
+  return NBODY_OK;
+}
+
 int count_kernel_nodes(cudaGraph_t g) {
   size_t nodes = 0;
   int kernels = 0;
@@ -930,13 +956,15 @@ nbody_status capture_steps(nbody_engine* e, int steps, bool timed, cudaGraphExec
         cudaEventRecordWithFlags(ev, e->stream, cudaEventRecordExternal) != cudaSuccess)
       s = fail(NBODY_ERR_CUDA, "event record during capture failed");
   };
+  const bool chain = can_chain_steps(e);  // one kernel between two steps instead of two
   for (int k = 0; k < steps && s == NBODY_OK; ++k) {
     rec(e->ev[0]);
-    if (s == NBODY_OK) s = enqueue_predict(e, e->stream);
+    if (s == NBODY_OK && (k == 0 || !chain)) s = enqueue_predict(e, e->stream);
     rec(e->ev[1]);
     if (s == NBODY_OK) s = launch_pair(e, e->tiling, 0, e->n, e->stream);
     rec(e->ev[2]);
-    if (s == NBODY_OK) s = enqueue_correct(e, e->stream);
+    if (s == NBODY_OK)
+      s = chain && k + 1 < steps ? enqueue_correct_predict(e, e->stream) : enqueue_correct(e, e->stream);
     rec(e->ev[3]);
   }
   cudaError_t ce = cudaStreamEndCapture(e->stream, &g);

@@ -170,20 +170,24 @@ static __global__ void pack_kernel(int n, int ld, SoA7 in, JBody64* __restrict__
   if (jbx2) jbx2[i] = make_jbx2(x, y, z, m, vx, vy, vz);
 }
 
+// One component's predicted position and velocity.
+__device__ __forceinline__ void predict_component(double dt, double x, double v, double a, double j,
+                                                  double& p, double& u) {
+  const double h2 = 0.5 * dt * dt;
+  const double h3 = dt * dt * dt * (1.0 / 6.0);
+  p = x + (v * dt + (a * h2 + j * h3));
+  u = v + (a * dt + j * h2);
+}
+
 // Predicted position p and velocity u of row i, written back to X, V and, if
 // not null, to XP ([6][ld]).
 __device__ __forceinline__ void predict_body(double dt, int ld, int i, double* __restrict__ X,
                                              double* __restrict__ V, const double* __restrict__ D,
                                              double p[3], double u[3],
                                              double* __restrict__ XP = nullptr) {
-  const double h2 = 0.5 * dt * dt;
-  const double h3 = dt * dt * dt * (1.0 / 6.0);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const double x = X[c * ld + i], v = V[c * ld + i];
-    const double a = D[c * ld + i], j = D[(3 + c) * ld + i];
-    p[c] = x + (v * dt + (a * h2 + j * h3));
-    u[c] = v + (a * dt + j * h2);
+    predict_component(dt, X[c * ld + i], V[c * ld + i], D[c * ld + i], D[(3 + c) * ld + i], p[c], u[c]);
     X[c * ld + i] = p[c];
     V[c * ld + i] = u[c];
     if (XP) {
@@ -275,13 +279,42 @@ __device__ __forceinline__ void slot_sums(const double* __restrict__ P, int ld, 
   }
 }
 
+// The corrector of row i (the calling thread's): snap/crackle from the pre-step
+// d = (a, j) and the new sums, corrected x, v in place; returns the Aarseth
+// criterion.
+__device__ __forceinline__ double correct_body(double dt, double eta, const double d[6],
+                                               const double sum[6], double x[3], double v[3]) {
+  const double idt2 = 1.0 / (dt * dt);
+  const double idt3 = idt2 / dt;
+  const double dt3 = dt * dt * dt, dt4 = dt3 * dt, dt5 = dt4 * dt;
+  double A2 = 0, J2 = 0, S2 = 0, C2 = 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double a1 = sum[c], j1 = sum[3 + c];
+    const double a = d[c], j = d[3 + c];
+    const double da = a - a1;
+    const double a2 = 2.0 * idt2 * (-3.0 * da - (2.0 * j + j1) * dt);
+    const double a3 = 6.0 * idt3 * (2.0 * da + (j + j1) * dt);
+    x[c] += a2 * dt4 * (1.0 / 24.0) + a3 * dt5 * (1.0 / 120.0);
+    v[c] += a2 * dt3 * (1.0 / 6.0) + a3 * dt4 * (1.0 / 24.0);
+    A2 += a * a; J2 += j * j; S2 += a2 * a2; C2 += a3 * a3;
+  }
+  const double num = sqrt(A2) * sqrt(S2) + J2;
+  const double den = sqrt(J2) * sqrt(C2) + S2;
+  return sqrt(eta * num / den);
+}
+
 // Corrector fused with the split-j reduction and the Aarseth criterion:
 // a1/j1 = sum over the row's slots of P; snap/crackle; correct X, V; D <- a1/j1.
-template <int GR>
+// PREDICT (fixed step only: an adaptive one is known when every row is done):
+// the next step's predictor on top, so X, V become its predicted state and jb64
+// its records; M: masses.
+template <int GR, bool PREDICT = false>
 static __global__ void __launch_bounds__(kSumThreads)
     correct_kernel(int n, int ld, RowSlots slots, const double* __restrict__ P,
                    double* __restrict__ X, double* __restrict__ V, double* __restrict__ D,
-                   StepCtl* __restrict__ ctl, double eta) {
+                   StepCtl* __restrict__ ctl, double eta, const double* __restrict__ M = nullptr,
+                   JBody64* __restrict__ jb64 = nullptr) {
   __shared__ double sh[GR > 1 ? 6 * kSumThreads : 32];
   grid_wait();
   grid_release();
@@ -299,26 +332,16 @@ static __global__ void __launch_bounds__(kSumThreads)
   slot_sums<GR>(P, ld, i < n ? slots.count(i) : 0, i, sum, sh);
   if (mine) {
     const double dt = ctl->dt;
-    const double idt2 = 1.0 / (dt * dt);
-    const double idt3 = idt2 / dt;
-    const double dt3 = dt * dt * dt, dt4 = dt3 * dt, dt5 = dt4 * dt;
-    double A2 = 0, J2 = 0, S2 = 0, C2 = 0;
+    crit = correct_body(dt, eta, d, sum, x, v);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const double a1 = sum[c], j1 = sum[3 + c];
-      const double a = d[c], j = d[3 + c];
-      const double da = a - a1;
-      const double a2 = 2.0 * idt2 * (-3.0 * da - (2.0 * j + j1) * dt);
-      const double a3 = 6.0 * idt3 * (2.0 * da + (j + j1) * dt);
-      X[c * ld + i] = x[c] + (a2 * dt4 * (1.0 / 24.0) + a3 * dt5 * (1.0 / 120.0));
-      V[c * ld + i] = v[c] + (a2 * dt3 * (1.0 / 6.0) + a3 * dt4 * (1.0 / 24.0));
-      D[c * ld + i] = a1;
-      D[(3 + c) * ld + i] = j1;
-      A2 += a * a; J2 += j * j; S2 += a2 * a2; C2 += a3 * a3;
+      if (PREDICT) predict_component(dt, x[c], v[c], sum[c], sum[3 + c], x[c], v[c]);
+      X[c * ld + i] = x[c];
+      V[c * ld + i] = v[c];
+      D[c * ld + i] = sum[c];
+      D[(3 + c) * ld + i] = sum[3 + c];
     }
-    const double num = sqrt(A2) * sqrt(S2) + J2;
-    const double den = sqrt(J2) * sqrt(C2) + S2;
-    crit = sqrt(eta * num / den);
+    if (PREDICT) store_jb64(jb64, i, x[0], x[1], x[2], M[i], v[0], v[1], v[2]);
   }
   if (GR > 1) __syncthreads();  // sh is reused
   finish_criterion(ctl, crit, true, sh);
@@ -377,9 +400,10 @@ static __global__ void __launch_bounds__(kSumThreads)
 }
 
 // Groups per row: eight from kSumGroupSlots slots, one below, where most
-// groups would have nothing to add.  Corrector with eight groups against one:
-// N = 1024 (26 slots) 3.9 against 10 us, N = 5003 (40) 6 against 16; N = 65536
-// (80), which the partials' bandwidth bounds, the same within 0.2 % of a step.
+// groups would have nothing to add.  Corrector with eight groups against one,
+// cold caches, N = 4096: 9.7 us over 44 slots against 18.6 over 32; a step at N =
+// 1024 39.4 against 42.4 us.  At N = 65536 (80 slots) the partials' bandwidth
+// bounds both, the same within 0.2 % of a step.
 constexpr int kSumGroupSlots = 8;
 inline bool sum_in_groups(const RowSlots& s) { return s.S + s.nb / 2 >= kSumGroupSlots; }
 
@@ -388,7 +412,7 @@ inline void launch_correct(cudaStream_t st, int n, int ld, RowSlots slots, const
                            bool chained = false) {
   if (sum_in_groups(slots) && chained)
     launch_chained(correct_kernel<8>, (n + kSumRows<8> - 1) / kSumRows<8>, kSumThreads, 0, st, n, ld,
-                   slots, P, X, V, D, ctl, eta);
+                   slots, P, X, V, D, ctl, eta, static_cast<const double*>(nullptr), static_cast<JBody64*>(nullptr));
   else if (sum_in_groups(slots))
     correct_kernel<8><<<(n + kSumRows<8> - 1) / kSumRows<8>, kSumThreads, 0, st>>>(
         n, ld, slots, P, X, V, D, ctl, eta);

@@ -486,8 +486,8 @@ struct __align__(128) SymSub {
 };
 static_assert(sizeof(SymSub) == 3200, "subtiles start 128-byte aligned");
 
-// Writes one subtile from the values of the calling CTA's 64 bodies (one per
-// thread; invalid ones are zero-mass padding at the centre).
+// Writes one subtile from the values of the calling CTA's first 64 threads' 64
+// bodies (invalid ones are zero-mass padding at the centre); called by all.
 __device__ __forceinline__ void write_subtile(SymSub* __restrict__ out, bool valid, const double p[3],
                                               const double u[3], double m) {
   __shared__ double box[6][2];
@@ -498,7 +498,7 @@ __device__ __forceinline__ void write_subtile(SymSub* __restrict__ out, bool val
   for (int k = 0; k < 6; ++k) {  // bounding box in double (empty subtile: +inf/-inf)
     double w = k < 3 ? (valid ? p[k] : INFINITY) : (valid ? p[k - 3] : -INFINITY);
     w = k < 3 ? warp_min(w) : warp_max(w);
-    if (lane == 0) box[k][warp] = w;
+    if (lane == 0 && warp < 2) box[k][warp] = w;
   }
   __syncthreads();
   double lo[3], hi[3];
@@ -516,7 +516,7 @@ __device__ __forceinline__ void write_subtile(SymSub* __restrict__ out, bool val
   float R = __double2float_ru(sqrt(r2));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
-  if (lane == 0) rmax[warp] = R;
+  if (lane == 0 && warp < 2) rmax[warp] = R;
   __syncthreads();
   if (tid == 0) {
 #pragma unroll
@@ -536,20 +536,22 @@ __device__ __forceinline__ void write_subtile(SymSub* __restrict__ out, bool val
     oh[k] = -dh;
     ol[k] = -dl;
   }
-  // body tid = half `warp` of lane `lane`'s pairs; word w of chunk q at [128 q + 2 w]
-  float* f = reinterpret_cast<float*>(&stage.v[0][lane]) + warp;
-  f[0] = oh[0];
-  f[2] = oh[1];
-  f[128] = oh[2];
-  f[130] = __double2float_rn(m);
-  f[256] = __double2float_rn(u[0]);
-  f[258] = __double2float_rn(u[1]);
-  f[384] = __double2float_rn(u[2]);
-  f[386] = 0.f;
-  f[512] = ol[0];
-  f[514] = ol[1];
-  f[640] = ol[2];
-  f[642] = 0.f;
+  if (tid < 64) {
+    // body tid = half `warp` of lane `lane`'s pairs; word w of chunk q at [128 q + 2 w]
+    float* f = reinterpret_cast<float*>(&stage.v[0][lane]) + warp;
+    f[0] = oh[0];
+    f[2] = oh[1];
+    f[128] = oh[2];
+    f[130] = __double2float_rn(m);
+    f[256] = __double2float_rn(u[0]);
+    f[258] = __double2float_rn(u[1]);
+    f[384] = __double2float_rn(u[2]);
+    f[386] = 0.f;
+    f[512] = ol[0];
+    f[514] = ol[1];
+    f[640] = ol[2];
+    f[642] = 0.f;
+  }
   if (tid < 22) stage.pad[tid] = 0.f;
   bulk_store_fence();
   __syncthreads();
@@ -560,8 +562,8 @@ __device__ __forceinline__ void write_subtile(SymSub* __restrict__ out, bool val
 // PREDICT: `in` is the state X, V (written), with its derivatives D and step
 // ctl, and the subtile is that of the predicted state (predict_kernel's
 // arithmetic): one pass instead of two.  Bound by its launch below some 10^5
-// bodies (104 B read, 48 + 50 written per body): N = 5003 5 us instead of 5 +
-// 5.  Zeroes near_count for the pair pass that follows.
+// bodies (104 B read, 48 + 50 written per body): the phase at N = 65536 9.6 us
+// instead of 12.6.  Zeroes near_count for the pair pass that follows.
 template <bool PREDICT>
 __global__ void __launch_bounds__(64)
     sym_tile_kernel(int n, SoA7 in, SymSub* __restrict__ out, int ld = 0, double* X = nullptr,
@@ -584,6 +586,57 @@ __global__ void __launch_bounds__(64)
     }
   }
   write_subtile(out + blockIdx.x, valid, p, u, m);
+}
+
+// correct_kernel<8, true> for the near/far records: corrector and the next
+// step's predictor on the 64 bodies of subtile blockIdx.x (64 rows times eight
+// groups of threads, the sums in correct_kernel<8>'s order), and the subtile.
+constexpr int kCorrectTileThreads = 512;
+static __global__ void __launch_bounds__(kCorrectTileThreads)
+    correct_tile_kernel(int n, int ld, RowSlots slots, const double* __restrict__ P,
+                        double* __restrict__ X, double* __restrict__ V, double* __restrict__ D,
+                        StepCtl* __restrict__ ctl, double eta, const double* __restrict__ M,
+                        SymSub* __restrict__ out, unsigned long long* near_count) {
+  __shared__ double sh[6 * kCorrectTileThreads];
+  const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int i = blockIdx.x * 64 + r;
+  const bool mine = i < n && g == 0;
+  if (near_count && blockIdx.x == 0 && threadIdx.x == 0) *near_count = 0;
+  double crit = __longlong_as_double(static_cast<long long>(kPosInfBits));
+  double x[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0}, d[6], m = 0.0;
+  if (mine) {
+    m = M[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      x[c] = X[c * ld + i]; v[c] = V[c * ld + i];
+      d[c] = D[c * ld + i]; d[3 + c] = D[(3 + c) * ld + i];
+    }
+  }
+  const int S = i < n ? slots.count(i) : 0;
+  double sum[6];
+  split_sums(P + static_cast<size_t>(g) * 6 * ld, ld, (S - g + 7) / 8, i, sum, 8);
+#pragma unroll
+  for (int c = 0; c < 6; ++c) sh[(g * 6 + c) * 64 + r] = sum[c];
+  __syncthreads();
+  if (mine) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q)
+#pragma unroll
+      for (int c = 0; c < 6; ++c) sum[c] += sh[(q * 6 + c) * 64 + r];
+    const double dt = ctl->dt;
+    crit = correct_body(dt, eta, d, sum, x, v);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      predict_component(dt, x[c], v[c], sum[c], sum[3 + c], x[c], v[c]);
+      X[c * ld + i] = x[c];
+      V[c * ld + i] = v[c];
+      D[c * ld + i] = sum[c];
+      D[(3 + c) * ld + i] = sum[3 + c];
+    }
+  }
+  write_subtile(out + blockIdx.x, mine, x, v, m);
+  __syncthreads();  // sh is reused
+  finish_criterion(ctl, crit, true, sh);
 }
 
 __device__ __forceinline__ uint64_t f2_dup(float v) { return f2_pack(v, v); }

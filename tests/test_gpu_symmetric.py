@@ -284,3 +284,24 @@ def test_ensemble_edges(precision, variant, tpi):
             assert ea.max() <= 1e-12 and ej.max() <= 1e-12, (c, n, ea.max(), ej.max())
         else:
             assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4 and np.median(ej) <= 1e-5, (c, n)
+
+
+# steps of one call share a kernel between the corrector and the next step's
+# predictor; steps of their own calls do not: the same arithmetic, bit for bit
+# (short last subtile and CTA, one body more than a CTA's rows, no full subtile)
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [33, 300, 1025, 4095, 16385])
+def test_chained_steps_equal_single_steps(n, precision):
+    s = bodies(n)
+    out = []
+    for calls in ([11], [1] * 11):
+        with nb.Engine(n, eps2=EPS2, precision=precision, dt=1 / 1024) as e:
+            e.set_state(s)
+            e.force_calculation()
+            for k in calls:
+                e.timestepping(k)
+            out.append((e.get_state(), e.get_derivs()))
+    (a, da), (b, db) = out
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
+    assert np.array_equal(da, db)
