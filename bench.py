@@ -61,19 +61,26 @@ FLOP_PER_INTERACTION = 60
 L2_FLUSH_BYTES = 256 << 20
 
 # Instructions per pair interaction of each pair kernel, counted from its
-# source (csrc/pair.cuh): FP32 (or FP64) pipe lane-operations and MUFU
-# operations.  record_format -> (pipe, lane ops, mufu ops).  The near/far
-# kernel (format 3) issues 25 lane-ops on a far tile and 31 on a near one
-# (double-single separation): roofline() weights them by the measured share.
+# source (csrc/pair.cuh, csrc/sympair.cuh): FP32 (or FP64) pipe lane-operations
+# and MUFU operations, without the shuffles.  Kernel -> (pipe, lane ops, mufu
+# ops, lane ops more on a near tile).  The symmetric kernels evaluate a pair
+# once for both of its interactions.  roofline() weights near tiles by their
+# measured share.
 ISSUED_OPS = {
-    0: ("fp64", 31, 1),   # pair_fp64_kernel: rsqrt.approx.f64 + one Householder step
-    1: ("fp32", 32, 1),   # pair_mixed_kernel: scalar hi/lo, y^2 by multiply
-    2: ("fp32", 31, 2),   # pair_mixed_x2_kernel: packed hi/lo, rsqrt + rcp on MUFU
-    3: ("fp32", 25, 2),   # pair_mixed_nf_kernel, far tiles: one add per separation component
+    "pair_sym_fp64_kernel": ("fp64", 19, 0.5, 0),   # rsqrt.approx.f64 + one Householder step
+    "pair_sym_nf_kernel": ("fp32", 16, 1, 3),       # near: double-single separations
+    "pair_mixed_kernel": ("fp32", 32, 1, 0),        # scalar hi/lo, y^2 by multiply
+    "pair_mixed_x2_kernel": ("fp32", 31, 2, 0),     # packed hi/lo, rsqrt + rcp on MUFU
+    "pair_mixed_nf_kernel": ("fp32", 25, 2, 6),     # variant 5: every tile taken as far
 }
-NEAR_EXTRA_OPS = 6        # near tiles: three adds per component instead of one
-KERNEL_NAMES = {0: "pair_fp64_kernel", 1: "pair_mixed_kernel", 2: "pair_mixed_x2_kernel",
-                3: "pair_mixed_nf_kernel"}
+
+
+def kernel_name(record_format, variant=0):
+    """The pair kernel of a full-row pass with an automatic or tuned tiling."""
+    return {0: "pair_sym_fp64_kernel", 1: "pair_mixed_kernel", 2: "pair_mixed_x2_kernel",
+            3: "pair_mixed_nf_kernel" if variant == 5 else "pair_sym_nf_kernel"}[record_format]
+
+
 VARIANT_NAMES = {1: "scalar hi/lo (pair_variant 1)", 2: "packed hi/lo (pair_variant 2)",
                  3: "packed hi/lo (pair_variant 3)",
                  4: "near/far tile-relative (pair_variant 4): far tiles one add per separation "
@@ -271,6 +278,7 @@ def run_arm(w, precision, state, torch, dist, world, dev, steps, warmup, variant
         "clocks": clk.summary(),
         "launches": int(launches),
         "record_format": tm["record_format"],
+        "kernel": kernel_name(tm["record_format"], variant),
         "near_tile_fraction": tm["near_tile_fraction"],
     }
 
@@ -317,23 +325,23 @@ def roofline(peaks, w, arm, prec):
     """60-flop convention against the measured FMA peak, plus the issued
     lane-operations of the kernel against the same pipe's lane-op peak."""
     inter = float(w.n) * w.n
-    fmt = arm["record_format"]
+    kernel = arm["kernel"]
     peak = peaks["fp32_tflops"] if prec == "mixed" else peaks["fp64_tflops"]
     achieved = FLOP_PER_INTERACTION * inter / (arm["pair_ms"] * 1e-3) / 1e12
-    pipe, lane_ops, mufu_ops = ISSUED_OPS[fmt]
-    near = arm.get("near_tile_fraction", 0.0) if fmt == 3 else 0.0
-    lane_ops = lane_ops + NEAR_EXTRA_OPS * near
+    pipe, lane_ops, mufu_ops, near_extra = ISSUED_OPS[kernel]
+    near = arm.get("near_tile_fraction", 0.0) if near_extra else 0.0
+    lane_ops = lane_ops + near_extra * near
     lane_peak = (max(peaks["fp32_tflops"], peaks["fp32x2_tflops"]) if pipe == "fp32"
                  else peaks["fp64_tflops"]) / 2 * 1e12       # FMA = 2 flop = 1 lane-op
     rate = inter / (arm["pair_ms"] * 1e-3)
     return {"bound": pipe, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-            "frac": achieved / peak, "traffic": traffic_per_launch(KERNEL_NAMES[fmt]),
-            "kernel": KERNEL_NAMES[fmt],
+            "frac": achieved / peak, "traffic": traffic_per_launch(kernel),
+            "kernel": kernel,
             "peak_source": "measured live by nbody_measure_peaks (FMA microkernel, this GPU)",
             "flop_per_interaction": FLOP_PER_INTERACTION,
             "issued_frac": rate * lane_ops / lane_peak,
             "issued": {"lane_ops_per_interaction": lane_ops, "mufu_ops_per_interaction": mufu_ops,
-                       "near_tile_fraction": near if fmt == 3 else None,
+                       "near_tile_fraction": near if near_extra else None,
                        "lane_op_peak_per_s": lane_peak,
                        "mufu_frac": rate * mufu_ops / (peaks["mufu_rsqrt_gops"] * 1e9)}}
 
@@ -379,7 +387,7 @@ def accuracy_block(w, state, dev, sample_rows=2048):
         dm, fmt = engine_derivs(w, state, "mixed", dev, v)
         out["all_bodies_vs_fp64_engine"][key] = {"acc": _stats(_vec_rel(dm[:3], d64[:3])),
                                                  "jerk": _stats(_vec_rel(dm[3:], d64[3:])),
-                                                 "kernel": KERNEL_NAMES[fmt]}
+                                                 "kernel": kernel_name(fmt, v)}
         out["sampled_vs_fp64"][key] = {"acc": _stats(_vec_rel(dm[:3, rows], ref[:3])),
                                        "jerk": _stats(_vec_rel(dm[3:, rows], ref[3:]))}
     out["sampled_vs_fp64"]["reference_f32"] = {"acc": _stats(_vec_rel(f32[:3], ref[:3])),
@@ -819,7 +827,7 @@ def large_n_block(a, peaks, torch, dev):
         out[k] = {"value": inter / (arm["ms_per_step"] * 1e-3) / 1e9, "unit": "Gint/s",
                   "ms_per_step": arm["ms_per_step"], "steps_per_s": 1e3 / arm["ms_per_step"],
                   "pair_ms": arm["pair_ms"],
-                  "kernel": KERNEL_NAMES[arm["record_format"]], "tiling": arm["tiling"],
+                  "kernel": arm["kernel"], "tiling": arm["tiling"],
                   "tiling_source": arm["tiling_source"], "roofline": roofline(peaks, w, arm, prec),
                   "clocks": arm["clocks"]}
         if k != "mixed_hilo" and tu > 0:
