@@ -210,26 +210,28 @@ __global__ void ens_key_kernel(int L, const int* __restrict__ cid, const int* __
   vals[r] = r;
 }
 
-// The slot sums of row r (CTAs of kSumThreads: kSumRows<8> rows of one cluster,
-// eight groups), valid in group 0 of real rows; returns the row's cluster or -1.
+// The slot sums of row r (CTAs of kSumThreads: kSumRows<GR> rows of one cluster,
+// GR groups), valid in group 0 of real rows; returns the row's cluster or -1.
+template <int GR>
 __device__ __forceinline__ int ens_slot_sums(int r, const int* __restrict__ cid,
                                              const ClusterDev* __restrict__ cl,
                                              const double* __restrict__ P, double sum[6], double* sh) {
   const int c = cid[r];
   const ClusterDev k = cl[max(c, 0)];
   const int i = c >= 0 ? r - k.row0 : 0;
-  slot_sums<8>(P + k.p_off, k.ld, c >= 0 ? RowSlots(k.S, k.block_rows, k.nb).count(i) : 0, i, sum, sh);
-  return threadIdx.x < kSumRows<8> ? c : -1;
+  slot_sums<GR>(P + k.p_off, k.ld, c >= 0 ? RowSlots(k.S, k.block_rows, k.nb).count(i) : 0, i, sum, sh);
+  return threadIdx.x < kSumRows<GR> ? c : -1;
 }
 
+template <int GR>
 __global__ void __launch_bounds__(kSumThreads)
     ens_correct_kernel(int L, const int* __restrict__ cid, const ClusterDev* __restrict__ cl,
                        const double* __restrict__ P, double* __restrict__ X, double* __restrict__ V,
                        double* __restrict__ D) {
-  __shared__ double sh[6 * kSumThreads];
-  const int r = blockIdx.x * kSumRows<8> + threadIdx.x % kSumRows<8>;
+  __shared__ double sh[GR > 1 ? 6 * kSumThreads : 1];
+  const int r = blockIdx.x * kSumRows<GR> + threadIdx.x % kSumRows<GR>;
   double sum[6];
-  const int c = ens_slot_sums(r, cid, cl, P, sum, sh);
+  const int c = ens_slot_sums<GR>(r, cid, cl, P, sum, sh);
   if (c < 0) return;
   const double dt = cl[c].dt;
   const double idt2 = 1.0 / (dt * dt), idt3 = idt2 / dt;
@@ -248,13 +250,14 @@ __global__ void __launch_bounds__(kSumThreads)
   }
 }
 
+template <int GR>
 __global__ void __launch_bounds__(kSumThreads)
     ens_reduce_kernel(int L, const int* __restrict__ cid, const ClusterDev* __restrict__ cl,
                       const double* __restrict__ P, double* __restrict__ D) {
-  __shared__ double sh[6 * kSumThreads];
-  const int r = blockIdx.x * kSumRows<8> + threadIdx.x % kSumRows<8>;
+  __shared__ double sh[GR > 1 ? 6 * kSumThreads : 1];
+  const int r = blockIdx.x * kSumRows<GR> + threadIdx.x % kSumRows<GR>;
   double sum[6];
-  if (ens_slot_sums(r, cid, cl, P, sum, sh) < 0) return;
+  if (ens_slot_sums<GR>(r, cid, cl, P, sum, sh) < 0) return;
 #pragma unroll
   for (int f = 0; f < 6; ++f) D[f * L + r] = sum[f];
 }
@@ -645,7 +648,15 @@ nbody_status launch_ens_pack(nbody_ensemble* e) {
   return ens_records(e, e->stream, false);
 }
 
-int sum_blocks(const nbody_ensemble* e) { return e->L / kSumRows<8>; }  // L is a multiple of 256
+// Whether the rows' slots are summed by eight groups of threads or by one thread:
+// as sum_in_groups (hermite.cuh), by the mean over the rows.  512 clusters of 256
+// to 8192 bodies, 1.2e6 rows of 3 slots on average: corrector 173 us in groups,
+// 57 by one thread.
+bool sum_by_groups(const nbody_ensemble* e) {
+  return e->p_doubles >= static_cast<size_t>(kSumGroupSlots) * 6 * e->L;
+}
+// L is a multiple of 256
+int sum_blocks(const nbody_ensemble* e, bool groups) { return e->L / (groups ? kSumRows<8> : kSumRows<1>); }
 
 int count_graph_kernels(cudaGraph_t g) {
   size_t nodes = 0;
@@ -665,7 +676,9 @@ int count_graph_kernels(cudaGraph_t g) {
 nbody_status ens_eval_current(nbody_ensemble* e) {
   EN_TRY(launch_ens_pack(e));
   EN_TRY(launch_ens_pair(e));
-  ens_reduce_kernel<<<sum_blocks(e), kSumThreads, 0, e->stream>>>(e->L, e->cid, e->cl, e->P, e->D);
+  const bool groups = sum_by_groups(e);
+  (groups ? ens_reduce_kernel<8> : ens_reduce_kernel<1>)<<<sum_blocks(e, groups), kSumThreads, 0, e->stream>>>(
+      e->L, e->cid, e->cl, e->P, e->D);
   EN_CUDA(cudaGetLastError());
   e->have_derivs = true;
   return NBODY_OK;
@@ -681,7 +694,9 @@ nbody_status ens_capture(nbody_ensemble* e, bool timed, cudaGraphExec_t* out) {
     s = nbody_set_error(NBODY_ERR_CUDA, "event record during capture failed");
   if (s == NBODY_OK) s = ens_records(e, e->stream, true);
   if (s == NBODY_OK) s = launch_ens_pair(e);
-  ens_correct_kernel<<<sum_blocks(e), kSumThreads, 0, e->stream>>>(e->L, e->cid, e->cl, e->P, e->X, e->V, e->D);
+  const bool groups = sum_by_groups(e);
+  (groups ? ens_correct_kernel<8> : ens_correct_kernel<1>)<<<sum_blocks(e, groups), kSumThreads, 0, e->stream>>>(
+      e->L, e->cid, e->cl, e->P, e->X, e->V, e->D);
   if (timed && s == NBODY_OK &&
       cudaEventRecordWithFlags(e->ev[1], e->stream, cudaEventRecordExternal) != cudaSuccess)
     s = nbody_set_error(NBODY_ERR_CUDA, "event record during capture failed");
