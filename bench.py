@@ -123,8 +123,8 @@ def parse():
     ap.add_argument("--heuristic", action="store_true",
                     help="tile the pair kernels by the heuristic instead of the autotuner")
     ap.add_argument("--variant", type=int, default=0,
-                    help="mixed pair kernel (nbody_config.pair_variant): 0 = automatic (near/far "
-                         "tile-relative from 16384 bodies), 1 = scalar hi/lo, 2/3 = packed hi/lo, "
+                    help="mixed pair kernel (nbody_config.pair_variant): 0 = automatic (symmetric "
+                         "near/far tile-relative), 1 = scalar hi/lo, 2/3 = packed hi/lo, "
                          "4 = near/far tile-relative, 5 = plain tile-relative; ensembles: 4 = "
                          "near/far, 5 = plain tile-relative, else packed hi/lo")
     ap.add_argument("--time-units", type=float, default=1.0,

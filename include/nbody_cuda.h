@@ -65,9 +65,11 @@ typedef struct {
   double eta0;        /* initial-dt criterion, default 1e-4 (nbody.h:15)    */
   int tune;           /* 1: time candidate tilings on first use (autotuner) */
   int threads, i_per_thread, j_tile, split_j; /* 0 = choose automatically   */
-  int pair_variant;   /* mixed only: 0 = automatic (variant 4 from 16384
-                         bodies, variant 3 below, where building the tiles
-                         costs more than it saves), 1 = scalar FP32 kernel
+  int pair_variant;   /* mixed only: 0 = automatic (the near/far kernel in
+                         its symmetric form, every unordered pair once;
+                         bodies in Hilbert order from 16384 of them on;
+                         with an explicit shape the one-sided variant 4
+                         from 16384 bodies, 3 below), 1 = scalar FP32 kernel
                          on hi/lo positions, 2 = packed-pair (f32x2) hi/lo
                          kernel, FP64 accumulators in registers, 3 = packed
                          hi/lo kernel, FP64 accumulators in shared memory,
@@ -79,9 +81,10 @@ typedef struct {
                          add per separation component, a near tile forms
                          the separation in double-single (hi/lo offsets),
                          so close pairs keep the hi/lo kernels' accuracy
-                         (the fastest for large systems), 5 = the same
-                         kernel with every tile taken as far (plain
-                         tile-relative offsets; a comparison)               */
+                         (symmetric as 0, bodies always in Hilbert order;
+                         one-sided with an explicit shape), 5 = one-sided
+                         with every tile taken as far (plain tile-relative
+                         offsets; a comparison)                             */
   int sort_every;     /* tile-relative kernels: re-order the bodies along
                          the Hilbert curve every this many steps (tile
                          centres and offsets are rebuilt every step);
@@ -111,7 +114,9 @@ typedef struct {
                                        0 FP64, 1 FP32 hi/lo, 2 packed hi/lo,
                                        3 packed near/far tile-relative
                                        (bodies kept in Hilbert order)       */
-  int step_kernels;                 /* kernel launches in one captured step */
+  int step_kernels;                 /* kernel launches in one step by itself
+                                       (small systems: steps of one call
+                                       share one between two steps)         */
   long long reorders;               /* Hilbert re-orderings run by steps     */
   int order_kernels;                /* kernel launches in one re-ordering   */
   double dt_crit;                   /* criterion of the last completed pass:
@@ -280,14 +285,15 @@ typedef struct {
   const double* dt;      /* fixed shared step per cluster (> 0)              */
   int precision;         /* nbody_precision                                  */
   int device;
-  int tiles_per_item;    /* j-tiles per work item; 0 = default 8, or (with the
-                            kernel shape) chosen by timing when tune = 1    */
+  int tiles_per_item;    /* j-tiles per work item; 0 = chosen so that the
+                            items fill the GPU (64 to 1024 bodies), or (with
+                            the kernel shape) by timing when tune = 1       */
   int tune;
-  int pair_variant;      /* mixed only: 0 = automatic (the packed hi/lo
-                            kernel, the faster one for clusters of up to a
-                            few thousand bodies), 3 = packed hi/lo kernel,
-                            4 = near/far tile-relative kernel (each cluster
-                            kept in Hilbert order within its segment),
+  int pair_variant;      /* mixed only: 0 = automatic (the one-sided
+                            packed hi/lo kernel), 3 = packed hi/lo kernel,
+                            4 = near/far tile-relative kernel, symmetric
+                            (each cluster kept in Hilbert order within its
+                            segment),
                             5 = tile-relative with every tile taken as far
                             (nbody_config numbering)                       */
   int sort_every;        /* variants 4, 5: re-order every this many steps;

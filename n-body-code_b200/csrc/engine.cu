@@ -3,10 +3,10 @@
 // One engine = one system of n bodies on one device, one CUDA stream, and
 // device memory allocated once at creation:
 //   state  [13][ld] float64  X(3) V(3) M(1) D(6)  (D = current acc, jerk)
-//   P      [S][6][ld]        split-j partial sums of the pair kernel
+//   P      [S][6][ld]        partial-sum slots of the pair kernel
 //   jb64   [ld] JBody64      FP64 j-records (also used by the potential)
 //   jb32   [ld] JBody32      mixed-precision j-records (mixed engines):
-//                            JBody32, JBodyX2, or tiles of JBodyNF
+//                            JBody32, JBodyX2, tiles of JBodyNF, or SymSub
 //   sort   keys, indices, CUB scratch of the Hilbert ordering (mixed engines)
 //   perm   [2][ld] int       position -> caller's body index (tile-relative
 //                            engines keep their state in Hilbert order)
@@ -15,11 +15,11 @@
 //   ctl    StepCtl           dt, t, Aarseth criterion, step counter
 // ld = n rounded up to a multiple of 256 (kPad).
 //
-// A Hermite step - predict (O(N), writes the j-records; the near/far
-// tile-relative kernel's records come from rel_tile_nf_kernel right after),
-// pair (O(N^2)), correct (O(N), fused split reduction + snap/crackle +
-// correction + dt criterion) - is captured once into a CUDA graph and
-// replayed.  The Hilbert re-ordering of a tile-relative engine's state is a
+// A Hermite step - predict (O(N), writes the j-records; the one-sided near/far
+// kernel's come from rel_tile_nf_kernel right after), pair (O(N^2)), correct
+// (O(N), fused slot sums + snap/crackle + correction + dt criterion) - is
+// captured into CUDA graphs and replayed: eight steps at a time, single ones,
+// and the last step of a call with event records.  The Hilbert re-ordering of a tile-relative engine's state is a
 // second captured graph, replayed ahead of every sort_every-th step.
 #include <cuda_runtime.h>
 

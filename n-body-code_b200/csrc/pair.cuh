@@ -1,4 +1,5 @@
-// O(N^2) pair acc + jerk kernels (the hot path).
+// O(N^2) pair acc + jerk kernels, one-sided: row ranges, explicit tilings and the
+// hi/lo variants.  (Full-row passes with an automatic tiling: sympair.cuh.)
 //
 // Physics (src/kernel.cpp:1187-1221 in the reference, restated): for every
 // i-row, a_i = sum_j m_j q r_ij and jerk_i = sum_j m_j q (v_ij + c r_ij) with
@@ -29,7 +30,7 @@
 //          accuracy however close two bodies are), velocities and the rest
 //          of the pair math in float with the MUFU rsqrt, float partial sums
 //          over one j-tile flushed into double accumulators after each tile.
-//   Mixed, near/far tile-relative (default for large systems): bodies in
+//   Mixed, near/far tile-relative: bodies in
 //          Hilbert order, j-tiles of float offsets from each tile's centre;
 //          the separation costs one add per component for tiles far from a
 //          warp's rows and is formed in double-single for near tiles

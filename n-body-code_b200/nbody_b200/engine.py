@@ -34,9 +34,10 @@ class Engine:
     """One system of n bodies on one GPU (wraps nbody_create/nbody_destroy).
 
     precision "mixed" takes pair_variant (nbody_config.pair_variant): 0 picks
-    the near/far tile-relative kernel (4) from 16384 bodies and the packed
-    hi/lo kernel (3) below; 1 and 2 are the other hi/lo forms; 5 is the
-    tile-relative kernel with every tile taken as far (a comparison).  The
+    the symmetric near/far tile-relative kernel (bodies in Hilbert order from
+    16384 of them on); 3 is packed hi/lo, 1 and 2 are its other forms; 4 is
+    near/far with the bodies always in order; 5 is the tile-relative kernel
+    with every tile taken as far (a comparison).  The
     tile-relative engines keep their bodies in Hilbert order on the device;
     get_state and get_derivs return them in the caller's order.  sort_every
     sets how often they re-order (0 = every 16 steps).  eps2 must be >= 1e-24
