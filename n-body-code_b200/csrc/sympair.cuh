@@ -111,11 +111,13 @@ struct SymRun {
 // would evaluate more of the pairs one-sided (1 / nb of them).
 constexpr int kMaxSymBlocks = 128;
 constexpr int kMaxSymSplits = 64;
-// Slots are further bounded by memory (8 GiB of P, at least 8 slots): larger
-// systems take fewer, larger blocks and fewer splits.
+// Slots are further bounded by memory (8 GiB of P): from 1.4e6 bodies on systems
+// take fewer, larger blocks and fewer splits.  At least 32 slots, 1536 bytes per
+// body: 32 blocks of 16 splits still fill the SMs, where the 8 that fit at 2e7
+// bodies would be 32 CTAs.
 inline int max_sym_slots(int n) {
   const double fit = 8.0 * (1 << 30) / (48.0 * n);
-  return fit > 2 * kMaxSymSplits ? 2 * kMaxSymSplits : std::max(8, static_cast<int>(fit));
+  return fit > 2 * kMaxSymSplits ? 2 * kMaxSymSplits : std::max(32, static_cast<int>(fit));
 }
 
 // The blocks of n bodies for a kernel whose CTAs hold `rows` rows.
