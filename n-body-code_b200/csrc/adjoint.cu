@@ -411,7 +411,7 @@ nbody_status fwd_initial(nbody_adjoint* a, cudaStream_t st) {
   if (a->cfg.precision == NBODY_FP64)
     pack_kernel<<<(a->ld + kBlock - 1) / kBlock, kBlock, 0, st>>>(a->n, a->ld, own_state(a), a->jb64, nullptr);
   else
-    sym_tile_kernel<false><<<a->ld / 64, 64, 0, st>>>(a->n, own_state(a), a->jsub);
+    sym_tile_kernel<false, false><<<a->ld / 64, 64, 0, st>>>(a->n, own_state(a), a->jsub);  // the caller's order
   AD_CUDA(cudaGetLastError());
   AD_TRY(fwd_eval(a, st));
   double* D = a->D;
@@ -427,7 +427,7 @@ nbody_status fwd_step(nbody_adjoint* a, cudaStream_t st, double* xp_out) {
     AD_CUDA(launch_chained(predict_kernel, (a->n + kPredictBlock - 1) / kPredictBlock, kPredictBlock, 0, st,
                            a->n, a->ld, a->ctl, a->X, a->V, a->M, a->D, a->jb64, nullptr, nullptr, xp_out));
   else
-    AD_CUDA(launch_chained(sym_tile_kernel<true>, a->ld / 64, 64, 0, st, a->n, own_state(a), a->jsub, a->ld,
+    AD_CUDA(launch_chained(sym_tile_kernel<true, false>, a->ld / 64, 64, 0, st, a->n, own_state(a), a->jsub, a->ld,
                            a->X, a->V, a->D, a->ctl, nullptr, xp_out));
   AD_TRY(fwd_eval(a, st));
   launch_correct(st, a->n, a->ld, a->fwd.slots(), a->P, a->X, a->V, a->D, a->ctl, 1.0, true);

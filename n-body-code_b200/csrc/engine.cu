@@ -557,7 +557,7 @@ nbody_status launch_pair(nbody_engine* e, const Tiling& t, int i_begin, int i_en
 }
 
 nbody_status launch_pack(nbody_engine* e, int n, const SoA7& in, cudaStream_t st, int fmt,
-                         int tj);
+                         int tj, bool ordered);
 nbody_status enqueue_reorder_state(nbody_engine* e, cudaStream_t st);
 
 // The tiling the autotuner cached for this engine's (device, precision,
@@ -616,7 +616,8 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
     // passes at each size from 1024 to 262144
     if (!k.sym || k.precision != e->cfg.precision) continue;
     const int s0 = plan_sym(e, k, rows).S;
-    NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj));
+    NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj,
+                       wants_order(e, e->n, e->order_min_bodies)));
     for (int s : {std::max(1, s0 / 2), s0, std::min(kMaxSplit, s0 * 2)}) {
       Tiling t{&k, s};
       NB_TRY(ensure_partials(e, partial_count(t, rows)));
@@ -784,10 +785,10 @@ nbody_status build_rel_tiles(nbody_engine* e, int n, const SoA7& in, cudaStream_
 // kernels: also theirs), or tiles of tj near/far records of `in`, which must
 // then be in Hilbert order.  (The energy diagnostic packs its own records.)
 nbody_status launch_pack(nbody_engine* e, int n, const SoA7& in, cudaStream_t st, int fmt,
-                         int tj) {
+                         int tj, bool ordered) {
   if (fmt == kRecSym) {
-    sym_tile_kernel<false><<<e->ld / 64, 64, 0, st>>>(n, in, static_cast<SymSub*>(e->jb32), 0, nullptr,
-                                                      nullptr, nullptr, nullptr, e->near_count);
+    (ordered ? sym_tile_kernel<false, true> : sym_tile_kernel<false, false>)<<<e->ld / 64, 64, 0, st>>>(
+        n, in, static_cast<SymSub*>(e->jb32), 0, nullptr, nullptr, nullptr, nullptr, e->near_count, nullptr);
     NB_CUDA(cudaGetLastError());
   } else if (fmt != kRecRel) {
     pack_kernel<<<(e->ld + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, st>>>(
@@ -815,7 +816,7 @@ nbody_status eval_foreign_rel(nbody_engine* e, const Tiling& t, int n, const SoA
   gather_rows_kernel<<<(n + kBlockO1 - 1) / kBlockO1, kBlockO1, 0, st>>>(n, ord, g, nullptr, nullptr);
   NB_CUDA(cudaGetLastError());
   const SoA7 sorted{g.dst[0], g.dst[1], g.dst[2], g.dst[3], g.dst[4], g.dst[5], g.dst[6]};
-  NB_TRY(launch_pack(e, n, sorted, st, t.k->fmt, t.k->tj));
+  NB_TRY(launch_pack(e, n, sorted, st, t.k->fmt, t.k->tj, true));
   NB_TRY(launch_pair(e, t, 0, n, st, &sorted, n));
   if (!reduce) return NBODY_OK;  // the caller sums the splits (rows in sort_idx + ld order)
   launch_reduce(st, 0, n, e->ld, row_slots(t, n), e->P, out, nullptr, ord);
@@ -854,7 +855,7 @@ nbody_status maybe_reorder(nbody_engine* e, cudaStream_t st) {
 nbody_status eval_current(nbody_engine* e) {
   NB_TRY(ensure_tiling(e));
   if (curve_resident(e) && !e->sorted) NB_TRY(enqueue_reorder_state(e, e->stream));
-  NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, tiling_fmt(e), tiling_tj(e)));
+  NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, tiling_fmt(e), tiling_tj(e), curve_resident(e)));
   if (!e->init_events) {
     NB_CUDA(cudaEventCreate(&e->ev_init[0]));
     NB_CUDA(cudaEventCreate(&e->ev_init[1]));
@@ -877,8 +878,9 @@ nbody_status eval_current(nbody_engine* e) {
 nbody_status enqueue_predict(nbody_engine* e, cudaStream_t st) {
   const int fmt = tiling_fmt(e);
   if (fmt == kRecSym) {
-    sym_tile_kernel<true><<<e->ld / 64, 64, 0, st>>>(e->n, own_inputs(e), static_cast<SymSub*>(e->jb32),
-                                                     e->ld, e->X, e->V, e->D, e->ctl, e->near_count);
+    (curve_resident(e) ? sym_tile_kernel<true, true> : sym_tile_kernel<true, false>)<<<e->ld / 64, 64, 0, st>>>(
+        e->n, own_inputs(e), static_cast<SymSub*>(e->jb32), e->ld, e->X, e->V, e->D, e->ctl, e->near_count,
+        nullptr);
     NB_CUDA(cudaGetLastError());
     return NBODY_OK;
   }
@@ -914,7 +916,8 @@ bool can_chain_steps(const nbody_engine* e) {
 nbody_status enqueue_correct_predict(nbody_engine* e, cudaStream_t st) {
   const RowSlots slots = row_slots(e->tiling, e->n);
   if (tiling_fmt(e) == kRecSym)
-    correct_tile_kernel<<<e->ld / 64, kCorrectTileThreads, 0, st>>>(
+    (curve_resident(e) ? correct_tile_kernel<true>
+                       : correct_tile_kernel<false>)<<<e->ld / 64, kCorrectTileThreads, 0, st>>>(
         e->n, e->ld, slots, e->P, e->X, e->V, e->D, e->ctl, e->cfg.eta, e->M,
         static_cast<SymSub*>(e->jb32), e->near_count);
   else
@@ -1235,7 +1238,7 @@ nbody_status nbody_set_state(nbody_engine* e, const double* x, const double* y, 
   }
   e->sorted = e->permuted = false;
   if (!curve_resident(e))
-    NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, tiling_fmt(e), tiling_tj(e)));
+    NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, tiling_fmt(e), tiling_tj(e), false));
   NB_CUDA(cudaStreamSynchronize(e->stream));
   e->have_state = true;
   e->have_derivs = false;
@@ -1475,7 +1478,7 @@ nbody_status nbody_acc_jerk_device(nbody_engine* e, int n, const double* x, cons
     NB_TRY(enqueue_curve_order(e, n, in, st, kDropInOrderLowBit));
     return eval_foreign_rel(e, t, n, in, out, st);
   }
-  NB_TRY(launch_pack(e, n, in, st, t.k->fmt, t.k->tj));
+  NB_TRY(launch_pack(e, n, in, st, t.k->fmt, t.k->tj, false));
   NB_TRY(launch_pair(e, t, 0, n, st, &in, n));
   launch_reduce(st, 0, n, e->ld, row_slots(t, n), e->P, out);
   NB_CUDA(cudaGetLastError());
@@ -1590,7 +1593,7 @@ extern "C" nbody_status nbody_force_calculation(int n, double eps2, int precisio
   if (n <= kDropInStageBodies && !order) {
     double* out[6] = {ax, ay, az, jx, jy, jz};
     NB_TRY(upload_state(e, src));
-    NB_TRY(launch_pack(e, n, own_inputs(e), e->stream, t.k->fmt, t.k->tj));
+    NB_TRY(launch_pack(e, n, own_inputs(e), e->stream, t.k->fmt, t.k->tj, false));
     NB_TRY(launch_pair(e, t, i_begin, i_end, e->stream));
     if (i_end > i_begin) {
       launch_reduce(e->stream, i_begin, i_end, e->ld, row_slots(t, n), e->P, own_derivs(e));
@@ -1626,7 +1629,7 @@ extern "C" nbody_status nbody_force_calculation(int n, double eps2, int precisio
   } else {
     for (int k = 0; k < 7; ++k)
       NB_CUDA(cudaMemcpyAsync(dst[k], src[k], b, cudaMemcpyHostToDevice, e->stream));
-    NB_TRY(launch_pack(e, n, own_inputs(e), e->stream, t.k->fmt, t.k->tj));
+    NB_TRY(launch_pack(e, n, own_inputs(e), e->stream, t.k->fmt, t.k->tj, false));
     NB_TRY(launch_pair(e, t, i_begin, i_end, e->stream));
   }
   // one field at a time: field k's download (second stream) overlaps the

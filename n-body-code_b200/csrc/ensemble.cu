@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(64)
       }
     }
   }
-  write_subtile(out + blockIdx.x, c >= 0, p, u, m);
+  write_subtile<true>(out + blockIdx.x, c >= 0, p, u, m);
 }
 
 // Predictor of the FP64 ensemble and of the one-sided kernels, with the records

@@ -482,6 +482,10 @@ __global__ void __launch_bounds__(32 * W)
 // l + 32 as packed pairs, so each 64-bit word is an f32x2 operand: chunks
 // 0 (-Dx, -Dy), 1 (-Dz, m), 2 (vx, vy), 3 (vz, -), 4 (-Dx_lo, -Dy_lo),
 // 5 (-Dz_lo, -), with (D, D_lo) = ds_offset(c, x_hi, x_lo).  50 bytes per body.
+// Bodies that are in no order get centre 0 and a box without end: D is then -x
+// itself and no subtile is far, so every separation has the accuracy of the
+// hi/lo kernels, whatever order the bodies are in and whatever shares a subtile
+// (beside an escaper at 1e10, D_lo holds the others' positions as mere floats).
 struct __align__(128) SymSub {
   float c[3], R, lo[3], hi[3], pad[22];
   ulonglong2 v[6][32];
@@ -490,44 +494,56 @@ static_assert(sizeof(SymSub) == 3200, "subtiles start 128-byte aligned");
 
 // Writes one subtile from the values of the calling CTA's first 64 threads' 64
 // bodies (invalid ones are zero-mass padding at the centre); called by all.
+// ORDERED: neighbours in space share a subtile.
+template <bool ORDERED>
 __device__ __forceinline__ void write_subtile(SymSub* __restrict__ out, bool valid, const double p[3],
                                               const double u[3], double m) {
-  __shared__ double box[6][2];
-  __shared__ float rmax[2];
   __shared__ SymSub stage;  // written out in one bulk copy
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float c[3] = {0.f, 0.f, 0.f};
+  if (ORDERED) {
+    __shared__ double box[6][2];
+    __shared__ float rmax[2];
 #pragma unroll
-  for (int k = 0; k < 6; ++k) {  // bounding box in double (empty subtile: +inf/-inf)
-    double w = k < 3 ? (valid ? p[k] : INFINITY) : (valid ? p[k - 3] : -INFINITY);
-    w = k < 3 ? warp_min(w) : warp_max(w);
-    if (lane == 0 && warp < 2) box[k][warp] = w;
-  }
-  __syncthreads();
-  double lo[3], hi[3];
-  float c[3];
-  double r2 = 0.0;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    lo[k] = fmin(box[k][0], box[k][1]);
-    hi[k] = fmax(box[3 + k][0], box[3 + k][1]);
-    const double mid = 0.5 * lo[k] + 0.5 * hi[k];
-    c[k] = isfinite(mid) ? static_cast<float>(mid) : 0.0f;
-    const double d = p[k] - static_cast<double>(c[k]);
-    r2 += valid ? d * d : 0.0;
-  }
-  float R = __double2float_ru(sqrt(r2));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
-  if (lane == 0 && warp < 2) rmax[warp] = R;
-  __syncthreads();
-  if (tid == 0) {
+    for (int k = 0; k < 6; ++k) {  // bounding box in double (empty subtile: +inf/-inf)
+      double w = k < 3 ? (valid ? p[k] : INFINITY) : (valid ? p[k - 3] : -INFINITY);
+      w = k < 3 ? warp_min(w) : warp_max(w);
+      if (lane == 0 && warp < 2) box[k][warp] = w;
+    }
+    __syncthreads();
+    double lo[3], hi[3];
+    double r2 = 0.0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      stage.c[k] = c[k];
-      stage.lo[k] = __double2float_rd(lo[k]);
-      stage.hi[k] = __double2float_ru(hi[k]);
+      lo[k] = fmin(box[k][0], box[k][1]);
+      hi[k] = fmax(box[3 + k][0], box[3 + k][1]);
+      const double mid = 0.5 * lo[k] + 0.5 * hi[k];
+      c[k] = isfinite(mid) ? static_cast<float>(mid) : 0.0f;
+      const double d = p[k] - static_cast<double>(c[k]);
+      r2 += valid ? d * d : 0.0;
     }
-    stage.R = fmaxf(rmax[0], rmax[1]);
+    float R = __double2float_ru(sqrt(r2));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
+    if (lane == 0 && warp < 2) rmax[warp] = R;
+    __syncthreads();
+    if (tid == 0) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        stage.c[k] = c[k];
+        stage.lo[k] = __double2float_rd(lo[k]);
+        stage.hi[k] = __double2float_ru(hi[k]);
+      }
+      stage.R = fmaxf(rmax[0], rmax[1]);
+    }
+  } else if (tid == 0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      stage.c[k] = 0.f;
+      stage.lo[k] = -INFINITY;
+      stage.hi[k] = INFINITY;
+    }
+    stage.R = 0.f;
   }
   float oh[3], ol[3];
 #pragma unroll
@@ -566,7 +582,7 @@ __device__ __forceinline__ void write_subtile(SymSub* __restrict__ out, bool val
 // arithmetic): one pass instead of two.  Bound by its launch below some 10^5
 // bodies (104 B read, 48 + 50 written per body): the phase at N = 65536 9.6 us
 // instead of 12.6.  Zeroes near_count for the pair pass that follows.
-template <bool PREDICT>
+template <bool PREDICT, bool ORDERED>
 __global__ void __launch_bounds__(64)
     sym_tile_kernel(int n, SoA7 in, SymSub* __restrict__ out, int ld = 0, double* X = nullptr,
                     double* V = nullptr, const double* __restrict__ D = nullptr,
@@ -587,13 +603,14 @@ __global__ void __launch_bounds__(64)
       u[0] = in.vx[slot]; u[1] = in.vy[slot]; u[2] = in.vz[slot];
     }
   }
-  write_subtile(out + blockIdx.x, valid, p, u, m);
+  write_subtile<ORDERED>(out + blockIdx.x, valid, p, u, m);
 }
 
 // correct_kernel<8, true> for the near/far records: corrector and the next
 // step's predictor on the 64 bodies of subtile blockIdx.x (64 rows times eight
 // groups of threads, the sums in correct_kernel<8>'s order), and the subtile.
 constexpr int kCorrectTileThreads = 512;
+template <bool ORDERED>
 static __global__ void __launch_bounds__(kCorrectTileThreads)
     correct_tile_kernel(int n, int ld, RowSlots slots, const double* __restrict__ P,
                         double* __restrict__ X, double* __restrict__ V, double* __restrict__ D,
@@ -636,7 +653,7 @@ static __global__ void __launch_bounds__(kCorrectTileThreads)
       D[(3 + c) * ld + i] = sum[3 + c];
     }
   }
-  write_subtile(out + blockIdx.x, mine, x, v, m);
+  write_subtile<ORDERED>(out + blockIdx.x, mine, x, v, m);
   __syncthreads();  // sh is reused
   finish_criterion(ctl, crit, true, sh);
 }
