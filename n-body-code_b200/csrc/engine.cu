@@ -352,10 +352,11 @@ int default_format(const nbody_engine* e) {
 
 bool tile_relative(int fmt) { return fmt == kRecRel || fmt == kRecSym; }
 
-// Whether tile-relative kernels of this engine get their bodies in Hilbert
-// order: the one-sided ones always, the automatic choice from `min` bodies.
-bool wants_order(const nbody_engine* e, int n, int min) {
-  return e->cfg.pair_variant >= 4 || n >= min;
+// Whether a pass over n bodies with records of format fmt gets them in Hilbert
+// order: the one-sided near/far kernels always, the symmetric ones from `min`
+// bodies or where pair_variant asks for it.
+bool wants_order(const nbody_engine* e, int fmt, int n, int min) {
+  return fmt == kRecRel || (fmt == kRecSym && (e->cfg.pair_variant >= 4 || n >= min));
 }
 
 // The engine keeps its bodies in Hilbert order (positions != body indices).
@@ -607,8 +608,7 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
   int best_idx = -1, best_split = 1;
   const auto& reg = registry();
   // the near/far kernel's cost depends on the order of the bodies
-  if (default_format(e) == kRecSym && e->have_state && !e->sorted &&
-      wants_order(e, e->n, e->order_min_bodies))
+  if (e->have_state && !e->sorted && wants_order(e, default_format(e), e->n, e->order_min_bodies))
     NB_TRY(enqueue_reorder_state(e, e->stream));
   for (size_t idx = 0; idx < reg.size(); ++idx) {
     const PairKernel& k = reg[idx];
@@ -617,7 +617,7 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
     if (!k.sym || k.precision != e->cfg.precision) continue;
     const int s0 = plan_sym(e, k, rows).S;
     NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj,
-                       wants_order(e, e->n, e->order_min_bodies)));
+                       wants_order(e, k.fmt, e->n, e->order_min_bodies)));
     for (int s : {std::max(1, s0 / 2), s0, std::min(kMaxSplit, s0 * 2)}) {
       Tiling t{&k, s};
       NB_TRY(ensure_partials(e, partial_count(t, rows)));
@@ -829,7 +829,7 @@ int tiling_tj(const nbody_engine* e) { return e->tiled ? e->tiling.k->tj : 0; }
 int sort_period(const nbody_engine* e) { return e->cfg.sort_every > 0 ? e->cfg.sort_every : 16; }
 
 bool curve_resident(const nbody_engine* e) {
-  return tile_relative(tiling_fmt(e)) && wants_order(e, e->n, e->order_min_bodies);
+  return wants_order(e, tiling_fmt(e), e->n, e->order_min_bodies);
 }
 
 // Before a step of the engine's own state: re-order when the order is stale
@@ -1473,7 +1473,7 @@ nbody_status nbody_acc_jerk_device(nbody_engine* e, int n, const double* x, cons
   NB_TRY(ensure_partials(e, partial_count(t, n)));
   const SoA7 in{x, y, z, m, vx, vy, vz};
   const SoA6 out{ax, ay, az, jx, jy, jz};
-  if (tile_relative(t.k->fmt) && wants_order(e, n, kForeignOrderMin)) {
+  if (wants_order(e, t.k->fmt, n, kForeignOrderMin)) {
     // Hilbert order of the caller's bodies, gathered into scratch
     NB_TRY(enqueue_curve_order(e, n, in, st, kDropInOrderLowBit));
     return eval_foreign_rel(e, t, n, in, out, st);
@@ -1589,7 +1589,7 @@ extern "C" nbody_status nbody_force_calculation(int n, double eps2, int precisio
   // order (the near/far kernel evaluates all rows in Hilbert order)
   if (!full && tile_relative(t.k->fmt)) NB_TRY(hilo_tiling(e, i_end - i_begin, &t));
   NB_TRY(ensure_partials(e, partial_count(t, n)));
-  const bool order = tile_relative(t.k->fmt) && wants_order(e, n, kForeignOrderMin);
+  const bool order = wants_order(e, t.k->fmt, n, kForeignOrderMin);
   if (n <= kDropInStageBodies && !order) {
     double* out[6] = {ax, ay, az, jx, jy, jz};
     NB_TRY(upload_state(e, src));

@@ -1,0 +1,45 @@
+"""Which kernel, order and work list a call gets."""
+import numpy as np
+import pytest
+
+import nbody_b200 as nb
+import oracle as O
+from _util import vec_rel
+
+pytestmark = pytest.mark.gpu
+
+EPS2 = 1e-4
+
+
+def device_arrays(s):
+    import torch
+    n = s["x"].size
+    return [torch.tensor(s[k], device="cuda") for k in nb.FIELDS], \
+        torch.empty(6, n, dtype=torch.float64, device="cuda")
+
+
+def stream():
+    import torch
+    return torch.cuda.current_stream().cuda_stream
+
+
+def test_one_sided_near_far_calls_get_their_bodies_in_order():
+    """An explicit shape of the near/far kernel between 16384 and 32768 bodies:
+    device-array calls order the caller's bodies (in no order, every tile of
+    128 of them is near)."""
+    import torch
+    n = 20000
+    s = nb.plummer(n, seed=5)
+    t, out = device_arrays(s)
+    with nb.Engine(n, eps2=EPS2, precision="mixed", dt=1.0, threads=128, i_per_thread=4, j_tile=128) as e:
+        e.set_state(s)
+        e.force_calculation()
+        own = e.timers()["near_tile_fraction"]
+        e.acc_jerk_device(*t, list(out), stream=stream())
+        torch.cuda.synchronize()
+        called = e.timers()["near_tile_fraction"]
+    assert own < 0.9 and called < 0.9, (own, called)
+    rows = np.arange(0, n, 97)
+    ref = O.force_rows(s, EPS2, rows)
+    ea = vec_rel(out.cpu().numpy()[:3, rows], ref[:3])
+    assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4
