@@ -257,9 +257,11 @@ int partial_count(const Tiling& t, int n) {
 }
 
 // Autotune results shared by all engines of the process: (device, precision,
-// record format, ld, rows) -> tiling.
+// record format, ld, rows, bodies in Hilbert order) -> tiling.  The order
+// decides how many subtiles are near, and with it which kernel is the faster.
+using TuneKey = std::tuple<int, int, int, int, int, bool>;
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int, int>, std::pair<int, int>> g_tuned;  // -> (kernel idx, split)
+std::map<TuneKey, std::pair<int, int>> g_tuned;  // -> (kernel idx, split)
 
 }  // namespace
 
@@ -561,10 +563,14 @@ nbody_status launch_pack(nbody_engine* e, int n, const SoA7& in, cudaStream_t st
                          int tj, bool ordered);
 nbody_status enqueue_reorder_state(nbody_engine* e, cudaStream_t st);
 
-// The tiling the autotuner cached for this engine's (device, precision,
-// record format, ld, rows), if any.
-bool tuned_lookup(const nbody_engine* e, int rows, Tiling* out, bool full = true) {
-  const auto key = std::make_tuple(e->dev, e->cfg.precision, default_format(e), e->ld, rows);
+TuneKey tune_key(const nbody_engine* e, int rows, int order_min) {
+  const int fmt = default_format(e);
+  return {e->dev, e->cfg.precision, fmt, e->ld, rows, wants_order(e, fmt, rows, order_min)};
+}
+
+// The tiling the autotuner cached for `rows` bodies on this engine, if any.
+bool tuned_lookup(const nbody_engine* e, int rows, int order_min, Tiling* out, bool full = true) {
+  const TuneKey key = tune_key(e, rows, order_min);
   std::lock_guard<std::mutex> g(g_tune_mu);
   auto it = g_tuned.find(key);
   if (it == g_tuned.end()) return false;
@@ -598,9 +604,10 @@ void choose_sym(const nbody_engine* e, int n, Tiling* out) {
   }
 }
 
-nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
-  const auto key = std::make_tuple(e->dev, e->cfg.precision, default_format(e), e->ld, rows);
-  if (tuned_lookup(e, rows, out)) return NBODY_OK;
+nbody_status autotune(nbody_engine* e, int rows, int order_min, Tiling* out) {
+  const TuneKey key = tune_key(e, rows, order_min);
+  if (tuned_lookup(e, rows, order_min, out)) return NBODY_OK;
+  const bool ordered = std::get<5>(key);
   cudaEvent_t a, b;
   NB_CUDA(cudaEventCreate(&a));
   NB_CUDA(cudaEventCreate(&b));
@@ -608,7 +615,7 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
   int best_idx = -1, best_split = 1;
   const auto& reg = registry();
   // the near/far kernel's cost depends on the order of the bodies
-  if (e->have_state && !e->sorted && wants_order(e, default_format(e), e->n, e->order_min_bodies))
+  if (e->have_state && !e->sorted && ordered)
     NB_TRY(enqueue_reorder_state(e, e->stream));
   for (size_t idx = 0; idx < reg.size(); ++idx) {
     const PairKernel& k = reg[idx];
@@ -616,8 +623,7 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
     // passes at each size from 1024 to 262144
     if (!k.sym || k.precision != e->cfg.precision) continue;
     const int s0 = plan_sym(e, k, rows).S;
-    NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj,
-                       wants_order(e, k.fmt, e->n, e->order_min_bodies)));
+    NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj, ordered));
     for (int s : {std::max(1, s0 / 2), s0, std::min(kMaxSplit, s0 * 2)}) {
       Tiling t{&k, s};
       NB_TRY(ensure_partials(e, partial_count(t, rows)));
@@ -656,8 +662,9 @@ nbody_status autotune(nbody_engine* e, int rows, Tiling* out) {
 }
 
 // Tiling for `rows` i-rows: explicit config, else tuned, else heuristic.
-// full: the rows are all the bodies of the pass (a symmetric kernel may serve).
-nbody_status get_tiling(nbody_engine* e, int rows, Tiling* out, bool full = true) {
+// full: the rows are all the bodies of the pass (a symmetric kernel may serve),
+// in Hilbert order from order_min of them on.
+nbody_status get_tiling(nbody_engine* e, int rows, int order_min, Tiling* out, bool full = true) {
   const nbody_config& c = e->cfg;
   // defaults: the best measured shape of each family (Plummer N = 65536);
   // small systems take half the rows per thread, which doubles their row
@@ -677,8 +684,8 @@ nbody_status get_tiling(nbody_engine* e, int rows, Tiling* out, bool full = true
                 "no compiled pair kernel for threads=%d i_per_thread=%d j_tile=%d variant=%d", nt,
                 ipt, tj, variant);
   const bool automatic = !explicit_shape(c) && !c.pair_variant;
-  if (c.tune && automatic && full) return autotune(e, rows, out);
-  if (e->tune_lookup && automatic && tuned_lookup(e, rows, out, full)) return NBODY_OK;
+  if (c.tune && automatic && full) return autotune(e, rows, order_min, out);
+  if (e->tune_lookup && automatic && tuned_lookup(e, rows, order_min, out, full)) return NBODY_OK;
   const bool near_far = c.precision == NBODY_MIXED && c.pair_variant == 4;
   if (full && (automatic || (near_far && !explicit_shape(c)))) {
     choose_sym(e, rows, out);
@@ -704,7 +711,7 @@ nbody_status hilo_tiling(nbody_engine* e, int rows, Tiling* out) {
 
 nbody_status ensure_tiling(nbody_engine* e) {
   if (e->tiled) return NBODY_OK;
-  NB_TRY(get_tiling(e, e->n, &e->tiling));
+  NB_TRY(get_tiling(e, e->n, e->order_min_bodies, &e->tiling));
   NB_TRY(ensure_partials(e, partial_count(e->tiling, e->n)));
   e->tiled = true;
   return NBODY_OK;
@@ -1168,7 +1175,7 @@ nbody_status nbody_create(nbody_engine** out, const nbody_config* cfg) {
     NB_CUDA(cudaMemsetAsync(e->status, 0, sizeof(int), e->stream));
     if (!explicit_shape(e->cfg) && e->cfg.tune == 0) {  // the slots of its own passes
       Tiling t;
-      NB_TRY(get_tiling(e.get(), e->n, &t));
+      NB_TRY(get_tiling(e.get(), e->n, e->order_min_bodies, &t));
       NB_TRY(ensure_partials(e.get(), partial_count(t, e->n)));
     }
     NB_CUDA(cudaStreamSynchronize(e->stream));
@@ -1469,7 +1476,7 @@ nbody_status nbody_acc_jerk_device(nbody_engine* e, int n, const double* x, cons
     if (!p) return fail(NBODY_ERR_INVALID_ARG, "null device array");
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : e->stream;
   Tiling t;
-  NB_TRY(get_tiling(e, n, &t));
+  NB_TRY(get_tiling(e, n, kForeignOrderMin, &t));
   NB_TRY(ensure_partials(e, partial_count(t, n)));
   const SoA7 in{x, y, z, m, vx, vy, vz};
   const SoA6 out{ax, ay, az, jx, jy, jz};
@@ -1584,7 +1591,7 @@ extern "C" nbody_status nbody_force_calculation(int n, double eps2, int precisio
   NB_TRY(ensure_tiling(e));
   Tiling t = e->tiling;
   const bool full = i_begin == 0 && i_end == n;
-  if (!full) NB_TRY(get_tiling(e, i_end - i_begin, &t, false));
+  if (!full) NB_TRY(get_tiling(e, i_end - i_begin, kForeignOrderMin, &t, false));
   // a row range: the packed hi/lo kernel, whose rows stay in the caller's
   // order (the near/far kernel evaluates all rows in Hilbert order)
   if (!full && tile_relative(t.k->fmt)) NB_TRY(hilo_tiling(e, i_end - i_begin, &t));

@@ -43,3 +43,23 @@ def test_one_sided_near_far_calls_get_their_bodies_in_order():
     ref = O.force_rows(s, EPS2, rows)
     ea = vec_rel(out.cpu().numpy()[:3, rows], ref[:3])
     assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4
+
+
+def test_tuned_tilings_of_ordered_and_unordered_passes_are_apart():
+    """Between 16384 and 32768 bodies an engine's passes run on bodies in
+    Hilbert order and a drop-in call's do not: neither takes the tiling that
+    was timed for the other."""
+    n = 20011
+    s = nb.plummer(n, seed=5)
+    nb.release_force_cache()
+    try:
+        nb.force_calculation_tune(s, eps2=EPS2, precision="mixed")
+        source = []
+        for _ in range(2):
+            with nb.Engine(n, eps2=EPS2, precision="mixed", dt=1.0, tune=True) as e:
+                e.set_state(s)
+                e.force_calculation()
+                source.append(e.timers()["tiling_source"])
+    finally:
+        nb.release_force_cache()
+    assert source == [2, 3]  # timed for this engine, then taken from the cache
