@@ -568,13 +568,12 @@ TuneKey tune_key(const nbody_engine* e, int rows, int order_min) {
   return {e->dev, e->cfg.precision, fmt, e->ld, rows, wants_order(e, fmt, rows, order_min)};
 }
 
-// The tiling the autotuner cached for `rows` bodies on this engine, if any.
-bool tuned_lookup(const nbody_engine* e, int rows, int order_min, Tiling* out, bool full = true) {
+// The tiling the autotuner cached for full passes over `rows` bodies, if any.
+bool tuned_lookup(const nbody_engine* e, int rows, int order_min, Tiling* out) {
   const TuneKey key = tune_key(e, rows, order_min);
   std::lock_guard<std::mutex> g(g_tune_mu);
   auto it = g_tuned.find(key);
   if (it == g_tuned.end()) return false;
-  if (!full && registry()[it->second.first].sym) return false;  // evaluates all rows only
   out->k = &registry()[it->second.first];
   out->split = it->second.second;
   out->source = 3;
@@ -685,7 +684,7 @@ nbody_status get_tiling(nbody_engine* e, int rows, int order_min, Tiling* out, b
                 ipt, tj, variant);
   const bool automatic = !explicit_shape(c) && !c.pair_variant;
   if (c.tune && automatic && full) return autotune(e, rows, order_min, out);
-  if (e->tune_lookup && automatic && tuned_lookup(e, rows, order_min, out, full)) return NBODY_OK;
+  if (e->tune_lookup && automatic && full && tuned_lookup(e, rows, order_min, out)) return NBODY_OK;
   const bool near_far = c.precision == NBODY_MIXED && c.pair_variant == 4;
   if (full && (automatic || (near_far && !explicit_shape(c)))) {
     choose_sym(e, rows, out);
