@@ -316,6 +316,11 @@ struct nbody_engine {
   // for the ordering.  An engine re-orders every sort_every steps; a drop-in
   // or device-array call on every call (kForeignOrderMin).
   int order_min_bodies = 16384;
+  // The device-array calls' last size and its tiling: planning takes 20 us at n
+  // = 40000 and 60 at 262144, on the host ahead of every launch.  The choice
+  // depends on the size and the engine's configuration only.
+  int foreign_n = 0;
+  Tiling foreign_tiling;
   // drop-in engines: reuse a tiling the autotuner chose for the same
   // (device, precision, record format, size) in this process; never tune
   bool tune_lookup = false;
@@ -1474,8 +1479,12 @@ nbody_status nbody_acc_jerk_device(nbody_engine* e, int n, const double* x, cons
   for (auto p : ptrs)
     if (!p) return fail(NBODY_ERR_INVALID_ARG, "null device array");
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : e->stream;
-  Tiling t;
-  NB_TRY(get_tiling(e, n, kForeignOrderMin, &t));
+  if (e->foreign_n != n) {
+    e->foreign_n = 0;
+    NB_TRY(get_tiling(e, n, kForeignOrderMin, &e->foreign_tiling));
+    e->foreign_n = n;
+  }
+  const Tiling& t = e->foreign_tiling;
   NB_TRY(ensure_partials(e, partial_count(t, n)));
   const SoA7 in{x, y, z, m, vx, vy, vz};
   const SoA6 out{ax, ay, az, jx, jy, jz};

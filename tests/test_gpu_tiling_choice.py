@@ -63,3 +63,20 @@ def test_tuned_tilings_of_ordered_and_unordered_passes_are_apart():
     finally:
         nb.release_force_cache()
     assert source == [2, 3]  # timed for this engine, then taken from the cache
+
+
+def test_device_calls_of_alternating_sizes():
+    """The kept tiling of a device-array call is that of its size."""
+    import torch
+    s = nb.plummer(3000, seed=5)
+    t, out = device_arrays(s)
+    with nb.Engine(3000, eps2=EPS2, dt=1.0) as e:
+        for n in (3000, 100, 2500, 2500, 3000):
+            sub = [a[:n] for a in t]
+            got = torch.empty(6, n, dtype=torch.float64, device="cuda")
+            e.acc_jerk_device(*sub, list(got), stream=stream())
+            with nb.Engine(3000, eps2=EPS2, dt=1.0) as f:
+                want = torch.empty_like(got)
+                f.acc_jerk_device(*sub, list(want), stream=stream())
+                torch.cuda.synchronize()
+            assert torch.equal(got, want), n
