@@ -75,6 +75,11 @@ constexpr int kStepsPerGraph = 8;
 constexpr int kStageInBodies = 16384;
 constexpr int kStageOutBodies = 65536;
 constexpr int kDropInStageBodies = 32768;
+// Slots that nbody_create allocates: those of systems up to about 400000 bodies,
+// whose first pass takes less than 0.2 s.  A larger one's (5.8 GB at 10^6
+// bodies) wait for its first pass, which an engine made for energies, or for
+// calls on fewer bodies, never runs.
+constexpr double kEagerSlotBytes = 2.0 * (1 << 30);
 // Calls on caller-owned bodies order them for the near/far kernel from this
 // many bodies: ordering costs about 0.09 ms a call and saves the pair pass
 // 0.02 ms at N = 16384.
@@ -343,13 +348,13 @@ bool explicit_shape(const nbody_config& c) {
   return c.threads || c.i_per_thread || c.j_tile || c.split_j || c.j_cluster;
 }
 
-// The mixed kernel family in use: pair_variant, 0 (automatic) being near/far;
-// with an explicit (one-sided) shape, packed hi/lo below order_min_bodies,
-// where the one-sided near/far kernel is the slower of the two.
-int effective_variant(const nbody_engine* e) {
+// The mixed kernel family of the one-sided kernels: pair_variant, 0 (automatic)
+// being near/far from order_min_bodies and packed hi/lo below, where the
+// one-sided near/far kernel is the slower of the two.
+int one_sided_variant(const nbody_engine* e) {
   const nbody_config& c = e->cfg;
   if (c.precision != NBODY_MIXED || c.pair_variant != 0) return c.pair_variant;
-  return explicit_shape(c) && e->n < e->order_min_bodies ? 3 : 4;
+  return e->n < e->order_min_bodies ? 3 : 4;
 }
 
 // Record format of the autotuner's family (the automatic choice).
@@ -470,9 +475,11 @@ void drop_step_graphs(nbody_engine* e) {
   }
 }
 
-// Grows P to `split` slots.
+// Grows P to `split` slots.  If they do not fit, the slots there were stay.
 nbody_status ensure_partials(nbody_engine* e, int split) {
   if (split <= e->p_splits) return NBODY_OK;
+  const size_t slot = sizeof(double) * 6 * static_cast<size_t>(e->ld);
+  const int before = e->p_splits;
   if (e->P) {
     NB_CUDA(cudaStreamSynchronize(e->stream));
     cudaFree(e->P);
@@ -480,8 +487,17 @@ nbody_status ensure_partials(nbody_engine* e, int split) {
   drop_step_graphs(e);  // the captured steps refer to the old buffer
   e->P = nullptr;
   e->p_splits = 0;
-  NB_CUDA(cudaMalloc(&e->P, sizeof(double) * 6 * static_cast<size_t>(e->ld) * split));
-  e->p_splits = split;
+  for (const int want : {split, before}) {
+    if (want == 0) break;
+    if (cudaMalloc(&e->P, slot * want) == cudaSuccess) {
+      e->p_splits = want;
+      break;
+    }
+    e->P = nullptr;
+    cudaGetLastError();  // reported below
+  }
+  if (e->p_splits < split)
+    return fail(NBODY_ERR_OOM, "no memory for %d partial-sum slots of %zu bytes", split, slot);
   return NBODY_OK;
 }
 
@@ -630,7 +646,9 @@ nbody_status autotune(nbody_engine* e, int rows, int order_min, Tiling* out) {
     NB_TRY(launch_pack(e, e->n, own_inputs(e), e->stream, k.fmt, k.tj, ordered));
     for (int s : {std::max(1, s0 / 2), s0, std::min(kMaxSplit, s0 * 2)}) {
       Tiling t{&k, s};
-      NB_TRY(ensure_partials(e, partial_count(t, rows)));
+      const nbody_status fits = ensure_partials(e, partial_count(t, rows));
+      if (fits == NBODY_ERR_OOM) continue;
+      NB_TRY(fits);
       NB_TRY(launch_pair(e, t, 0, rows, e->stream));  // warm-up
       NB_CUDA(cudaEventRecord(a, e->stream));
       for (int r = 0; r < 3; ++r) NB_TRY(launch_pair(e, t, 0, rows, e->stream));
@@ -656,7 +674,7 @@ nbody_status autotune(nbody_engine* e, int rows, int order_min, Tiling* out) {
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   NB_TRY(check_status_word(e));
-  if (best_idx < 0) return fail(NBODY_ERR_STATE, "autotune found no kernel");
+  if (best_idx < 0) return fail(NBODY_ERR_OOM, "no memory for the partial-sum slots of any symmetric kernel");
   out->k = &reg[best_idx];
   out->split = best_split;
   out->source = 2;
@@ -674,7 +692,7 @@ nbody_status get_tiling(nbody_engine* e, int rows, int order_min, Tiling* out, b
   // small systems take half the rows per thread, which doubles their row
   // blocks (FP64 below 32768 rows: N = 4096 40 vs 48 us per launch;
   // tile-relative below 8192 rows)
-  const int variant = effective_variant(e);
+  const int variant = one_sided_variant(e);
   const bool rel = c.precision == NBODY_MIXED && variant == 4;
   int nt = c.threads ? c.threads : 128;
   int ipt = c.i_per_thread ? c.i_per_thread
@@ -713,10 +731,23 @@ nbody_status hilo_tiling(nbody_engine* e, int rows, Tiling* out) {
   return NBODY_OK;
 }
 
+// Tiling of a full pass over n bodies with its slots in place.  Where the
+// symmetric kernels' slots (up to 128, 48 bytes per body each) find no memory,
+// the pass is one-sided, with as many splits as fit.
+nbody_status settle_tiling(nbody_engine* e, int n, int order_min, Tiling* out) {
+  nbody_status s = get_tiling(e, n, order_min, out);
+  if (s == NBODY_OK) s = ensure_partials(e, partial_count(*out, n));
+  if (s != NBODY_ERR_OOM || explicit_shape(e->cfg)) return s;
+  NB_TRY(get_tiling(e, n, order_min, out, false));
+  for (;; out->split = (out->split + 1) / 2) {
+    s = ensure_partials(e, partial_count(*out, n));
+    if (s != NBODY_ERR_OOM || out->split == 1) return s;
+  }
+}
+
 nbody_status ensure_tiling(nbody_engine* e) {
-  if (e->tiled) return NBODY_OK;
-  NB_TRY(get_tiling(e, e->n, e->order_min_bodies, &e->tiling));
-  NB_TRY(ensure_partials(e, partial_count(e->tiling, e->n)));
+  if (e->tiled) return ensure_partials(e, partial_count(e->tiling, e->n));
+  NB_TRY(settle_tiling(e, e->n, e->order_min_bodies, &e->tiling));
   e->tiled = true;
   return NBODY_OK;
 }
@@ -1180,7 +1211,11 @@ nbody_status nbody_create(nbody_engine** out, const nbody_config* cfg) {
     if (!explicit_shape(e->cfg) && e->cfg.tune == 0) {  // the slots of its own passes
       Tiling t;
       NB_TRY(get_tiling(e.get(), e->n, e->order_min_bodies, &t));
-      NB_TRY(ensure_partials(e.get(), partial_count(t, e->n)));
+      const int slots = partial_count(t, e->n);
+      if (48.0 * ld * slots <= kEagerSlotBytes) {
+        const nbody_status fits = ensure_partials(e.get(), slots);
+        if (fits != NBODY_ERR_OOM) NB_TRY(fits);  // else: settle_tiling at the first pass
+      }
     }
     NB_CUDA(cudaStreamSynchronize(e->stream));
     return NBODY_OK;
@@ -1481,7 +1516,7 @@ nbody_status nbody_acc_jerk_device(nbody_engine* e, int n, const double* x, cons
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : e->stream;
   if (e->foreign_n != n) {
     e->foreign_n = 0;
-    NB_TRY(get_tiling(e, n, kForeignOrderMin, &e->foreign_tiling));
+    NB_TRY(settle_tiling(e, n, kForeignOrderMin, &e->foreign_tiling));
     e->foreign_n = n;
   }
   const Tiling& t = e->foreign_tiling;

@@ -1,0 +1,66 @@
+"""Partial-sum slots on a device with little memory left."""
+import numpy as np
+import pytest
+
+import nbody_b200 as nb
+import oracle as O
+from _util import derivs_rel, vec_rel
+
+pytestmark = pytest.mark.gpu
+
+EPS2 = 1e-4
+
+
+@pytest.fixture
+def crowded():
+    """Leaves `keep` bytes of device memory free."""
+    import torch
+    held = []
+
+    def hold(keep):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free, _ = torch.cuda.mem_get_info()
+        assert free > keep
+        held.append(torch.empty(int(free - keep), dtype=torch.uint8, device="cuda"))
+    yield hold
+    held.clear()
+    torch.cuda.empty_cache()
+
+
+def test_the_largest_engine_is_created():
+    """2^28 bodies, the largest n: 62 GB of state and records; the slots of a
+    symmetric pass (up to 412 GB) wait for a pass."""
+    with nb.Engine(1 << 28, eps2=EPS2, dt=1.0) as e:
+        assert e.timers()["tiling_source"] == 0
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_passes_without_room_for_the_symmetric_slots(precision, crowded):
+    """600001 bodies want 2.5 GB and more of slots: with 1.2 GB left the pass is
+    one-sided; device-array calls likewise."""
+    import torch
+    n = 600001
+    s = nb.plummer(n, seed=2)
+    rows = np.arange(0, n, 9973)
+    ref = O.force_rows(s, EPS2, rows)
+    t = [torch.tensor(s[k], device="cuda") for k in nb.FIELDS]
+    out = torch.empty(6, n, dtype=torch.float64, device="cuda")
+    crowded(1.2e9)
+    got = []
+    with nb.Engine(n, eps2=EPS2, precision=precision, dt=1.0) as e:
+        e.set_state(s)
+        e.force_calculation()
+        got.append(e.get_derivs()[:, rows])
+        assert e.timers()["split_j"] * 48 * n < 1.2e9
+    with nb.Engine(n, eps2=EPS2, precision=precision, dt=1.0) as e:
+        e.acc_jerk_device(*t, list(out), stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        got.append(out.cpu().numpy()[:, rows])
+    for d in got:
+        if precision == "fp64":
+            ea, ej = derivs_rel(d, ref)
+            assert ea <= 1e-12 and ej <= 1e-12, (ea, ej)
+        else:
+            ea = vec_rel(d[:3], ref[:3])
+            assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4, (np.median(ea), ea.max())
