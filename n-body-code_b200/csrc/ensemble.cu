@@ -60,6 +60,9 @@ constexpr int kBlock = 256;
 // 2.89 (512); 256 of 256-1024 302 us (1024), 193 (512); 16 of 256-2048 284 us
 // (1024), 152 (512), 56 (128).
 constexpr int kItemBodies[] = {1024, 512, 256, 128, 64};
+// A j-tile of the interface (tiles_per_item, info's j_tile) in tiles of the
+// kernel: FP64 items are given in tiles of 128 bodies, whatever the kernel streams.
+constexpr int kFp64ItemTile = 128;
 constexpr double kItemsPerCta = 2.5;
 constexpr int kWideCtasPerSm = 6;  // resident CTAs of the four-row near/far shape
 
@@ -423,6 +426,7 @@ struct nbody_ensemble {
   cudaGraphExec_t order_graph = nullptr;
   int order_kernels = 0;
   long long reorders = 0;
+  int tile_unit() const { return precision == NBODY_FP64 ? kFp64ItemTile / kSymTile64 : 1; }
 };
 
 namespace {
@@ -951,7 +955,8 @@ nbody_status nbody_ensemble_create(nbody_ensemble** out, const nbody_ensemble_co
       if (first) break;
       first = &k;
     }
-    return build_items(raw, cfg->tiles_per_item > 0 ? cfg->tiles_per_item : default_tiles_per_item(raw));
+    if (cfg->tiles_per_item == 0) return build_items(raw, default_tiles_per_item(raw));
+    return build_items(raw, std::min(cfg->tiles_per_item, 1 << 28) * raw->tile_unit());
   };
   nbody_status s = body();
   if (s != NBODY_OK) {
@@ -1061,8 +1066,9 @@ nbody_status nbody_ensemble_info(nbody_ensemble* e, nbody_ensemble_info_t* out) 
   out->nclusters = e->C;
   out->padded_rows = e->L;
   out->items = e->n_items;
-  out->tiles_per_item = e->tiles_per_item;
-  out->j_tile = e->kern->tile;
+  const int unit = e->tile_unit();
+  out->tiles_per_item = e->tiles_per_item < 0 ? -1 : (e->tiles_per_item + unit - 1) / unit;
+  out->j_tile = e->kern->tile * unit;
   out->threads = e->kern->nt;
   out->grid = e->grid;
   out->interactions_per_step = static_cast<double>(e->interactions);

@@ -80,3 +80,25 @@ def test_device_calls_of_alternating_sizes():
                 f.acc_jerk_device(*sub, list(want), stream=stream())
                 torch.cuda.synchronize()
             assert torch.equal(got, want), n
+
+
+@pytest.mark.parametrize("tpi", [1, 8, 100])
+def test_fp64_ensemble_items_are_given_in_tiles_of_128_bodies(tpi):
+    """tiles_per_item = 8: 1024 bodies per item, as the packed hi/lo ensembles'."""
+    sizes = [5000, 700, 100]
+    s = [nb.plummer(n, seed=n) for n in sizes]
+    with nb.Ensemble(sizes, EPS2, 1 / 512, precision="fp64", tiles_per_item=tpi) as e:
+        e.set_state({k: np.concatenate([p[k] for p in s]) for k in nb.FIELDS})
+        e.force_calculation()
+        info, d, off = e.info(), e.get_derivs(), e.offsets
+    assert info["tiles_per_item"] == tpi and info["j_tile"] == 128
+    items = 0
+    for n in sizes:
+        blocks, tiles = -(-n // 256), -(-n // 32)  # tiles of the kernel
+        first = min((blocks // 2 + 1) * 8, tiles)  # the first block's run
+        items += blocks * -(-first // (4 * tpi))
+    assert info["items"] == items
+    for c, p in enumerate(s):
+        rows = np.arange(0, sizes[c], 7)
+        got, ref = d[:, off[c]:off[c + 1]][:, rows], O.force_rows(p, EPS2, rows)
+        assert vec_rel(got[:3], ref[:3]).max() <= 1e-12
