@@ -751,8 +751,10 @@ nbody_status ens_build_graph(nbody_ensemble* e) {
   return NBODY_OK;
 }
 
-// Times the pair launch for every (kernel shape, item size) pair; keeps the
-// fastest.  Items count j-tiles, so tiles_per_item x tile = j per item.
+// Times the pair launch for every (kernel shape, item size) pair, the default's
+// sizes among them, and keeps the pair with the least time of launch and slot
+// sums (short items leave many slots).  Items count j-tiles, so tiles_per_item
+// x tile = j per item.
 nbody_status ens_autotune(nbody_ensemble* e) {
   EN_TRY(launch_ens_pack(e));
   cudaEvent_t a, b;
@@ -765,8 +767,14 @@ nbody_status ens_autotune(nbody_ensemble* e) {
     if (k.precision != e->precision || k.fmt != e->fmt) continue;
     EN_TRY(use_kernel(e, &k));
     if (e->fmt == kRecRel) EN_TRY(ens_records(e, e->stream, false));  // this kernel's tile size
-    for (int j_per_item : {256, 512, 1024, 2048, 4096, 8192}) {
+    // shorter items than 256 bodies only where the default takes them: they
+    // leave the most slots
+    const int least = std::min(std::max(1, 256 / k.tile), default_tiles_per_item(e));
+    int last_tpi = 0;
+    for (int j_per_item : {64, 128, 256, 512, 1024, 2048, 4096, 8192}) {
       const int tpi = std::max(1, j_per_item / k.tile);
+      if (tpi == last_tpi || tpi < least) continue;
+      last_tpi = tpi;
       EN_TRY(build_items(e, tpi));
       EN_TRY(launch_ens_pair(e));
       EN_CUDA(cudaEventRecord(a, e->stream));
@@ -775,9 +783,11 @@ nbody_status ens_autotune(nbody_ensemble* e) {
       EN_CUDA(cudaEventSynchronize(b));
       float ms = 0;
       EN_CUDA(cudaEventElapsedTime(&ms, a, b));
+      const float pair_ms = ms / 2;
+      ms = pair_ms + static_cast<float>(8.0 * e->p_doubles / kSplitSumBytesPerMs);
       if (getenv("NBODY_TUNE_VERBOSE"))
-        fprintf(stderr, "[nbody ens tune] nt=%d tile=%d tiles_per_item=%d  %.4f ms\n", k.nt, k.tile,
-                tpi, ms / 2);
+        fprintf(stderr, "[nbody ens tune] nt=%d tile=%d tiles_per_item=%d  %.4f ms (pair %.4f)\n", k.nt,
+                k.tile, tpi, ms, pair_ms);
       if (ms < best) {
         best = ms;
         best_k = &k;

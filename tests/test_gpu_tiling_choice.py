@@ -102,3 +102,27 @@ def test_fp64_ensemble_items_are_given_in_tiles_of_128_bodies(tpi):
         rows = np.arange(0, sizes[c], 7)
         got, ref = d[:, off[c]:off[c + 1]][:, rows], O.force_rows(p, EPS2, rows)
         assert vec_rel(got[:3], ref[:3]).max() <= 1e-12
+
+
+@pytest.mark.parametrize("precision,variant", [("fp64", 0), ("mixed", 0), ("mixed", 4)])
+def test_ensemble_tuning_tries_the_default_item_size(precision, variant, capfd, monkeypatch):
+    """A small ensemble's default items are shorter than 256 bodies."""
+    rng = np.random.default_rng(1)
+    sizes = rng.integers(256, 2048, 16)
+    parts = [nb.plummer(int(n), seed=int(n)) for n in sizes]
+    state = {k: np.concatenate([p[k] for p in parts]) for k in nb.FIELDS}
+    kw = dict(precision=precision, pair_variant=variant)
+    with nb.Ensemble(sizes, EPS2, 1 / 512, **kw) as e:
+        default = e.info()
+    bodies = default["tiles_per_item"] * default["j_tile"]
+    assert bodies <= 128
+    monkeypatch.setenv("NBODY_TUNE_VERBOSE", "1")
+    with nb.Ensemble(sizes, EPS2, 1 / 512, tune=True, **kw) as e:
+        e.set_state(state)
+        e.force_calculation()
+    tried = []
+    for line in capfd.readouterr().err.splitlines():
+        if "[nbody ens tune]" in line:
+            f = dict(w.split("=") for w in line.split() if "=" in w)
+            tried.append(int(f["tile"]) * int(f["tiles_per_item"]))
+    assert tried and any(t <= bodies for t in tried), (bodies, sorted(set(tried)))
