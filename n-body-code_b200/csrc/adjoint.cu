@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "../../include/nbody_cuda.h"
+#include "devptr.h"
 #include "errors.h"
 #include "hermite.cuh"
 #include "pair.cuh"
@@ -451,9 +452,27 @@ nbody_status vjp(nbody_adjoint* a, cudaStream_t st) {
   return NBODY_OK;
 }
 
+bool all_local(const nbody_adjoint* a, const double* const* p, int count) {
+  return std::all_of(p, p + count, [&](const double* q) {
+    return !q || local_to(q, a->cfg.device, [](cudaPointerAttributes* at, const void* r) {
+      return cudaPointerGetAttributes(at, r);
+    });
+  });
+}
+
 // The caller's `count` arrays (n each; null: zeros) into consecutive [ld]
-// arrays, padding rows zero.
+// arrays, padding rows zero.  Arrays that are not this device's own memory go
+// through the runtime's copies, which reach a peer's memory and refuse what
+// they cannot read.
 nbody_status copy_rows(nbody_adjoint* a, cudaStream_t st, const double* const* src, double* dst, int count) {
+  if (!all_local(a, src, count)) {
+    AD_CUDA(cudaMemsetAsync(dst, 0, sizeof(double) * a->ld * count, st));
+    for (int k = 0; k < count; ++k)
+      if (src[k])
+        AD_CUDA(cudaMemcpyAsync(dst + static_cast<size_t>(k) * a->ld, src[k], sizeof(double) * a->n,
+                                cudaMemcpyDeviceToDevice, st));
+    return NBODY_OK;
+  }
   GatherArgs g{};
   g.arrays = count;
   for (int k = 0; k < count; ++k) {
@@ -466,6 +485,12 @@ nbody_status copy_rows(nbody_adjoint* a, cudaStream_t st, const double* const* s
 }
 // And back: consecutive [ld] arrays to the caller's.
 nbody_status copy_out(nbody_adjoint* a, cudaStream_t st, const double* src, double* const* dst, int count) {
+  if (!all_local(a, dst, count)) {
+    for (int k = 0; k < count; ++k)
+      AD_CUDA(cudaMemcpyAsync(dst[k], src + static_cast<size_t>(k) * a->ld, sizeof(double) * a->n,
+                              cudaMemcpyDeviceToDevice, st));
+    return NBODY_OK;
+  }
   GatherArgs g{};
   g.arrays = count;
   for (int k = 0; k < count; ++k) {

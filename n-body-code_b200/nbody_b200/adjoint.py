@@ -37,13 +37,16 @@ def _f(name):
     return _lib.bind(name, _SIGS[name])
 
 
-def _p(t):
-    assert t.is_cuda and t.dtype.is_floating_point and t.is_contiguous()
+def _p(t, n):
+    """Address of a contiguous float64 CUDA array of at least n values."""
+    assert t.is_cuda and t.dtype.is_floating_point and t.element_size() == 8
+    assert t.is_contiguous() and t.numel() >= n
     return _vp(t.data_ptr())
 
 
-def _rows(t):
-    return [t[k] for k in range(t.shape[0])]
+def _rows(t, n):
+    assert t.shape[0] == 3
+    return [_p(t[k], n) for k in range(3)]
 
 
 class Adjoint:
@@ -70,21 +73,22 @@ class Adjoint:
             pass
 
     def forward(self, x, v, m, x1, v1, stream: int):
-        check(_f("nbody_adjoint_forward")(self._h, *map(_p, _rows(x)), _p(m), *map(_p, _rows(v)),
-                                          *map(_p, _rows(x1)), *map(_p, _rows(v1)), _vp(stream)),
+        n = self.n
+        check(_f("nbody_adjoint_forward")(self._h, *_rows(x, n), _p(m, n), *_rows(v, n),
+                                          *_rows(x1, n), *_rows(v1, n), _vp(stream)),
               "nbody_adjoint_forward")
 
     def backward(self, gx1, gv1, gx0, gv0, gm, stream: int):
-        check(_f("nbody_adjoint_backward")(self._h, *map(_p, _rows(gx1)), *map(_p, _rows(gv1)),
-                                           *map(_p, _rows(gx0)), *map(_p, _rows(gv0)), _p(gm),
-                                           _vp(stream)),
+        n = self.n
+        check(_f("nbody_adjoint_backward")(self._h, *_rows(gx1, n), *_rows(gv1, n), *_rows(gx0, n),
+                                           *_rows(gv0, n), _p(gm, n), _vp(stream)),
               "nbody_adjoint_backward")
 
     def vjp_acc_jerk(self, x, v, m, abar, jbar, gx, gv, gm, stream: int):
-        check(_f("nbody_adjoint_vjp_acc_jerk")(self._h, *map(_p, _rows(x)), _p(m), *map(_p, _rows(v)),
-                                               *map(_p, _rows(abar)), *map(_p, _rows(jbar)),
-                                               *map(_p, _rows(gx)), *map(_p, _rows(gv)), _p(gm),
-                                               _vp(stream)),
+        n = self.n
+        check(_f("nbody_adjoint_vjp_acc_jerk")(self._h, *_rows(x, n), _p(m, n), *_rows(v, n),
+                                               *_rows(abar, n), *_rows(jbar, n), *_rows(gx, n),
+                                               *_rows(gv, n), _p(gm, n), _vp(stream)),
               "nbody_adjoint_vjp_acc_jerk")
 
 
