@@ -20,6 +20,7 @@
 #include <utility>
 
 #include "pair.cuh"
+#include "symplan.h"
 
 namespace nbody {
 
@@ -215,22 +216,6 @@ static __global__ void predict_kernel(int n, int ld, const StepCtl* __restrict__
   if (jb32) jb32[i] = make_jb32(p[0], p[1], p[2], m, u[0], u[1], u[2]);
   if (jbx2) jbx2[i] = make_jbx2(p[0], p[1], p[2], m, u[0], u[1], u[2]);
 }
-
-// Partial-sum slots of a row: S of every row and, where the symmetric pair
-// kernels (sympair.cuh) wrote them, one per block at distance 1, 2, ... ahead
-// of which the row's block lies.
-struct RowSlots {
-  int S;           // splits
-  int block_rows;  // rows per block of the symmetric schedule
-  int nb;          // its blocks; 0: no such slots
-  __host__ __device__ RowSlots(int splits, int rows = 1, int blocks = 0)
-      : S(splits), block_rows(rows), nb(blocks) {}
-  __device__ __forceinline__ int count(int i) const {
-    if (nb == 0) return S;
-    const int half = nb / 2;  // an even nb's last distance reaches the upper half only
-    return S + ((nb & 1) ? half : half - (i / block_rows < half ? 1 : 0));
-  }
-};
 
 // sum[c] = sum over slots s = 0, 1, ..., S-1 (in that order) of
 // P[s * step][c][i], for the F fields at once: one pass over the splits with
