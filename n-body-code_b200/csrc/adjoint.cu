@@ -325,17 +325,18 @@ struct SymLaunch {
   size_t smem = 0;
   int rows = 0, tj = 0, S = 1, subs = 1, nb = 1, block_rows = 1;
   double ms = 0;  // predicted
-  cudaError_t plan(const void* f, size_t sm, int rows_, int tj_, int n, int sms, double rate, double tail) {
+  cudaError_t plan(const void* f, size_t sm, int rows_, int tj_, int n, int sms, double rate, double tail,
+                   int most_slots) {
     fn = f; smem = sm; rows = rows_; tj = tj_;
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
     if (e != cudaSuccess) return e;
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, 32 * kW, sm);
     if (e != cudaSuccess) return e;
-    const SymPlan p = sym_plan(sms, std::max(occ, 1), rows, tj, n, rate, tail);
+    const SymPlan p = sym_plan(sms, std::max(occ, 1), rows, tj, n, rate, tail, most_slots);
     S = p.S;
     ms = p.ms;
-    const SymGrid g(rows, n);
+    const SymGrid g(rows, n, most_slots);
     subs = g.subs; nb = g.nb; block_rows = g.block_rows;
     return cudaSuccess;
   }
@@ -371,8 +372,9 @@ struct nbody_adjoint {
   double* adj = nullptr;    // [13][ld] xb vb ab jb, mb
   double* ab1 = nullptr;    // [6][ld] caller's acc/jerk adjoints (vjp_acc_jerk)
   double* mb = nullptr;     // adj's last array
-  double* P = nullptr;      // forward slots [..][6][ld]
-  double* Pv = nullptr;     // VJP slots [..][7][ld]
+  // Slots of the forward pass, [..][6][ld], or of the VJP, [..][7][ld]: each
+  // pass's are summed by the kernel after it
+  double* P = nullptr;
   JBody64* jb64 = nullptr;
   SymSub* jsub = nullptr;
   JAdj* jadj = nullptr;
@@ -398,6 +400,26 @@ SymArgs sym_args(const nbody_adjoint* a, double* out) {
 SoA7 own_state(const nbody_adjoint* a) {
   const size_t ld = a->ld;
   return SoA7{a->X, a->X + ld, a->X + 2 * ld, a->M, a->V, a->V + ld, a->V + 2 * ld};
+}
+
+// The forward's kernel and splits (the engine's choice) and the VJP's, of at most
+// most_slots partial-sum slots each.
+cudaError_t plan_passes(nbody_adjoint* a, int most_slots) {
+  const bool fp64 = a->cfg.precision == NBODY_FP64;
+  for (const bool wide : {false, true}) {
+    if (a->n < sym_min_bodies(wide)) continue;
+    const size_t smem = fp64 ? (wide ? sym_fp64_smem<4, kW, 2>() : sym_fp64_smem<2, kW, 4>())
+                             : (wide ? sym_nf_smem<4, kW, 2>() : sym_nf_smem<2, kW, 1>());
+    SymLaunch l;
+    const cudaError_t e =
+        l.plan(fp64 ? fwd_fp64(wide) : fwd_mixed(wide), smem, 32 * kW * (wide ? 4 : 2),
+               fp64 ? kSymTile64 : wide ? 128 : 64, a->n, a->sms, sym_rate(fp64, wide),
+               fp64 ? kSymTail64 : kSymTailNF, most_slots);
+    if (e != cudaSuccess) return e;
+    if (!wide || l.ms < a->fwd.ms) a->fwd = l;
+  }
+  return a->rev.plan(vjp_fn(), vjp_smem<2, kW>(), 32 * kW * 2, kVjpTile, a->n, a->sms, 3.3e8, kSymTail64,
+                     most_slots);
 }
 
 nbody_status fwd_eval(nbody_adjoint* a, cudaStream_t st) {
@@ -441,14 +463,14 @@ nbody_status link(nbody_adjoint* a, cudaStream_t st, bool sum, bool post, AdjPac
                   const double* XV = nullptr, const double* AB = nullptr) {
   constexpr int rows = kSumRows<8>;
   AD_CUDA(launch_chained(adj_link_kernel, (a->ld + rows - 1) / rows, kSumThreads, 0, st, a->n, a->ld,
-                         a->cfg.dt, a->rev.slots(), sum, a->Pv, post, a->adj, a->mb,
+                         a->cfg.dt, a->rev.slots(), sum, a->P, post, a->adj, a->mb,
                          static_cast<int>(pack), XV, a->M, AB, a->jadj));
   return NBODY_OK;
 }
 
 // Slots of the pair VJP at the packed records.
 nbody_status vjp(nbody_adjoint* a, cudaStream_t st) {
-  AD_CUDA(a->rev.launch(a->jadj, sym_args(a, a->Pv), st));
+  AD_CUDA(a->rev.launch(a->jadj, sym_args(a, a->P), st));
   return NBODY_OK;
 }
 
@@ -530,7 +552,7 @@ nbody_status nbody_adjoint_destroy(nbody_adjoint* a) {
   if (!a) return NBODY_OK;
   cudaSetDevice(a->cfg.device);
   cudaDeviceSynchronize();
-  void* bufs[] = {a->state, a->ckpt, a->segxv, a->adj, a->ab1, a->P, a->Pv,
+  void* bufs[] = {a->state, a->ckpt, a->segxv, a->adj, a->ab1, a->P,
                   a->jb64, a->jsub, a->jadj, a->ctl, a->status};
   for (void* p : bufs) cudaFree(p);
   delete a;
@@ -567,17 +589,6 @@ nbody_status nbody_adjoint_create(nbody_adjoint** out, const nbody_adjoint_confi
   auto body = [&]() -> nbody_status {
     const size_t ld = r->ld;
     const bool fp64 = cfg->precision == NBODY_FP64;
-    for (const bool wide : {false, true}) {  // the engine's choice
-      if (r->n < sym_min_bodies(wide)) continue;
-      const size_t smem = fp64 ? (wide ? sym_fp64_smem<4, kW, 2>() : sym_fp64_smem<2, kW, 4>())
-                               : (wide ? sym_nf_smem<4, kW, 2>() : sym_nf_smem<2, kW, 1>());
-      SymLaunch l;
-      AD_CUDA(l.plan(fp64 ? fwd_fp64(wide) : fwd_mixed(wide), smem, 32 * kW * (wide ? 4 : 2),
-                     fp64 ? kSymTile64 : wide ? 128 : 64, r->n, r->sms, sym_rate(fp64, wide),
-                     fp64 ? kSymTail64 : kSymTailNF));
-      if (!wide || l.ms < r->fwd.ms) r->fwd = l;
-    }
-    AD_CUDA(r->rev.plan(vjp_fn(), vjp_smem<2, kW>(), 32 * kW * 2, kVjpTile, r->n, r->sms, 3.3e8, kSymTail64));
     AD_CUDA(cudaMalloc(&r->state, sizeof(double) * 13 * ld));
     AD_CUDA(cudaMemset(r->state, 0, sizeof(double) * 13 * ld));
     r->X = r->state;
@@ -589,15 +600,22 @@ nbody_status nbody_adjoint_create(nbody_adjoint** out, const nbody_adjoint_confi
     AD_CUDA(cudaMalloc(&r->adj, sizeof(double) * 13 * ld));
     r->mb = r->adj + 12 * ld;
     AD_CUDA(cudaMalloc(&r->ab1, sizeof(double) * 6 * ld));
-    AD_CUDA(cudaMalloc(&r->P, sizeof(double) * 6 * ld * r->fwd.count()));
-    AD_CUDA(cudaMalloc(&r->Pv, sizeof(double) * 7 * ld * r->rev.count()));
     if (fp64) AD_CUDA(cudaMalloc(&r->jb64, sizeof(JBody64) * ld));
     else AD_CUDA(cudaMalloc(&r->jsub, sizeof(SymSub) * (ld / 64)));
     AD_CUDA(cudaMalloc(&r->jadj, sizeof(JAdj) * ld));
     AD_CUDA(cudaMalloc(&r->ctl, sizeof(StepCtl)));
     AD_CUDA(cudaMalloc(&r->status, sizeof(int)));
     AD_CUDA(cudaMemset(r->status, 0, sizeof(int)));
-    return NBODY_OK;
+    // where memory is short, schedules of fewer blocks and splits
+    for (int most = max_sym_slots(r->n);; most /= 2) {
+      AD_CUDA(plan_passes(r, most));
+      const size_t fields = std::max(6 * r->fwd.count(), 7 * r->rev.count());
+      const cudaError_t e = cudaMalloc(&r->P, sizeof(double) * ld * fields);
+      if (e == cudaSuccess) return NBODY_OK;
+      r->P = nullptr;
+      if (e != cudaErrorMemoryAllocation || most <= 4) AD_CUDA(e);
+      cudaGetLastError();
+    }
   };
   nbody_status s = body();
   if (s != NBODY_OK) {

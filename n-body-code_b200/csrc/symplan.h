@@ -83,10 +83,12 @@ inline int max_sym_slots(int n) {
 }
 
 // The blocks of n bodies for a kernel whose CTAs hold `rows` rows.
+// most_slots: bound on its partial-sum slots.
 struct SymGrid {
   int subs, block_rows, nb;
-  SymGrid(int rows, int n) {
-    const long most = static_cast<long>(std::min(kMaxSymBlocks, max_sym_slots(n))) * rows;
+  SymGrid(int rows, int n) : SymGrid(rows, n, max_sym_slots(n)) {}
+  SymGrid(int rows, int n, int most_slots) {
+    const long most = static_cast<long>(std::min(kMaxSymBlocks, most_slots)) * rows;
     subs = static_cast<int>((n + most - 1) / most);
     block_rows = subs * rows;
     nb = (n + block_rows - 1) / block_rows;
@@ -164,12 +166,12 @@ struct SymPlan {
   int S;
   double ms;
 };
-inline SymPlan sym_plan(int sms, int occ, int rows, int tj, int n, double rate, double tail) {
-  const SymGrid g(rows, n);
+inline SymPlan sym_plan(int sms, int occ, int rows, int tj, int n, double rate, double tail, int most_slots) {
+  const SymGrid g(rows, n, most_slots);
   const long slots = static_cast<long>(sms) * occ;
   const double tile_ms = 2.0 * rows * tj * slots / rate;
   SymPlan best{1, 1e300};
-  for_sym_splits(g, tj, n, std::min(kMaxSymSplits, max_sym_slots(n) / 2), [&](const SymSplit& p) {
+  for_sym_splits(g, tj, n, std::min(kMaxSymSplits, std::max(1, most_slots / 2)), [&](const SymSplit& p) {
     const double one = static_cast<double>(p.tps) * g.subs + kSymCtaTiles;
     const double mean = p.mean * g.subs + kSymCtaTiles;
     const long last = (p.ctas + 1) % slots;
@@ -183,6 +185,9 @@ inline SymPlan sym_plan(int sms, int occ, int rows, int tj, int n, double rate, 
     if (ms < best.ms) best = {p.S, ms};
   });
   return best;
+}
+inline SymPlan sym_plan(int sms, int occ, int rows, int tj, int n, double rate, double tail) {
+  return sym_plan(sms, occ, rows, tj, n, rate, tail, max_sym_slots(n));
 }
 
 // Splits of the potential kernel, which leaves no slots and keeps 7 to 10 CTAs

@@ -64,3 +64,29 @@ def test_passes_without_room_for_the_symmetric_slots(precision, crowded):
         else:
             ea = vec_rel(d[:3], ref[:3])
             assert np.median(ea) <= 2e-6 and ea.max() <= 2e-4, (np.median(ea), ea.max())
+
+
+def test_adjoint_without_room_for_all_slots(crowded):
+    """200003 bodies want 1.3 GB of slots; with less left the schedules get fewer
+    blocks and splits.  Same sums in another order: 1e-11 of each kind's
+    largest value."""
+    import torch
+    n = 200003
+    s = nb.plummer(n, seed=2)
+    rng = np.random.default_rng(3)
+    x, v, a, j = (torch.tensor(w, device="cuda") for w in
+                  (np.stack([s[k] for k in "xyz"]), np.stack([s[k] for k in ("vx", "vy", "vz")]),
+                   rng.normal(size=(3, n)), rng.normal(size=(3, n))))
+    m = torch.tensor(s["m"], device="cuda")
+    out = []
+    for crowd in (False, True):
+        g = [torch.empty_like(x), torch.empty_like(x), torch.empty_like(m), torch.empty_like(x), torch.empty_like(x)]
+        if crowd:
+            crowded(0.7e9)
+        adj = nb.Adjoint(n, EPS2, 1 / 256, 1, 1)
+        adj.vjp_acc_jerk(x, v, m, a, j, g[0], g[1], g[2], torch.cuda.current_stream().cuda_stream)
+        adj.forward(x, v, m, g[3], g[4], torch.cuda.current_stream().cuda_stream)
+        adj.close()
+        out.append([w.cpu().numpy() for w in g])
+    for p, q in zip(*out):
+        assert np.abs(p - q).max() <= 1e-11 * np.abs(p).max()
