@@ -38,7 +38,8 @@ def local():
     src, so = os.path.join(BUILD, "devptr_check.cpp"), os.path.join(BUILD, "devptr_check.so")
     with open(src, "w") as f:
         f.write(SHIM)
-    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(CUDA, "include"),
+    # -Bsymbolic: its own cudaGetLastError, not that of a CUDA runtime already loaded
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", os.path.join(CUDA, "include"),
                     "-I", os.path.join(ROOT, "n-body-code_b200", "csrc"), "-o", so, src], check=True)
     return C.CDLL(so).local
 
