@@ -296,9 +296,11 @@ __global__ void copy_rows_kernel(int n, int ld, GatherArgs g, bool pad) {
 #define AD_CUDA(call)                                                                      \
   do {                                                                                     \
     cudaError_t e_ = (call);                                                               \
-    if (e_ != cudaSuccess)                                                                 \
+    if (e_ != cudaSuccess) {                                                               \
+      cudaGetLastError(); /* returned here, not by the next call's check of its launches */ \
       return nbody_set_error(e_ == cudaErrorMemoryAllocation ? NBODY_ERR_OOM : NBODY_ERR_CUDA, \
                              "%s failed: %s", #call, cudaGetErrorString(e_));              \
+    }                                                                                      \
   } while (0)
 #define AD_TRY(expr)               \
   do {                             \
@@ -613,8 +615,8 @@ nbody_status nbody_adjoint_create(nbody_adjoint** out, const nbody_adjoint_confi
       const cudaError_t e = cudaMalloc(&r->P, sizeof(double) * ld * fields);
       if (e == cudaSuccess) return NBODY_OK;
       r->P = nullptr;
-      if (e != cudaErrorMemoryAllocation || most <= 4) AD_CUDA(e);
       cudaGetLastError();
+      if (e != cudaErrorMemoryAllocation || most <= 4) AD_CUDA(e);
     }
   };
   nbody_status s = body();

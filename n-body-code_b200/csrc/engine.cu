@@ -100,9 +100,11 @@ nbody_status fail(nbody_status s, const char* fmt, ...) {
 #define NB_CUDA(call)                                                                        \
   do {                                                                                       \
     cudaError_t e_ = (call);                                                                 \
-    if (e_ != cudaSuccess)                                                                   \
+    if (e_ != cudaSuccess) {                                                                 \
+      cudaGetLastError(); /* returned here, not by the next call's check of its launches */  \
       return fail(e_ == cudaErrorMemoryAllocation ? NBODY_ERR_OOM : NBODY_ERR_CUDA,          \
                   "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                                        \
   } while (0)
 
 #define NB_TRY(expr)                 \

@@ -76,9 +76,11 @@ struct ClusterDev {
 #define EN_CUDA(call)                                                                      \
   do {                                                                                     \
     cudaError_t e_ = (call);                                                               \
-    if (e_ != cudaSuccess)                                                                 \
+    if (e_ != cudaSuccess) {                                                               \
+      cudaGetLastError(); /* returned here, not by the next call's check of its launches */ \
       return nbody_set_error(e_ == cudaErrorMemoryAllocation ? NBODY_ERR_OOM : NBODY_ERR_CUDA, \
                              "%s failed: %s", #call, cudaGetErrorString(e_));              \
+    }                                                                                      \
   } while (0)
 #define EN_TRY(expr)               \
   do {                             \

@@ -90,3 +90,21 @@ def test_adjoint_without_room_for_all_slots(crowded):
         out.append([w.cpu().numpy() for w in g])
     for p, q in zip(*out):
         assert np.abs(p - q).max() <= 1e-11 * np.abs(p).max()
+
+
+def test_a_create_without_memory_leaves_nothing_behind(crowded):
+    """Each kind of object that finds no memory says so; the calls after it work."""
+    s = nb.plummer(1000, seed=1)
+    ref = O.force(s, EPS2)
+    crowded(2e9)
+    for refused in (lambda: nb.Engine(1 << 28, eps2=EPS2, dt=1.0),
+                    lambda: nb.Ensemble([1 << 20] * 40, EPS2, 1 / 512),
+                    lambda: nb.Adjoint(1 << 22, EPS2, 1 / 256, 160, 16)):
+        with pytest.raises(nb.NBodyError) as err:
+            refused()
+        assert "OOM" in str(err.value)
+        with nb.Engine(1000, eps2=EPS2, dt=1.0) as e:
+            e.set_state(s)
+            e.force_calculation()
+            ea, ej = derivs_rel(e.get_derivs(), ref)
+        assert ea <= 1e-12 and ej <= 1e-12
