@@ -17,7 +17,11 @@
  *   - Host arrays are borrowed for the duration of a call only.  The engine
  *     owns its device memory from nbody_create to nbody_destroy; no entry
  *     point allocates after nbody_create (the autotuner, graph capture and
- *     ensemble set-up allocate once, on first use).
+ *     ensemble set-up allocate once, on first use, and so does the first
+ *     full pass of a system of more than about 400000 bodies: its
+ *     partial-sum slots are up to 6 KB per body, 5.8 GB at 10^6 bodies,
+ *     1.5 KB per body from 5.6e6 on; without room for them the pass is
+ *     one-sided, which takes 48 bytes per body and split).
  *   - An engine is not thread-safe; it serialises all work on its own CUDA
  *     stream.  Several engines may coexist.
  *   - Array layout is SoA float64: x, y, z, m, vx, vy, vz and ax, ay, az,
@@ -67,7 +71,9 @@ typedef struct {
   int threads, i_per_thread, j_tile, split_j; /* 0 = choose automatically   */
   int pair_variant;   /* mixed only: 0 = automatic (the near/far kernel in
                          its symmetric form, every unordered pair once;
-                         bodies in Hilbert order from 16384 of them on;
+                         bodies in Hilbert order from 16384 of them on,
+                         below in the caller's order with every separation
+                         in double-single, as 3;
                          with an explicit shape the one-sided variant 4
                          from 16384 bodies, 3 below), 1 = scalar FP32 kernel
                          on hi/lo positions, 2 = packed-pair (f32x2) hi/lo
@@ -113,7 +119,8 @@ typedef struct {
   int record_format;                /* j-records of the pair kernel in use:
                                        0 FP64, 1 FP32 hi/lo, 2 packed hi/lo,
                                        3 packed near/far tile-relative
-                                       (bodies kept in Hilbert order)       */
+                                       (the automatic choice below 16384
+                                       bodies: in the caller's order)       */
   int step_kernels;                 /* kernel launches in one step by itself
                                        (small systems: steps of one call
                                        share one between two steps)         */
@@ -206,10 +213,11 @@ const char* nbody_status_string(nbody_status s);
  * 240-246) gets the complete result.  A cached engine per (thread, device)
  * is reused, so repeated calls allocate nothing after the first.  Copies
  * host->device and back inside the call (the reference contract).
- * precision = NBODY_MIXED: the near/far tile-relative kernel from 32768
- * bodies over the full row range (each call orders the bodies along the
- * Hilbert curve in device memory and returns results in the caller's order),
- * the packed hi/lo kernel below that and for partial row ranges.  The
+ * precision = NBODY_MIXED: over the full row range the symmetric near/far
+ * kernel, from 32768 bodies on bodies that each call orders along the Hilbert
+ * curve in device memory (results come back in the caller's order), below in
+ * the caller's order with every separation in double-single; the packed hi/lo
+ * kernel for partial row ranges.  The
  * tiling is the heuristic one unless the autotuner has chosen one for the same
  * device, precision and n in this process (nbody_force_calculation_tune, or an
  * engine created with tune = 1); the call itself never runs the autotuner. */
@@ -285,7 +293,8 @@ typedef struct {
   const double* dt;      /* fixed shared step per cluster (> 0)              */
   int precision;         /* nbody_precision                                  */
   int device;
-  int tiles_per_item;    /* j-tiles per work item; 0 = chosen so that the
+  int tiles_per_item;    /* j-tiles per work item (128 bodies each in FP64 and
+                            hi/lo, 64 in variants 4 and 5); 0 = chosen so that the
                             items fill the GPU (64 to 1024 bodies), or (with
                             the kernel shape) by timing when tune = 1       */
   int tune;
@@ -301,7 +310,9 @@ typedef struct {
 } nbody_ensemble_config;
 typedef struct {
   int nclusters, padded_rows, items, tiles_per_item, grid;
-  int threads, j_tile;           /* persistent kernel shape in use */
+  int threads, j_tile;           /* persistent kernel shape in use; bodies per
+                                    tile of tiles_per_item (rounded up in FP64,
+                                    where an item may be shorter than one)   */
   double interactions_per_step;  /* sum of n[c]^2 */
   long long steps;
   double last_step_ms;           /* CUDA events around the last graph step */
@@ -334,8 +345,9 @@ nbody_status nbody_ensemble_get_stream(nbody_ensemble* ens, void** stream);
  * positions, velocities and masses.  The forward keeps the state every
  * checkpoint_every steps; the backward recomputes each segment and runs the
  * hand-written adjoint kernels (pair acc/jerk VJP in FP64, reverse corrector
- * and predictor).  All arrays are float64 device pointers of n values on the
- * adjoint's device; work is ordered on `stream` (cudaStream_t, NULL = legacy
+ * and predictor).  A mixed forward takes the bodies in the caller's order, with
+ * every separation in double-single.  All arrays are float64 device pointers of
+ * n values on the adjoint's device; work is ordered on `stream` (cudaStream_t, NULL = legacy
  * default stream); the calls return after their work completes. */
 typedef struct nbody_adjoint nbody_adjoint;
 typedef struct {

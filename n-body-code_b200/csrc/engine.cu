@@ -3,7 +3,8 @@
 // One engine = one system of n bodies on one device, one CUDA stream, and
 // device memory allocated once at creation:
 //   state  [13][ld] float64  X(3) V(3) M(1) D(6)  (D = current acc, jerk)
-//   P      [S][6][ld]        partial-sum slots of the pair kernel
+//   P      [S][6][ld]        partial-sum slots of the pair kernel (large ones
+//                            at the first pass, kEagerSlotBytes)
 //   jb64   [ld] JBody64      FP64 j-records (also used by the potential)
 //   jb32   [ld] JBody32      mixed-precision j-records (mixed engines):
 //                            JBody32, JBodyX2, tiles of JBodyNF, or SymSub
@@ -19,8 +20,9 @@
 // kernel's come from rel_tile_nf_kernel right after), pair (O(N^2)), correct
 // (O(N), fused slot sums + snap/crackle + correction + dt criterion) - is
 // captured into CUDA graphs and replayed: eight steps at a time, single ones,
-// and the last step of a call with event records.  The Hilbert re-ordering of a tile-relative engine's state is a
-// second captured graph, replayed ahead of every sort_every-th step.
+// and the last step of a call with event records.  The Hilbert re-ordering of a
+// tile-relative engine's state is a second captured graph, replayed ahead of
+// every sort_every-th step.
 #include <cuda_runtime.h>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -319,8 +321,8 @@ struct nbody_engine {
   cudaGraphExec_t many = nullptr;       // kStepsPerGraph steps
   int graph_kernels = 0;  // kernel nodes of the captured step
   // automatic mixed kernel (pair_variant 0): bodies in Hilbert order from this
-  // many, in the caller's below, where too few subtiles would be far to pay
-  // for the ordering.  An engine re-orders every sort_every steps; a drop-in
+  // many, in the caller's below (every separation in double-single), where too
+  // few subtiles would be far to pay for the ordering.  An engine re-orders every sort_every steps; a drop-in
   // or device-array call on every call (kForeignOrderMin).
   int order_min_bodies = 16384;
   // The device-array calls' last size and its tiling: planning takes 20 us at n
@@ -826,8 +828,9 @@ nbody_status build_rel_tiles(nbody_engine* e, int n, const SoA7& in, cudaStream_
 }
 
 // Writes the j-records of a pair kernel's format: FP64 records (hi/lo
-// kernels: also theirs), or tiles of tj near/far records of `in`, which must
-// then be in Hilbert order.  (The energy diagnostic packs its own records.)
+// kernels: also theirs), tiles of tj near/far records of `in`, which must then
+// be in Hilbert order, or subtiles of `in`, in Hilbert order or not (ordered).
+// (The energy diagnostic packs its own records.)
 nbody_status launch_pack(nbody_engine* e, int n, const SoA7& in, cudaStream_t st, int fmt,
                          int tj, bool ordered) {
   if (fmt == kRecSym) {

@@ -7,10 +7,10 @@
 // cluster comes from cid[row] (-1 on padding rows).
 //
 // Work list: item = (cluster, 256-row block, range of at most `tiles_per_item`
-// j-tiles; in the symmetric schedule, sympair.cuh, of the block's run).  Items are sorted by cost (longest first) and a fixed grid of
-// SMs x resident CTAs takes them from an atomic counter, so a 256-body cluster
-// and an 8192-body cluster share one launch without the small one idling the
-// GPU.  The partial-sum slots of cluster c live at P + p_off_c ([slot][6][ld_c])
+// j-tiles; in the symmetric schedule, sympair.cuh, of the block's run).  Items
+// are sorted by cost (longest first) and a fixed grid of SMs x resident CTAs
+// takes them from an atomic counter, so a 256-body cluster and an 8192-body
+// cluster share one launch without the small one idling the GPU.  The partial-sum slots of cluster c live at P + p_off_c ([slot][6][ld_c])
 // and are added in a fixed order by the corrector, so results are bitwise
 // reproducible.
 //
@@ -322,12 +322,16 @@ __global__ void ens_energy_sum_kernel(const ClusterDev* __restrict__ cl, const d
 // Persistent-kernel shapes (all with 256-row items = one padding unit); the
 // default is the first of a (precision, record format) or, for large near/far
 // ensembles, the second; the autotuner times all of them.  The packed hi/lo
-// default stays one-sided with tiles of 128: its float sums are those of the
-// single-system hi/lo kernel bit for bit, and in clusters with close pairs
-// (softening 4/N) any other order of them moves a body's result by more than
-// its own error against FP64.  Two rows per thread, j-loop unrolled four
-// times: pair launch of 256 clusters of 256-8192 bodies 2.64 ms, four rows
-// 2.74; the symmetric near/far kernel (pair_variant 4) takes 1.92.
+// default is one-sided with tiles of 128 by contract: its float sums, tile by
+// tile, are those of the single-system hi/lo kernel (pair_variant 3), and its
+// results stay what they are.  A symmetric hi/lo form sums in another order: it
+// moved the worst body of 256 clusters (softening 4/N) by 8.5e-8 in 8 steps, a
+// distance between the two forms and not an error.  Against FP64 sums the default
+// has acc errors of 5.0e-8 / 2.7e-7 / 1.9e-6 (median / p99 / max, 32 clusters of
+// 256-8192 bodies), the symmetric near/far kernel 4.3e-8 / 2.3e-7 / 1.7e-6; who
+// wants its speed asks for pair_variant 4 (pair launch of 256 clusters of
+// 256-8192 bodies 1.92 ms; hi/lo with two rows per thread and the j-loop
+// unrolled four times 2.64, with four rows 2.74).
 struct EnsKernel {
   int precision, nt, tile;
   int fmt;  // RecordFormat of its j-records

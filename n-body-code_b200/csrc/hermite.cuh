@@ -387,8 +387,9 @@ static __global__ void __launch_bounds__(kSumThreads)
 // Groups per row: eight from kSumGroupSlots slots, one below, where most
 // groups would have nothing to add.  Corrector with eight groups against one,
 // cold caches, N = 4096: 9.7 us over 44 slots against 18.6 over 32; a step at N =
-// 1024 39.4 against 42.4 us.  At N = 65536 (80 slots) the partials' bandwidth
-// bounds both, the same within 0.2 % of a step.
+// 1024 39.4 against 42.4 us.  At N = 65536 the partials' bandwidth bounds both:
+// the same within 0.2 % of a step over 80 slots; over the 116 (mixed) and 106
+// (FP64) of the automatic splits eight groups take 96 and 92 us, 3.9 TB/s.
 constexpr int kSumGroupSlots = 8;
 inline bool sum_in_groups(const RowSlots& s) { return s.S + s.nb / 2 >= kSumGroupSlots; }
 

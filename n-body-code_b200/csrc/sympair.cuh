@@ -26,7 +26,7 @@
 // s in slot s, the sums a block at distance d adds to its partners in slot
 // S + d - 1.  Every (slot, row) is written by exactly one thread, and slot
 // sums run in slot order, so results are bitwise reproducible.  A row's slot
-// count is RowSlots::count.
+// count is RowSlots::count.  The schedule's arithmetic is in symplan.h.
 //
 // Large systems: a block is `subs` sub-blocks of 32 * IPT * W rows, which the
 // CTA works through one after another over the same tiles, adding to the slots
@@ -535,10 +535,10 @@ __device__ __forceinline__ void sym_rotate(uint64_t* b, int next) {
 // separation with one add per component, near ones in double-single; a
 // (warp, subtile) pair is far when their boxes are apart by at least R / 2.
 // Float sums (a row's over one tile of 64 SUB bodies in two halves, a
-// j-body's over the warp's 32 IPT rows) are flushed into double: fewer terms
-// per float sum than the one-sided kernel's 128, and smaller errors (N =
-// 65536 median / p99 / rms acc error 2.3e-8 / 1.2e-7 / 3.8e-8, one-sided
-// 3.0e-8 / 1.6e-7 / 5.0e-8).  Jerk likewise.
+// j-body's over the warp's 32 IPT rows) are flushed into double: at most 128
+// terms per float sum, as in the one-sided kernel, most sums fewer, and smaller
+// errors (N = 65536 median / p99 / rms acc error 2.3e-8 / 1.2e-7 / 3.8e-8,
+// one-sided 3.0e-8 / 1.6e-7 / 5.0e-8).  Jerk likewise.
 //
 // Two j-bodies per lane are packed, the i-rows are held in both halves of
 // their registers: the packed j-operands and their sums come from shared

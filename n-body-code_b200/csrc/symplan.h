@@ -76,7 +76,8 @@ constexpr int kMaxSymSplits = 64;
 // Slots are further bounded by memory (8 GiB of P): from 1.4e6 bodies on systems
 // take fewer, larger blocks and fewer splits.  At least 32 slots, 1536 bytes per
 // body: 32 blocks of 16 splits still fill the SMs, where the 8 that fit at 2e7
-// bodies would be 32 CTAs.
+// bodies would be 32 CTAs.  Where the slots find no memory, an engine's pass is
+// one-sided and an adjoint's schedule is planned with half of them.
 inline int max_sym_slots(int n) {
   const double fit = 8.0 * (1 << 30) / (48.0 * n);
   return fit > 2 * kMaxSymSplits ? 2 * kMaxSymSplits : std::max(32, static_cast<int>(fit));
@@ -97,8 +98,8 @@ struct SymGrid {
   int count(int S) const { return S + nb / 2; }
 };
 
-// Rate at which the corrector sums slots (104 slots at N = 65536: 327 MB in 84
-// us): the price of each partial a tiling leaves.
+// Rate at which the corrector sums slots (116 slots at N = 65536: 380 MB with the
+// state in 96 us): the price of each partial a tiling leaves.
 constexpr double kSplitSumBytesPerMs = 3.9e9;
 
 // Interactions per ms of a GPU full of a pass's CTAs (fitted, see sym_plan).
@@ -157,7 +158,8 @@ inline void for_sym_splits(const SymGrid& g, int tj, int n, int max_s, F&& f) {
 // kernels at 19 (mixed, 1500 to 262144 bodies) and 13 sizes (FP64, 1024 to
 // 100000): 5 % rms; the kernel and split with the least time are on average
 // 0.6 % (4 % at most) slower than the measured best of all, at 12 sizes not
-// fitted (FP64, 1500 to 10000) 3 %, at worst 26 % (N = 4679).  Pass and sums in
+// fitted (FP64, 1500 to 10000) 3 %, at worst 26 % (N = 4679, where a step takes
+// 60 us, one-sided 84).  Pass and sums in
 // us against a fixed line between the kernels at 16384 bodies and a model that
 // counted idle CTAs: FP64 N = 3000 25 / 28, 5003 48 / 51, 8192 107 / 122, 12000
 // 219 / 234, 65536 5744 / 5794; mixed 5003 33 / 34, 8192 69 / 73, 18001 267 /
