@@ -278,10 +278,14 @@ struct RowsFP64 {
     eps2 = e2;
   }
 
+  // Group by group, so that a record's chunks lie at fixed offsets from one
+  // running pointer.
   __device__ __forceinline__ void consume(const JB* tile) {
+#pragma unroll 1
+    for (int g = 0; g < TJ; g += 32)
 #pragma unroll JU
-    for (int j = 0; j < TJ; ++j) {
-      const double2* r = jb64_at(tile, j);
+    for (int j = 0; j < 32; ++j) {
+      const double2* r = reinterpret_cast<const double2*>(tile + g) + j;
       const double2 p0 = r[0], p1 = r[32], p2 = r[64], p3 = r[96];
       const double xj = p0.x, yj = p0.y, zj = p1.x, mj = p1.y;
       const double uj = p2.x, vj = p2.y, wj = p3.x;
