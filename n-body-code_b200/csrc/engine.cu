@@ -1456,7 +1456,9 @@ nbody_status nbody_get_timers(nbody_engine* e, nbody_timers* out) {
     out->record_format = e->tiling.k->fmt == kRecSym ? kRecRel : e->tiling.k->fmt;
     out->tiling_source = e->tiling.source;
     const PairKernel& k = *e->tiling.k;
-    if (tile_relative(k.fmt) && k.near) {
+    if (k.fmt == kRecSym && !curve_resident(e)) {
+      out->near_tile_fraction = e->have_derivs ? 1.0 : 0.0;  // without a copy: about 10 us
+    } else if (tile_relative(k.fmt) && k.near) {
       unsigned long long near = 0;
       NB_CUDA(cudaMemcpy(&near, e->near_count, sizeof near, cudaMemcpyDeviceToHost));
       // classified per (warp, tile): warps = row blocks x NT / 32; the
