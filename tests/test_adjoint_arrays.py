@@ -79,3 +79,27 @@ def test_arrays_are_checked_before_a_call():
                 Array(10, contiguous=False)):
         with pytest.raises(AssertionError):
             adjoint._p(bad, 10)
+
+
+class Matrix(Array):
+    """Three rows of n values, `row` apart."""
+
+    def __init__(self, n, row=None, column=1, rows=3, **kw):
+        super().__init__(n, **kw)
+        self.shape, self.strides = (rows, n), (row or n, column)
+
+    def stride(self):
+        return self.strides
+
+
+def test_rows_are_checked_before_a_call():
+    def at(t, n):
+        return [p.value for p in adjoint._rows(t, n)]
+    assert at(Matrix(10), 10) == [4096, 4096 + 80, 4096 + 160]
+    assert at(Matrix(10, row=16), 10) == [4096, 4096 + 128, 4096 + 256]  # columns of a wider matrix
+    assert at(Matrix(12), 10) == [4096, 4096 + 96, 4096 + 192]
+    assert at(Matrix(1, row=3, column=3), 1) == [4096, 4096 + 24, 4096 + 48]
+    for bad in (Matrix(9), Matrix(10, size=4), Matrix(10, cuda=False), Matrix(10, floating=False),
+                Matrix(10, column=3, row=1), Matrix(10, rows=2)):
+        with pytest.raises(AssertionError):
+            adjoint._rows(bad, 10)
