@@ -511,7 +511,7 @@ nbody_status build_items(nbody_ensemble* e, int tpi) {
         it.nb = k.nb;
         it.subs = k.subs;
         it.split = s;
-        it.p_off = p_off;
+        it.p_off = kern.sym ? p_off : p_off + static_cast<long long>(s) * 6 * e->ld[c];
         it.eps2 = e->eps2[c];
         const int q0 = s * tpi;
         it.t_begin = kern.sym ? rb * (k.block / kern.tile) + q0 : q0;

@@ -915,7 +915,8 @@ struct EnsItem {
   int t_begin, nt;    // first j-tile (cluster-relative; symmetric kernels: cyclic) and count
   int S, nb, subs;    // the cluster's splits, (symmetric) blocks and 256-row sub-blocks per block
   int split;          // the item's split
-  long long p_off;    // doubles from the partial-sum base to the cluster's slots
+  long long p_off;    // doubles from the partial-sum base to the cluster's slots or,
+                      // one-sided kernels, to the item's own slot
   double eps2;
 };
 
@@ -945,8 +946,7 @@ __global__ void __launch_bounds__(R::NT) ensemble_pair_kernel(const typename R::
     if (!pipe.run(cj + static_cast<size_t>(it.t_begin) * R::TJ, it.nt, status,
                   [&](const JB* tile) { r.consume(tile); }))
       return;
-    r.store(P + it.p_off + static_cast<long long>(it.split) * 6 * it.ld, static_cast<size_t>(it.ld), row,
-            it.rows_end);
+    r.store(P + it.p_off, static_cast<size_t>(it.ld), row, it.rows_end);
   }
 }
 
@@ -978,8 +978,7 @@ __global__ void __launch_bounds__(R::NT, MINB) ensemble_pair_nf_kernel(
                  smem_raw + 2 * kRecs * sizeof(JBodyNF));
     const JBodyNF* ct = jt + static_cast<size_t>(it.jrow0 / R::TJ + it.t_begin) * kRecs;
     if (!pipe.run(ct, it.nt, status, [&](const JBodyNF* tile) { r.consume(tile); })) return;
-    r.store(P + it.p_off + static_cast<long long>(it.split) * 6 * it.ld, static_cast<size_t>(it.ld),
-            it.rows_end);
+    r.store(P + it.p_off, static_cast<size_t>(it.ld), it.rows_end);
   }
 }
 
