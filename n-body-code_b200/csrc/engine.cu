@@ -322,8 +322,9 @@ struct nbody_engine {
   int graph_kernels = 0;  // kernel nodes of the captured step
   // automatic mixed kernel (pair_variant 0): bodies in Hilbert order from this
   // many, in the caller's below (every separation in double-single), where too
-  // few subtiles would be far to pay for the ordering.  An engine re-orders every sort_every steps; a drop-in
-  // or device-array call on every call (kForeignOrderMin).
+  // few subtiles would be far to pay for the ordering.  An engine re-orders
+  // every sort_every steps; a drop-in or device-array call on every call
+  // (kForeignOrderMin).
   int order_min_bodies = 16384;
   // The device-array calls' last size and its tiling: planning takes 20 us at n
   // = 40000 and 60 at 262144, on the host ahead of every launch.  The choice
